@@ -181,7 +181,7 @@ def _mid_run(st, rng):
     F[:, 5] = F[:, 7] = t[:, 4]
     F[:, 2] = F[:, 6] = t[:, 5]
     V0 = torch.from_numpy(st["vol0"][idx]).to(dev)
-    V = V0 * torch.linalg.det(F.view(-1, 3, 3))
+    V = V0 * _det(F)
     eng = torch.tensor([1.0, 1.0, 1.0, 2.0, 2.0, 2.0], dtype=torch.float64, device=dev)
     new = {"pos": xb + _waves(rng, y, 3, 0.4 * h), "vel": _waves(rng, y, 3, 4.0), "stress": sig, "backstress": R,
            "F": F, "vol": V, "strain": t * eng, "eps_p": ep * eng,
@@ -192,6 +192,13 @@ def _mid_run(st, rng):
     for k, v in new.items():
         st[k][idx] = v.cpu().numpy()
     st["fext"][:] = 0.0
+
+
+def _det(F):
+    """Determinants of 3 x 3 matrices given as n x 9 (rows or columns in turn)."""
+    a = F.unbind(1)
+    return (a[0] * (a[4] * a[8] - a[5] * a[7]) - a[1] * (a[3] * a[8] - a[5] * a[6]) +
+            a[2] * (a[3] * a[7] - a[4] * a[6]))
 
 
 def _states(case, seed):
@@ -520,7 +527,7 @@ class _Sim:
         self.rate = e / dt
         F = P["F"].view(-1, 3, 3).transpose(1, 2)  # stored column by column
         F = F + (D @ F if self.contact else F @ D)
-        V = torch.where(go, torch.linalg.det(F) * P["vol0"], P["vol"])
+        V = torch.where(go, _det(F.reshape(-1, 9)) * P["vol0"], P["vol"])
         P["F"] = F.transpose(1, 2).reshape(-1, 9)
         E, nu, R, s = M["E"], M["nu"], P["backstress"], P["stress"]
         G = 0.5 * E / (1.0 + nu)
