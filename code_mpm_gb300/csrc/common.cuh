@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fpmap.h"
 #include "fpsplit.h"
 
 namespace mpm {
@@ -134,6 +135,7 @@ struct MatConst {
     double inv_E, nu_over_E, inv_G;
     // RN32 images of the constants the FP32 form uses
     float fC, fone_m_nu, fnu, fhalf_m_nu, fk0, fs23C1, fC0, finv_E, fnu_over_E, finv_G;
+    fps_map_const map;  // the return map in pairs of floats (FP32 form's fallback path)
 };
 
 inline void set_float_constants(MatConst& k) {
@@ -147,6 +149,7 @@ inline void set_float_constants(MatConst& k) {
     k.finv_E = (float)k.inv_E;
     k.fnu_over_E = (float)k.nu_over_E;
     k.finv_G = (float)k.inv_G;
+    fps_map_constants(k.E, k.nu, k.Y, k.C0, k.C1, &k.map);
 }
 
 // An increment of the form's type as a double (exact in both forms).

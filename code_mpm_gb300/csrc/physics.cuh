@@ -176,7 +176,7 @@ __device__ __forceinline__ double len3_rn(const double a[3]) { return __dsqrt_rn
 //
 // FP64 (plain) form, the reference's arithmetic: diagonal strain increment
 // (1 + L_ii dt) - 1 (…MPLocks.cpp:206-219); non-contact F <- F (I + L dt)
-// (:242); contact F <- F + (L F) dt (…_Contact.cpp:464); V = det(F) V0 with
+// (:242); contact F <- F + (L dt) F (…_Contact.cpp:464); V = det(F) V0 with
 // glm's cofactor determinant.
 //
 // FP32 (chosen) form: the same mathematics rearranged so FP32 keeps the
@@ -191,8 +191,7 @@ struct Kinematics;
 template <>
 struct Kinematics<double> {
     static __device__ __forceinline__ double strain_diag(double x) { return __dadd_rn(__dadd_rn(1.0, x), -1.0); }
-    static __device__ __forceinline__ void update(bool contact, const double F[9], const double L[9],
-                                                  const double Ldt[9], double dt, double Fn[9]) {
+    static __device__ __forceinline__ void update(bool contact, const double F[9], const double Ldt[9], double Fn[9]) {
         if (!contact) {
 #pragma unroll
             for (int c = 0; c < 3; ++c)
@@ -209,7 +208,7 @@ struct Kinematics<double> {
 #pragma unroll
                 for (int r = 0; r < 3; ++r)
                     Fn[3 * c + r] =
-                        F[3 * c + r] + (L[r] * F[3 * c] + L[3 + r] * F[3 * c + 1] + L[6 + r] * F[3 * c + 2]) * dt;
+                        F[3 * c + r] + Ldt[r] * F[3 * c] + Ldt[3 + r] * F[3 * c + 1] + Ldt[6 + r] * F[3 * c + 2];
         }
     }
     static __device__ __forceinline__ double det(const double m[9]) {
@@ -222,8 +221,7 @@ template <>
 struct Kinematics<float> {
     static __device__ __forceinline__ float strain_diag(float x) { return x; }
     // H (= F - I) in, Hn out
-    static __device__ __forceinline__ void update(bool contact, const float H[9], const float L[9], const float Ldt[9],
-                                                  float dt, float Hn[9]) {
+    static __device__ __forceinline__ void update(bool contact, const float H[9], const float Ldt[9], float Hn[9]) {
 #pragma unroll
         for (int c = 0; c < 3; ++c)
 #pragma unroll
@@ -297,9 +295,10 @@ __device__ __forceinline__ void cr_trial(const MatConst& m, T R, const T sig[6],
 // (…_PerfectlyPlastic.cpp:4-76, radius k0); von Mises with explicit
 // isotropic hardening (…_VonMisesHardening.cpp:4-92, radius k0 + R/sqrt 2,
 // dR = C0 (sqrt(2/3) C1 - R) sqrt(2/3 sum deps_p^2) when positive), from
-// the trial state.
+// the trial state.  Returns whether the increment is plastic (elastic: deps_p
+// and dR are zero).
 template <typename T>
-__device__ __forceinline__ void cr_return(const MatConst& m, T R, const T sig[6], const T e[6], const CrTrial<T>& t,
+__device__ __forceinline__ bool cr_return(const MatConst& m, T R, const T sig[6], const T e[6], const CrTrial<T>& t,
                                           CrOut<T>& o) {
     o.dR = (T)0;
 #pragma unroll
@@ -307,7 +306,7 @@ __device__ __forceinline__ void cr_return(const MatConst& m, T R, const T sig[6]
     if (m.type == 0 || t.J2 <= t.rad * t.rad) {
 #pragma unroll
         for (int i = 0; i < 6; ++i) o.dsig[i] = t.dtr[i];
-        return;
+        return false;
     }
     const T hyd = (T)(1.0 / 3.0) * (t.tr[0] + t.tr[1] + t.tr[2]);
     const T sc = t.rad / sqrt(t.J2);
@@ -333,13 +332,14 @@ __device__ __forceinline__ void cr_return(const MatConst& m, T R, const T sig[6]
     ee[5] = o.dsig[5] * iG;
 #pragma unroll
     for (int i = 0; i < 6; ++i) o.deps_p[i] = e[i] - ee[i];
-    if (m.type != 4) return;
+    if (m.type != 4) return true;
     T ep = (T)0;
 #pragma unroll
     for (int i = 0; i < 6; ++i) ep += o.deps_p[i] * o.deps_p[i];
     ep = sqrt(ep * (T)(2.0 / 3.0));
     const T sat = form_const<T>(m.s23C1, m.fs23C1) - R;
     o.dR = (sat > (T)0) ? form_const<T>(m.C0, m.fC0) * sat * ep : (T)0;
+    return true;
 }
 
 template <typename T>
@@ -349,8 +349,8 @@ __device__ __forceinline__ void cr_increment(const MatConst& m, T R, const T sig
     cr_return<T>(m, R, sig, e, t, o);
 }
 
-// The exact map in FP64 on FP32 state (the chosen form's fallback path and
-// the judge of the learned map): the float inputs widened exactly, the
+// The exact map in FP64 on FP32 state (the judge of the learned map and the
+// guard's replacement of its results): the float inputs widened exactly, the
 // increment computed in double (cr_increment<double>, the plain form's
 // arithmetic), each output rounded once to float.
 __device__ __forceinline__ void cr_increment_wide(const MatConst& m, float R, const float sig[6], const float e[6],
@@ -371,6 +371,25 @@ __device__ __forceinline__ void cr_narrow(const CrOut<double>& w, CrOut<float>& 
         o.deps_p[i] = __double2float_rn(w.deps_p[i]);
     }
     o.dR = __double2float_rn(w.dR);
+}
+
+// The same map on the chosen form's fallback path, in pairs of floats
+// (fpmap.h).  In FP64 it held pass 2 to the FP64 pipe wherever a warp had one
+// particle near the yield surface: of a solid block of 1.07M particles with a
+// quarter of them on the surface, pass 2 took 212 us, 119 us with the pairs;
+// 5.08M particles of honeycombs, 536 and 408 us.  Returns whether the
+// increment is plastic.
+__device__ __forceinline__ bool cr_increment_pairs(const MatConst& m, float R, const float sig[6], const float e[6],
+                                                   CrOut<float>& o) {
+    fps_map_out w;
+    const int plastic = fps_vmh_map(&m.map, R, sig, e, &w);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        o.dsig[i] = w.dsig[i];
+        o.deps_p[i] = w.deps_p[i];
+    }
+    o.dR = w.dR;
+    return plastic != 0;
 }
 
 // ---------------------------------------------------------------------------

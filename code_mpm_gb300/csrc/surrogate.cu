@@ -459,7 +459,8 @@ __global__ void k_exact_fp32(long long n, const float* __restrict__ in, MatConst
 }
 
 // the exact return map in FP64 on physical rows, outputs rounded once to
-// float: the arithmetic of the FP32 form's fallback path (cr_increment_wide)
+// float (cr_increment_wide); the FP32 form's fallback path computes the same
+// map in pairs of floats (cr_increment_pairs)
 __global__ void k_exact_wide(long long n, const float* __restrict__ in, MatConst M, float* __restrict__ out) {
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= n) return;

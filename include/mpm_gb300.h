@@ -73,8 +73,8 @@ extern "C" {
 #define MPM_OPT_P2G_REDUCE 3     /* P2G: 0 = one atomic per particle, 1 = sum each cell's run across lanes first, 2 = stage the block in shared memory and sum each (cell, corner) in one thread, 3 (default) / 4 = as 2 with each thread summing 2 / 4 corners of a cell */
 #define MPM_OPT_P2G_BLOCK 4      /* P2G threads per block (128, 256 or 512) */
 #define MPM_OPT_PASS_BLOCK 5     /* G2P pass-2 threads per block (128, 256 (default) or 512) */
-#define MPM_OPT_GATHER 6         /* pass-2 (G2P) mode: 0 = node gathers one corner at a time, 1 = several corners'
-                                    loads issued together, 2 = (FP32 form) as 0 with the block's particle fields
+#define MPM_OPT_GATHER 6         /* pass-2 (G2P) mode: 0 = node gathers one (x, y) pair of corners at a time, 1 = several
+                                    pairs' loads issued together, 2 = (FP32 form) as 0 with the block's particle fields
                                     brought into shared memory by bulk copies first */
 #define MPM_OPT_GRAPH 7          /* 1 (default): mpm_advance replays a captured two-step CUDA graph in the steady state; 0: launch every kernel */
 #define MPM_OPT_REORDER 8        /* FP32 form: store particles in cell order after each particle upload (0, default), also every N steps (N > 0), or never (-1); results stay in the caller's order */
@@ -82,7 +82,8 @@ extern "C" {
 #define MPM_OPT_PASS1_BLOCK 11   /* cell-run G2P pass 1: threads per block (128, 256 or 512) */
 #define MPM_OPT_LARGE_STRAIN 12  /* FP64 form, non-contact loop: 1 runs the large-strain pass 2 (G2P_P2_LargeStrain, PhysicsEngine_runSimulation_Classic_DoublePass_MPLocks.cpp:281-437), which the reference ships disabled (:605); 0 (default) the small-strain pass */
 #define MPM_OPT_FP64_FALLBACK 13 /* FP32 form: 1 (default) computes the von Mises hardening return map
-                                    (…_VonMisesHardening.cpp:4-92) in FP64 for particles whose FP32 trial yield
+                                    (…_VonMisesHardening.cpp:4-92) as FP64 gives it, rounded to float (in pairs of
+                                    floats, 48 bits), for particles whose FP32 trial yield
                                     function is above -0.001 x k0 and that the network does not take: with a
                                     network the states up to its band (mpm_attach_surrogate, 0.02 by default) past
                                     the surface, every plastic state without one, and the elastic states just

@@ -89,8 +89,8 @@ int mpm_net_loss_grad(mpm_net* net, const float* x, const float* t, int64_t n, f
 /* Inference on device rows (inputs n x 13, outputs n x 7, physical units).
  * kernel: 0 = BF16 tcgen05, 1 = FP32 CUDA cores (reference), 2 = the exact
  * FP32 return map (the method without the network), 3 = the exact return map
- * in FP64 on the float inputs, outputs rounded once to float (the FP32 form's
- * fallback path and the judge of the network, MPM_OPT_FP64_FALLBACK). */
+ * in FP64 on the float inputs, outputs rounded once to float (the judge of the
+ * network; what the FP32 form's fallback path reproduces, MPM_OPT_FP64_FALLBACK). */
 int mpm_net_infer(mpm_net* net, const float* d_in, float* d_out, int64_t n, int kernel, void* stream);
 /* Normalisation in use: physical input = normalised x in_scale; physical
  * output = normalised x out_scale + out_shift (+ D de for the stress). */
