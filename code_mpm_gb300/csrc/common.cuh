@@ -36,6 +36,7 @@ struct Geom {
     float ih_lo[3];   // RN32(inv_h - inv_hf): inv_hf + ih_lo is inv_h to 2^-48
     int nn[3];        // nodes per axis = cells + 1
     int kd[3];        // cell-key extents = cells + 2 (base cells -1..cells)
+    unsigned kd_mul[2], kd_shift[2];  // division of a key by kd[0], kd[1] (set_key_division)
     unsigned key_max; // total key count over all specimens: the key of a particle with no node in range
     long long n_nodes;  // total node count over all specimens
     const double* xtab;
@@ -53,6 +54,22 @@ inline void set_float_geometry(Geom& g, int a) {
     g.ih_lo[a] = (float)(g.inv_h[a] - (double)g.inv_hf[a]);
 }
 
+// Multiplier and shift for exact division of any 32-bit number by d >= 2
+// (Granlund and Montgomery, PLDI 1994, figure 4.1).
+inline void set_key_division(Geom& g) {
+    for (int a = 0; a < 2; ++a) {
+        const unsigned long long d = (unsigned long long)g.kd[a];
+        unsigned l = 0;
+        while ((1ull << l) < d) ++l;
+        g.kd_mul[a] = (unsigned)(((((1ull << l) - d) << 32) / d) + 1ull);
+        g.kd_shift[a] = l - 1u;
+    }
+}
+__device__ __forceinline__ unsigned key_div(unsigned n, unsigned mul, unsigned shift) {
+    const unsigned t = __umulhi(mul, n);
+    return (t + ((n - t) >> 1)) >> shift;
+}
+
 // The geometry of particle p's specimen.
 __device__ __forceinline__ const Geom& spec_geom(const Geom& g, const uint16_t* __restrict__ sid, long long p) {
     return (g.nspec > 1) ? g.tab[sid[p]] : g;
@@ -60,11 +77,12 @@ __device__ __forceinline__ const Geom& spec_geom(const Geom& g, const uint16_t* 
 
 // Decode a cell key into the base (bottom-left-far) cell index of its specimen.
 __device__ __forceinline__ void key_to_base(unsigned key, const Geom& g, int b[3]) {
-    unsigned k = key - g.key_off;
-    b[0] = (int)(k % (unsigned)g.kd[0]) - 1;
-    k /= (unsigned)g.kd[0];
-    b[1] = (int)(k % (unsigned)g.kd[1]) - 1;
-    b[2] = (int)(k / (unsigned)g.kd[1]) - 1;
+    const unsigned k = key - g.key_off;
+    const unsigned r = key_div(k, g.kd_mul[0], g.kd_shift[0]);  // row
+    const unsigned z = key_div(r, g.kd_mul[1], g.kd_shift[1]);
+    b[0] = (int)(k - r * (unsigned)g.kd[0]) - 1;
+    b[1] = (int)(r - z * (unsigned)g.kd[1]) - 1;
+    b[2] = (int)z - 1;
 }
 
 __device__ __forceinline__ double node_coord(const Geom& g, int a, int n) { return g.xtab[g.xoff[a] + n + 1]; }
@@ -77,33 +95,31 @@ __device__ __forceinline__ long long corner_node(const Geom& g, const int b[3], 
     return g.node_off + (long long)nx + (long long)ny * g.nn[0] + (long long)nz * g.nn[0] * g.nn[1];
 }
 
-// A cell's corner nodes in a form the cell-run kernels stage per slot:
-// corner k = 4 ix + 2 iy + iz is node n0 + ix + iy sy + iz sz, in range when
-// bit k of mask is set (the same nodes corner_node gives).
+// A cell's corner nodes: corner k = 4 ix + 2 iy + iz is node n0 + ix + iy sy +
+// iz sz, in range when bit k of mask is set (the same nodes corner_node
+// gives).  Node numbers fit 32 bits (a context holds fewer than 2^32 - 1); n0
+// of a base cell at -1 wraps and comes back in range with its valid corners.
 struct CellNodes {
-    long long n0, sz;
-    int sy;
-    unsigned mask;
+    unsigned n0, sy, sz, mask;
 };
 
 __device__ __forceinline__ CellNodes cell_nodes(const Geom& g, const int b[3]) {
     CellNodes c;
-    c.sy = g.nn[0];
-    c.sz = (long long)g.nn[0] * g.nn[1];
-    c.n0 = g.node_off + (long long)b[0] + (long long)b[1] * c.sy + (long long)b[2] * c.sz;
-    c.mask = 0u;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int nx = b[0] + ((k >> 2) & 1), ny = b[1] + ((k >> 1) & 1), nz = b[2] + (k & 1);
-        if (nx >= 0 && ny >= 0 && nz >= 0 && nx <= g.nn[0] - 1 && ny <= g.nn[1] - 1 && nz <= g.nn[2] - 1)
-            c.mask |= 1u << k;
-    }
+    c.sy = (unsigned)g.nn[0];
+    c.sz = (unsigned)g.nn[0] * (unsigned)g.nn[1];
+    c.n0 = (unsigned)g.node_off + (unsigned)b[0] + (unsigned)b[1] * c.sy + (unsigned)b[2] * c.sz;
+    // base cells run from -1 to cells: the lower node of an axis is in range
+    // unless b = -1, the upper one unless b = cells
+    const unsigned mx = (b[0] >= 0 ? 0x0fu : 0u) | (b[0] < g.nn[0] - 1 ? 0xf0u : 0u);
+    const unsigned my = (b[1] >= 0 ? 0x33u : 0u) | (b[1] < g.nn[1] - 1 ? 0xccu : 0u);
+    const unsigned mz = (b[2] >= 0 ? 0x55u : 0u) | (b[2] < g.nn[2] - 1 ? 0xaau : 0u);
+    c.mask = mx & my & mz;
     return c;
 }
 
 // corner k's node (in range: bit k of c.mask)
-__device__ __forceinline__ long long cell_node(const CellNodes& c, int k) {
-    return c.n0 + ((k >> 2) & 1) + (long long)(((k >> 1) & 1) * c.sy) + ((k & 1) ? c.sz : 0ll);
+__device__ __forceinline__ unsigned cell_node(const CellNodes& c, int k) {
+    return c.n0 + ((k >> 2) & 1) + (((k >> 1) & 1) ? c.sy : 0u) + ((k & 1) ? c.sz : 0u);
 }
 
 // Specimen owning global node i (binary search over the node offsets).

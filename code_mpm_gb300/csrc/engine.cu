@@ -53,9 +53,12 @@ struct mpm_ctx {
     // options
     int floor_friction = 0;
     int profile = 0;
-    // defaults: the autotuner's choice on the 256-specimen honeycomb batch
-    int p2g_reduce = 3, p2g_block = 128, pass_block = 256, gather_batch = 0;
-    int pass1_corners = 2, pass1_block = 128;  // cell-run pass 1 (P2G modes 2-4)
+    // block sizes: 0 = chosen by the particle count (auto_block) unless the
+    // caller or the autotuner sets one; modes: the autotuner's choice on the
+    // 256-specimen honeycomb batch
+    int p2g_reduce = 3, p2g_block = 0, pass_block = 0, gather_batch = 0;
+    int pass1_corners = 2, pass1_block = 0;  // cell-run pass 1 (P2G modes 2-4)
+    bool have_fext = false;  // some particle carries an external force
     // simulation scalars
     mpm_sim sim{0.0, 1.0e-3, 0.0, 0.0, 10.0, 0};
     // counts
@@ -91,6 +94,7 @@ struct mpm_ctx {
     DevBuf staging2;
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t xfer_ev[4] = {nullptr, nullptr, nullptr, nullptr};  // per buffer: copy done, kernel done
+    DevBuf fext_any;
     DevBuf work_acc;  // boundary work since the last particle upload (FP64): displacement control, friction
     int nsurf = 0;
     bool have_mon = false;
@@ -151,7 +155,7 @@ struct mpm_ctx {
                           &g_state, &g_fixed, &g_friction, &g_ratio, &g_q, &g_owner, &g_nowner, &g_need, &g_list, &g_count, &rs_chunk, &cstart,
                           &cend, &keys0, &vals0, &keys1, &vals1, &keys_copy, &counts, &dclist, &mats, &staging, &staging2, &tune_backup, &surf, &mon_mask, &mon_acc, &loc, &geom_tab, &sid, &alist, &acount,
                           &q_in, &q_out, &q_vol, &q_pidx, &q_count, &sg_acc, &hv_count,
-                          &dsim, &tl_dev, &orig, &ptmp, &Fe, &work_acc};
+                          &dsim, &tl_dev, &orig, &ptmp, &Fe, &work_acc, &fext_any};
         all.assign(std::begin(list), std::end(list));
     }
 };
@@ -313,24 +317,25 @@ int prof_resolve(mpm_ctx* c) {
         kernel<<<(grid), (block), (smem), c->stream>>>(__VA_ARGS__);       \
     } while (0)
 
-// A cell-run kernel template <T, corners per thread, block size> launched for
-// the runtime choice of both (1, 2 or 4 corners; 128, 256 or 512 threads).
-#define LAUNCH_CELLS(name, K, T, cpt, bs, grid, smem, ...)                                              \
-    do {                                                                                                \
-        if ((bs) == 128) {                                                                              \
-            if ((cpt) == 1) LAUNCH_SMEM(name, (K<T, 1, 128>), grid, 128, smem, __VA_ARGS__);            \
-            else if ((cpt) == 2) LAUNCH_SMEM(name, (K<T, 2, 128>), grid, 128, smem, __VA_ARGS__);       \
-            else LAUNCH_SMEM(name, (K<T, 4, 128>), grid, 128, smem, __VA_ARGS__);                       \
-        } else if ((bs) == 256) {                                                                       \
-            if ((cpt) == 1) LAUNCH_SMEM(name, (K<T, 1, 256>), grid, 256, smem, __VA_ARGS__);            \
-            else if ((cpt) == 2) LAUNCH_SMEM(name, (K<T, 2, 256>), grid, 256, smem, __VA_ARGS__);       \
-            else LAUNCH_SMEM(name, (K<T, 4, 256>), grid, 256, smem, __VA_ARGS__);                       \
-        } else {                                                                                        \
-            if ((cpt) == 1) LAUNCH_SMEM(name, (K<T, 1, 512>), grid, 512, smem, __VA_ARGS__);            \
-            else if ((cpt) == 2) LAUNCH_SMEM(name, (K<T, 2, 512>), grid, 512, smem, __VA_ARGS__);       \
-            else LAUNCH_SMEM(name, (K<T, 4, 512>), grid, 512, smem, __VA_ARGS__);                       \
-        }                                                                                               \
+// A kernel template <T, block size, FE> launched for the runtime block size: 128,
+// 256 or 512 threads, and in the FP64 form also 32 and 64 (auto_block).
+#define LAUNCH_BS(name, K, T, FE, bs, grid, smem, ...)                                  \
+    do {                                                                                \
+        if ((bs) == 128) LAUNCH_SMEM(name, (K<T, 128, FE>), grid, 128, smem, __VA_ARGS__);  \
+        else if ((bs) == 256) LAUNCH_SMEM(name, (K<T, 256, FE>), grid, 256, smem, __VA_ARGS__); \
+        else if ((bs) == 512) LAUNCH_SMEM(name, (K<T, 512, FE>), grid, 512, smem, __VA_ARGS__); \
+        else if constexpr (sizeof(T) == 8) {                                            \
+            if ((bs) == 64) LAUNCH_SMEM(name, (K<T, 64, FE>), grid, 64, smem, __VA_ARGS__); \
+            else LAUNCH_SMEM(name, (K<T, 32, FE>), grid, 32, smem, __VA_ARGS__);            \
+        }                                                                               \
     } while (0)
+template <typename T, int BS>
+using Pass1Kernel = void (*)(PView<T>, NView<T>, Geom, const unsigned*, const unsigned*, long long, T, int);
+// pass 1 with the option's corners per thread (1, 2 or 4)
+template <typename T, int BS>
+Pass1Kernel<T, BS> pass1_kernel(int cpt) {
+    return cpt == 1 ? k_pass1_cells<T, 1, BS> : cpt == 2 ? k_pass1_cells<T, 2, BS> : k_pass1_cells<T, 4, BS>;
+}
 
 // ---- host-side timeline (TimeLine::getVelocity, TimeLine.h:33-46) ----------
 void timeline_velocity(const mpm_ctx* c, double t, double out[3]) {
@@ -506,6 +511,15 @@ __global__ void k_specimen_ids(const int32_t* __restrict__ in, long long n, int 
         return;
     }
     out[i] = (uint16_t)s;
+}
+
+// *any = 1 when one of the n values is not zero
+template <typename T>
+__global__ void k_any_nonzero(const T* __restrict__ v, long long n, unsigned* __restrict__ any) {
+    bool f = false;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        f |= v[i] != (T)0;
+    if (__any_sync(FULL_MASK, f) && (threadIdx.x & 31) == 0) *any = 1u;
 }
 
 __global__ void k_clear_flag(uint8_t* __restrict__ pflags, long long n, uint8_t bits) {
@@ -827,6 +841,22 @@ void graph_reset(mpm_ctx* c) {
     }
 }
 
+// The block size of a particle kernel: the caller's (or the autotuner's), else
+// 128 threads in the FP32 form.  The FP64 form's kernels are bound by the FP64
+// pipe, two lanes per clock of each SM, so what counts is that every SM gets
+// its share of the warps: smaller blocks until there are AUTO_WAVES of them
+// per SM.  A 40,000-particle bar took 129.5 us per step with 2, 122.8 with 4
+// (blocks of 64), 130.8 with 8 and 16 (blocks of 32, whose cell runs are cut
+// more often), 286k particles 475 us with 2 to 8, 490 with 16.
+constexpr int AUTO_WAVES = 4;
+int auto_block(const mpm_ctx* c, int chosen) {
+    if (chosen) return chosen;
+    if (c->form != MPM_FORM_FP64) return 128;
+    int b = 128;
+    while (b > 32 && c->n < (long long)AUTO_WAVES * b * c->sm_count) b >>= 1;
+    return b;
+}
+
 // output: the step is an output step, the last of an advance, whose results
 // the caller can see.  Only an output step runs the contact path's contact
 // detection (node mass gradients, particle and node normals, node contact
@@ -884,7 +914,7 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
         bool pairs_done = false;
         if constexpr (sizeof(T) == 4) {
             if (c->p2g_reduce >= 5) {  // runs reduced in registers and by a pair shuffle (mode 6: tile staged)
-                const int bs = c->p2g_block;
+                const int bs = auto_block(c, c->p2g_block);
                 const unsigned pg = (unsigned)((n + 4LL * bs - 1) / (4LL * bs));
                 const bool st = c->p2g_reduce == 6;
 #define PAIRS(B, MGV, STV)                                                                                       \
@@ -907,21 +937,36 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
                 pairs_done = true;
             }
         }
+        const int bp = auto_block(c, c->p2g_block);
         if (pairs_done) {
-        } else if (c->p2g_reduce >= 2) {  // shared-memory cell runs, 1 / 2 / 4 corners per thread
-            const int bs = c->p2g_block, cpt = 1 << std::min(2, c->p2g_reduce - 2);
-            if (mg_in_p2g)
-                LAUNCH_CELLS("p2g", k_p2g_cells_mg, T, cpt, bs, blocks_for(n, bs), p2g_cells_smem<T>(bs), P, N, g,
-                             skeys, perm, n, fp32);
-            else
-                LAUNCH_CELLS("p2g", k_p2g_cells, T, cpt, bs, blocks_for(n, bs), p2g_cells_smem<T>(bs), P, N, g, skeys,
-                             perm, n, fp32);
+        } else if (c->p2g_reduce >= 2) {  // shared-memory cell runs
+            bool mg_done = false;
+            if constexpr (sizeof(T) == 4) {
+                if (mg_in_p2g) {
+                    const size_t sm = p2g_cells_smem<float>(bp, true);
+                    if (bp == 128)
+                        LAUNCH_SMEM("p2g", k_p2g_cells_mg<128>, blocks_for(n, bp), bp, sm, P, N, g, skeys, perm, n,
+                                    fp32);
+                    else if (bp == 256)
+                        LAUNCH_SMEM("p2g", k_p2g_cells_mg<256>, blocks_for(n, bp), bp, sm, P, N, g, skeys, perm, n,
+                                    fp32);
+                    else
+                        LAUNCH_SMEM("p2g", k_p2g_cells_mg<512>, blocks_for(n, bp), bp, sm, P, N, g, skeys, perm, n,
+                                    fp32);
+                    mg_done = true;
+                }
+            }
+            const size_t sm = p2g_cells_smem<T>(bp);
+            if (!mg_done && c->have_fext)
+                LAUNCH_BS("p2g", k_p2g_cells, T, true, bp, blocks_for(n, bp), sm, P, N, g, skeys, perm, n, fp32);
+            else if (!mg_done)
+                LAUNCH_BS("p2g", k_p2g_cells, T, false, bp, blocks_for(n, bp), sm, P, N, g, skeys, perm, n, fp32);
         }
         else if (c->p2g_reduce == 1)
-            LAUNCH("p2g", (k_p2g<T, 1>), blocks_for(n, c->p2g_block), c->p2g_block, P, N, g, skeys, perm, n,
+            LAUNCH("p2g", (k_p2g<T, 1>), blocks_for(n, bp), bp, P, N, g, skeys, perm, n,
                    mg_in_p2g, fp32);
         else
-            LAUNCH("p2g", (k_p2g<T, 0>), blocks_for(n, c->p2g_block), c->p2g_block, P, N, g, skeys, perm, n,
+            LAUNCH("p2g", (k_p2g<T, 0>), blocks_for(n, bp), bp, P, N, g, skeys, perm, n,
                    mg_in_p2g, fp32);
         CK(cudaMemsetAsync(c->acount.p, 0, 4, c->stream));
         LAUNCH("active_list", k_compact_state, (unsigned)((nn + CS_THREADS * CS_ROUNDS - 1) / (CS_THREADS * CS_ROUNDS)),
@@ -967,7 +1012,7 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
                (double*)c->work_acc.p, dt);
         if (sizeof(T) == 4 && c->p2g_reduce >= 5) {  // the same runs as P2G, reduced by lane pairs
             if constexpr (sizeof(T) == 4) {
-                const int b1 = c->pass1_block;
+                const int b1 = auto_block(c, c->pass1_block);
                 const unsigned pg = (unsigned)((n + 4LL * b1 - 1) / (4LL * b1));
                 if (b1 == 128)
                     LAUNCH("pass1_remap", k_pass1_pairs<128>, pg, 128, P, N, g, skeys, perm, n, (float)dt, contact);
@@ -977,9 +1022,21 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
                     LAUNCH("pass1_remap", k_pass1_pairs<512>, pg, 512, P, N, g, skeys, perm, n, (float)dt, contact);
             }
         } else if (c->p2g_reduce >= 2) {  // the same reduction as P2G: shared-memory cell runs
-            const int b1 = c->pass1_block;
-            LAUNCH_CELLS("pass1_remap", k_pass1_cells, T, c->pass1_corners, b1, blocks_for(n, b1),
-                         pass1_cells_smem<T>(b1), P, N, g, skeys, perm, n, (T)dt, mm, contact);
+            const int cpt = c->pass1_corners, b1 = std::max(auto_block(c, c->pass1_block), cpt == 2 ? 32 : 128);
+            const unsigned gb = blocks_for(n, b1);
+            const size_t sm = pass1_cells_smem<T>(b1);
+            if (b1 == 128)
+                LAUNCH_SMEM("pass1_remap", (pass1_kernel<T, 128>(cpt)), gb, 128, sm, P, N, g, skeys, perm, n, (T)dt, contact);
+            else if (b1 == 256)
+                LAUNCH_SMEM("pass1_remap", (pass1_kernel<T, 256>(cpt)), gb, 256, sm, P, N, g, skeys, perm, n, (T)dt, contact);
+            else if (b1 == 512)
+                LAUNCH_SMEM("pass1_remap", (pass1_kernel<T, 512>(cpt)), gb, 512, sm, P, N, g, skeys, perm, n, (T)dt, contact);
+            else if constexpr (sizeof(T) == 8) {
+                if (b1 == 64)
+                    LAUNCH_SMEM("pass1_remap", (k_pass1_cells<T, 2, 64>), gb, 64, sm, P, N, g, skeys, perm, n, (T)dt, contact);
+                else
+                    LAUNCH_SMEM("pass1_remap", (k_pass1_cells<T, 2, 32>), gb, 32, sm, P, N, g, skeys, perm, n, (T)dt, contact);
+            }
         }
         else if (c->gather_batch)
             LAUNCH("pass1_remap", (k_pass1_remap<T, 1>), blocks_for(n), NTHREADS, P, N, g, skeys, perm, n, (T)dt, mm,
@@ -1031,7 +1088,8 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
             a.sg_acc = (SurrogateAcc*)c->sg_acc.p;
         }
         {
-            const unsigned pb = blocks_for(n, c->pass_block);
+            const int b2 = auto_block(c, c->pass_block);
+            const unsigned pb = blocks_for(n, b2);
             unsigned* kc = (unsigned*)c->keys_copy.p;
             const MatConst* mats = (const MatConst*)c->mats.p;
 #define PASS2(B, S) LAUNCH("pass2", (k_pass2<T, B, S>), pb, S, P, N, g, kc, keys_next, mats, c->nmat, a, err)
@@ -1046,22 +1104,24 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
             if (large) {
             } else if (c->gather_batch == 2 && sizeof(T) == 4) {
                 if constexpr (sizeof(T) == 4) {
-                    if (c->pass_block == 128)
+                    if (b2 == 128)
                         LAUNCH_SMEM("pass2", k_pass2_staged<128>, pb, 128, Pass2Stage<128>::SMEM, P, N, g, kc,
                                     keys_next, mats, c->nmat, a, err);
-                    else if (c->pass_block == 256)
+                    else if (b2 == 256)
                         LAUNCH_SMEM("pass2", k_pass2_staged<256>, pb, 256, Pass2Stage<256>::SMEM, P, N, g, kc,
                                     keys_next, mats, c->nmat, a, err);
                     else
                         LAUNCH_SMEM("pass2", k_pass2_staged<512>, pb, 512, Pass2Stage<512>::SMEM, P, N, g, kc,
                                     keys_next, mats, c->nmat, a, err);
                 }
-            } else if (c->pass_block == 128) {
+            } else if (b2 == 128) {
                 if (c->gather_batch == 1) PASS2(1, 128); else PASS2(0, 128);
-            } else if (c->pass_block == 256) {
+            } else if (b2 == 256) {
                 if (c->gather_batch == 1) PASS2(1, 256); else PASS2(0, 256);
-            } else {
+            } else if (b2 == 512) {
                 if (c->gather_batch == 1) PASS2(1, 512); else PASS2(0, 512);
+            } else if constexpr (sizeof(T) == 8) {
+                if (b2 == 64) PASS2(0, 64); else PASS2(0, 32);
             }
 #undef PASS2
         }
@@ -1228,14 +1288,19 @@ int alloc_particles(mpm_ctx* c, long long n) {
 // =============================================================================
 // C ABI
 // =============================================================================
-// The cell-run kernels stage up to 512 slots in shared memory (P2G: 123 KB
-// in FP64, pass 1: 54 KB): allow each instantiation its dynamic shared memory.
-template <typename T, int CPT, int BS>
+// The cell-run kernels stage up to 512 slots in shared memory (P2G: 101 KB
+// in FP64, pass 1: 52 KB): allow each instantiation its dynamic shared memory.
+template <typename T, int BS>
 bool cells_attr() {
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    return cudaFuncSetAttribute(k_p2g_cells<T, CPT, BS>, a, (int)p2g_cells_smem<T>(BS)) == cudaSuccess &&
-           cudaFuncSetAttribute(k_p2g_cells_mg<T, CPT, BS>, a, (int)p2g_cells_smem<T>(BS)) == cudaSuccess &&
-           cudaFuncSetAttribute(k_pass1_cells<T, CPT, BS>, a, (int)pass1_cells_smem<T>(BS)) == cudaSuccess;
+    bool ok = cudaFuncSetAttribute(k_p2g_cells<T, BS, false>, a, (int)p2g_cells_smem<T>(BS)) == cudaSuccess &&
+              cudaFuncSetAttribute(k_p2g_cells<T, BS, true>, a, (int)p2g_cells_smem<T>(BS)) == cudaSuccess &&
+              cudaFuncSetAttribute(k_pass1_cells<T, 1, BS>, a, (int)pass1_cells_smem<T>(BS)) == cudaSuccess &&
+              cudaFuncSetAttribute(k_pass1_cells<T, 2, BS>, a, (int)pass1_cells_smem<T>(BS)) == cudaSuccess &&
+              cudaFuncSetAttribute(k_pass1_cells<T, 4, BS>, a, (int)pass1_cells_smem<T>(BS)) == cudaSuccess;
+    if constexpr (sizeof(T) == 4)
+        ok = ok && cudaFuncSetAttribute(k_p2g_cells_mg<BS>, a, (int)p2g_cells_smem<T>(BS, true)) == cudaSuccess;
+    return ok;
 }
 template <int BS>
 bool pairs_attr() {
@@ -1253,9 +1318,7 @@ bool pass2_staged_attrs() {
 }
 template <typename T>
 bool cells_attrs() {
-    return cells_attr<T, 1, 128>() && cells_attr<T, 2, 128>() && cells_attr<T, 4, 128>() &&
-           cells_attr<T, 1, 256>() && cells_attr<T, 2, 256>() && cells_attr<T, 4, 256>() &&
-           cells_attr<T, 1, 512>() && cells_attr<T, 2, 512>() && cells_attr<T, 4, 512>();
+    return cells_attr<T, 128>() && cells_attr<T, 256>() && cells_attr<T, 512>();
 }
 
 extern "C" {
@@ -1310,7 +1373,6 @@ int mpm_create_batch(const mpm_grid_desc* grids, int32_t nspec, int form, mpm_ct
     c->tsize = form == MPM_FORM_FP64 ? 8 : 4;
     if (form == MPM_FORM_FP32) {  // the autotuner's choice on the honeycomb batch
         c->gather_batch = 2;
-        c->pass_block = 128;
     }
     c->nspec = nspec;
     cudaGetDevice(&c->device);
@@ -1345,6 +1407,7 @@ int mpm_create_batch(const mpm_grid_desc* grids, int32_t nspec, int form, mpm_ct
             g.xoff[a] = (int)tab.size();
             for (int i = -1; i <= g.nn[a]; ++i) tab.push_back(i * gd.length[a] / gd.cells[a]);
         }
+        set_key_division(g);
         g.key_off = key_off;
         g.node_off = node_off;
         key_off += (unsigned)ks;
@@ -1382,7 +1445,7 @@ int mpm_create_batch(const mpm_grid_desc* grids, int32_t nspec, int form, mpm_ct
     Geom& g = c->g;
     if ((rc = ensure(c, c->err_word, 4))) return bail(rc);
     cudaMemset(c->err_word.p, 0, 4);
-    if (cudaMallocHost((void**)&c->h_err, sizeof(unsigned)) != cudaSuccess) return bail(MPM_ERR_CUDA);
+    if (cudaMallocHost((void**)&c->h_err, 2 * sizeof(unsigned)) != cudaSuccess) return bail(MPM_ERR_CUDA);
     const size_t t = c->tsize, nn = (size_t)c->nn;
     struct {
         DevBuf* b;
@@ -1657,9 +1720,21 @@ int mpm_upload_particles(mpm_ctx* c, const mpm_particles* p, int64_t n) {
         LAUNCH("fill", k_compact_flag, blocks_for(n), NTHREADS, (const uint8_t*)c->pflags.p, (long long)n,
                (uint8_t)MPM_PF_SURFACE, (unsigned*)c->surf.p, (unsigned*)c->g_count.p);
     CK(cudaMemcpyAsync(c->h_err, c->g_count.p, 4, cudaMemcpyDeviceToHost, c->stream));
+    // whether any particle carries an external force (without one P2G does not read the forces)
+    if ((rc = ensure(c, c->fext_any, 4))) return rc;
+    CK(cudaMemsetAsync(c->fext_any.p, 0, 4, c->stream));
+    if (p->fext && n > 0) {
+        const unsigned fb = (unsigned)std::min<long long>(blocks_for(3 * n), (long long)c->sm_count * 8);
+        if (f64)
+            LAUNCH("fill", k_any_nonzero<double>, fb, NTHREADS, (const double*)c->fext.p, 3 * n, (unsigned*)c->fext_any.p);
+        else
+            LAUNCH("fill", k_any_nonzero<float>, fb, NTHREADS, (const float*)c->fext.p, 3 * n, (unsigned*)c->fext_any.p);
+    }
+    CK(cudaMemcpyAsync(c->h_err + 1, c->fext_any.p, 4, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->stream));
-    c->nsurf = (int)*c->h_err;
+    c->nsurf = (int)c->h_err[0];
+    c->have_fext = c->h_err[1] != 0u;
     c->have_particles = true;
     c->keys_valid = false;
     c->have_orig = false;  // the upload is in the caller's order
@@ -2102,7 +2177,8 @@ int mpm_autotune(mpm_ctx* c, int32_t steps, double dt, int contact, mpm_tune_res
         c->sim = sim0;
         return r;
     };
-    const int blocks[3] = {128, 256, 512}, corners[3] = {1, 2, 4};
+    // block candidates: 0 is 128, or fewer where the FP64 form's auto_block says so
+    const int blocks[3] = {0, 256, 512}, corners[3] = {1, 2, 4};
     const int p2g_modes = c->form == MPM_FORM_FP32 ? 7 : 5;
     for (int red = 0; red < p2g_modes && rc == MPM_OK; ++red)
         for (int pb = 0; pb < 3 && rc == MPM_OK; ++pb) rc = trial(0, red, 1, blocks[pb]);
@@ -2125,10 +2201,10 @@ int mpm_autotune(mpm_ctx* c, int32_t steps, double dt, int contact, mpm_tune_res
     for (int i = 0; i < 6; ++i) *opt[i] = best[i];
     if (out) {
         out->p2g_reduce = best[0];
-        out->p2g_block = best[1];
+        out->p2g_block = best[1] ? best[1] : 128;
         out->pass1_corners = best[2];
-        out->pass1_block = best[3];
-        out->pass_block = best[4];
+        out->pass1_block = best[3] ? best[3] : 128;
+        out->pass_block = best[4] ? best[4] : 128;
         out->gather_batch = best[5];
         out->candidates = ncand;
         out->best_ms_per_step = best_ms;

@@ -259,17 +259,28 @@ __global__ void __launch_bounds__(512) k_p2g(PView<T> P, NView<T> nd, Geom g, co
 }
 
 // ---------------------------------------------------------------------------
-// P2G, cell-centric (P2G_REDUCE = 2).  A block takes blockDim.x consecutive
-// sorted slots.  Phase 1: each slot's thread stages its particle's per-axis
-// bases (N and dN/du for both nodes of each axis) and transfer quantities
-// (m, m v, -V sigma, f_ext) in shared memory.  Phase 2: one thread per
-// (run of equal cell keys, corner) sums that corner's contributions over the
-// run's particles in slot order and issues one atomic per field.  Same
-// per-particle arithmetic as k_p2g; the cross-lane shuffles of REDUCE = 1
-// become shared-memory reads, and the atomics are issued by full warps.
-// Shared memory: (12 + 13) values per slot (the 12 base rows padded to an odd
-// stride) plus each slot's cell nodes and key, and the run starts
-// (p2g_cells_smem); phase 2 takes the run's nodes from its first slot.
+// P2G, cell-centric (P2G modes 2 to 4).  A block takes BS consecutive slots.
+// Phase 1: each slot's thread stages its particle's shape factors and transfer
+// quantities in shared memory.  Phase 2: four threads per run of equal cell
+// keys sum the run's contributions in slot order and issue one atomic per
+// corner and field.
+//
+// What the four threads sum is the run's moments, not its corners.  With v =
+// -V sigma and the trilinear N a corner's force is
+//   -(sx FX(iy, iz) + sy FY(ix, iz) + sz FZ(ix, iy)) + sum N f_ext,
+// s = +1/h at the lower and -1/h at the upper node of an axis, FX = sum over
+// the particles of Ny Nz (v_xx, v_xy, v_xz) and FY, FZ likewise.  Thread (a, b)
+// = (0..1, 0..1) keeps mass and momentum of the corners (ix, iy) = (a, b), iz =
+// 0, 1, and the moments FX(a, b), FY(a, b), FZ(a, b): 22 multiply-adds per
+// particle and thread against 39 when each thread formed its corners' forces,
+// and the moments are exchanged by shuffles once per run.  This is what bounds
+// the FP64 form (its FP64 pipe) and shortens the FP32 form's issue-bound sums.
+//
+// The gradient factors of a particle within 1e-12 of a node plane are zero
+// (GridPoint_Mediator.cpp:118-133).  Its quantities are then staged as zero for
+// that axis.  Where rounding leaves one of the axis' two factors (FP32: a
+// cell-local coordinate below 3e-8), the staging thread adds that factor's
+// share to the nodes itself (rare: one particle in some ten million).
 // ---------------------------------------------------------------------------
 // Runs of equal cell keys among the block's first nslots slots (keys staged
 // in shared memory, a __syncthreads after the staging): run r covers slots
@@ -302,10 +313,6 @@ __device__ __forceinline__ int block_runs(const unsigned* skey, int nslots, int*
     return R;
 }
 
-// Per slot, beside the values: the cell's nodes (n0, sz, sy, mask: 24 bytes)
-// and the key; then the run starts (bs + 1) and the warp counts.
-constexpr size_t CELL_SLOT_BYTES = 28;
-
 // FP32 cell-run value rows: slot s is stored at row position s ^ ((s >> 3) & 7),
 // a permutation inside each aligned group of 8 slots (block sizes are multiples
 // of 8).  The cell runs one warp sums start 8 slots apart when cells hold 8
@@ -314,280 +321,263 @@ constexpr size_t CELL_SLOT_BYTES = 28;
 // eight distinct bank groups.  Sums still run in slot order.
 __device__ __forceinline__ int slot_swz(int s) { return s ^ ((s >> 3) & 7); }
 
-template <typename T>
-__host__ __device__ constexpr size_t p2g_cells_smem(int bs) {
-    return (sizeof(T) == 4 ? (size_t)25 * bs * 4 : ((size_t)12 * (bs + 1) + (size_t)13 * bs) * sizeof(T)) +
-           (size_t)bs * CELL_SLOT_BYTES + (size_t)(bs + 1) * 4 + 64 * 4;
-}
-
-// The slot arrays that follow the values (8-byte aligned: even bs).
+// The run arrays that follow the values: the slots' cell keys, the run starts
+// (bs + 1) and 32 warp counts with their total.
 struct CellSlots {
-    long long *n0, *sz;
-    int* sy;
-    unsigned *mask, *key;
+    unsigned* key;
     int *run_start, *wsum;
     __device__ __forceinline__ CellSlots(unsigned char* at, int bs) {
-        n0 = reinterpret_cast<long long*>(at);
-        sz = n0 + bs;
-        sy = reinterpret_cast<int*>(sz + bs);
-        mask = reinterpret_cast<unsigned*>(sy + bs);
-        key = mask + bs;
-        run_start = reinterpret_cast<int*>(key + bs);  // bs + 1
-        wsum = run_start + bs + 1;                     // 32 warp counts + total
-    }
-    __device__ __forceinline__ void put(int t, const CellNodes& c) const {
-        n0[t] = c.n0;
-        sz[t] = c.sz;
-        sy[t] = c.sy;
-        mask[t] = c.mask;
-    }
-    // corner k's node of the cell staged at slot a, or -1 out of range
-    __device__ __forceinline__ long long node(int a, int k) const {
-        if (!((mask[a] >> k) & 1u)) return -1;
-        CellNodes c;
-        c.n0 = n0[a];
-        c.sz = sz[a];
-        c.sy = sy[a];
-        return cell_node(c, k);
+        key = reinterpret_cast<unsigned*>(at);
+        run_start = reinterpret_cast<int*>(key + bs);
+        wsum = run_start + bs + 1;
     }
 };
+__host__ __device__ constexpr size_t cell_slots_bytes(int bs) { return (size_t)bs * 4 + (size_t)(bs + 1) * 4 + 64 * 4; }
 
-// CPT corners per phase-2 thread (1, 2 or 4): the corners sharing the
-// thread's x (CPT 4) or x and y (CPT 2) bases, so a particle's quantities are
-// read from shared memory 8 / CPT times instead of 8.  BS, the block size, is
-// a compile-time constant so the shared-memory rows sit at fixed offsets from
-// one address.
-// A cell-run P2G block of BS slots in shared memory: the per-axis bases, the
-// transfer quantities (m, m v (3), -V sigma (6), f_ext (3)) and the slots
-// (cell nodes, key, runs).  FP64: 12 rows of BS + 1 bases (the odd stride puts
-// the two nodes' values of an axis in different banks; Nx0 Nx1 Ny0 Ny1 Nz0
-// Nz1 gx0 gx1 gy0 gy1 gz0 gz1) and 13 rows of BS quantities.  FP32: six rows
-// of BS float4 ({Nx0 Nx1 gx0 gx1}, y, z, {m, m v}, {-V sigma 0..3},
-// {-V sigma 4..5, f_ext 0..1}) and a row of f_ext 2, so a scatter thread reads
-// a particle with seven shared loads.
-template <typename T, int BS>
+// A slot's staged values, in rows of four (Quad): {m, m v}, {-V sigma xx xy zx,
+// Nx0}, {xy yy yz, Ny0}, {zx yz zz, Nz0} (an axis' row zeroed when its gradient
+// factors are), {f_ext, 0}; FP64: {Nx1, Ny1, Nz1, 0} (FP32: N1 = 1 - |u - 1| is
+// 1 - N0 to the bit); FP32 with mass gradients: {m or 0 per axis, 0}.
+// FP32: the axis rows carry the factor 1/h and the slot's corner nodes are
+// staged too, so a run needs no geometry of its own; FP64: the 1/h and the
+// nodes come once per run (nine FP64 products per particle less).
+template <typename T>
+__host__ __device__ constexpr int p2g_rows(bool mg) {
+    return sizeof(T) == 8 || mg ? 6 : 5;
+}
+template <typename T>
+__host__ __device__ constexpr size_t p2g_cells_smem(int bs, bool mg = false) {
+    return (size_t)p2g_rows<T>(mg) * bs * 4 * sizeof(T) + (sizeof(T) == 4 ? bs * sizeof(CellNodes) : 0) +
+           cell_slots_bytes(bs);
+}
+
+template <typename T>
+__device__ __forceinline__ T quad_shfl(T v, int src) {
+    return __shfl_sync(FULL_MASK, v, src);
+}
+
+template <typename T, int BS, bool FE, bool MG>
 struct P2GBlock {
-    static constexpr int S = BS + 1;
-    T* sw;
-    T* sq;
+    using Q = Quad<T>;
+    static constexpr bool F32 = sizeof(T) == 4;
+    Q* row;
+    CellNodes* nodes;  // FP32
     CellSlots cs;
     __device__ __forceinline__ explicit P2GBlock(unsigned char* raw)
-        : sw(reinterpret_cast<T*>(raw)), sq(sw + (sizeof(T) == 4 ? 24 * BS : 12 * S)),
-          cs(reinterpret_cast<unsigned char*>(sq + (sizeof(T) == 4 ? BS : 13 * BS)), BS) {}
+        : row(reinterpret_cast<Q*>(raw)),
+          nodes(reinterpret_cast<CellNodes*>(row + p2g_rows<T>(MG) * BS)),
+          cs(reinterpret_cast<unsigned char*>(nodes + (F32 ? BS : 0)), BS) {
+        static_assert(!MG || sizeof(T) == 4, "mass gradients: FP32 form");
+    }
 
-    // slot t's particle: bases, mass m, volume V, velocity v, external force fe, stress sig, its cell's nodes
-    __device__ __forceinline__ void stage(int t, const Bases<T>& B, T m, T V, const T v[3], const T fe[3],
-                                          const T sig[6], const CellNodes& cn) const {
-        if constexpr (sizeof(T) == 4) {
-            static_assert(BS % 8 == 0, "slot swizzle groups");
-            float4* sv = reinterpret_cast<float4*>(sw);
-            const int u = slot_swz(t);
-            sv[u] = make_float4(B.Nx[0], B.Nx[1], B.gx[0], B.gx[1]);
-            sv[BS + u] = make_float4(B.Ny[0], B.Ny[1], B.gy[0], B.gy[1]);
-            sv[2 * BS + u] = make_float4(B.Nz[0], B.Nz[1], B.gz[0], B.gz[1]);
-            sv[3 * BS + u] = make_float4(m, m * v[0], m * v[1], m * v[2]);
-            sv[4 * BS + u] = make_float4(-V * sig[0], -V * sig[1], -V * sig[2], -V * sig[3]);
-            sv[5 * BS + u] = make_float4(-V * sig[4], -V * sig[5], fe[0], fe[1]);
-            sq[u] = fe[2];
-            cs.put(t, cn);
-            return;
-        }
-        sw[0 * S + t] = B.Nx[0];
-        sw[1 * S + t] = B.Nx[1];
-        sw[2 * S + t] = B.Ny[0];
-        sw[3 * S + t] = B.Ny[1];
-        sw[4 * S + t] = B.Nz[0];
-        sw[5 * S + t] = B.Nz[1];
-        sw[6 * S + t] = B.gx[0];
-        sw[7 * S + t] = B.gx[1];
-        sw[8 * S + t] = B.gy[0];
-        sw[9 * S + t] = B.gy[1];
-        sw[10 * S + t] = B.gz[0];
-        sw[11 * S + t] = B.gz[1];
-        sq[t] = m;
+    // One gradient factor of an axis is zero and the other is not: the other's
+    // share of the particle's force (and mass gradient), added to its four
+    // nodes.  bit, step: the axis' corner bit and node stride; p, q: the other two
+    // axes' shape factors, bits and strides.
+    static __device__ __forceinline__ void lone_factor(const NView<T>& nd, const CellNodes& cn, int axis, int bit,
+                                                       unsigned step, const T G[2], const T Np[2], int bitp,
+                                                       unsigned stepp, const T Nq[2], int bitq, unsigned stepq, T v0,
+                                                       T v1, T v2, T m) {
+        const bool up = G[1] != (T)0;
+        const T g = up ? G[1] : G[0];
+        const unsigned n0 = cn.n0 + (up ? step : 0u);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            sq[(1 + c) * BS + t] = m * v[c];
-            sq[(10 + c) * BS + t] = fe[c];
+        for (int c = 0; c < 4; ++c) {
+            const int op = c >> 1, oq = c & 1;
+            const int k = (up ? bit : 0) | (op ? bitp : 0) | (oq ? bitq : 0);
+            if (!((cn.mask >> k) & 1u)) continue;
+            const long long nid = n0 + (op ? stepp : 0u) + (oq ? stepq : 0u);
+            const T w = -(Np[op] * Nq[oq]) * g;
+            atomicAdd(nd.acc + 8 * nid + 4, w * v0);
+            atomicAdd(nd.acc + 8 * nid + 5, w * v1);
+            atomicAdd(nd.acc + 8 * nid + 6, w * v2);
+            if constexpr (MG) atomicAdd(nd.mg + axis * nd.nn + nid, w * m);
         }
+    }
+
+    // slot t's particle: bases, mass m, volume V, velocity v, external force fe, stress sig
+    __device__ __forceinline__ void stage(int t, const NView<T>& nd, const Geom& g, const int b[3], const Bases<T>& B,
+                                          T m, T V, const T v[3], const T fe[3], const T sig[6]) const {
+        static_assert(BS % 8 == 0, "slot swizzle groups");
+        const int u = slot_swz(t);
+        const bool x0 = B.gx[0] != (T)0, y0 = B.gy[0] != (T)0, z0 = B.gz[0] != (T)0;
+        const bool x1 = B.gx[1] != (T)0, y1 = B.gy[1] != (T)0, z1 = B.gz[1] != (T)0;
+        T s[6];
 #pragma unroll
-        for (int c = 0; c < 6; ++c) sq[(4 + c) * BS + t] = -V * sig[c];
-        cs.put(t, cn);
+        for (int c = 0; c < 6; ++c) s[c] = -V * sig[c];
+        if (x0 != x1 || y0 != y1 || z0 != z1) {
+            const CellNodes cn = cell_nodes(g, b);
+            if (x0 != x1) lone_factor(nd, cn, 0, 4, 1u, B.gx, B.Ny, 2, cn.sy, B.Nz, 1, cn.sz, s[0], s[3], s[5], m);
+            if (y0 != y1) lone_factor(nd, cn, 1, 2, cn.sy, B.gy, B.Nx, 4, 1u, B.Nz, 1, cn.sz, s[3], s[1], s[4], m);
+            if (z0 != z1) lone_factor(nd, cn, 2, 1, cn.sz, B.gz, B.Nx, 4, 1u, B.Ny, 2, cn.sy, s[5], s[4], s[2], m);
+        }
+        const bool x = x0 && x1, y = y0 && y1, z = z0 && z1;
+        const T o = (T)0;
+        row[u] = Q{m, m * v[0], m * v[1], m * v[2]};
+        if constexpr (F32) {
+            const T hx = x ? B.gx[0] : o, hy = y ? B.gy[0] : o, hz = z ? B.gz[0] : o;
+            row[BS + u] = Q{hx * s[0], hx * s[3], hx * s[5], B.Nx[0]};
+            row[2 * BS + u] = Q{hy * s[3], hy * s[1], hy * s[4], B.Ny[0]};
+            row[3 * BS + u] = Q{hz * s[5], hz * s[4], hz * s[2], B.Nz[0]};
+            nodes[t] = cell_nodes(g, b);
+        } else {
+            row[BS + u] = Q{x ? s[0] : o, x ? s[3] : o, x ? s[5] : o, B.Nx[0]};
+            row[2 * BS + u] = Q{y ? s[3] : o, y ? s[1] : o, y ? s[4] : o, B.Ny[0]};
+            row[3 * BS + u] = Q{z ? s[5] : o, z ? s[4] : o, z ? s[2] : o, B.Nz[0]};
+        }
+        if constexpr (FE) row[4 * BS + u] = Q{fe[0], fe[1], fe[2], o};
+        if constexpr (MG)
+            row[5 * BS + u] = Q{x ? B.gx[0] * m : o, y ? B.gy[0] * m : o, z ? B.gz[0] * m : o, o};
+        if constexpr (sizeof(T) == 8) row[5 * BS + u] = Q{B.Nx[1], B.Ny[1], B.Nz[1], o};
     }
 
     // After the staging and a __syncthreads (keys in cs.key for the first nslots
-    // slots, out of range where nothing was staged): one thread per (cell run,
-    // CPT corners) sums the run's contributions in slot order and issues one
-    // atomic per field; mark_active also marks the corners active.  MG: also the
-    // node mass gradients.
+    // slots, out of range where nothing was staged): the runs' sums and their
+    // atomics; mark_active also marks the corners active.  MG: also the node
+    // mass gradients.  sid: the slots' specimens from the block's first slot on
+    // (perm: through the sort order), for the runs' geometry.
     //
-    // FP32: a warp holds consecutive runs, the TPR threads of a run in
-    // adjacent lanes.  When run r's cell follows run r - 1's in x (key + 1),
-    // the x = 1 corners of r - 1 are the x = 0 corners of r: one shuffle of
-    // the sums, TPR / 2 lanes up, adds them to r's, and only r's lanes issue
-    // the atomics (in the batch about three runs in four have such a
-    // neighbour, so a third of the corner atomics go).
-    template <int CPT, bool MG>
-    __device__ __forceinline__ void scatter(const NView<T>& nd, const Geom& g, int nslots, int mark_active) const {
-        static_assert(CPT == 1 || CPT == 2 || CPT == 4, "corners per thread");
-        constexpr int bs = BS;
+    // FP32: a warp holds consecutive runs, the threads of a run in adjacent
+    // lanes.  When run r's cell follows run r - 1's in x (key + 1), the x = 1
+    // corners of r - 1 are the x = 0 corners of r: one shuffle of the sums, two
+    // lanes up, adds them to r's, and only r's lanes issue the atomics (in the
+    // honeycomb batch about three runs in four have such a neighbour, so a
+    // third of the corner atomics go).
+    __device__ __forceinline__ void scatter(const NView<T>& nd, const Geom& g, const uint16_t* __restrict__ sid,
+                                            const unsigned* __restrict__ perm, long long s0, int nslots,
+                                            int mark_active) const {
         const int t = threadIdx.x, lane = t & 31;
         const long long nn = nd.nn;
         const unsigned* skey = cs.key;
         const int R = block_runs(skey, nslots, cs.run_start, cs.wsum);
-        constexpr int TPR = 8 / CPT;  // threads per run
-        const int nitems = R * TPR;
-        // whole warps take the loop together (the merge shuffles)
-        for (int item = t; item - lane < nitems; item += bs) {
+        const int nitems = R * 4;
+        const int quad = lane & ~3, a = (t >> 1) & 1, b = t & 1;
+        // whole warps take the loop together (the shuffles)
+        for (int item = t; item - lane < nitems; item += BS) {
             const bool live = item < nitems;
-            const int r = live ? item / TPR : 0, kq = item % TPR, k0 = kq * CPT;  // corners k0 .. k0 + CPT - 1
-            const int a = cs.run_start[r];
+            const int r = live ? item >> 2 : 0;
+            const int first = cs.run_start[r];
+            const unsigned key = skey[first];
             // slots outside the grid (and lanes past the items) sum nothing
-            const bool inb = live && skey[a] < g.key_max;
-            const int e = inb ? cs.run_start[r + 1] : a;
-            T am[CPT], ap0[CPT], ap1[CPT], ap2[CPT], af0[CPT], af1[CPT], af2[CPT], g0[CPT], g1[CPT], g2[CPT];
-    #pragma unroll
-            for (int j = 0; j < CPT; ++j) am[j] = ap0[j] = ap1[j] = ap2[j] = af0[j] = af1[j] = af2[j] = g0[j] = g1[j] = g2[j] = 0;
-            for (int i = a; i < e; ++i) {
-                T m, mv0, mv1, mv2, v0, v1, v2, v3, v4, v5, fe0, fe1, fe2;
-                float4 X, Y, Z;
-                if constexpr (sizeof(T) == 4) {
-                    const float4* sv = reinterpret_cast<const float4*>(sw);
-                    const int u = slot_swz(i);
-                    X = sv[u];
-                    Y = sv[BS + u];
-                    Z = sv[2 * BS + u];
-                    const float4 q0 = sv[3 * BS + u], q1 = sv[4 * BS + u], q2 = sv[5 * BS + u];
-                    m = q0.x, mv0 = q0.y, mv1 = q0.z, mv2 = q0.w;
-                    v0 = q1.x, v1 = q1.y, v2 = q1.z, v3 = q1.w;
-                    v4 = q2.x, v5 = q2.y, fe0 = q2.z, fe1 = q2.w;
-                    fe2 = sq[u];
+            const bool inb = live && key < g.key_max;
+            const int e = inb ? cs.run_start[r + 1] : first;
+            T c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0};          // {m, m v} of the corners iz = 0, 1
+            T fx[3] = {0, 0, 0}, fy[3] = {0, 0, 0}, fz[3] = {0, 0, 0};  // moments (a, b)
+            T e0[3] = {0, 0, 0}, e1[3] = {0, 0, 0};                // N f_ext
+            T mx = 0, my = 0, mz = 0;                              // mass moments (MG)
+#pragma unroll 1
+            for (int i = first; i < e; ++i) {
+                const int u = slot_swz(i);
+                const Q q = row[u], X = row[BS + u], Y = row[2 * BS + u], Z = row[3 * BS + u];
+                T nx1, ny1, nz1;
+                if constexpr (sizeof(T) == 8) {
+                    const Q N = row[5 * BS + u];
+                    nx1 = N.x, ny1 = N.y, nz1 = N.z;
                 } else {
-                    m = sq[i], mv0 = sq[1 * bs + i], mv1 = sq[2 * bs + i], mv2 = sq[3 * bs + i];
-                    v0 = sq[4 * bs + i], v1 = sq[5 * bs + i], v2 = sq[6 * bs + i];
-                    v3 = sq[7 * bs + i], v4 = sq[8 * bs + i], v5 = sq[9 * bs + i];
-                    fe0 = sq[10 * bs + i], fe1 = sq[11 * bs + i], fe2 = sq[12 * bs + i];
+                    nx1 = (T)1 - X.w, ny1 = (T)1 - Y.w, nz1 = (T)1 - Z.w;
                 }
-                if constexpr (sizeof(T) == 4 && CPT >= 2) {
-                    // FP32, corners sharing x (and y) bases: the products are
-                    // regrouped around the z factor.  With A = Nx Ny, Bx = Ny gx,
-                    // By = Nx gy a corner's N = A Nz, G = -(Bx Nz, By Nz, A gz),
-                    // so its seven sums are N m, N m v and Nz c + gz d, with
-                    // c and d formed once per slot and (x, y) pair.
-                    const int ix = (k0 >> 2) & 1;
-                    const float nx = ix ? X.y : X.x, gxv = ix ? X.w : X.z;
+                const T nx = a ? nx1 : X.w, nya = a ? ny1 : Y.w, nyb = b ? ny1 : Y.w;
+                const T nz0 = Z.w, nzb = b ? nz1 : nz0;
+                const T A = nx * nyb, w0 = A * nz0, w1 = A * nz1, wx = nya * nzb, wy = nx * nzb;
+                c0[0] += w0 * q.x, c0[1] += w0 * q.y, c0[2] += w0 * q.z, c0[3] += w0 * q.w;
+                c1[0] += w1 * q.x, c1[1] += w1 * q.y, c1[2] += w1 * q.z, c1[3] += w1 * q.w;
+                fx[0] += wx * X.x, fx[1] += wx * X.y, fx[2] += wx * X.z;
+                fy[0] += wy * Y.x, fy[1] += wy * Y.y, fy[2] += wy * Y.z;
+                fz[0] += A * Z.x, fz[1] += A * Z.y, fz[2] += A * Z.z;
+                if constexpr (FE) {
+                    const Q f = row[4 * BS + u];
+                    e0[0] += w0 * f.x, e0[1] += w0 * f.y, e0[2] += w0 * f.z;
+                    e1[0] += w1 * f.x, e1[1] += w1 * f.y, e1[2] += w1 * f.z;
+                }
+                if constexpr (MG) {
+                    const Q M = row[5 * BS + u];
+                    mx += wx * M.x, my += wy * M.y, mz += A * M.z;
+                }
+            }
+            // the run's geometry and corner nodes
+            CellNodes cn{0u, 0u, 0u, 0u};
+            T hx = 1, hy = 1, hz = 1;  // 1/h where the staged rows do not carry it
+            if constexpr (F32) {
+                if (inb) cn = nodes[first];
+            } else if (inb) {
+                const Geom& gs = (g.nspec > 1) ? g.tab[sid[perm ? perm[s0 + first] : s0 + first]] : g;
+                int base[3];
+                key_to_base(key, gs, base);
+                cn = cell_nodes(gs, base);
+                hx = gs.inv_h[0];
+                hy = gs.inv_h[1];
+                hz = gs.inv_h[2];
+            }
+            if (a == 0) hx = -hx;  // -s of this thread's corners (ix, iy) = (a, b)
+            if (b == 0) hy = -hy;
+            T p0[3], p1[3], g0[3], g1[3];
 #pragma unroll
-                    for (int jy = 0; jy < CPT / 2; ++jy) {
-                        const int iy = CPT == 4 ? jy : ((k0 >> 1) & 1);
-                        const float ny = iy ? Y.y : Y.x, gyv = iy ? Y.w : Y.z;
-                        const float A = nx * ny, Bx = ny * gxv, By = nx * gyv;
-                        const float Am = A * m, Am0 = A * mv0, Am1 = A * mv1, Am2 = A * mv2;
-                        const float c0 = A * fe0 - Bx * v0 - By * v3;
-                        const float c1 = A * fe1 - By * v1 - Bx * v3;
-                        const float c2 = A * fe2 - Bx * v5 - By * v4;
-                        const float d0 = -A * v5, d1 = -A * v4, d2 = -A * v2;
-#pragma unroll
-                        for (int iz = 0; iz < 2; ++iz) {
-                            const int j = 2 * jy + iz;
-                            const float nz = iz ? Z.y : Z.x, gzv = iz ? Z.w : Z.z;
-                            am[j] += nz * Am;
-                            ap0[j] += nz * Am0;
-                            ap1[j] += nz * Am1;
-                            ap2[j] += nz * Am2;
-                            af0[j] = fmaf(gzv, d0, fmaf(nz, c0, af0[j]));
-                            af1[j] = fmaf(gzv, d1, fmaf(nz, c1, af1[j]));
-                            af2[j] = fmaf(gzv, d2, fmaf(nz, c2, af2[j]));
-                            if constexpr (MG) {
-                                g0[j] -= nz * (Bx * m);
-                                g1[j] -= nz * (By * m);
-                                g2[j] -= gzv * Am;
-                            }
-                        }
-                    }
-                    continue;
-                }
-    #pragma unroll
-                for (int j = 0; j < CPT; ++j) {
-                    const int k = k0 + j;
-                    const int ix = (k >> 2) & 1, iy = (k >> 1) & 1, iz = k & 1;
-                    T nx, ny, nz, gxv, gyv, gzv;
-                    if constexpr (sizeof(T) == 4) {
-                        nx = ix ? X.y : X.x, gxv = ix ? X.w : X.z;
-                        ny = iy ? Y.y : Y.x, gyv = iy ? Y.w : Y.z;
-                        nz = iz ? Z.y : Z.x, gzv = iz ? Z.w : Z.z;
-                    } else {
-                        nx = sw[ix * S + i], ny = sw[(2 + iy) * S + i], nz = sw[(4 + iz) * S + i];
-                        gxv = sw[(6 + ix) * S + i], gyv = sw[(8 + iy) * S + i], gzv = sw[(10 + iz) * S + i];
-                    }
-                    const T N = nx * ny * nz;
-                    const T G0 = -(ny * nz) * gxv;
-                    const T G1 = -(nx * nz) * gyv;
-                    const T G2 = -(nx * ny) * gzv;
-                    am[j] += N * m;
-                    ap0[j] += N * mv0;
-                    ap1[j] += N * mv1;
-                    ap2[j] += N * mv2;
-                    af0[j] += G0 * v0 + G1 * v3 + G2 * v5 + N * fe0;
-                    af1[j] += G1 * v1 + G0 * v3 + G2 * v4 + N * fe1;
-                    af2[j] += G2 * v2 + G0 * v5 + G1 * v4 + N * fe2;
-                    if constexpr (MG) {
-                        g0[j] += G0 * m;
-                        g1[j] += G1 * m;
-                        g2[j] += G2 * m;
-                    }
-                }
+            for (int c = 0; c < 3; ++c) {
+                const T X0 = quad_shfl(fx[c], quad + 2 * b), X1 = quad_shfl(fx[c], quad + 2 * b + 1);
+                const T Y0 = quad_shfl(fy[c], quad + 2 * a), Y1 = quad_shfl(fy[c], quad + 2 * a + 1);
+                p0[c] = e0[c] + (hx * X0 + hy * Y0 - hz * fz[c]);
+                p1[c] = e1[c] + (hx * X1 + hy * Y1 + hz * fz[c]);
+            }
+            if constexpr (MG) {
+                g0[0] = hx * quad_shfl(mx, quad + 2 * b), g1[0] = hx * quad_shfl(mx, quad + 2 * b + 1);
+                g0[1] = hy * quad_shfl(my, quad + 2 * a), g1[1] = hy * quad_shfl(my, quad + 2 * a + 1);
+                g0[2] = -hz * mz, g1[2] = hz * mz;
             }
             bool skip = !inb;
             if constexpr (sizeof(T) == 4) {
-                constexpr int SH = TPR / 2;  // lanes from run r - 1's x = 1 corners to run r's x = 0 corners
-                const bool recv = inb && kq < SH && lane >= SH && r > 0 && skey[cs.run_start[r - 1]] + 1u == skey[a];
+                constexpr int SH = 2;  // lanes from run r - 1's x = 1 corners to run r's x = 0 corners
+                const bool recv = inb && !a && lane >= SH && r > 0 && skey[cs.run_start[r - 1]] + 1u == key;
 #pragma unroll
-                for (int j = 0; j < CPT; ++j) {
-                    const float x0 = __shfl_up_sync(FULL_MASK, am[j], SH), x1 = __shfl_up_sync(FULL_MASK, ap0[j], SH);
-                    const float x2 = __shfl_up_sync(FULL_MASK, ap1[j], SH), x3 = __shfl_up_sync(FULL_MASK, ap2[j], SH);
-                    const float x4 = __shfl_up_sync(FULL_MASK, af0[j], SH), x5 = __shfl_up_sync(FULL_MASK, af1[j], SH);
-                    const float x6 = __shfl_up_sync(FULL_MASK, af2[j], SH);
-                    if (recv) {
-                        am[j] += x0, ap0[j] += x1, ap1[j] += x2, ap2[j] += x3;
-                        af0[j] += x4, af1[j] += x5, af2[j] += x6;
-                    }
+                for (int c = 0; c < 4; ++c) {
+                    const float x0 = __shfl_up_sync(FULL_MASK, c0[c], SH), x1 = __shfl_up_sync(FULL_MASK, c1[c], SH);
+                    if (recv) c0[c] += x0, c1[c] += x1;
+                }
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const float x0 = __shfl_up_sync(FULL_MASK, p0[c], SH), x1 = __shfl_up_sync(FULL_MASK, p1[c], SH);
+                    if (recv) p0[c] += x0, p1[c] += x1;
                     if constexpr (MG) {
-                        const float y0 = __shfl_up_sync(FULL_MASK, g0[j], SH);
-                        const float y1 = __shfl_up_sync(FULL_MASK, g1[j], SH);
-                        const float y2 = __shfl_up_sync(FULL_MASK, g2[j], SH);
-                        if (recv) g0[j] += y0, g1[j] += y1, g2[j] += y2;
+                        const float y0 = __shfl_up_sync(FULL_MASK, g0[c], SH);
+                        const float y1 = __shfl_up_sync(FULL_MASK, g1[c], SH);
+                        if (recv) g0[c] += y0, g1[c] += y1;
                     }
                 }
                 // a sender's sums went to the lane SH up (lanes near the warp's top read their own false)
-                if (__shfl_down_sync(FULL_MASK, recv ? 1 : 0, SH) && kq >= SH) skip = true;
+                if (__shfl_down_sync(FULL_MASK, recv ? 1 : 0, SH) && a) skip = true;
             }
             if (skip) continue;
+            const unsigned n0 = cn.n0 + a + (b ? cn.sy : 0u);
+            const unsigned ok = cn.mask >> (4 * a + 2 * b);
 #pragma unroll
-            for (int j = 0; j < CPT; ++j) {
-                const long long nid = cs.node(a, k0 + j);
-                if (nid < 0) continue;
+            for (int iz = 0; iz < 2; ++iz) {
+                if (!((ok >> iz) & 1u)) continue;
+                const long long nid = iz ? n0 + cn.sz : n0;
+                const T* c = iz ? c1 : c0;
+                const T* f = iz ? p1 : p0;
                 // active nodes: the in-range corners of occupied cells (b_Active, …MPLocks.cpp:36)
                 if (mark_active) atomicOr(&nd.state[nid], 1u);  // a reduction: no load to wait for
-                acc_add<T>(nd.acc, nid, am[j], ap0[j], ap1[j], ap2[j], af0[j], af1[j], af2[j]);
+                acc_add<T>(nd.acc, nid, c[0], c[1], c[2], c[3], f[0], f[1], f[2]);
                 if constexpr (MG) {
-                    atomicAdd(&nd.mg[nid], g0[j]);
-                    atomicAdd(&nd.mg[nn + nid], g1[j]);
-                    atomicAdd(&nd.mg[2 * nn + nid], g2[j]);
+                    const T* gm = iz ? g1 : g0;
+                    atomicAdd(&nd.mg[nid], gm[0]);
+                    atomicAdd(&nd.mg[nn + nid], gm[1]);
+                    atomicAdd(&nd.mg[2 * nn + nid], gm[2]);
                 }
             }
         }
     }
 };
 
-// MG: also the contact path's node mass gradients (output steps only).
-template <typename T, int CPT, int BS, bool MG>
+// FE: some particle carries an external force (uploaded; without one the forces are not read).  MG: also the contact
+// path's node mass gradients (output steps of the FP32 form).
+template <typename T, int BS, bool FE, bool MG>
 __device__ __forceinline__ void p2g_cells_run(const PView<T>& P, const NView<T>& nd, const Geom& g,
                                               const unsigned* __restrict__ skeys, const unsigned* __restrict__ perm,
                                               long long n, int mark_active) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const P2GBlock<T, BS> blk(smem_raw);
+    const P2GBlock<T, BS, FE, MG> blk(smem_raw);
     const int t = threadIdx.x;
-    const long long s = blockIdx.x * (long long)BS + t;
+    const long long s0 = blockIdx.x * (long long)BS, s = s0 + t;
     const unsigned key = (s < n) ? skeys[s] : 0xffffffffu;
     const long long np = P.n;
     if (key < g.key_max) {
@@ -597,40 +587,39 @@ __device__ __forceinline__ void p2g_cells_run(const PView<T>& P, const NView<T>&
         key_to_base(key, gs, b);
         Bases<T> B;
         particle_bases<T>(P, gs, p, b, B);
-        T v[3], fe[3], sig[6];
+        T v[3], fe[3] = {0, 0, 0}, sig[6];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            v[c] = P.vel[c * np + p];
-            fe[c] = P.fext[c * np + p];
+        for (int c = 0; c < 3; ++c) v[c] = P.vel[c * np + p];
+        if constexpr (FE) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) fe[c] = P.fext[c * np + p];
         }
 #pragma unroll
         for (int c = 0; c < 6; ++c) sig[c] = P.stress[c * np + p];
-        blk.stage(t, B, P.mass[p], P.vol[p], v, fe, sig, cell_nodes(gs, b));
+        blk.stage(t, nd, gs, b, B, P.mass[p], P.vol[p], v, fe, sig);
     }
     blk.cs.key[t] = key;
     __syncthreads();
-    blk.template scatter<CPT, MG>(nd, g, (int)min((long long)BS, n - blockIdx.x * (long long)BS), mark_active);
+    blk.scatter(nd, g, P.sid, perm, s0, (int)min((long long)BS, n - s0), mark_active);
 }
 
-// FP32 with 1 or 2 corners per thread: registers capped for 1536 resident
-// threads per SM (40 registers, no spills at 2 corners), which hides more of
-// the staging loads' latency than 48 registers at 1280 threads.
-template <typename T, int CPT>
-__host__ __device__ constexpr int cells_min_blocks(int bs) {
-    return sizeof(T) == 4 && CPT < 4 ? 1536 / bs : 1;
+// Threads resident per SM that the FP32 kernels are built for (P2G: 1280 at 48
+// registers; 5.08M particles of honeycombs, 138 us, against 140 us for 1536 at
+// 40 registers with spills and 176 us for 1024).  Before the moments P2G took
+// 154 us there, 39.1 us (now 33.7) on a solid block of 1.07M particles; FP64
+// form, a solid block of 286k particles: 233 us before, 115 now.
+template <typename T, int BS, bool FE>
+__global__ void __launch_bounds__(BS, sizeof(T) == 4 ? 1280 / BS : 1) k_p2g_cells(
+    PView<T> P, NView<T> nd, Geom g, const unsigned* __restrict__ skeys, const unsigned* __restrict__ perm, long long n,
+    int mark_active) {
+    p2g_cells_run<T, BS, FE, false>(P, nd, g, skeys, perm, n, mark_active);
 }
 
-template <typename T, int CPT, int BS>
-__global__ void __launch_bounds__(BS, cells_min_blocks<T, CPT>(BS)) k_p2g_cells(PView<T> P, NView<T> nd, Geom g, const unsigned* __restrict__ skeys,
-                                                   const unsigned* __restrict__ perm, long long n, int mark_active) {
-    p2g_cells_run<T, CPT, BS, false>(P, nd, g, skeys, perm, n, mark_active);
-}
-
-template <typename T, int CPT, int BS>
-__global__ void __launch_bounds__(BS) k_p2g_cells_mg(PView<T> P, NView<T> nd, Geom g,
+template <int BS>
+__global__ void __launch_bounds__(BS) k_p2g_cells_mg(PView<float> P, NView<float> nd, Geom g,
                                                       const unsigned* __restrict__ skeys,
                                                       const unsigned* __restrict__ perm, long long n, int mark_active) {
-    p2g_cells_run<T, CPT, BS, true>(P, nd, g, skeys, perm, n, mark_active);
+    p2g_cells_run<float, BS, true, true>(P, nd, g, skeys, perm, n, mark_active);
 }
 
 // ---------------------------------------------------------------------------
@@ -843,51 +832,54 @@ __global__ void __launch_bounds__(256) k_pass1_remap(PView<T> P, NView<T> nd, Ge
 }
 
 // ---------------------------------------------------------------------------
-// G2P pass 1 + velocity remap, cell-centric (used with P2G mode 2): each slot's
-// thread updates its particle's velocity from the node records (in corner
-// order, as k_pass1_remap) and stages N (per axis) and m v in shared memory;
-// one thread per (cell run, corner) then sums N m v over the run in slot order
-// and issues three atomics.  Skipped particles (platen on the contact path)
-// stay in their run with zero weight.
+// G2P pass 1 + velocity remap, cell-centric (used with P2G modes 2 to 4): each
+// slot's thread updates its particle's velocity from the node records and
+// stages N (per axis) and m v in shared memory; one thread per (cell run, CPT
+// corners) then sums N m v over the run in slot order and issues one vector
+// (FP64: three) atomics per corner.  Skipped particles (platen on the contact
+// path) stay in their run with zero weight.
+// Both forms work on the (x, y) pairs of corners: A = Nx Ny once, then N = A Nz
+// (FP64: 96 operations per particle on the pipe that bounds it, from 190
+// corner by corner with the records' thresholds tested; a record's r is zero
+// where m <= mass_min).  A solid block of 286k particles in the FP64 form:
+// 107 us before, 77 now.
 // ---------------------------------------------------------------------------
+// The slots' corner nodes, staged beside the keys: the first node, and the
+// strides and mask of the cell.
 template <typename T>
 __host__ __device__ constexpr size_t pass1_cells_smem(int bs) {
-    return (sizeof(T) == 4 ? (size_t)9 * bs * 4 : ((size_t)6 * (bs + 1) + (size_t)3 * bs) * sizeof(T)) +
-           (size_t)bs * CELL_SLOT_BYTES + (size_t)(bs + 1) * 4 + 64 * 4;
+    return (size_t)(sizeof(T) == 4 ? 9 : 10) * bs * sizeof(T) + (size_t)bs * sizeof(CellNodes) + cell_slots_bytes(bs);
 }
 
 // FP32 with 1 or 2 corners per thread: registers capped for 1536 resident
-// threads per SM (40 registers, a few bytes spilled), about 10% faster than
-// 56 registers at 1152 threads: the kernel waits on its record gathers, and
-// more resident warps keep more of them in flight.
+// threads per SM (40 registers), about 10% faster than 56 registers at 1152
+// threads: the kernel waits on its record gathers, and more resident warps
+// keep more of them in flight.
 template <typename T, int CPT, int BS>
-__global__ void __launch_bounds__(BS, cells_min_blocks<T, CPT>(BS)) k_pass1_cells(PView<T> P, NView<T> nd, Geom g,
+__global__ void __launch_bounds__(BS, sizeof(T) == 4 && CPT < 4 ? 1536 / BS : 1) k_pass1_cells(PView<T> P, NView<T> nd, Geom g,
                                                      const unsigned* __restrict__ skeys,
-                                                     const unsigned* __restrict__ perm, long long n, T dt,
-                                                     T mass_min, int contact) {
+                                                     const unsigned* __restrict__ perm, long long n, T dt, int contact) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int bs = BS;
     const int t = threadIdx.x;
-    // FP64: 6 rows of S = bs + 1 (odd stride: the two nodes' values of an axis
-    // in different banks) Nx0 Nx1 Ny0 Ny1 Nz0 Nz1, then 3 rows of bs m v.
+    // FP64: rows of bs pairs {Nx0 Nx1} {Ny0 Ny1} {Nz0 Nz1} {mv0 mv1} {mv2 0}.
     // FP32: two rows of bs float4 {Nx0 Nx1 Ny0 Ny1} {Nz0 Nz1 mv0 mv1} and a row of mv2.
-    constexpr int S = bs + 1;
     constexpr bool F32 = sizeof(T) == 4;
-    T* sn = reinterpret_cast<T*>(smem_raw);
-    T* smv = sn + (F32 ? 8 * bs : 6 * S);
-    CellSlots cs(reinterpret_cast<unsigned char*>(smv + (F32 ? bs : 3 * bs)), bs);
+    static_assert(BS % 8 == 0, "slot swizzle groups");
+    CellNodes* scn = reinterpret_cast<CellNodes*>(smem_raw);
+    T* sn = reinterpret_cast<T*>(scn + bs);
+    CellSlots cs(reinterpret_cast<unsigned char*>(sn + (F32 ? 9 : 10) * bs), bs);
     unsigned* skey = cs.key;
     const long long s = blockIdx.x * (long long)bs + t;
     const unsigned key = (s < n) ? skeys[s] : 0xffffffffu;
-    const bool key_ok = key < g.key_max;
-    const long long np = P.n, nn = nd.nn;
-    if (key_ok) {
+    const long long np = P.n;
+    if (key < g.key_max) {
         const long long p = perm ? perm[s] : s;
         const Geom& gs = spec_geom(g, P.sid, p);
         int b[3];
         key_to_base(key, gs, b);
         const CellNodes cn = cell_nodes(gs, b);
-        cs.put(t, cn);
+        scn[t] = cn;
         const bool valid = !(contact && (P.pflags[p] & 8u));
         T N6[6] = {0, 0, 0, 0, 0, 0}, mv[3] = {0, 0, 0};
         if (valid) {
@@ -895,6 +887,7 @@ __global__ void __launch_bounds__(BS, cells_min_blocks<T, CPT>(BS)) k_pass1_cell
             particle_bases<T>(P, gs, p, b, B);
             const T m = P.mass[p];
             T v[3] = {P.vel[p], P.vel[np + p], P.vel[2 * np + p]};
+            T dv[3] = {0, 0, 0};
             // four corners' records requested before any is used; summed in corner order
 #pragma unroll(F32 ? 2 : 1)
             for (int h = 0; h < 2; ++h) {
@@ -903,20 +896,20 @@ __global__ void __launch_bounds__(BS, cells_min_blocks<T, CPT>(BS)) k_pass1_cell
                 for (int j = 0; j < 4; ++j) {
                     const int k = 4 * h + j;
                     const Quad<T> z{(T)0, (T)0, (T)0, (T)0};
-                    rq[j] = ((cn.mask >> k) & 1u) ? ld_quad(nd.rec + 8 * cell_node(cn, k)) : z;
+                    rq[j] = ((cn.mask >> k) & 1u) ? ld_quad(nd.rec + 8ll * cell_node(cn, k)) : z;
                 }
+                const T nx = h ? B.Nx[1] : B.Nx[0];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    if (!(rq[j].w != (T)0)) continue;
-                    T N, G[3];
-                    B.corner(4 * h + j, N, G);
-                    v[0] = v[0] + N * rq[j].x * dt;
-                    v[1] = v[1] + N * rq[j].y * dt;
-                    v[2] = v[2] + N * rq[j].z * dt;
+                    const T N = nx * ((j & 2) ? B.Ny[1] : B.Ny[0]) * ((j & 1) ? B.Nz[1] : B.Nz[0]);
+                    dv[0] += N * rq[j].x;
+                    dv[1] += N * rq[j].y;
+                    dv[2] += N * rq[j].z;
                 }
             }
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
+                v[c] += dv[c] * dt;
                 P.vel[c * np + p] = v[c];
                 mv[c] = m * v[c];
             }
@@ -927,18 +920,19 @@ __global__ void __launch_bounds__(BS, cells_min_blocks<T, CPT>(BS)) k_pass1_cell
             N6[4] = B.Nz[0];
             N6[5] = B.Nz[1];
         }
+        const int u = slot_swz(t);
         if constexpr (F32) {
-            static_assert(BS % 8 == 0, "slot swizzle groups");
             float4* sv = reinterpret_cast<float4*>(sn);
-            const int u = slot_swz(t);
             sv[u] = make_float4(N6[0], N6[1], N6[2], N6[3]);
             sv[bs + u] = make_float4(N6[4], N6[5], mv[0], mv[1]);
-            smv[u] = mv[2];
+            sn[8 * bs + u] = mv[2];
         } else {
-#pragma unroll
-            for (int c = 0; c < 6; ++c) sn[c * S + t] = N6[c];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) smv[c * bs + t] = mv[c];
+            double2* sv = reinterpret_cast<double2*>(sn);
+            sv[u] = make_double2(N6[0], N6[1]);
+            sv[bs + u] = make_double2(N6[2], N6[3]);
+            sv[2 * bs + u] = make_double2(N6[4], N6[5]);
+            sv[3 * bs + u] = make_double2(mv[0], mv[1]);
+            sv[4 * bs + u] = make_double2(mv[2], 0.0);
         }
     }
     skey[t] = key;
@@ -953,36 +947,34 @@ __global__ void __launch_bounds__(BS, cells_min_blocks<T, CPT>(BS)) k_pass1_cell
 #pragma unroll
         for (int j = 0; j < CPT; ++j) q0[j] = q1[j] = q2[j] = 0;
         for (int i = a; i < e; ++i) {
-            T mv0, mv1, mv2;
-            float4 A, B;
+            const int u = slot_swz(i);
+            T mv0, mv1, mv2, X[2], Y[2], Z[2];
             if constexpr (F32) {
                 const float4* sv = reinterpret_cast<const float4*>(sn);
-                const int u = slot_swz(i);
-                A = sv[u];
-                B = sv[bs + u];
-                mv0 = B.z, mv1 = B.w, mv2 = smv[u];
+                const float4 A = sv[u], B = sv[bs + u];
+                X[0] = A.x, X[1] = A.y, Y[0] = A.z, Y[1] = A.w, Z[0] = B.x, Z[1] = B.y;
+                mv0 = B.z, mv1 = B.w, mv2 = sn[8 * bs + u];
             } else {
-                mv0 = smv[i], mv1 = smv[bs + i], mv2 = smv[2 * bs + i];
+                const double2* sv = reinterpret_cast<const double2*>(sn);
+                const double2 A = sv[u], B = sv[bs + u], C = sv[2 * bs + u], D = sv[3 * bs + u];
+                X[0] = A.x, X[1] = A.y, Y[0] = B.x, Y[1] = B.y, Z[0] = C.x, Z[1] = C.y;
+                mv0 = D.x, mv1 = D.y, mv2 = sv[4 * bs + u].x;
             }
+            const T nx = (k0 & 4) ? X[1] : X[0];
 #pragma unroll
             for (int j = 0; j < CPT; ++j) {
                 const int k = k0 + j;
-                const int ix = (k >> 2) & 1, iy = (k >> 1) & 1, iz = k & 1;
-                T N;
-                if constexpr (F32)
-                    N = (ix ? A.y : A.x) * (iy ? A.w : A.z) * (iz ? B.y : B.x);
-                else
-                    N = sn[ix * S + i] * sn[(2 + iy) * S + i] * sn[(4 + iz) * S + i];
+                const T N = nx * ((k & 2) ? Y[1] : Y[0]) * ((k & 1) ? Z[1] : Z[0]);
                 q0[j] += N * mv0;
                 q1[j] += N * mv1;
                 q2[j] += N * mv2;
             }
         }
+        const CellNodes cn = scn[a];
 #pragma unroll
         for (int j = 0; j < CPT; ++j) {
-            const long long nid = cs.node(a, k0 + j);
-            if (nid < 0) continue;
-            q_add<T>(nd.q, nid, q0[j], q1[j], q2[j]);
+            const int k = k0 + j;
+            if ((cn.mask >> k) & 1u) q_add<T>(nd.q, cell_node(cn, k), q0[j], q1[j], q2[j]);
         }
     }
 }
@@ -1631,7 +1623,7 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
                     const Quad<T> z{(T)0, (T)0, (T)0, (T)0};
                     rq[j] = z;
                     vq[j] = z;
-                    if ((cn.mask >> (2 * h + j)) & 1u) ld_record(nd.rec + 8 * cell_node(cn, 2 * h + j), rq[j], vq[j]);
+                    if ((cn.mask >> (2 * h + j)) & 1u) ld_record(nd.rec + 8ll * cell_node(cn, 2 * h + j), rq[j], vq[j]);
                 }
                 const bool ix = (h >> 1) & 1, iy = h & 1;
                 const T nx = ix ? B.Nx[1] : B.Nx[0], ny = iy ? B.Ny[1] : B.Ny[0];

@@ -12,38 +12,21 @@ namespace mpm {
 // [0,1]; the gradient factor is sign(d)/h when 1e-12 < |d/h| < 1 - 1e-12,
 // else 0.  Here d/h is formed as d * (1/h): within a few ulp of the
 // reference, which the parity tolerance covers.
+//
+// FP64 form: the comparisons and the sign are taken on the bit patterns
+// (non-negative doubles order as their bits), which leaves six operations per
+// axis on the FP64 pipe, whose rate bounds that form's kernels, instead of 26.
 // ---------------------------------------------------------------------------
-template <typename T>
-__device__ __forceinline__ void axis_bases(const Geom& g, int a, double x, int b, T N[2], T gf[2]) {
+__device__ __forceinline__ void axis_bases(const Geom& g, int a, double x, int b, double N[2], double gf[2]) {
+    const unsigned long long lo = fps_d2u(1.0e-12), hi = fps_d2u(1.0 - 1.0e-12);
 #pragma unroll
     for (int o = 0; o < 2; ++o) {
-        double d = x - node_coord(g, a, b + o);
-        T r = (T)(d * g.inv_h[a]);
-        T ar = r >= (T)0 ? r : -r;
-        T nv = (T)1 - ar;
-        if (nv < (T)0 || nv > (T)1) nv = (T)0;
-        N[o] = nv;
-        T s = (T)((d > 0.0) - (d < 0.0));
-        gf[o] = (ar > (T)1.0e-12 && ar < (T)(1.0 - 1.0e-12)) ? s * (T)g.inv_h[a] : (T)0;
-    }
-}
-
-// FP32 (chosen) form: one FP64 subtraction and product per axis give the
-// cell-local coordinate u = (x - X_b)/h in [0, 1); both nodes' bases follow
-// in FP32 (d/h = u and u - 1).  FP64 instructions cost ~60 FP32 ones on this
-// part, so the chosen form keeps them to this one pair per axis.
-__device__ __forceinline__ void axis_bases_local(const Geom& g, int a, double x, int b, float N[2], float gf[2]) {
-    const float u = (float)((x - node_coord(g, a, b)) * g.inv_h[a]);
-    const float r[2] = {u, u - 1.0f};
-    const float ih = (float)g.inv_h[a];
-#pragma unroll
-    for (int o = 0; o < 2; ++o) {
-        float ar = fabsf(r[o]);
-        float nv = 1.0f - ar;
-        if (nv < 0.0f || nv > 1.0f) nv = 0.0f;
-        N[o] = nv;
-        float s = (float)((r[o] > 0.0f) - (r[o] < 0.0f));
-        gf[o] = (ar > 1.0e-12f && ar < (float)(1.0 - 1.0e-12)) ? s * ih : 0.0f;
+        const double d = x - node_coord(g, a, b + o);
+        const unsigned long long ar = fps_d2u(d * g.inv_h[a]) & 0x7fffffffffffffffull;  // |d/h|
+        const double nv = 1.0 - fps_u2d(ar);
+        N[o] = (long long)fps_d2u(nv) < 0 ? 0.0 : nv;
+        const unsigned long long s = (fps_d2u(d) & 0x8000000000000000ull) ^ fps_d2u(g.inv_h[a]);
+        gf[o] = (ar > lo && ar < hi) ? fps_u2d(s) : 0.0;
     }
 }
 
@@ -65,15 +48,9 @@ struct Bases {
     T Nx[2], Ny[2], Nz[2];
     T gx[2], gy[2], gz[2];
     __device__ __forceinline__ void init(const Geom& g, const double x[3], const int b[3]) {
-        if constexpr (sizeof(T) == 4) {
-            axis_bases_local(g, 0, x[0], b[0], Nx, gx);
-            axis_bases_local(g, 1, x[1], b[1], Ny, gy);
-            axis_bases_local(g, 2, x[2], b[2], Nz, gz);
-        } else {
-            axis_bases<T>(g, 0, x[0], b[0], Nx, gx);
-            axis_bases<T>(g, 1, x[1], b[1], Ny, gy);
-            axis_bases<T>(g, 2, x[2], b[2], Nz, gz);
-        }
+        axis_bases(g, 0, x[0], b[0], Nx, gx);
+        axis_bases(g, 1, x[1], b[1], Ny, gy);
+        axis_bases(g, 2, x[2], b[2], Nz, gz);
     }
     // FP32 form: bases from the cell-local coordinate stored by the previous step
     __device__ __forceinline__ void init_local(const Geom& g, const float u[3]) {

@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(BS) k_pass1_pairs(PView<float> P, NView<float>
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
                 const Quad<float> z{0.0f, 0.0f, 0.0f, 0.0f};
-                rq[k] = ((cn.mask >> k) & 1u) ? ld_quad(nd.rec + 8 * cell_node(cn, k)) : z;
+                rq[k] = ((cn.mask >> k) & 1u) ? ld_quad(nd.rec + 8ll * cell_node(cn, k)) : z;
             }
             for (int j = a + par; j < e; j += 2) {
                 const long long p = perm ? (long long)perm[s0 + j] : s0 + j;

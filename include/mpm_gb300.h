@@ -70,16 +70,16 @@ extern "C" {
 /* Options for mpm_set_option. */
 #define MPM_OPT_FLOOR_FRICTION 1 /* contact path: Coulomb friction on x/y of z-fixed nodes (extension; default 0) */
 #define MPM_OPT_PROFILE 2        /* 1: time every kernel with CUDA events (default 0) */
-#define MPM_OPT_P2G_REDUCE 3     /* P2G: 0 = one atomic per particle, 1 = sum each cell's run across lanes first, 2 = stage the block in shared memory and sum each (cell, corner) in one thread, 3 (default) / 4 = as 2 with each thread summing 2 / 4 corners of a cell */
-#define MPM_OPT_P2G_BLOCK 4      /* P2G threads per block (128, 256 or 512) */
-#define MPM_OPT_PASS_BLOCK 5     /* G2P pass-2 threads per block (128, 256 (default) or 512) */
+#define MPM_OPT_P2G_REDUCE 3     /* P2G: 0 = one atomic per particle, 1 = sum each cell's run across lanes first, 2, 3 (default), 4 = stage the block in shared memory and sum each cell's run in four threads (one kernel; the three values differ in nothing any more), 5 / 6 (FP32 form) = sum the runs in registers by lane pairs, with the tile read from global memory / staged by bulk copies */
+#define MPM_OPT_P2G_BLOCK 4      /* P2G threads per block: 128 (default), 256 or 512; by default the FP64 form takes 64 or 32 where the particles are few */
+#define MPM_OPT_PASS_BLOCK 5     /* G2P pass-2 threads per block: 128 (default), 256 or 512; by default the FP64 form takes 64 or 32 where the particles are few */
 #define MPM_OPT_GATHER 6         /* pass-2 (G2P) mode: 0 = node gathers one (x, y) pair of corners at a time, 1 = several
                                     pairs' loads issued together, 2 = (FP32 form) as 0 with the block's particle fields
                                     brought into shared memory by bulk copies first */
 #define MPM_OPT_GRAPH 7          /* 1 (default): mpm_advance replays a captured two-step CUDA graph in the steady state; 0: launch every kernel */
 #define MPM_OPT_REORDER 8        /* FP32 form: store particles in cell order after each particle upload (0, default), also every N steps (N > 0), or never (-1); results stay in the caller's order */
 #define MPM_OPT_PASS1_CORNERS 10 /* cell-run G2P pass 1 (P2G modes 2-4): corners per thread, 1, 2 (default) or 4 */
-#define MPM_OPT_PASS1_BLOCK 11   /* cell-run G2P pass 1: threads per block (128, 256 or 512) */
+#define MPM_OPT_PASS1_BLOCK 11   /* cell-run G2P pass 1: threads per block, as MPM_OPT_P2G_BLOCK */
 #define MPM_OPT_LARGE_STRAIN 12  /* FP64 form, non-contact loop: 1 runs the large-strain pass 2 (G2P_P2_LargeStrain, PhysicsEngine_runSimulation_Classic_DoublePass_MPLocks.cpp:281-437), which the reference ships disabled (:605); 0 (default) the small-strain pass */
 #define MPM_OPT_FP64_FALLBACK 13 /* FP32 form: 1 (default) computes the von Mises hardening return map
                                     (…_VonMisesHardening.cpp:4-92) as FP64 gives it, rounded to float (in pairs of
