@@ -139,13 +139,14 @@ struct mpm_ctx {
     float* hv_rows = nullptr;
     long long hv_cap = 0;
     DevBuf hv_count;
-    // particles stored in cell order (FP32 form): orig[slot] = the caller's index
+    // particles stored in cell order: orig[slot] = the caller's index
     DevBuf orig, ptmp;
     bool have_orig = false, reorder_pending = false;
     int reorder_interval = 0;  // -1: never; 0: after each particle upload; N: also every N steps
-    bool cell_sort = false;    // FP32 form, P2G modes 2-4: false = take the storage order as the cell order
+    bool cell_sort = false;    // P2G modes 2-6: false = take the storage order as the cell order
     bool large_strain = false; // FP64 form, non-contact loop: the large-strain pass 2
     long long steps_since_reorder = 0;
+    long long steps_asked = 0;  // steps asked of mpm_advance since the last particle upload
     bool owner_clean = false;  // displacement-control claims all zero (phase B clears them after use)
 
     mpm_ctx() {
@@ -744,7 +745,7 @@ int sort_cells(mpm_ctx* c, const unsigned** skeys_out, const unsigned** perm_out
 
 void graph_reset(mpm_ctx* c);
 
-// Store the particles in cell order (FP32 form).  After a sort every
+// Store the particles in cell order.  After a sort every
 // particle array is permuted into sorted order and `orig` keeps each slot's
 // index as the caller numbers it; the displacement-control list is remapped
 // and the surface list rebuilt.  Later sorts find the particles nearly in
@@ -755,30 +756,33 @@ int reorder(mpm_ctx* c) {
     c->reorder_pending = false;
     c->steps_since_reorder = 0;
     const long long n = c->n;
-    if (n <= 0 || c->form != MPM_FORM_FP32) return MPM_OK;
+    if (n <= 0) return MPM_OK;
     graph_reset(c);
     const unsigned *skeys = nullptr, *perm = nullptr;
-    int rc = sort_cells(c, &skeys, &perm);
-    if (rc) return rc;
-    if ((rc = ensure(c, c->orig, (size_t)n * 4)) || (rc = ensure(c, c->ptmp, (size_t)n * 36))) return rc;
+    int rc;
+    if ((rc = ensure(c, c->orig, (size_t)n * 4)) || (rc = ensure(c, c->ptmp, (size_t)n * 9 * c->tsize))) return rc;
+    if ((rc = sort_cells(c, &skeys, &perm))) return rc;
     if (!c->have_orig) {
         LAUNCH("reorder", k_iota, blocks_for(n), NTHREADS, (unsigned*)c->orig.p, n);
         c->have_orig = true;
     }
+    const int t = (int)c->tsize;
     struct {
         DevBuf* b;
         int k, es;
-    } fields[] = {{&c->pos, 3, 8},        {&c->vel, 3, 4},       {&c->fext, 3, 4},         {&c->mass, 1, 4},
-                  {&c->vol, 1, 4},        {&c->vol0, 1, 4},      {&c->F, 9, 4},            {&c->stress, 6, 4},
-                  {&c->strain, 6, 4},     {&c->eps_p, 6, 4},     {&c->e_strain, 1, 8},     {&c->e_strain_max, 1, 8},
-                  {&c->e_strain_ti, 1, 8}, {&c->e_plastic, 1, 8}, {&c->backstress, 1, 4},   {&c->mp_mg, 3, 4},
-                  {&c->strain_rate, 6, 4}, {&c->material, 1, 4}, {&c->pflags, 1, 1},       {&c->dc_mult, 1, 4},
-                  {&c->loc, 3, 4},        {&c->keys_copy, 1, 4}, {&c->orig, 1, 4},         {&c->sid, 1, 2},
-                  {&c->mon_mask, 1, 1}};
+    } fields[] = {{&c->pos, 3, 8},         {&c->vel, 3, t},       {&c->fext, 3, t},       {&c->mass, 1, t},
+                  {&c->vol, 1, t},         {&c->vol0, 1, t},      {&c->F, 9, t},          {&c->stress, 6, t},
+                  {&c->strain, 6, t},      {&c->eps_p, 6, t},     {&c->e_strain, 1, 8},   {&c->e_strain_max, 1, 8},
+                  {&c->e_strain_ti, 1, 8}, {&c->e_plastic, 1, 8}, {&c->backstress, 1, t}, {&c->mp_mg, 3, t},
+                  {&c->strain_rate, 6, t}, {&c->material, 1, 4},  {&c->pflags, 1, 1},     {&c->dc_mult, 1, 4},
+                  {&c->loc, 3, 4},         {&c->Fe, 9, 8},        {&c->keys_copy, 1, 4},  {&c->orig, 1, 4},
+                  {&c->sid, 1, 2},         {&c->mon_mask, 1, 1}};
     const unsigned grid = (unsigned)std::min<long long>(blocks_for(n * 3), (long long)c->sm_count * 32);
     for (auto& f : fields) {
         if (f.b == &c->sid && c->nspec <= 1) continue;
         if (f.b == &c->mon_mask && !c->have_mon) continue;
+        if (f.b == &c->loc && c->form != MPM_FORM_FP32) continue;
+        if (f.b == &c->Fe && c->form != MPM_FORM_FP64) continue;
         void* src = f.b->p;
         switch (f.es) {
             case 8: LAUNCH("reorder", k_permute<8>, grid, NTHREADS, src, c->ptmp.p, perm, n, f.k); break;
@@ -886,30 +890,29 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
         c->grid_dirty = false;
     }
     if (n > 0) {
-        // The FP32 form's cell-run kernels accept slots out of cell order (a
-        // cell met twice is summed in two runs), so with particles stored in
-        // cell order it can skip the sort and take the storage order as it is.
-        const bool sort = !(c->form == MPM_FORM_FP32 && !c->cell_sort && c->p2g_reduce >= 2);
+        const int fp32 = c->form == MPM_FORM_FP32 ? 1 : 0;
+        const bool detecting = contact && output;
+        // The cell-run kernels accept slots out of cell order (a cell met twice
+        // is summed in two runs), so with particles stored in cell order a step
+        // can skip the sort and take the storage order as it is.  The FP64
+        // form sorts until its particles are stored in cell order, and on the
+        // steps that detect contact, whose exact gather needs cell ranges.
+        const bool sort = c->cell_sort || c->p2g_reduce < 2 || (!fp32 && (!c->have_orig || detecting));
         const unsigned *skeys = nullptr, *perm = nullptr;
         if (int rs = sort_cells(c, &skeys, &perm, sort)) return rs;
         // pass 2 writes the next step's sort input into the buffer not holding skeys
         unsigned* keys_next = (skeys == (unsigned*)c->keys0.p) ? (unsigned*)c->keys1.p : (unsigned*)c->keys0.p;
         c->key_buf = (keys_next == (unsigned*)c->keys1.p) ? 1 : 0;
         const unsigned* keys = (const unsigned*)c->keys_copy.p;
-        // FP32 form: the contact mass gradient is accumulated by P2G itself
-        // and P2G marks the active nodes; the FP64 form marks them here and
-        // records the per-cell ranges its bit-exact ordered gather reads.
-        const int fp32 = c->form == MPM_FORM_FP32 ? 1 : 0;
-        const bool detecting = contact && output;
+        // P2G marks the active nodes.  FP32 form: the contact mass gradient is
+        // accumulated by P2G itself; the FP64 form records the per-cell ranges
+        // its bit-exact ordered gather reads.
         const int mg_in_p2g = (detecting && fp32) ? 1 : 0;
-        if (!fp32) {
-            if (detecting) {
-                CK(cudaMemsetAsync(c->cstart.p, 0, (size_t)g.key_max * 4, c->stream));
-                CK(cudaMemsetAsync(c->cend.p, 0, (size_t)g.key_max * 4, c->stream));
-            }
-            LAUNCH("cell_ranges", k_cell_ranges, blocks_for(n), NTHREADS, skeys, n, g, N.state,
-                   detecting ? (unsigned*)c->cstart.p : nullptr, detecting ? (unsigned*)c->cend.p : nullptr, perm,
-                   P.sid);
+        if (detecting && !fp32) {
+            CK(cudaMemsetAsync(c->cstart.p, 0, (size_t)g.key_max * 4, c->stream));
+            CK(cudaMemsetAsync(c->cend.p, 0, (size_t)g.key_max * 4, c->stream));
+            LAUNCH("cell_ranges", k_cell_ranges, blocks_for(n), NTHREADS, skeys, n, g, (unsigned*)c->cstart.p,
+                   (unsigned*)c->cend.p);
         }
         bool pairs_done = false;
         if constexpr (sizeof(T) == 4) {
@@ -918,7 +921,7 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
                 const unsigned pg = (unsigned)((n + 4LL * bs - 1) / (4LL * bs));
                 const bool st = c->p2g_reduce == 6;
 #define PAIRS(B, MGV, STV)                                                                                       \
-    LAUNCH_SMEM("p2g", (k_p2g_pairs<B, MGV, STV>), pg, B, p2g_pairs_smem<B>(STV), P, N, g, skeys, perm, n, 1, err)
+    LAUNCH_SMEM("p2g", (k_p2g_pairs<B, MGV, STV>), pg, B, p2g_pairs_smem<B>(STV), P, N, g, skeys, perm, n, err)
 #define PAIRS_BS(B)                            \
     do {                                       \
         if (mg_in_p2g) {                       \
@@ -945,29 +948,26 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
                 if (mg_in_p2g) {
                     const size_t sm = p2g_cells_smem<float>(bp, true);
                     if (bp == 128)
-                        LAUNCH_SMEM("p2g", k_p2g_cells_mg<128>, blocks_for(n, bp), bp, sm, P, N, g, skeys, perm, n,
-                                    fp32);
+                        LAUNCH_SMEM("p2g", k_p2g_cells_mg<128>, blocks_for(n, bp), bp, sm, P, N, g, skeys, perm, n);
                     else if (bp == 256)
-                        LAUNCH_SMEM("p2g", k_p2g_cells_mg<256>, blocks_for(n, bp), bp, sm, P, N, g, skeys, perm, n,
-                                    fp32);
+                        LAUNCH_SMEM("p2g", k_p2g_cells_mg<256>, blocks_for(n, bp), bp, sm, P, N, g, skeys, perm, n);
                     else
-                        LAUNCH_SMEM("p2g", k_p2g_cells_mg<512>, blocks_for(n, bp), bp, sm, P, N, g, skeys, perm, n,
-                                    fp32);
+                        LAUNCH_SMEM("p2g", k_p2g_cells_mg<512>, blocks_for(n, bp), bp, sm, P, N, g, skeys, perm, n);
                     mg_done = true;
                 }
             }
             const size_t sm = p2g_cells_smem<T>(bp);
             if (!mg_done && c->have_fext)
-                LAUNCH_BS("p2g", k_p2g_cells, T, true, bp, blocks_for(n, bp), sm, P, N, g, skeys, perm, n, fp32);
+                LAUNCH_BS("p2g", k_p2g_cells, T, true, bp, blocks_for(n, bp), sm, P, N, g, skeys, perm, n);
             else if (!mg_done)
-                LAUNCH_BS("p2g", k_p2g_cells, T, false, bp, blocks_for(n, bp), sm, P, N, g, skeys, perm, n, fp32);
+                LAUNCH_BS("p2g", k_p2g_cells, T, false, bp, blocks_for(n, bp), sm, P, N, g, skeys, perm, n);
         }
         else if (c->p2g_reduce == 1)
             LAUNCH("p2g", (k_p2g<T, 1>), blocks_for(n, bp), bp, P, N, g, skeys, perm, n,
-                   mg_in_p2g, fp32);
+                   mg_in_p2g);
         else
             LAUNCH("p2g", (k_p2g<T, 0>), blocks_for(n, bp), bp, P, N, g, skeys, perm, n,
-                   mg_in_p2g, fp32);
+                   mg_in_p2g);
         CK(cudaMemsetAsync(c->acount.p, 0, 4, c->stream));
         LAUNCH("active_list", k_compact_state, (unsigned)((nn + CS_THREADS * CS_ROUNDS - 1) / (CS_THREADS * CS_ROUNDS)),
                CS_THREADS, (const unsigned*)N.state, nn, 1u, (unsigned*)c->alist.p, (unsigned*)c->acount.p);
@@ -1161,12 +1161,20 @@ int step(mpm_ctx* c, double dt, int contact, bool graph = false, bool output = t
 // graph.  Capturing records two steps without running them while the host
 // state advances by two steps; launching the graph once then brings the
 // device to the same point.
-// Steps between periodic reorders (FP32 form; 0: none).  Without the
+// Steps between periodic reorders (0: none).  Without the
 // per-step sort the storage order is the only cell order, so it is restored
 // every SORT_FREE_REORDER steps unless the caller chose an interval.
 constexpr int SORT_FREE_REORDER = 256;
+// The FP64 form stores its particles in cell order once this many steps have
+// been asked for since the upload: a reorder costs about as much as the sorts
+// of this many steps, and a caller that uploads for every few steps is served
+// by the sort.  With the per-step sort (62 us of a 123 us step) the
+// 40,000-particle bar took 123 us per step, without it 82; 1,043 particles 99
+// and 85, 286k particles 475 and 434, 406k particles 703 and 653.
+constexpr long long FP64_REORDER_STEPS = 8;
 int reorder_every(const mpm_ctx* c) {
-    if (c->form != MPM_FORM_FP32 || c->reorder_interval < 0) return 0;
+    if (c->reorder_interval < 0) return 0;
+    if (c->form == MPM_FORM_FP64 && !c->have_orig) return 0;  // not yet stored in cell order
     if (c->reorder_interval > 0) return c->reorder_interval;
     return (!c->cell_sort && c->p2g_reduce >= 2) ? SORT_FREE_REORDER : 0;
 }
@@ -1174,9 +1182,12 @@ int reorder_every(const mpm_ctx* c) {
 int advance_graph(mpm_ctx* c, int nsteps, double dt, int contact, bool between_reorders = false,
                   bool output_last = true) {
     if (!between_reorders) {
-        if (c->reorder_pending && c->have_particles) {
+        c->steps_asked += nsteps;
+        if (c->reorder_pending && c->have_particles &&
+            (c->form == MPM_FORM_FP32 || c->steps_asked >= FP64_REORDER_STEPS)) {
             int rc = reorder(c);
-            if (rc) return rc;
+            // no room to store the FP64 form's particles in cell order: it goes on sorting every step
+            if (rc && !(rc == MPM_ERR_NOMEM && c->form == MPM_FORM_FP64)) return rc;
         }
         const int every = reorder_every(c);
         if (every > 0) {  // periodic: advance in runs between reorders
@@ -1738,7 +1749,8 @@ int mpm_upload_particles(mpm_ctx* c, const mpm_particles* p, int64_t n) {
     c->have_particles = true;
     c->keys_valid = false;
     c->have_orig = false;  // the upload is in the caller's order
-    c->reorder_pending = c->form == MPM_FORM_FP32 && c->reorder_interval >= 0;
+    c->reorder_pending = c->reorder_interval >= 0;
+    c->steps_asked = 0;
     c->last_perm = c->last_skeys = nullptr;
     return MPM_OK;
 }
@@ -2111,7 +2123,7 @@ int mpm_autotune(mpm_ctx* c, int32_t steps, double dt, int contact, mpm_tune_res
     if (!c->have_particles) return fail(c, MPM_ERR_STATE, "no particles uploaded");
     if (c->reorder_pending) {  // the trials time the storage order the run will have
         int r0 = reorder(c);
-        if (r0) return r0;
+        if (r0 && !(r0 == MPM_ERR_NOMEM && c->form == MPM_FORM_FP64)) return r0;
     }
     const long long since0 = c->steps_since_reorder;
     // everything a step writes that outlives the step

@@ -4,9 +4,10 @@
 // maps onto:
 //   k_reset_grid        ResetGrid (:4-22)
 //   k_cell_keys         FindAGPs cell lookup, floor(x/h) (GridPoint_Mediator.cpp:8)
-//   radix sort          particles ordered by cell key
-//   k_cell_ranges       active-node marking (b_Active, :36) + per-cell particle ranges
-//   k_p2g               M2G (:48-89): warp-segmented reduction, then one atomic per run
+//   radix sort          particles ordered by cell key (on reorders, and where a step needs sorted cells)
+//   k_cell_ranges       per-cell particle ranges (FP64 form, steps that detect contact)
+//   k_p2g_cells         M2G (:48-89): each cell run's moments, then one atomic per corner and field;
+//                       active-node marking (b_Active, :36)
 //   k_dc_claim          DisplacementControl (:143-174), last writer in list order
 //   k_node_phase_a      displacement control, IntegrateGrid (:90-142; contact :242-277),
 //                       f/m per node (the divisor of G2P pass 1)
@@ -98,28 +99,17 @@ static __global__ void k_cell_keys(const double* __restrict__ pos, long long n, 
 }
 
 // ---------------------------------------------------------------------------
-// Active nodes (the union of the in-range corners of every occupied cell) and
-// per-cell [start, end) ranges in sorted order.
+// Per-cell [start, end) ranges in sorted order (for the FP64 form's exact
+// contact gather, on output steps).
 // ---------------------------------------------------------------------------
-static __global__ void k_cell_ranges(const unsigned* __restrict__ skeys, long long n, Geom g, unsigned* __restrict__ state,
-                              unsigned* __restrict__ cstart, unsigned* __restrict__ cend,
-                              const unsigned* __restrict__ perm, const uint16_t* __restrict__ sid) {
+static __global__ void k_cell_ranges(const unsigned* __restrict__ skeys, long long n, Geom g,
+                                     unsigned* __restrict__ cstart, unsigned* __restrict__ cend) {
     long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (s >= n) return;
     unsigned key = skeys[s];
     if (key >= g.key_max) return;
-    if (s == 0 || skeys[s - 1] != key) {
-        if (cstart) cstart[key] = (unsigned)s;
-        const Geom& gs = (g.nspec > 1) ? g.tab[sid[perm[s]]] : g;
-        int b[3];
-        key_to_base(key, gs, b);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            long long nid = corner_node(gs, b, k);
-            if (nid >= 0) atomicOr(&state[nid], 1u);
-        }
-    }
-    if (cend && (s == n - 1 || skeys[s + 1] != key)) cend[key] = (unsigned)(s + 1);
+    if (s == 0 || skeys[s - 1] != key) cstart[key] = (unsigned)s;
+    if (s == n - 1 || skeys[s + 1] != key) cend[key] = (unsigned)(s + 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -191,8 +181,7 @@ __device__ __forceinline__ void prefetch_l2(const void* base, int es, long long 
 // ---------------------------------------------------------------------------
 template <typename T, int REDUCE>
 __global__ void __launch_bounds__(512) k_p2g(PView<T> P, NView<T> nd, Geom g, const unsigned* __restrict__ skeys,
-                                             const unsigned* __restrict__ perm, long long n, int with_mg,
-                                             int mark_active) {
+                                             const unsigned* __restrict__ perm, long long n, int with_mg) {
     long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     unsigned key = (s < n) ? skeys[s] : 0xffffffffu;
     const bool valid = key < g.key_max;
@@ -246,7 +235,7 @@ __global__ void __launch_bounds__(512) k_p2g(PView<T> P, NView<T> nd, Geom g, co
         if (valid && (!REDUCE || run.tail)) {
             long long nid = corner_node(*gsp, b, k);
             if (nid >= 0) {
-                if (mark_active) atomicOr(&nd.state[nid], 1u);  // a reduction: no load to wait for
+                atomicOr(&nd.state[nid], 1u);  // a reduction: no load to wait for
                 acc_add<T>(nd.acc, nid, c[0], c[1], c[2], c[3], c[4], c[5], c[6]);
                 if (nf == 10) {
                     atomicAdd(&nd.mg[nid], c[7]);
@@ -433,7 +422,7 @@ struct P2GBlock {
 
     // After the staging and a __syncthreads (keys in cs.key for the first nslots
     // slots, out of range where nothing was staged): the runs' sums and their
-    // atomics; mark_active also marks the corners active.  MG: also the node
+    // atomics, which also mark the corners active.  MG: also the node
     // mass gradients.  sid: the slots' specimens from the block's first slot on
     // (perm: through the sort order), for the runs' geometry.
     //
@@ -444,8 +433,7 @@ struct P2GBlock {
     // honeycomb batch about three runs in four have such a neighbour, so a
     // third of the corner atomics go).
     __device__ __forceinline__ void scatter(const NView<T>& nd, const Geom& g, const uint16_t* __restrict__ sid,
-                                            const unsigned* __restrict__ perm, long long s0, int nslots,
-                                            int mark_active) const {
+                                            const unsigned* __restrict__ perm, long long s0, int nslots) const {
         const int t = threadIdx.x, lane = t & 31;
         const long long nn = nd.nn;
         const unsigned* skey = cs.key;
@@ -555,7 +543,7 @@ struct P2GBlock {
                 const T* c = iz ? c1 : c0;
                 const T* f = iz ? p1 : p0;
                 // active nodes: the in-range corners of occupied cells (b_Active, …MPLocks.cpp:36)
-                if (mark_active) atomicOr(&nd.state[nid], 1u);  // a reduction: no load to wait for
+                atomicOr(&nd.state[nid], 1u);  // a reduction: no load to wait for
                 acc_add<T>(nd.acc, nid, c[0], c[1], c[2], c[3], f[0], f[1], f[2]);
                 if constexpr (MG) {
                     const T* gm = iz ? g1 : g0;
@@ -573,7 +561,7 @@ struct P2GBlock {
 template <typename T, int BS, bool FE, bool MG>
 __device__ __forceinline__ void p2g_cells_run(const PView<T>& P, const NView<T>& nd, const Geom& g,
                                               const unsigned* __restrict__ skeys, const unsigned* __restrict__ perm,
-                                              long long n, int mark_active) {
+                                              long long n) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const P2GBlock<T, BS, FE, MG> blk(smem_raw);
     const int t = threadIdx.x;
@@ -600,7 +588,7 @@ __device__ __forceinline__ void p2g_cells_run(const PView<T>& P, const NView<T>&
     }
     blk.cs.key[t] = key;
     __syncthreads();
-    blk.scatter(nd, g, P.sid, perm, s0, (int)min((long long)BS, n - s0), mark_active);
+    blk.scatter(nd, g, P.sid, perm, s0, (int)min((long long)BS, n - s0));
 }
 
 // Threads resident per SM that the FP32 kernels are built for (P2G: 1280 at 48
@@ -610,16 +598,15 @@ __device__ __forceinline__ void p2g_cells_run(const PView<T>& P, const NView<T>&
 // form, a solid block of 286k particles: 233 us before, 115 now.
 template <typename T, int BS, bool FE>
 __global__ void __launch_bounds__(BS, sizeof(T) == 4 ? 1280 / BS : 1) k_p2g_cells(
-    PView<T> P, NView<T> nd, Geom g, const unsigned* __restrict__ skeys, const unsigned* __restrict__ perm, long long n,
-    int mark_active) {
-    p2g_cells_run<T, BS, FE, false>(P, nd, g, skeys, perm, n, mark_active);
+    PView<T> P, NView<T> nd, Geom g, const unsigned* __restrict__ skeys, const unsigned* __restrict__ perm, long long n) {
+    p2g_cells_run<T, BS, FE, false>(P, nd, g, skeys, perm, n);
 }
 
 template <int BS>
 __global__ void __launch_bounds__(BS) k_p2g_cells_mg(PView<float> P, NView<float> nd, Geom g,
                                                       const unsigned* __restrict__ skeys,
-                                                      const unsigned* __restrict__ perm, long long n, int mark_active) {
-    p2g_cells_run<float, BS, true, true>(P, nd, g, skeys, perm, n, mark_active);
+                                                      const unsigned* __restrict__ perm, long long n) {
+    p2g_cells_run<float, BS, true, true>(P, nd, g, skeys, perm, n);
 }
 
 // ---------------------------------------------------------------------------
@@ -1910,42 +1897,48 @@ static __global__ void k_contact_compact(const unsigned* __restrict__ need, long
     if (take) list[base + __popc(m & ((1u << lane) - 1u))] = (unsigned)i;
 }
 
-// One warp per needed node: gather the particle ids of the eight surrounding
-// cells into shared memory, rank them by id, compute each pair's exact
-// grad N * m in parallel, then add them in id order on one lane.  Nodes with
-// more than CG_CAP contributors take the one-lane merge below.
+// One warp per needed node: gather the slots of the eight surrounding cells'
+// particles into shared memory, rank them by the caller's particle index (the
+// slot itself when particles are not stored in cell order), compute each
+// pair's exact grad N * m in parallel, then add them in index order on one
+// lane.  Nodes with more than CG_CAP contributors take the selection below:
+// the warp looks for the next larger index among all of them, one at a time.
 constexpr int CG_WARPS = 4;
 constexpr int CG_CAP = 256;
 
 template <typename T>
-__device__ __noinline__ void mass_gradient_merge(const PView<T>& P, const Geom& g, const int node[3],
-                                                 const unsigned* __restrict__ perm, const unsigned cs[8],
-                                                 const unsigned ce[8], double gsum[3]) {
+__device__ __forceinline__ unsigned caller_index(const PView<T>& P, unsigned slot) {
+    return P.orig ? P.orig[slot] : slot;
+}
+
+template <typename T>
+__device__ __noinline__ void mass_gradient_select(const PView<T>& P, const Geom& g, const int node[3],
+                                                  const unsigned* __restrict__ perm, const unsigned seg[8],
+                                                  const unsigned off[8], unsigned total, double gsum[3]) {
     const long long np = P.n;
-    unsigned cur[8], end[8];
-    for (int k = 0; k < 8; ++k) {
-        cur[k] = cs[k];
-        end[k] = ce[k];
-    }
+    const int lane = threadIdx.x & 31;
     gsum[0] = gsum[1] = gsum[2] = 0.0;
-    while (true) {
-        int best = -1;
-        unsigned bp = 0xffffffffu;
-        for (int c = 0; c < 8; ++c) {
-            if (cur[c] < end[c]) {
-                unsigned pp = perm[cur[c]];
-                if (pp < bp) {
-                    bp = pp;
-                    best = c;
-                }
+    long long last = -1;
+    for (unsigned done = 0; done < total; ++done) {
+        unsigned best = 0xffffffffu, slot = 0;
+        for (unsigned e = lane; e < total; e += 32) {
+            int k = 0;
+            for (int kk = 1; kk < 8; ++kk)
+                if (e >= off[kk]) k = kk;
+            const unsigned sl = perm[seg[k] + (e - off[k])], id = caller_index(P, sl);
+            if ((long long)id > last && id < best) {
+                best = id;
+                slot = sl;
             }
         }
-        if (best < 0) break;
-        cur[best]++;
-        double x[3] = {P.pos[bp], P.pos[np + bp], P.pos[2 * np + bp]};
+        const unsigned next = __reduce_min_sync(FULL_MASK, best);
+        const unsigned from = __ballot_sync(FULL_MASK, best == next);
+        slot = __shfl_sync(FULL_MASK, slot, __ffs(from) - 1);
+        last = next;
+        const double x[3] = {P.pos[slot], P.pos[np + slot], P.pos[2 * np + slot]};
         double G[3];
         exact_gradient(g, x, node, G);
-        double m = (double)P.mass[bp];
+        const double m = (double)P.mass[slot];
         for (int c = 0; c < 3; ++c) gsum[c] = __dadd_rn(gsum[c], __dmul_rn(G[c], m));
     }
 }
@@ -1957,7 +1950,7 @@ __global__ void __launch_bounds__(CG_WARPS * 32) k_contact_mass_gradient(PView<T
                                                                          const unsigned* __restrict__ perm,
                                                                          const unsigned* __restrict__ cstart,
                                                                          const unsigned* __restrict__ cend) {
-    __shared__ unsigned s_id[CG_WARPS][CG_CAP];
+    __shared__ unsigned s_id[CG_WARPS][CG_CAP];  // the caller's index
     __shared__ double s_c[CG_WARPS][CG_CAP][3];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long np = P.n, nn = nd.nn;
@@ -1996,27 +1989,25 @@ __global__ void __launch_bounds__(CG_WARPS * 32) k_contact_mass_gradient(PView<T
         }
         double gsum[3] = {0.0, 0.0, 0.0};
         if (total > (unsigned)CG_CAP) {
-            if (lane == 0) {
-                unsigned cs[8], ce[8];
-                for (int k = 0; k < 8; ++k) {
-                    cs[k] = segs[k];
-                    ce[k] = segs[k] + ((k < 7 ? offs[k + 1] : total) - offs[k]);
-                }
-                mass_gradient_merge<T>(P, gs, node, perm, cs, ce, gsum);
-            }
+            mass_gradient_select<T>(P, gs, node, perm, segs, offs, total, gsum);
         } else {
             for (unsigned e = lane; e < total; e += 32) {
                 int k = 0;
 #pragma unroll
                 for (int kk = 1; kk < 8; ++kk)
                     if (e >= offs[kk]) k = kk;
-                s_id[w][e] = perm[segs[k] + (e - offs[k])];
+                s_id[w][e] = caller_index(P, perm[segs[k] + (e - offs[k])]);
             }
             __syncwarp();
             for (unsigned e = lane; e < total; e += 32) {
-                const unsigned id = s_id[w][e];
+                const unsigned key = s_id[w][e];
+                int k = 0;
+#pragma unroll
+                for (int kk = 1; kk < 8; ++kk)
+                    if (e >= offs[kk]) k = kk;
+                const unsigned id = perm[segs[k] + (e - offs[k])];
                 unsigned rank = 0;
-                for (unsigned j = 0; j < total; ++j) rank += s_id[w][j] < id ? 1u : 0u;
+                for (unsigned j = 0; j < total; ++j) rank += s_id[w][j] < key ? 1u : 0u;
                 double x[3] = {P.pos[id], P.pos[np + id], P.pos[2 * np + id]};
                 double G[3];
                 exact_gradient(gs, x, node, G);

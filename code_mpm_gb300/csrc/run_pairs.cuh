@@ -221,7 +221,7 @@ __device__ __forceinline__ void pair_exchange(float v[8], int par) {
 template <int BS, bool MG, bool STAGE>
 __global__ void __launch_bounds__(BS) k_p2g_pairs(PView<float> P, NView<float> nd, Geom g,
                                                    const unsigned* __restrict__ skeys,
-                                                   const unsigned* __restrict__ perm, long long n, int mark_active,
+                                                   const unsigned* __restrict__ perm, long long n,
                                                    unsigned* err) {
     constexpr int TS = PAIR_TILE_PER_THREAD * BS;
     using S = PairStage<TS>;
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(BS) k_p2g_pairs(PView<float> P, NView<float> n
             if (!((cn.mask >> k) & 1u)) continue;
             const long long nid = cell_node(cn, k);
             // active nodes: the in-range corners of occupied cells (b_Active, …MPLocks.cpp:36)
-            if (mark_active) atomicOr(&nd.state[nid], 1u);
+            atomicOr(&nd.state[nid], 1u);
             acc_add<float>(nd.acc, nid, am[j], ap0[j], ap1[j], ap2[j], af0[j], af1[j], af2[j]);
             if constexpr (MG) {
                 atomicAdd(&nd.mg[nid], g0[j]);

@@ -77,7 +77,7 @@ extern "C" {
                                     pairs' loads issued together, 2 = (FP32 form) as 0 with the block's particle fields
                                     brought into shared memory by bulk copies first */
 #define MPM_OPT_GRAPH 7          /* 1 (default): mpm_advance replays a captured two-step CUDA graph in the steady state; 0: launch every kernel */
-#define MPM_OPT_REORDER 8        /* FP32 form: store particles in cell order after each particle upload (0, default), also every N steps (N > 0), or never (-1); results stay in the caller's order */
+#define MPM_OPT_REORDER 8        /* store particles in cell order after each particle upload (0, default; FP64 form: once 8 steps have been asked for), also every N steps (N > 0), or never (-1); results stay in the caller's order */
 #define MPM_OPT_PASS1_CORNERS 10 /* cell-run G2P pass 1 (P2G modes 2-4): corners per thread, 1, 2 (default) or 4 */
 #define MPM_OPT_PASS1_BLOCK 11   /* cell-run G2P pass 1: threads per block, as MPM_OPT_P2G_BLOCK */
 #define MPM_OPT_LARGE_STRAIN 12  /* FP64 form, non-contact loop: 1 runs the large-strain pass 2 (G2P_P2_LargeStrain, PhysicsEngine_runSimulation_Classic_DoublePass_MPLocks.cpp:281-437), which the reference ships disabled (:605); 0 (default) the small-strain pass */
@@ -91,7 +91,7 @@ extern "C" {
 #define MPM_OPT_SURROGATE_GUARD 14 /* FP32 form with the learned return map: tolerance of the guard on the network's
                                       results as a fraction of k0 (default 0.001; 0 turns the guard off), see
                                       mpm_attach_surrogate */
-#define MPM_OPT_CELL_SORT 9      /* FP32 form, P2G modes 2-4: 1 sorts the particles by cell every step; 0 (default) takes the storage order as it is (a cell whose particles are not adjacent is summed in several runs) and, with MPM_OPT_REORDER 0, restores the cell order every 256 steps */
+#define MPM_OPT_CELL_SORT 9      /* P2G modes 2-6: 1 sorts the particles by cell every step; 0 (default) takes the storage order as it is (a cell whose particles are not adjacent is summed in several runs) and, with MPM_OPT_REORDER 0, restores the cell order every 256 steps (FP64 form: particles not stored in cell order, and steps that detect contact, are sorted all the same) */
 
 typedef struct mpm_ctx mpm_ctx;
 
