@@ -131,7 +131,9 @@ struct mpm_ctx {
     int g_contact[2] = {-1, -1};
     long long g_launches[2] = {0, 0};
     DevBuf dsim, tl_dev;
-    double* h_sim = nullptr;  // pinned: time, dt, step (as double bits), tv[3]
+    double* h_sim = nullptr;  // pinned DevSim
+    cudaStream_t clock_stream = nullptr;  // the clock kernels' branch of a capture
+    cudaEvent_t clock_ev[2] = {nullptr, nullptr};
     // harvesting of return-map inputs
     int hv_on = 0;
     unsigned hv_mats = 0;
@@ -240,7 +242,7 @@ NView<T> nview(mpm_ctx* c) {
     v.owner = (unsigned*)c->g_owner.p;
     v.nowner = (unsigned*)c->g_nowner.p;
     v.alist = c->use_alist ? (const unsigned*)c->alist.p : nullptr;
-    v.acount = (const unsigned*)c->acount.p;
+    v.acount = (unsigned*)c->acount.p;
     v.nn = c->nn;
     return v;
 }
@@ -318,16 +320,38 @@ int prof_resolve(mpm_ctx* c) {
         kernel<<<(grid), (block), (smem), c->stream>>>(__VA_ARGS__);       \
     } while (0)
 
+// A step kernel (one that begins with step_enter): may be placed while the
+// kernel before it drains.
+template <typename... Ex, typename... Act>
+void launch_step(mpm_ctx* c, void (*kernel)(Ex...), unsigned grid, unsigned block, size_t smem, Act&&... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c->stream;
+    cfg.attrs = at;
+    cfg.numAttrs = c->profile ? 0 : 1;  // per-kernel times: one after the other
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<Act>(args)...);
+}
+#define LAUNCH_STEP(name, kernel, grid, block, smem, ...)                \
+    do {                                                                 \
+        Launch l_(c, name);                                              \
+        launch_step(c, kernel, (grid), (block), (smem), __VA_ARGS__);    \
+    } while (0)
+
 // A kernel template <T, block size, FE> launched for the runtime block size: 128,
 // 256 or 512 threads, and in the FP64 form also 32 and 64 (auto_block).
 #define LAUNCH_BS(name, K, T, FE, bs, grid, smem, ...)                                  \
     do {                                                                                \
-        if ((bs) == 128) LAUNCH_SMEM(name, (K<T, 128, FE>), grid, 128, smem, __VA_ARGS__);  \
-        else if ((bs) == 256) LAUNCH_SMEM(name, (K<T, 256, FE>), grid, 256, smem, __VA_ARGS__); \
-        else if ((bs) == 512) LAUNCH_SMEM(name, (K<T, 512, FE>), grid, 512, smem, __VA_ARGS__); \
+        if ((bs) == 128) LAUNCH_STEP(name, (K<T, 128, FE>), grid, 128, smem, __VA_ARGS__);  \
+        else if ((bs) == 256) LAUNCH_STEP(name, (K<T, 256, FE>), grid, 256, smem, __VA_ARGS__); \
+        else if ((bs) == 512) LAUNCH_STEP(name, (K<T, 512, FE>), grid, 512, smem, __VA_ARGS__); \
         else if constexpr (sizeof(T) == 8) {                                            \
-            if ((bs) == 64) LAUNCH_SMEM(name, (K<T, 64, FE>), grid, 64, smem, __VA_ARGS__); \
-            else LAUNCH_SMEM(name, (K<T, 32, FE>), grid, 32, smem, __VA_ARGS__);            \
+            if ((bs) == 64) LAUNCH_STEP(name, (K<T, 64, FE>), grid, 64, smem, __VA_ARGS__); \
+            else LAUNCH_STEP(name, (K<T, 32, FE>), grid, 32, smem, __VA_ARGS__);            \
         }                                                                               \
     } while (0)
 template <typename T, int BS>
@@ -453,52 +477,6 @@ __global__ void k_compact_flag(const uint8_t* __restrict__ pflags, long long n, 
     if (lane == leader) base = atomicAdd(count, (unsigned)__popc(m));
     base = __shfl_sync(m, base, leader);
     if (take) list[base + __popc(m & ((1u << lane) - 1u))] = (unsigned)i;
-}
-// Active-node list: a block of CS_THREADS compacts a tile of CS_THREADS x
-// CS_ROUNDS consecutive nodes in node order and reserves its range with one
-// atomic (a counter shared by every warp would serialise tens of thousands of
-// atomics at one L2 address).  Each warp takes 32 x CS_ROUNDS consecutive
-// nodes, loads all its state words before counting (the loads overlap), and
-// writes its entries after the warps before it.
-constexpr int CS_THREADS = 256, CS_ROUNDS = 16;
-__global__ void __launch_bounds__(CS_THREADS) k_compact_state(const unsigned* __restrict__ state, long long n,
-                                                              unsigned bit, unsigned* __restrict__ list,
-                                                              unsigned* __restrict__ count) {
-    __shared__ unsigned woff[CS_THREADS / 32];
-    __shared__ unsigned base;
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const long long wbase = blockIdx.x * (long long)(CS_THREADS * CS_ROUNDS) + (long long)w * 32 * CS_ROUNDS;
-    unsigned v[CS_ROUNDS], m[CS_ROUNDS];
-#pragma unroll
-    for (int r = 0; r < CS_ROUNDS; ++r) {
-        const long long i = wbase + (long long)r * 32 + lane;
-        v[r] = i < n ? state[i] : 0u;
-    }
-    unsigned cnt = 0;
-#pragma unroll
-    for (int r = 0; r < CS_ROUNDS; ++r) {
-        m[r] = __ballot_sync(FULL_MASK, (v[r] & bit) != 0u);
-        cnt += __popc(m[r]);
-    }
-    if (lane == 0) woff[w] = cnt;
-    __syncthreads();
-    if (t == 0) {
-        unsigned total = 0;
-        for (int k = 0; k < CS_THREADS / 32; ++k) {
-            const unsigned c = woff[k];
-            woff[k] = total;
-            total += c;
-        }
-        base = total ? atomicAdd(count, total) : 0u;
-    }
-    __syncthreads();
-    unsigned off = base + woff[w];
-    const unsigned below = (1u << lane) - 1u;
-#pragma unroll
-    for (int r = 0; r < CS_ROUNDS; ++r) {
-        if (v[r] & bit) list[off + __popc(m[r] & below)] = (unsigned)(wbase + (long long)r * 32 + lane);
-        off += __popc(m[r]);
-    }
 }
 // Specimen ids of an upload (int32 from the caller) to the 16-bit device
 // array; the smallest index of an id outside [0, nspec) goes to *bad.
@@ -810,16 +788,22 @@ int reorder(mpm_ctx* c) {
     return MPM_OK;
 }
 
-// Device copy of the clock for graph replay: time, dt, step and the
-// timeline velocity at the step's start, computed with the host's exact
+// Device clock of the replayed two-step graph, computed with the host's exact
 // operations (timeline_velocity), so device and host clocks stay identical.
+// A replay takes the timeline velocities and step numbers of its two steps
+// from `ahead`, which the host fills for the first replay and each replay for
+// the one after it: the clock kernels run beside the steps, not between them.
 struct DevSim {
-    double time, dt;
+    double time, dt;            // the time of the next step to look ahead to
     unsigned long long step;
-    double tv[3];
+    struct Steps {
+        double tv[2][3];
+        unsigned long long step[2];
+    } now, ahead;
 };
 
-__global__ void k_step_begin(DevSim* d, const double* __restrict__ tl_t, const double* __restrict__ tl_v, int nt) {
+// look ahead: the timeline velocity at the clock's time, for step j of the next replay
+__global__ void k_step_begin(DevSim* d, const double* __restrict__ tl_t, const double* __restrict__ tl_v, int nt, int j) {
     const double t = d->time;
     double out[3] = {0.0, 0.0, 0.0};
     for (int k = 0; k + 1 < nt; ++k) {
@@ -829,12 +813,83 @@ __global__ void k_step_begin(DevSim* d, const double* __restrict__ tl_t, const d
                 out[a] = __dadd_rn(__dmul_rn(__dsub_rn(1.0, s), tl_v[3 * k + a]), __dmul_rn(s, tl_v[3 * (k + 1) + a]));
         }
     }
-    for (int a = 0; a < 3; ++a) d->tv[a] = out[a];
+    for (int a = 0; a < 3; ++a) d->ahead.tv[j][a] = out[a];
+    d->ahead.step[j] = d->step;
 }
 
 __global__ void k_step_end(DevSim* d) {
     d->time = __dadd_rn(d->time, d->dt);
     d->step += 1;
+}
+
+// What a step needs between P2G and the node phases, in one launch (two
+// kernels and the counter's memset before, each a launch's latency on a small
+// scene):
+//  * blocks [0, ncompact): the active-node list.  A block compacts a tile of
+//    CS_THREADS x CS_ROUNDS consecutive nodes in node order and reserves its
+//    range with one atomic (a counter shared by every warp would serialise tens
+//    of thousands of atomics at one L2 address).  Each warp takes 32 x
+//    CS_ROUNDS consecutive nodes, loads all its state words before counting
+//    (the loads overlap), and writes its entries after the warps before it;
+//  * the blocks after them: the displacement-control claims, one particle of
+//    the list per thread (they set another bit of the state words);
+//  * the first step of a replay takes over its clock (clock given).
+constexpr int CS_THREADS = 256, CS_ROUNDS = 16;
+struct ClaimArgs {
+    const unsigned* dclist;
+    int ndc;
+    const unsigned* keys;
+    const uint8_t* pflags;
+    unsigned* owner;
+    int contact;
+    const uint16_t* sid;
+};
+template <bool EARLY>
+__global__ void __launch_bounds__(CS_THREADS) k_step_lists(unsigned* state, long long n, unsigned ncompact,
+                                                           unsigned* __restrict__ list, unsigned* count, ClaimArgs dc,
+                                                           Geom g, DevSim* clock) {
+    __shared__ unsigned woff[CS_THREADS / 32];
+    __shared__ unsigned base;
+    step_enter<EARLY>();
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    if (clock && blockIdx.x == gridDim.x - 1 && t == 0) clock->now = clock->ahead;
+    if (blockIdx.x >= ncompact) {
+        const int k = (int)(blockIdx.x - ncompact) * CS_THREADS + t;
+        if (k < dc.ndc) dc_claim(k, dc.dclist, dc.keys, dc.pflags, g, dc.owner, n, dc.contact, dc.sid, state);
+        return;
+    }
+    const long long wbase = blockIdx.x * (long long)(CS_THREADS * CS_ROUNDS) + (long long)w * 32 * CS_ROUNDS;
+    unsigned v[CS_ROUNDS], m[CS_ROUNDS];
+#pragma unroll
+    for (int r = 0; r < CS_ROUNDS; ++r) {
+        const long long i = wbase + (long long)r * 32 + lane;
+        v[r] = i < n ? state[i] & 1u : 0u;
+    }
+    unsigned cnt = 0;
+#pragma unroll
+    for (int r = 0; r < CS_ROUNDS; ++r) {
+        m[r] = __ballot_sync(FULL_MASK, v[r] != 0u);
+        cnt += __popc(m[r]);
+    }
+    if (lane == 0) woff[w] = cnt;
+    __syncthreads();
+    if (t == 0) {
+        unsigned total = 0;
+        for (int k = 0; k < CS_THREADS / 32; ++k) {
+            const unsigned c = woff[k];
+            woff[k] = total;
+            total += c;
+        }
+        base = total ? atomicAdd(count, total) : 0u;
+    }
+    __syncthreads();
+    unsigned off = base + woff[w];
+    const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+    for (int r = 0; r < CS_ROUNDS; ++r) {
+        if (v[r]) list[off + __popc(m[r] & below)] = (unsigned)(wbase + (long long)r * 32 + lane);
+        off += __popc(m[r]);
+    }
 }
 
 void graph_reset(mpm_ctx* c) {
@@ -861,6 +916,7 @@ int auto_block(const mpm_ctx* c, int chosen) {
     return b;
 }
 
+// graph: 0, or which of the two captured steps this is (1, 2).
 // output: the step is an output step, the last of an advance, whose results
 // the caller can see.  Only an output step runs the contact path's contact
 // detection (node mass gradients, particle and node normals, node contact
@@ -871,7 +927,7 @@ int auto_block(const mpm_ctx* c, int chosen) {
 // node values: the others zero their active nodes once the records are formed
 // (pass 2 reads only the records), so the next step needs no grid reset.
 template <typename T>
-int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
+int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
     const long long n = c->n, nn = c->nn;
     PView<T> P = pview<T>(c);
     NView<T> N = nview<T>(c);
@@ -879,14 +935,13 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
     unsigned* err = (unsigned*)c->err_word.p;
 
     DevSim* dsim = (DevSim*)c->dsim.p;
-    if (graph) LAUNCH("step_clock", k_step_begin, 1, 1, dsim, (const double*)c->tl_dev.p, (const double*)c->tl_dev.p + c->tl_t.size(), (int)c->tl_t.size());
     // node kernels sweep the active-node list; the reset uses the previous step's
     const unsigned nodeblocks = (unsigned)std::min<long long>(blocks_for(nn), (long long)c->sm_count * 16);
     N.alist = c->have_alist ? (const unsigned*)c->alist.p : nullptr;
     // after an upload the reset clears the uploaded active nodes only
     const int vel_zero = c->have_alist ? 1 : 0;
     if (c->grid_dirty) {  // after a step that left its node values (or an upload); clean steps zero their own
-        LAUNCH("reset_grid", k_reset_grid<T>, c->have_alist ? nodeblocks : blocks_for(nn), NTHREADS, N, contact);
+        LAUNCH_STEP("reset_grid", k_reset_grid<T>, c->have_alist ? nodeblocks : blocks_for(nn), NTHREADS, 0, N, contact);
         c->grid_dirty = false;
     }
     if (n > 0) {
@@ -921,7 +976,7 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
                 const unsigned pg = (unsigned)((n + 4LL * bs - 1) / (4LL * bs));
                 const bool st = c->p2g_reduce == 6;
 #define PAIRS(B, MGV, STV)                                                                                       \
-    LAUNCH_SMEM("p2g", (k_p2g_pairs<B, MGV, STV>), pg, B, p2g_pairs_smem<B>(STV), P, N, g, skeys, perm, n, err)
+    LAUNCH_STEP("p2g", (k_p2g_pairs<B, MGV, STV>), pg, B, p2g_pairs_smem<B>(STV), P, N, g, skeys, perm, n, err)
 #define PAIRS_BS(B)                            \
     do {                                       \
         if (mg_in_p2g) {                       \
@@ -948,11 +1003,11 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
                 if (mg_in_p2g) {
                     const size_t sm = p2g_cells_smem<float>(bp, true);
                     if (bp == 128)
-                        LAUNCH_SMEM("p2g", k_p2g_cells_mg<128>, blocks_for(n, bp), bp, sm, P, N, g, skeys, perm, n);
+                        LAUNCH_STEP("p2g", k_p2g_cells_mg<128>, blocks_for(n, bp), bp, sm, P, N, g, skeys, perm, n);
                     else if (bp == 256)
-                        LAUNCH_SMEM("p2g", k_p2g_cells_mg<256>, blocks_for(n, bp), bp, sm, P, N, g, skeys, perm, n);
+                        LAUNCH_STEP("p2g", k_p2g_cells_mg<256>, blocks_for(n, bp), bp, sm, P, N, g, skeys, perm, n);
                     else
-                        LAUNCH_SMEM("p2g", k_p2g_cells_mg<512>, blocks_for(n, bp), bp, sm, P, N, g, skeys, perm, n);
+                        LAUNCH_STEP("p2g", k_p2g_cells_mg<512>, blocks_for(n, bp), bp, sm, P, N, g, skeys, perm, n);
                     mg_done = true;
                 }
             }
@@ -963,22 +1018,35 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
                 LAUNCH_BS("p2g", k_p2g_cells, T, false, bp, blocks_for(n, bp), sm, P, N, g, skeys, perm, n);
         }
         else if (c->p2g_reduce == 1)
-            LAUNCH("p2g", (k_p2g<T, 1>), blocks_for(n, bp), bp, P, N, g, skeys, perm, n,
+            LAUNCH_STEP("p2g", (k_p2g<T, 1>), blocks_for(n, bp), bp, 0, P, N, g, skeys, perm, n,
                    mg_in_p2g);
         else
-            LAUNCH("p2g", (k_p2g<T, 0>), blocks_for(n, bp), bp, P, N, g, skeys, perm, n,
+            LAUNCH_STEP("p2g", (k_p2g<T, 0>), blocks_for(n, bp), bp, 0, P, N, g, skeys, perm, n,
                    mg_in_p2g);
-        CK(cudaMemsetAsync(c->acount.p, 0, 4, c->stream));
-        LAUNCH("active_list", k_compact_state, (unsigned)((nn + CS_THREADS * CS_ROUNDS - 1) / (CS_THREADS * CS_ROUNDS)),
-               CS_THREADS, (const unsigned*)N.state, nn, 1u, (unsigned*)c->alist.p, (unsigned*)c->acount.p);
-        N.alist = (const unsigned*)c->alist.p;
-        c->have_alist = true;
         if (c->ndc > 0) {
             if (!c->owner_clean) CK(cudaMemsetAsync(c->g_owner.p, 0, (size_t)3 * nn * 4, c->stream));
             c->owner_clean = false;  // claims in use until phase B clears them
-            LAUNCH("dc_claim", k_dc_claim, blocks_for(c->ndc), NTHREADS, (const unsigned*)c->dclist.p, c->ndc, keys,
-                   (const uint8_t*)c->pflags.p, g, (unsigned*)c->g_owner.p, nn, contact, P.sid, (unsigned*)N.state);
         }
+        const unsigned ncompact = (unsigned)((nn + CS_THREADS * CS_ROUNDS - 1) / (CS_THREADS * CS_ROUNDS));
+        const unsigned nclaim = (unsigned)((c->ndc + CS_THREADS - 1) / CS_THREADS);
+        const ClaimArgs dc{(const unsigned*)c->dclist.p, c->ndc, keys, (const uint8_t*)c->pflags.p,
+                           (unsigned*)c->g_owner.p, contact, P.sid};
+        LAUNCH_STEP("step_lists", k_step_lists<sizeof(T) == 4>, ncompact + nclaim, CS_THREADS, 0, N.state, nn,
+                    ncompact, (unsigned*)c->alist.p, N.acount, dc, g, graph == 1 ? dsim : (DevSim*)nullptr);
+        if (graph == 1) {  // the next replay's clock, on a branch beside the two steps
+            const double* tl = (const double*)c->tl_dev.p;
+            const int nt = (int)c->tl_t.size();
+            CK(cudaEventRecord(c->clock_ev[0], c->stream));
+            CK(cudaStreamWaitEvent(c->clock_stream, c->clock_ev[0], 0));
+            for (int j = 0; j < 2; ++j) {
+                c->launches += 2;
+                k_step_begin<<<1, 1, 0, c->clock_stream>>>(dsim, tl, tl + nt, nt, j);
+                k_step_end<<<1, 1, 0, c->clock_stream>>>(dsim);
+            }
+            CK(cudaEventRecord(c->clock_ev[1], c->clock_stream));
+        }
+        N.alist = (const unsigned*)c->alist.p;
+        c->have_alist = true;
         if (detecting) {
             const unsigned* surf = (const unsigned*)c->surf.p;
             const int ns = c->nsurf;
@@ -1007,7 +1075,7 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
         // the mass threshold in the form's type (FP32: rounded down, so float masses compare exactly)
         const T mm = sizeof(T) == 4 ? (T)fps_float_threshold(c->sim.mass_min) : (T)c->sim.mass_min;
         // displacement control, grid update, displacement control, f/m: one pass over the active nodes
-        LAUNCH("node_phase_a", k_node_phase_a<T>, nodeblocks, NTHREADS, N, (T)dt, c->sim.damping, contact,
+        LAUNCH_STEP("node_phase_a", k_node_phase_a<T>, nodeblocks, NTHREADS, 0, N, (T)dt, c->sim.damping, contact,
                c->floor_friction, (const unsigned*)c->dclist.p, c->ndc, (const T*)c->vel.p, n, mm, output ? 0 : 1,
                (double*)c->work_acc.p, dt);
         if (sizeof(T) == 4 && c->p2g_reduce >= 5) {  // the same runs as P2G, reduced by lane pairs
@@ -1015,37 +1083,37 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
                 const int b1 = auto_block(c, c->pass1_block);
                 const unsigned pg = (unsigned)((n + 4LL * b1 - 1) / (4LL * b1));
                 if (b1 == 128)
-                    LAUNCH("pass1_remap", k_pass1_pairs<128>, pg, 128, P, N, g, skeys, perm, n, (float)dt, contact);
+                    LAUNCH_STEP("pass1_remap", k_pass1_pairs<128>, pg, 128, 0, P, N, g, skeys, perm, n, (float)dt, contact);
                 else if (b1 == 256)
-                    LAUNCH("pass1_remap", k_pass1_pairs<256>, pg, 256, P, N, g, skeys, perm, n, (float)dt, contact);
+                    LAUNCH_STEP("pass1_remap", k_pass1_pairs<256>, pg, 256, 0, P, N, g, skeys, perm, n, (float)dt, contact);
                 else
-                    LAUNCH("pass1_remap", k_pass1_pairs<512>, pg, 512, P, N, g, skeys, perm, n, (float)dt, contact);
+                    LAUNCH_STEP("pass1_remap", k_pass1_pairs<512>, pg, 512, 0, P, N, g, skeys, perm, n, (float)dt, contact);
             }
         } else if (c->p2g_reduce >= 2) {  // the same reduction as P2G: shared-memory cell runs
             const int cpt = c->pass1_corners, b1 = std::max(auto_block(c, c->pass1_block), cpt == 2 ? 32 : 128);
             const unsigned gb = blocks_for(n, b1);
             const size_t sm = pass1_cells_smem<T>(b1);
             if (b1 == 128)
-                LAUNCH_SMEM("pass1_remap", (pass1_kernel<T, 128>(cpt)), gb, 128, sm, P, N, g, skeys, perm, n, (T)dt, contact);
+                LAUNCH_STEP("pass1_remap", (pass1_kernel<T, 128>(cpt)), gb, 128, sm, P, N, g, skeys, perm, n, (T)dt, contact);
             else if (b1 == 256)
-                LAUNCH_SMEM("pass1_remap", (pass1_kernel<T, 256>(cpt)), gb, 256, sm, P, N, g, skeys, perm, n, (T)dt, contact);
+                LAUNCH_STEP("pass1_remap", (pass1_kernel<T, 256>(cpt)), gb, 256, sm, P, N, g, skeys, perm, n, (T)dt, contact);
             else if (b1 == 512)
-                LAUNCH_SMEM("pass1_remap", (pass1_kernel<T, 512>(cpt)), gb, 512, sm, P, N, g, skeys, perm, n, (T)dt, contact);
+                LAUNCH_STEP("pass1_remap", (pass1_kernel<T, 512>(cpt)), gb, 512, sm, P, N, g, skeys, perm, n, (T)dt, contact);
             else if constexpr (sizeof(T) == 8) {
                 if (b1 == 64)
-                    LAUNCH_SMEM("pass1_remap", (k_pass1_cells<T, 2, 64>), gb, 64, sm, P, N, g, skeys, perm, n, (T)dt, contact);
+                    LAUNCH_STEP("pass1_remap", (k_pass1_cells<T, 2, 64>), gb, 64, sm, P, N, g, skeys, perm, n, (T)dt, contact);
                 else
-                    LAUNCH_SMEM("pass1_remap", (k_pass1_cells<T, 2, 32>), gb, 32, sm, P, N, g, skeys, perm, n, (T)dt, contact);
+                    LAUNCH_STEP("pass1_remap", (k_pass1_cells<T, 2, 32>), gb, 32, sm, P, N, g, skeys, perm, n, (T)dt, contact);
             }
         }
         else if (c->gather_batch)
-            LAUNCH("pass1_remap", (k_pass1_remap<T, 1>), blocks_for(n), NTHREADS, P, N, g, skeys, perm, n, (T)dt, mm,
+            LAUNCH_STEP("pass1_remap", (k_pass1_remap<T, 1>), blocks_for(n), NTHREADS, 0, P, N, g, skeys, perm, n, (T)dt, mm,
                    contact);
         else
-            LAUNCH("pass1_remap", (k_pass1_remap<T, 0>), blocks_for(n), NTHREADS, P, N, g, skeys, perm, n, (T)dt, mm,
+            LAUNCH_STEP("pass1_remap", (k_pass1_remap<T, 0>), blocks_for(n), NTHREADS, 0, P, N, g, skeys, perm, n, (T)dt, mm,
                    contact);
         // remap, displacement control and BC in the path's order, p/m and v: one pass
-        LAUNCH("node_phase_b", k_node_phase_b<T>, nodeblocks, NTHREADS, N, contact, (const unsigned*)c->dclist.p,
+        LAUNCH_STEP("node_phase_b", k_node_phase_b<T>, nodeblocks, NTHREADS, 0, N, contact, (const unsigned*)c->dclist.p,
                c->ndc, (const T*)c->vel.p, n, mm, output ? 0 : 1, vel_zero);
         if (output) c->grid_dirty = true;  // the last step of an advance keeps its node values for the caller
         if (c->ndc > 0) c->owner_clean = true;
@@ -1055,7 +1123,7 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
         a.dt_f = (float)dt;
         a.mass_min_f = fps_float_threshold(c->sim.mass_min);
         timeline_velocity(c, c->sim.time, a.tv);
-        a.tv_dev = graph ? dsim->tv : nullptr;
+        a.tv_dev = graph ? dsim->now.tv[graph - 1] : nullptr;
         a.has_timeline = c->tl_t.empty() ? 0 : 1;
         a.contact = contact;
         a.sg_on = 0;
@@ -1092,11 +1160,11 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
             const unsigned pb = blocks_for(n, b2);
             unsigned* kc = (unsigned*)c->keys_copy.p;
             const MatConst* mats = (const MatConst*)c->mats.p;
-#define PASS2(B, S) LAUNCH("pass2", (k_pass2<T, B, S>), pb, S, P, N, g, kc, keys_next, mats, c->nmat, a, err)
+#define PASS2(B, S) LAUNCH_STEP("pass2", (k_pass2<T, B, S>), pb, S, 0, P, N, g, kc, keys_next, mats, c->nmat, a, err)
             bool large = false;
             if constexpr (sizeof(T) == 8) {
                 if (c->large_strain && !contact) {  // non-contact loop only, as in the reference
-                    LAUNCH("pass2", k_pass2_ls<128>, blocks_for(n, 128), 128, P, N, g, kc, keys_next, mats, c->nmat,
+                    LAUNCH_STEP("pass2", k_pass2_ls<128>, blocks_for(n, 128), 128, 0, P, N, g, kc, keys_next, mats, c->nmat,
                            a, err);
                     large = true;
                 }
@@ -1105,13 +1173,13 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
             } else if (c->gather_batch == 2 && sizeof(T) == 4) {
                 if constexpr (sizeof(T) == 4) {
                     if (b2 == 128)
-                        LAUNCH_SMEM("pass2", k_pass2_staged<128>, pb, 128, Pass2Stage<128>::SMEM, P, N, g, kc,
+                        LAUNCH_STEP("pass2", k_pass2_staged<128>, pb, 128, Pass2Stage<128>::SMEM, P, N, g, kc,
                                     keys_next, mats, c->nmat, a, err);
                     else if (b2 == 256)
-                        LAUNCH_SMEM("pass2", k_pass2_staged<256>, pb, 256, Pass2Stage<256>::SMEM, P, N, g, kc,
+                        LAUNCH_STEP("pass2", k_pass2_staged<256>, pb, 256, Pass2Stage<256>::SMEM, P, N, g, kc,
                                     keys_next, mats, c->nmat, a, err);
                     else
-                        LAUNCH_SMEM("pass2", k_pass2_staged<512>, pb, 512, Pass2Stage<512>::SMEM, P, N, g, kc,
+                        LAUNCH_STEP("pass2", k_pass2_staged<512>, pb, 512, Pass2Stage<512>::SMEM, P, N, g, kc,
                                     keys_next, mats, c->nmat, a, err);
                 }
             } else if (b2 == 128) {
@@ -1135,13 +1203,12 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
                 if (rq) return rq;
                 LAUNCH("net_finish", k_sg_finish, (unsigned)c->sm_count * 8, 256, P, a.q, net_material(c->net),
                        contact, dt, 1.0 / (double)net_yield(c->net), c->sg_recheck, (unsigned long long)c->sim.step,
-                       graph ? &dsim->step : (const unsigned long long*)nullptr, a.sg_acc,
+                       graph ? &dsim->now.step[graph - 1] : (const unsigned long long*)nullptr, a.sg_acc,
                        net_guard(c->net, c->sg_guard));
             }
         }
         c->keys_valid = true;
     }
-    if (graph) LAUNCH("step_clock", k_step_end, 1, 1, dsim);
     c->steps_since_reorder += 1;
     CK(cudaGetLastError());
     // d_Time += dTimeIncrement; i_TimeCycle++ (…MPLocks.cpp:802-803)
@@ -1150,7 +1217,7 @@ int step_impl(mpm_ctx* c, double dt, int contact, bool graph, bool output) {
     return MPM_OK;
 }
 
-int step(mpm_ctx* c, double dt, int contact, bool graph = false, bool output = true) {
+int step(mpm_ctx* c, double dt, int contact, int graph = 0, bool output = true) {
     return c->form == MPM_FORM_FP64 ? step_impl<double>(c, dt, contact, graph, output)
                                     : step_impl<float>(c, dt, contact, graph, output);
 }
@@ -1203,7 +1270,7 @@ int advance_graph(mpm_ctx* c, int nsteps, double dt, int contact, bool between_r
         }
     }
     int s = 0;
-    auto one = [&]() -> int { return step(c, dt, contact, false, output_last && s == nsteps - 1); };
+    auto one = [&]() -> int { return step(c, dt, contact, 0, output_last && s == nsteps - 1); };
     // launches the remaining steps one by one, the last as the output step
     auto plain = [&]() -> int {
         for (; s < nsteps; ++s)
@@ -1227,17 +1294,38 @@ int advance_graph(mpm_ctx* c, int nsteps, double dt, int contact, bool between_r
         cudaGetLastError();
         return plain();
     }
+    if (!c->clock_stream && cudaStreamCreateWithFlags(&c->clock_stream, cudaStreamNonBlocking) != cudaSuccess) {
+        cudaGetLastError();
+        c->clock_stream = nullptr;
+        return plain();
+    }
+    for (auto& e : c->clock_ev)
+        if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            e = nullptr;
+            return plain();
+        }
     // the device clock from the host's
     CK(cudaStreamSynchronize(c->stream));
-    DevSim hs{c->sim.time, dt, (unsigned long long)c->sim.step, {0.0, 0.0, 0.0}};
+    DevSim hs{};
+    hs.time = c->sim.time;
+    hs.dt = dt;
+    hs.step = (unsigned long long)c->sim.step;
+    for (int j = 0; j < 2; ++j) {  // the first replay's two steps
+        timeline_velocity(c, hs.time, hs.ahead.tv[j]);
+        hs.ahead.step[j] = hs.step;
+        hs.time += dt;
+        hs.step += 1;
+    }
     memcpy(c->h_sim, &hs, sizeof(hs));
     CK(cudaMemcpyAsync(c->dsim.p, c->h_sim, sizeof(DevSim), cudaMemcpyHostToDevice, c->stream));
     if (!c->gexec[par]) {
         const long long l0 = c->launches;
         cudaGraph_t gr = nullptr;
         CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
-        int r1 = step(c, dt, contact, true, false);
-        int r2 = r1 ? r1 : step(c, dt, contact, true, false);
+        int r1 = step(c, dt, contact, 1, false);
+        int r2 = r1 ? r1 : step(c, dt, contact, 2, false);
+        if (!r2 && cudaStreamWaitEvent(c->stream, c->clock_ev[1], 0) != cudaSuccess) r2 = MPM_ERR_CUDA;
         cudaError_t ec = cudaStreamEndCapture(c->stream, &gr);
         if (r2 || ec != cudaSuccess) {
             cudaGetLastError();
@@ -1505,6 +1593,9 @@ void mpm_destroy(mpm_ctx* c) {
     for (auto e : c->xfer_ev)
         if (e) cudaEventDestroy(e);
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
+    for (auto e : c->clock_ev)
+        if (e) cudaEventDestroy(e);
+    if (c->clock_stream) cudaStreamDestroy(c->clock_stream);
     delete c;
 }
 
@@ -2164,10 +2255,10 @@ int mpm_autotune(mpm_ctx* c, int32_t steps, double dt, int contact, mpm_tune_res
         for (int i = 0; i < 6; ++i) *opt[i] = best[i];
         *opt[i0] = v0;
         *opt[i1] = v1;
-        int r = step(c, dt, contact, false, false);  // the run's steps: not output steps
+        int r = step(c, dt, contact, 0, false);  // the run's steps: not output steps
         if (r == MPM_OK) {
             cudaEventRecord(a, c->stream);
-            for (int s = 0; s < steps && r == MPM_OK; ++s) r = step(c, dt, contact, false, false);
+            for (int s = 0; s < steps && r == MPM_OK; ++s) r = step(c, dt, contact, 0, false);
             cudaEventRecord(b, c->stream);
         }
         if (r == MPM_OK) {

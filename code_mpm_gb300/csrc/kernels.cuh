@@ -8,7 +8,8 @@
 //   k_cell_ranges       per-cell particle ranges (FP64 form, steps that detect contact)
 //   k_p2g_cells         M2G (:48-89): each cell run's moments, then one atomic per corner and field;
 //                       active-node marking (b_Active, :36)
-//   k_dc_claim          DisplacementControl (:143-174), last writer in list order
+//   k_step_lists        active-node list; DisplacementControl's claims (:143-174, last writer in
+//                       list order); the device clock of a replayed step (engine.cu)
 //   k_node_phase_a      displacement control, IntegrateGrid (:90-142; contact :242-277),
 //                       f/m per node (the divisor of G2P pass 1)
 //   k_pass1_remap       G2P pass 1 (:489-510) fused with the velocity remap (:539-564)
@@ -31,6 +32,7 @@ namespace mpm {
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void k_reset_grid(NView<T> nd, int contact) {
+    step_enter<sizeof(T) == 4>();
     const long long nn = nd.nn;
     NODE_LOOP(nd, i) {
         unsigned st = nd.state[i];
@@ -182,6 +184,8 @@ __device__ __forceinline__ void prefetch_l2(const void* base, int es, long long 
 template <typename T, int REDUCE>
 __global__ void __launch_bounds__(512) k_p2g(PView<T> P, NView<T> nd, Geom g, const unsigned* __restrict__ skeys,
                                              const unsigned* __restrict__ perm, long long n, int with_mg) {
+    step_enter<sizeof(T) == 4>();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *nd.acount = 0u;
     long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     unsigned key = (s < n) ? skeys[s] : 0xffffffffu;
     const bool valid = key < g.key_max;
@@ -564,7 +568,9 @@ __device__ __forceinline__ void p2g_cells_run(const PView<T>& P, const NView<T>&
                                               long long n) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const P2GBlock<T, BS, FE, MG> blk(smem_raw);
+    step_enter<sizeof(T) == 4>();
     const int t = threadIdx.x;
+    if (blockIdx.x == 0 && t == 0) *nd.acount = 0u;
     const long long s0 = blockIdx.x * (long long)BS, s = s0 + t;
     const unsigned key = (s < n) ? skeys[s] : 0xffffffffu;
     const long long np = P.n;
@@ -613,30 +619,32 @@ __global__ void __launch_bounds__(BS) k_p2g_cells_mg(PView<float> P, NView<float
 // Displacement control (…MPLocks.cpp:143-174; contact :283-297, :416-432).
 // The reference overwrites node velocity/momentum/force from each controlled
 // particle in list order, so a node shared by several keeps the last one's.
-// k_dc_claim records, per node and axis, the largest list position writing
+// dc_claim records, per node and axis, the largest list position writing
 // it, and marks the node (NODE_CLAIMED in its state word) so the node phases
 // read the claims of marked nodes only; node_dc lets only the claiming
 // particle write.  contact: every particle claims all three axes, so the axis-0
 // claim word stands for the three (one atomic per corner instead of three).
 // ---------------------------------------------------------------------------
-static __global__ void k_dc_claim(const unsigned* __restrict__ dclist, int ndc, const unsigned* __restrict__ keys,
-                           const uint8_t* __restrict__ pflags, Geom g, unsigned* __restrict__ owner, long long nn,
-                           int contact, const uint16_t* __restrict__ sid, unsigned* __restrict__ state) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= ndc) return;
-    unsigned p = dclist[k];
-    unsigned key = keys[p];
+__device__ __forceinline__ void dc_claim(int k, const unsigned* __restrict__ dclist, const unsigned* __restrict__ keys,
+                                         const uint8_t* __restrict__ pflags, const Geom& g, unsigned* owner,
+                                         long long nn, int contact, const uint16_t* __restrict__ sid,
+                                         unsigned* state) {
+    const unsigned p = dclist[k];
+    const unsigned key = keys[p];
     if (key >= g.key_max) return;
     const Geom& gs = spec_geom(g, sid, p);
-    unsigned axes = contact ? 7u : (pflags[p] & 7u);
+    const unsigned axes = contact ? 7u : (pflags[p] & 7u);
+    if (!axes) return;
     int b[3];
     key_to_base(key, gs, b);
+    const CellNodes cn = cell_nodes(gs, b);
+#pragma unroll
     for (int c8 = 0; c8 < 8; ++c8) {
-        long long nid = corner_node(gs, b, c8);
-        if (nid < 0) continue;
+        if (!((cn.mask >> c8) & 1u)) continue;
+        const long long nid = cell_node(cn, c8);
         for (int a = 0; a < 3; ++a)
             if ((axes & (1u << a)) && !(contact && a > 0)) atomicMax(&owner[a * nn + nid], (unsigned)k + 1u);
-        if (axes) atomicOr(&state[nid], NODE_CLAIMED);
+        atomicOr(&state[nid], NODE_CLAIMED);
     }
 }
 
@@ -740,6 +748,7 @@ __global__ void __launch_bounds__(256) k_pass1_remap(PView<T> P, NView<T> nd, Ge
                                                      const unsigned* __restrict__ skeys,
                                                      const unsigned* __restrict__ perm, long long n, T dt,
                                                      T mass_min, int contact) {
+    step_enter<sizeof(T) == 4>();
     long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     unsigned key = (s < n) ? skeys[s] : 0xffffffffu;
     Runs run;
@@ -857,6 +866,7 @@ __global__ void __launch_bounds__(BS, sizeof(T) == 4 && CPT < 4 ? 1536 / BS : 1)
     T* sn = reinterpret_cast<T*>(scn + bs);
     CellSlots cs(reinterpret_cast<unsigned char*>(sn + (F32 ? 9 : 10) * bs), bs);
     unsigned* skey = cs.key;
+    step_enter<sizeof(T) == 4>();
     const long long s = blockIdx.x * (long long)bs + t;
     const unsigned key = (s < n) ? skeys[s] : 0xffffffffu;
     const long long np = P.n;
@@ -967,7 +977,7 @@ __global__ void __launch_bounds__(BS, sizeof(T) == 4 && CPT < 4 ? 1536 / BS : 1)
 }
 
 // Displacement control from the node's side: for each axis whose last-writer
-// claim (list position + 1, k_dc_claim) is set, the claiming platen particle's
+// claim (list position + 1, dc_claim) is set, the claiming platen particle's
 // velocity v, momentum m v and zero force.
 template <typename T>
 __device__ __forceinline__ void node_dc_regs(const unsigned own[3], const unsigned* __restrict__ dclist,
@@ -1030,6 +1040,7 @@ template <typename T>
 __global__ void __launch_bounds__(256, 4) k_node_phase_a(NView<T> nd, T dt, double damping, int contact, int floor_friction,
                                const unsigned* __restrict__ dclist, int ndc, const T* __restrict__ pvel, long long np,
                                T mass_min, int clean, double* work, double dtd) {
+    step_enter<sizeof(T) == 4>();
     const long long nn = nd.nn;
     double w_dc = 0.0, w_fr = 0.0;
     NODE_LOOP_AHEAD(nd, i) {
@@ -1111,6 +1122,7 @@ __global__ void __launch_bounds__(256, 4) k_node_phase_a(NView<T> nd, T dt, doub
 template <typename T>
 __global__ void __launch_bounds__(256, 4) k_node_phase_b(NView<T> nd, int contact, const unsigned* __restrict__ dclist, int ndc,
                                const T* __restrict__ pvel, long long np, T mass_min, int clean, int vel_zero) {
+    step_enter<sizeof(T) == 4>();
     const long long nn = nd.nn;
     NODE_LOOP_AHEAD(nd, i) {
         const unsigned st = nd.state[i];
@@ -1135,7 +1147,7 @@ __global__ void __launch_bounds__(256, 4) k_node_phase_b(NView<T> nd, int contac
         if (ndc && (st & NODE_CLAIMED)) {
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                if (contact && a > 0) {  // one claim word for the three axes (k_dc_claim)
+                if (contact && a > 0) {  // one claim word for the three axes (dc_claim)
                     own[a] = own[0];
                     continue;
                 }
@@ -1782,6 +1794,7 @@ template <typename T, int BATCH, int BS>
 __global__ void __launch_bounds__(BS, sizeof(T) == 4 ? 1280 / BS : 1) k_pass2(PView<T> P, NView<T> nd, Geom g, unsigned* __restrict__ keys,
                                                unsigned* __restrict__ keys_next, const MatConst* __restrict__ mats,
                                                int nmat, StepArgs a, unsigned* err) {
+    step_enter<sizeof(T) == 4>();
     const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (threadIdx.x < 32) pass2_prefetch<T>(P, blockIdx.x * (long long)blockDim.x, blockDim.x, a.contact);
     if (p >= P.n) return;
@@ -1816,6 +1829,7 @@ __global__ void __launch_bounds__(BS, pass2_staged_blocks<BS>()) k_pass2_staged(
     const long long p0 = blockIdx.x * (long long)BS, p = p0 + t;
     float u[3];
     bool queued;
+    step_enter<true>();
     if (!S::usable(P, keys, p0)) {
         if (t < 32) pass2_prefetch<float>(P, p0, BS, a.contact);
         if (p < P.n) pass2_particle<float, 0>(P, nd, g, keys, keys_next, mats, nmat, a, err, p, u, queued);
@@ -1850,6 +1864,7 @@ template <int BS>
 __global__ void __launch_bounds__(BS) k_pass2_ls(PView<double> P, NView<double> nd, Geom g, unsigned* __restrict__ keys,
                                                  unsigned* __restrict__ keys_next, const MatConst* __restrict__ mats,
                                                  int nmat, StepArgs a, unsigned* err) {
+    step_enter<false>();
     const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (p >= P.n) return;
     float u[3];

@@ -232,6 +232,8 @@ __global__ void __launch_bounds__(BS) k_p2g_pairs(PView<float> P, NView<float> n
     int* wsum = run_start + TS + 1;                       // 33
     unsigned long long* bar_mem = reinterpret_cast<unsigned long long*>(smem_raw + (STAGE ? S::BYTES : 0) +
                                                                          ((size_t)TS * 8 + 4 + 33 * 4 + 15) / 16 * 16);
+    step_enter<true>();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *nd.acount = 0u;
     const int t = threadIdx.x, lane = t & 31;
     const long long s0 = blockIdx.x * (long long)TS;
     const int nslots = (int)min((long long)TS, n - s0);
@@ -339,6 +341,7 @@ __global__ void __launch_bounds__(BS) k_pass1_pairs(PView<float> P, NView<float>
                                                      const unsigned* __restrict__ skeys,
                                                      const unsigned* __restrict__ perm, long long n, float dt,
                                                      int contact) {
+    step_enter<true>();
     constexpr int TS = PAIR_TILE_PER_THREAD * BS;
     __shared__ unsigned skey[TS];
     __shared__ int run_start[TS + 1];
