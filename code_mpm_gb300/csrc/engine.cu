@@ -82,7 +82,7 @@ struct mpm_ctx {
         backstress, mp_mg, strain_rate, material, pflags, dc_mult,
         Fe;  // FP64 form: elastic deformation gradient (large-strain pass 2)
     // nodes
-    DevBuf g_acc, g_vel, g_ftemp, g_mg, g_state, g_fixed, g_friction, g_ratio, g_q, g_owner,
+    DevBuf g_acc, g_vel, g_ftemp, g_mg, g_state, g_amark, g_fixed, g_friction, g_ratio, g_q, g_owner,
         g_nowner, g_need, g_list, g_count, rs_chunk;
     int sm_count = 152;
     DevBuf cstart, cend;
@@ -158,7 +158,7 @@ struct mpm_ctx {
                           &g_state, &g_fixed, &g_friction, &g_ratio, &g_q, &g_owner, &g_nowner, &g_need, &g_list, &g_count, &rs_chunk, &cstart,
                           &cend, &keys0, &vals0, &keys1, &vals1, &keys_copy, &counts, &dclist, &mats, &staging, &staging2, &tune_backup, &surf, &mon_mask, &mon_acc, &loc, &geom_tab, &sid, &alist, &acount,
                           &q_in, &q_out, &q_vol, &q_pidx, &q_count, &sg_acc, &hv_count,
-                          &dsim, &tl_dev, &orig, &ptmp, &Fe, &work_acc, &fext_any};
+                          &dsim, &tl_dev, &orig, &ptmp, &Fe, &work_acc, &fext_any, &g_amark};
         all.assign(std::begin(list), std::end(list));
     }
 };
@@ -235,6 +235,7 @@ NView<T> nview(mpm_ctx* c) {
     v.ftemp = (T*)c->g_ftemp.p;
     v.mg = (T*)c->g_mg.p;
     v.state = (unsigned*)c->g_state.p;
+    v.amark = (uint8_t*)c->g_amark.p;
     v.fixed = (uint8_t*)c->g_fixed.p;
     v.friction = (double*)c->g_friction.p;
     v.rec = (T*)c->g_ratio.p;
@@ -825,16 +826,18 @@ __global__ void k_step_end(DevSim* d) {
 // What a step needs between P2G and the node phases, in one launch (two
 // kernels and the counter's memset before, each a launch's latency on a small
 // scene):
-//  * blocks [0, ncompact): the active-node list.  A block compacts a tile of
-//    CS_THREADS x CS_ROUNDS consecutive nodes in node order and reserves its
-//    range with one atomic (a counter shared by every warp would serialise tens
-//    of thousands of atomics at one L2 address).  Each warp takes 32 x
-//    CS_ROUNDS consecutive nodes, loads all its state words before counting
-//    (the loads overlap), and writes its entries after the warps before it;
+//  * blocks [0, ncompact): the active-node list from P2G's marks, 16 nodes per
+//    thread (a byte per node; the state words cost four: on a grid of 32M nodes,
+//    6% of them active, list and claims took 39-48 us from the state words,
+//    21 from the marks).  A block
+//    reserves its range with one atomic (a counter shared by every warp would
+//    serialise tens of thousands of atomics at one L2 address), so the list is
+//    in node order within each 4,096 nodes.  The marks are cleared for the next
+//    step; an output step also sets the nodes' state bits, which its caller sees;
 //  * the blocks after them: the displacement-control claims, one particle of
 //    the list per thread (they set another bit of the state words);
 //  * the first step of a replay takes over its clock (clock given).
-constexpr int CS_THREADS = 256, CS_ROUNDS = 16;
+constexpr int CS_THREADS = 256;
 struct ClaimArgs {
     const unsigned* dclist;
     int ndc;
@@ -845,9 +848,10 @@ struct ClaimArgs {
     const uint16_t* sid;
 };
 template <bool EARLY>
-__global__ void __launch_bounds__(CS_THREADS) k_step_lists(unsigned* state, long long n, unsigned ncompact,
-                                                           unsigned* __restrict__ list, unsigned* count, ClaimArgs dc,
-                                                           Geom g, DevSim* clock) {
+__global__ void __launch_bounds__(CS_THREADS) k_step_lists(uint8_t* amark, unsigned* state, long long nn,
+                                                           unsigned ncompact, unsigned* __restrict__ list,
+                                                           unsigned* count, int output, ClaimArgs dc, Geom g,
+                                                           DevSim* clock) {
     __shared__ unsigned woff[CS_THREADS / 32];
     __shared__ unsigned base;
     step_enter<EARLY>();
@@ -855,23 +859,30 @@ __global__ void __launch_bounds__(CS_THREADS) k_step_lists(unsigned* state, long
     if (clock && blockIdx.x == gridDim.x - 1 && t == 0) clock->now = clock->ahead;
     if (blockIdx.x >= ncompact) {
         const int k = (int)(blockIdx.x - ncompact) * CS_THREADS + t;
-        if (k < dc.ndc) dc_claim(k, dc.dclist, dc.keys, dc.pflags, g, dc.owner, n, dc.contact, dc.sid, state);
+        if (k < dc.ndc) dc_claim(k, dc.dclist, dc.keys, dc.pflags, g, dc.owner, nn, dc.contact, dc.sid, state);
         return;
     }
-    const long long wbase = blockIdx.x * (long long)(CS_THREADS * CS_ROUNDS) + (long long)w * 32 * CS_ROUNDS;
-    unsigned v[CS_ROUNDS], m[CS_ROUNDS];
-#pragma unroll
-    for (int r = 0; r < CS_ROUNDS; ++r) {
-        const long long i = wbase + (long long)r * 32 + lane;
-        v[r] = i < n ? state[i] & 1u : 0u;
+    const long long at = (blockIdx.x * (long long)CS_THREADS + t) * 16;
+    unsigned bits = 0u;  // this thread's marked nodes
+    if (at < nn) {       // (the marks are padded to whole groups of 16)
+        uint4* p = reinterpret_cast<uint4*>(amark + at);
+        const uint4 m = *p;
+        if (m.x | m.y | m.z | m.w) {
+            *p = make_uint4(0u, 0u, 0u, 0u);
+            // bytes of value 0 or 1: the product gathers a word's four into its top nibble
+            bits = ((m.x * 0x10204080u) >> 28) | ((m.y * 0x10204080u) >> 28) << 4 |
+                   ((m.z * 0x10204080u) >> 28) << 8 | ((m.w * 0x10204080u) >> 28) << 12;
+        }
     }
-    unsigned cnt = 0;
+    // entries of this warp's threads before this one
+    const unsigned cnt = __popc(bits);
+    unsigned incl = cnt;
 #pragma unroll
-    for (int r = 0; r < CS_ROUNDS; ++r) {
-        m[r] = __ballot_sync(FULL_MASK, v[r] != 0u);
-        cnt += __popc(m[r]);
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned o = __shfl_up_sync(FULL_MASK, incl, d);
+        if (lane >= d) incl += o;
     }
-    if (lane == 0) woff[w] = cnt;
+    if (lane == 31) woff[w] = incl;
     __syncthreads();
     if (t == 0) {
         unsigned total = 0;
@@ -883,12 +894,19 @@ __global__ void __launch_bounds__(CS_THREADS) k_step_lists(unsigned* state, long
         base = total ? atomicAdd(count, total) : 0u;
     }
     __syncthreads();
-    unsigned off = base + woff[w];
-    const unsigned below = (1u << lane) - 1u;
-#pragma unroll
-    for (int r = 0; r < CS_ROUNDS; ++r) {
-        if (v[r]) list[off + __popc(m[r] & below)] = (unsigned)(wbase + (long long)r * 32 + lane);
-        off += __popc(m[r]);
+    const unsigned off = base + woff[w] + incl - cnt;
+    // the warp writes the nodes of two threads at a time
+    const unsigned first = (unsigned)((blockIdx.x * (long long)CS_THREADS + (t - lane)) * 16);
+    const int half = lane >> 4, l16 = lane & 15;
+    const unsigned have = __ballot_sync(FULL_MASK, bits != 0u);
+    for (unsigned pairs = (have | have >> 1) & 0x55555555u; pairs; pairs &= pairs - 1u) {
+        const int src = __ffs(pairs) - 1 + half;
+        const unsigned b = __shfl_sync(FULL_MASK, bits, src), o = __shfl_sync(FULL_MASK, off, src);
+        if ((b >> l16) & 1u) {
+            const unsigned node = first + 16u * src + l16;
+            list[o + __popc(b & ((1u << l16) - 1u))] = node;
+            if (output) atomicOr(&state[node], 1u);
+        }
     }
 }
 
@@ -1027,12 +1045,13 @@ int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
             if (!c->owner_clean) CK(cudaMemsetAsync(c->g_owner.p, 0, (size_t)3 * nn * 4, c->stream));
             c->owner_clean = false;  // claims in use until phase B clears them
         }
-        const unsigned ncompact = (unsigned)((nn + CS_THREADS * CS_ROUNDS - 1) / (CS_THREADS * CS_ROUNDS));
+        const unsigned ncompact = (unsigned)((nn + 16 * CS_THREADS - 1) / (16 * CS_THREADS));
         const unsigned nclaim = (unsigned)((c->ndc + CS_THREADS - 1) / CS_THREADS);
         const ClaimArgs dc{(const unsigned*)c->dclist.p, c->ndc, keys, (const uint8_t*)c->pflags.p,
                            (unsigned*)c->g_owner.p, contact, P.sid};
-        LAUNCH_STEP("step_lists", k_step_lists<sizeof(T) == 4>, ncompact + nclaim, CS_THREADS, 0, N.state, nn,
-                    ncompact, (unsigned*)c->alist.p, N.acount, dc, g, graph == 1 ? dsim : (DevSim*)nullptr);
+        LAUNCH_STEP("step_lists", k_step_lists<sizeof(T) == 4>, ncompact + nclaim, CS_THREADS, 0, N.amark, N.state,
+                    nn, ncompact, (unsigned*)c->alist.p, N.acount, output ? 1 : 0, dc, g,
+                    graph == 1 ? dsim : (DevSim*)nullptr);
         if (graph == 1) {  // the next replay's clock, on a branch beside the two steps
             const double* tl = (const double*)c->tl_dev.p;
             const int nt = (int)c->tl_t.size();
@@ -1551,7 +1570,7 @@ int mpm_create_batch(const mpm_grid_desc* grids, int32_t nspec, int form, mpm_ct
         size_t bytes;
     } plan[] = {{&c->g_acc, 8 * nn * t},   {&c->g_vel, 3 * nn * t},
                 {&c->g_ftemp, 3 * nn * t}, {&c->g_mg, 3 * nn * t},
-                {&c->g_state, nn * 4},     {&c->g_fixed, nn},        {&c->g_friction, nn * 8},
+                {&c->g_state, nn * 4},     {&c->g_amark, (nn + 15) / 16 * 16}, {&c->g_fixed, nn},        {&c->g_friction, nn * 8},
                 {&c->g_ratio, 8 * nn * t}, {&c->g_q, 4 * nn * t},    {&c->g_owner, 3 * nn * 4},
                 {&c->g_nowner, nn * 4},    {&c->g_need, nn * 4},     {&c->g_list, nn * 4},
                 {&c->g_count, 4},          {&c->alist, nn * 4},       {&c->acount, 4},

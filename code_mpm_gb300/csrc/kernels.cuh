@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(512) k_p2g(PView<T> P, NView<T> nd, Geom g, co
         if (valid && (!REDUCE || run.tail)) {
             long long nid = corner_node(*gsp, b, k);
             if (nid >= 0) {
-                atomicOr(&nd.state[nid], 1u);  // a reduction: no load to wait for
+                mark_active(nd.amark, (unsigned)nid);
                 acc_add<T>(nd.acc, nid, c[0], c[1], c[2], c[3], c[4], c[5], c[6]);
                 if (nf == 10) {
                     atomicAdd(&nd.mg[nid], c[7]);
@@ -547,7 +547,7 @@ struct P2GBlock {
                 const T* c = iz ? c1 : c0;
                 const T* f = iz ? p1 : p0;
                 // active nodes: the in-range corners of occupied cells (b_Active, …MPLocks.cpp:36)
-                atomicOr(&nd.state[nid], 1u);  // a reduction: no load to wait for
+                mark_active(nd.amark, (unsigned)nid);
                 acc_add<T>(nd.acc, nid, c[0], c[1], c[2], c[3], f[0], f[1], f[2]);
                 if constexpr (MG) {
                     const T* gm = iz ? g1 : g0;

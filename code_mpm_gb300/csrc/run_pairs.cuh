@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(BS) k_p2g_pairs(PView<float> P, NView<float> n
             if (!((cn.mask >> k) & 1u)) continue;
             const long long nid = cell_node(cn, k);
             // active nodes: the in-range corners of occupied cells (b_Active, …MPLocks.cpp:36)
-            atomicOr(&nd.state[nid], 1u);
+            mark_active(nd.amark, (unsigned)nid);
             acc_add<float>(nd.acc, nid, am[j], ap0[j], ap1[j], ap2[j], af0[j], af1[j], af2[j]);
             if constexpr (MG) {
                 atomicAdd(&nd.mg[nid], g0[j]);
