@@ -516,7 +516,7 @@ int upload_field(mpm_ctx* c, DevBuf& dst, const double* host, long long n, int k
     size_t esz = fp64 ? 8 : 4;
     const bool acc = acc_comp >= 0;
     const long long off = acc ? acc_comp : 0, cs = acc ? 1 : n, ps = acc ? 8 : 1;
-    int rc = acc ? MPM_OK : ensure(c, dst, (size_t)n * k * esz);
+    int rc = acc ? MPM_OK : ensure(c, dst, (size_t)n * k * esz);  // (particle arrays: already there, padded)
     if (rc) return rc;
     if (n == 0) return MPM_OK;
     if (acc && !host) return MPM_OK;  // accumulator components are only written from host rows
@@ -1179,7 +1179,24 @@ int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
             const unsigned pb = blocks_for(n, b2);
             unsigned* kc = (unsigned*)c->keys_copy.p;
             const MatConst* mats = (const MatConst*)c->mats.p;
-#define PASS2(B, S) LAUNCH_STEP("pass2", (k_pass2<T, B, S>), pb, S, 0, P, N, g, kc, keys_next, mats, c->nmat, a, err)
+            // FP32: the corner pairs' loads are issued together either way
+#define PASS2(B, S)                                                                                              \
+    do {                                                                                                         \
+        constexpr int B_ = sizeof(T) == 4 ? 0 : (B);                                                             \
+        if (contact)                                                                                             \
+            LAUNCH_STEP("pass2", (k_pass2<T, B_, S, true>), pb, S, 0, P, N, g, kc, keys_next, mats, c->nmat, a, err); \
+        else                                                                                                     \
+            LAUNCH_STEP("pass2", (k_pass2<T, B_, S, false>), pb, S, 0, P, N, g, kc, keys_next, mats, c->nmat, a, err); \
+    } while (0)
+#define PASS2_STAGED(S)                                                                                          \
+    do {                                                                                                         \
+        if (contact)                                                                                             \
+            LAUNCH_STEP("pass2", (k_pass2_staged<S, true>), pb, S, Pass2Stage<S>::SMEM, P, N, g, kc, keys_next, mats, \
+                        c->nmat, a, err);                                                                        \
+        else                                                                                                     \
+            LAUNCH_STEP("pass2", (k_pass2_staged<S, false>), pb, S, Pass2Stage<S>::SMEM, P, N, g, kc, keys_next, mats, \
+                        c->nmat, a, err);                                                                        \
+    } while (0)
             bool large = false;
             if constexpr (sizeof(T) == 8) {
                 if (c->large_strain && !contact) {  // non-contact loop only, as in the reference
@@ -1191,15 +1208,9 @@ int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
             if (large) {
             } else if (c->gather_batch == 2 && sizeof(T) == 4) {
                 if constexpr (sizeof(T) == 4) {
-                    if (b2 == 128)
-                        LAUNCH_STEP("pass2", k_pass2_staged<128>, pb, 128, Pass2Stage<128>::SMEM, P, N, g, kc,
-                                    keys_next, mats, c->nmat, a, err);
-                    else if (b2 == 256)
-                        LAUNCH_STEP("pass2", k_pass2_staged<256>, pb, 256, Pass2Stage<256>::SMEM, P, N, g, kc,
-                                    keys_next, mats, c->nmat, a, err);
-                    else
-                        LAUNCH_STEP("pass2", k_pass2_staged<512>, pb, 512, Pass2Stage<512>::SMEM, P, N, g, kc,
-                                    keys_next, mats, c->nmat, a, err);
+                    if (b2 == 128) PASS2_STAGED(128);
+                    else if (b2 == 256) PASS2_STAGED(256);
+                    else PASS2_STAGED(512);
                 }
             } else if (b2 == 128) {
                 if (c->gather_batch == 1) PASS2(1, 128); else PASS2(0, 128);
@@ -1210,6 +1221,7 @@ int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
             } else if constexpr (sizeof(T) == 8) {
                 if (b2 == 64) PASS2(0, 64); else PASS2(0, 32);
             }
+#undef PASS2_STAGED
 #undef PASS2
         }
         if constexpr (sizeof(T) == 4) {
@@ -1391,7 +1403,7 @@ int alloc_particles(mpm_ctx* c, long long n) {
                 {&c->keys0, 4},       {&c->vals0, 4},          {&c->keys1, 4},           {&c->vals1, 4},
                 {&c->keys_copy, 4},   {&c->loc, c->form == MPM_FORM_FP32 ? 12u : 0u}};
     for (auto& e : plan) {
-        int rc = ensure(c, *e.b, (size_t)n * e.bytes);
+        int rc = ensure(c, *e.b, (size_t)n * e.bytes + PARTICLE_PAD);
         if (rc) return rc;
     }
     const long long nblocks = std::max<long long>(1, (n + RS_TILE - 1) / RS_TILE);
@@ -1428,11 +1440,11 @@ bool pairs_attr() {
            cudaFuncSetAttribute(k_p2g_pairs<BS, false, true>, a, (int)p2g_pairs_smem<BS>(true)) == cudaSuccess &&
            cudaFuncSetAttribute(k_p2g_pairs<BS, true, true>, a, (int)p2g_pairs_smem<BS>(true)) == cudaSuccess;
 }
-bool pass2_staged_attrs() {
+template <int BS>
+bool pass2_staged_attr() {
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    return cudaFuncSetAttribute(k_pass2_staged<128>, a, Pass2Stage<128>::SMEM) == cudaSuccess &&
-           cudaFuncSetAttribute(k_pass2_staged<256>, a, Pass2Stage<256>::SMEM) == cudaSuccess &&
-           cudaFuncSetAttribute(k_pass2_staged<512>, a, Pass2Stage<512>::SMEM) == cudaSuccess;
+    return cudaFuncSetAttribute(k_pass2_staged<BS, false>, a, Pass2Stage<BS>::SMEM) == cudaSuccess &&
+           cudaFuncSetAttribute(k_pass2_staged<BS, true>, a, Pass2Stage<BS>::SMEM) == cudaSuccess;
 }
 template <typename T>
 bool cells_attrs() {
@@ -1496,7 +1508,7 @@ int mpm_create_batch(const mpm_grid_desc* grids, int32_t nspec, int form, mpm_ct
     cudaGetDevice(&c->device);
     cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device);
     if (c->sm_count <= 0) c->sm_count = 152;
-    if (!cells_attrs<double>() || !cells_attrs<float>() || !pass2_staged_attrs() || !pairs_attr<128>() ||
+    if (!cells_attrs<double>() || !cells_attrs<float>() || !pass2_staged_attr<128>() || !pass2_staged_attr<256>() || !pass2_staged_attr<512>() || !pairs_attr<128>() ||
         !pairs_attr<256>() || !pairs_attr<512>()) {
         cudaGetLastError();
         delete c;
@@ -1763,7 +1775,7 @@ int mpm_upload_particles(mpm_ctx* c, const mpm_particles* p, int64_t n) {
             const long long i = *c->h_err;
             return fail(c, MPM_ERR_ARG, "particle %lld: specimen %d out of range", i, p->specimen[i]);
         }
-        if ((rc = ensure(c, c->sid, (size_t)std::max<int64_t>(1, n) * 2))) return rc;
+        if ((rc = ensure(c, c->sid, (size_t)n * 2 + PARTICLE_PAD))) return rc;
         if (n > 0)
             CK(cudaMemcpyAsync(c->sid.p, stg + in_bytes, (size_t)n * 2, cudaMemcpyDeviceToDevice, c->stream));
     }

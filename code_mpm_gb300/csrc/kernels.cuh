@@ -1249,9 +1249,7 @@ struct DirectSrc {
     __device__ __forceinline__ float loc(const PView<T>& P, int k, long long p) const { return P.loc[k * P.n + p]; }
     __device__ __forceinline__ T F(const PView<T>& P, int k, long long p) const { return P.F[k * P.n + p]; }
     __device__ __forceinline__ T stress(const PView<T>& P, int k, long long p) const { return P.stress[k * P.n + p]; }
-    __device__ __forceinline__ T strain(const PView<T>& P, int k, long long p) const { return P.strain[k * P.n + p]; }
     __device__ __forceinline__ double pos(const PView<T>& P, int k, long long p) const { return P.pos[k * P.n + p]; }
-    __device__ __forceinline__ double e_strain(const PView<T>& P, long long p) const { return P.e_strain[p]; }
 };
 
 __device__ __forceinline__ uint32_t shared_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -1278,30 +1276,23 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
 // for one memory round trip instead of one per dependent load.  One segment
 // per (field, component): BS elements plus 16 bytes, copied from the 16-byte
 // boundary at or below the block's first element (component k of an n-element
-// array starts (k n es) mod 16 bytes into its segment).  A block may stage
-// only if p0 + BS + 16 <= n (every copy then stays inside its array) and
-// every array starts on a 16-byte boundary.
+// array starts (k n es) mod 16 bytes into its segment).  Every array starts on
+// a 16-byte boundary (cudaMalloc) and is allocated PARTICLE_PAD bytes longer
+// than its n elements, so the last block's copies, which reach up to BS
+// elements plus 16 bytes past the end of a component, stay inside.
+constexpr size_t PARTICLE_PAD = 512 * 8 + 16;  // the largest block's elements of the widest type, and 16 bytes
+
 template <int BS>
 struct Pass2Stage {
+    static_assert((size_t)BS * 8 + 16 <= PARTICLE_PAD, "padding of the particle arrays");
     static constexpr int SEG1 = BS + 16, SEG2 = 2 * BS + 16, SEG4 = 4 * BS + 16, SEG8 = 8 * BS + 16;
     static constexpr int O_FLAGS = 0, O_SID = O_FLAGS + SEG1, O_KEYS = O_SID + SEG2, O_MAT = O_KEYS + SEG4;
     static constexpr int O_VOL0 = O_MAT + SEG4, O_BACK = O_VOL0 + SEG4, O_LOC = O_BACK + SEG4;
-    static constexpr int O_F = O_LOC + 3 * SEG4, O_STRESS = O_F + 9 * SEG4, O_STRAIN = O_STRESS + 6 * SEG4;
-    static constexpr int O_POS = O_STRAIN + 6 * SEG4, O_ES = O_POS + 3 * SEG8, BYTES = O_ES + SEG8;
-    static constexpr int NSEG = 34;  // flags, sid, keys, material, vol0, back stress, 3 loc, 9 F, 2 x 6 tensors, 3 pos, strain energy
+    static constexpr int O_F = O_LOC + 3 * SEG4, O_STRESS = O_F + 9 * SEG4;
+    static constexpr int O_POS = O_STRESS + 6 * SEG4, BYTES = O_POS + 3 * SEG8;
+    static constexpr int NSEG = 27;  // flags, sid, keys, material, vol0, back stress, 3 loc, 9 F, 6 stress, 3 pos
     static constexpr int SMEM = BYTES + 16;  // and the mbarrier
 
-    static __device__ __forceinline__ bool usable(const PView<float>& P, const unsigned* keys, long long p0) {
-        const unsigned long long a = (unsigned long long)P.pflags | (unsigned long long)P.sid |
-                                     (unsigned long long)keys | (unsigned long long)P.material |
-                                     (unsigned long long)P.vol0 | (unsigned long long)P.backstress |
-                                     (unsigned long long)P.loc | (unsigned long long)P.F |
-                                     (unsigned long long)P.stress | (unsigned long long)P.strain |
-                                     (unsigned long long)P.pos | (unsigned long long)P.e_strain;
-        const bool all = P.pflags && keys && P.material && P.vol0 && P.backstress && P.loc && P.F && P.stress &&
-                         P.strain && P.eps_p && P.pos && P.e_strain && P.e_plastic;
-        return all && (a & 15ull) == 0 && p0 + BS + 16 <= P.n;
-    }
     // segment i: its array, element size, component and shared offset
     static __device__ __forceinline__ void segment(int i, const PView<float>& P, const unsigned* keys, const void*& base,
                                                    int& es, int& k, int& off) {
@@ -1315,9 +1306,7 @@ struct Pass2Stage {
         else if (i < 9) { base = P.loc; es = 4; k = i - 6; off = O_LOC; }
         else if (i < 18) { base = P.F; es = 4; k = i - 9; off = O_F; }
         else if (i < 24) { base = P.stress; es = 4; k = i - 18; off = O_STRESS; }
-        else if (i < 30) { base = P.strain; es = 4; k = i - 24; off = O_STRAIN; }
-        else if (i < 33) { base = P.pos; es = 8; k = i - 30; off = O_POS; }
-        else { base = P.e_strain; es = 8; off = O_ES; }
+        else { base = P.pos; es = 8; k = i - 24; off = O_POS; }
         off += k * (BS * es + 16);
     }
     // bytes the block's copies deliver (no specimen ids with one specimen)
@@ -1366,13 +1355,9 @@ struct StagedSrc {
     __device__ __forceinline__ float stress(const PView<float>& P, int k, long long) const {
         return at<float, S::O_STRESS, 4>(P, k);
     }
-    __device__ __forceinline__ float strain(const PView<float>& P, int k, long long) const {
-        return at<float, S::O_STRAIN, 4>(P, k);
-    }
     __device__ __forceinline__ double pos(const PView<float>& P, int k, long long) const {
         return at<double, S::O_POS, 8>(P, k);
     }
-    __device__ __forceinline__ double e_strain(const PView<float>& P, long long) const { return at<double, S::O_ES, 8>(P, 0); }
 };
 
 // Apply a constitutive increment o to particle p (stress, plastic strain,
@@ -1382,10 +1367,13 @@ struct StagedSrc {
 // leaves the plastic strain, the plastic energy and the back stress as they
 // are: they are neither read nor written (68 of the FP32 form's 324 bytes per
 // particle).
-template <typename T, class SRC = DirectSrc<T>>
+// Sums that nothing in the step reads back (plastic strain and energy, on the
+// contact path the strain energy, in pass 2 the strain) are added by
+// reductions: the value is neither waited for nor held, and the FP64 form
+// saves its FP64 pipe the addition.
+template <typename T>
 __device__ __forceinline__ void apply_increment(const PView<T>& P, long long p, const T sig[6], const T e[6],
-                                                const CrOut<T>& o, T V, T R, bool plastic, int contact, double dt,
-                                                const SRC& src = SRC{}) {
+                                                const CrOut<T>& o, T V, T R, bool plastic, bool contact, double dt) {
     const long long np = P.n;
     T dEs = 0;
 #pragma unroll
@@ -1394,9 +1382,11 @@ __device__ __forceinline__ void apply_increment(const PView<T>& P, long long p, 
         P.stress[k * np + p] = sn;
         dEs += (contact ? sn : sn - (T)0.5 * o.dsig[k]) * e[k];
     }
-    const double es = src.e_strain(P, p) + fps_f2d_form(dEs * V);
-    P.e_strain[p] = es;
-    if (!contact) {
+    if (contact) {
+        atomicAdd(&P.e_strain[p], fps_f2d_form(dEs * V));
+    } else {
+        const double es = P.e_strain[p] + fps_f2d_form(dEs * V);
+        P.e_strain[p] = es;
         P.e_strain_ti[p] += es * dt;
         if (es > P.e_strain_max[p]) P.e_strain_max[p] = es;
     }
@@ -1405,10 +1395,10 @@ __device__ __forceinline__ void apply_increment(const PView<T>& P, long long p, 
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
         const T sn = sig[k] + o.dsig[k];
-        P.eps_p[k * np + p] += o.deps_p[k];
+        atomicAdd(&P.eps_p[k * np + p], o.deps_p[k]);
         dEp += (contact ? sn : sn - (T)0.5 * o.dsig[k]) * o.deps_p[k];
     }
-    P.e_plastic[p] += fps_f2d_form(dEp * V);
+    atomicAdd(&P.e_plastic[p], fps_f2d_form(dEp * V));
     P.backstress[p] = R + o.dR;
 }
 
@@ -1461,26 +1451,23 @@ __device__ __forceinline__ void pass2_prefetch(const PView<T>& P, long long p0, 
     } else if (t < 18) {
         base = P.stress;
         comp = t - 12;
-    } else if (t < 24) {
-        base = P.strain;
-        comp = t - 18;
-    } else if (t == 24) {
+    } else if (t == 18) {
         base = P.vol0;
-    } else if (t == 25) {
+    } else if (t == 19) {
         base = P.backstress;
-    } else if (t == 26) {
-        base = P.e_strain;
-        es = 8;
-    } else if (t == 27) {
+    } else if (t == 20) {
         base = P.material;
         es = 4;
-    } else if (t == 28) {
+    } else if (t == 21) {
         base = P.pflags;
         es = 1;
-    } else if (t == 29 && !contact) {
+    } else if (t == 22 && !contact) {
+        base = P.e_strain;
+        es = 8;
+    } else if (t == 23 && !contact) {
         base = P.e_strain_ti;
         es = 8;
-    } else if (t == 30 && !contact) {
+    } else if (t == 24 && !contact) {
         base = P.e_strain_max;
         es = 8;
     }
@@ -1559,7 +1546,7 @@ __device__ __forceinline__ void large_strain_update(const PView<T>& P, long long
             const double sn = (1.0 / det) * o.dsig[k];
             P.strain[k * np + p] = et[k];
             P.stress[k * np + p] = sn;
-            P.eps_p[k * np + p] += o.deps_p[k];
+            atomicAdd(&P.eps_p[k * np + p], o.deps_p[k]);
             es += sn * einc[k] * V;
         }
 #pragma unroll
@@ -1572,7 +1559,7 @@ __device__ __forceinline__ void large_strain_update(const PView<T>& P, long long
 
 // One particle of pass 2; returns the new cell key (u: the new cell-local
 // coordinate; queued: its stress increment waits for the network).
-template <typename T, int BATCH, bool LS = false, class SRC = DirectSrc<T>>
+template <typename T, int BATCH, bool CONTACT, bool LS = false, class SRC = DirectSrc<T>>
 __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NView<T>& nd, const Geom& g,
                                                    unsigned* __restrict__ keys, unsigned* __restrict__ keys_next,
                                                    const MatConst* __restrict__ mats, int nmat, const StepArgs& a,
@@ -1582,7 +1569,7 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
     queued = false;
     const unsigned fl = src.pflags(P, p);
     const T dt = form_const<T>(a.dt, a.dt_f);
-    const bool skip = a.contact && (fl & 8u);
+    const bool skip = CONTACT && (fl & 8u);
     const Geom& gs = (g.nspec > 1) ? g.tab[src.sid(P, p)] : g;
     // the position stays in registers until the new cell key is formed
     double x[3] = {src.pos(P, 0, p), src.pos(P, 1, p), src.pos(P, 2, p)};
@@ -1669,21 +1656,21 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
         T V = 0;
         // strain, F and V: on the contact path before the material check
         // (…_Contact.cpp:464-484), else with a material only (…MPLocks.cpp:226-258)
-        if (a.contact || have_mat) {
+        if (CONTACT || have_mat) {
             T F[9], Fn[9];
 #pragma unroll
             for (int k = 0; k < 9; ++k) F[k] = src.F(P, k, p);
-            Kinematics<T>::update(a.contact != 0, F, Ldt, Fn);
+            Kinematics<T>::update(CONTACT, F, Ldt, Fn);
 #pragma unroll
             for (int k = 0; k < 9; ++k) P.F[k * np + p] = Fn[k];
             V = Kinematics<T>::det(Fn) * src.vol0(P, p);
             P.vol[p] = V;
 #pragma unroll
-            for (int k = 0; k < 6; ++k) P.strain[k * np + p] = src.strain(P, k, p) + e[k];
+            for (int k = 0; k < 6; ++k) atomicAdd(&P.strain[k * np + p], e[k]);
         }
         if (have_mat) {
             const MatConst& M = mats[mi];
-            if (a.contact && a.outputs) {
+            if (CONTACT && a.outputs) {
 #pragma unroll
                 for (int k = 0; k < 6; ++k) P.strain_rate[k * np + p] = e[k] / dt;
             }
@@ -1749,9 +1736,9 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
                 } else {
                     plastic = cr_return<T>(M, R, sig, e, tr, o);
                 }
-                apply_increment<T>(P, p, sig, e, o, V, R, plastic, a.contact, a.dt, src);
+                apply_increment<T>(P, p, sig, e, o, V, R, plastic, CONTACT, a.dt);
             }
-        } else if (!a.contact) {
+        } else if (!CONTACT) {
             atomicOr(err, ERR_BAD_MATERIAL);
         }
         }
@@ -1759,7 +1746,7 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
     // platen timeline (…MPLocks.cpp:766-789; contact :531-540)
     if (fl & PF_IN_DC) {
         const double* tv = a.tv_dev ? a.tv_dev : a.tv;
-        if (!a.contact) {
+        if constexpr (!CONTACT) {
             if (a.has_timeline) {
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
@@ -1789,35 +1776,39 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
 
 // BS: the block size; the FP32 form asks for 1280 / BS blocks per SM (48
 // registers: a few spill, and the extra resident warps hide more of the
-// gathers' latency).
-template <typename T, int BATCH, int BS>
+// gathers' latency).  CONTACT: the loop's path, apart so that each kernel holds
+// one path's code (pass 2's warps also wait for instructions).
+template <typename T, int BATCH, int BS, bool CONTACT>
 __global__ void __launch_bounds__(BS, sizeof(T) == 4 ? 1280 / BS : 1) k_pass2(PView<T> P, NView<T> nd, Geom g, unsigned* __restrict__ keys,
                                                unsigned* __restrict__ keys_next, const MatConst* __restrict__ mats,
                                                int nmat, StepArgs a, unsigned* err) {
     step_enter<sizeof(T) == 4>();
     const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (threadIdx.x < 32) pass2_prefetch<T>(P, blockIdx.x * (long long)blockDim.x, blockDim.x, a.contact);
+    if (threadIdx.x < 32) pass2_prefetch<T>(P, blockIdx.x * (long long)blockDim.x, blockDim.x, CONTACT);
     if (p >= P.n) return;
     float u[3];
     bool queued;
-    pass2_particle<T, BATCH>(P, nd, g, keys, keys_next, mats, nmat, a, err, p, u, queued);
+    pass2_particle<T, BATCH, CONTACT>(P, nd, g, keys, keys_next, mats, nmat, a, err, p, u, queued);
 }
 
 // FP32 pass 2 with the block's particle fields staged in shared memory
 // (Pass2Stage): warp 0 issues the bulk copies, every thread waits once on the
-// mbarrier, then runs pass2_particle reading from shared memory.  Blocks that
-// cannot stage (the last ones, or unaligned arrays) read global memory.
+// mbarrier, then runs pass2_particle reading from shared memory.  The arrays
+// are allocated with room for the last block's copies (PARTICLE_PAD).
 // Blocks per SM: as many as the staging buffers fit (228 KB of shared memory,
 // 1 KB reserved per block), but no more than 1024 threads, which leaves 64
-// registers per thread.  At 7, 8, 9 and 10 blocks of 128 the step of a solid
-// block of 1.07M particles in mid-crush took 187.6, 186.4, 187.0 and 188.6 us.
+// registers per thread.  At 6, 7, 8, 9 and 10 blocks of 128 the step of a solid
+// block of 1.07M particles in mid-crush took 147.8, 145.5, 145.8, 146.1 and
+// 150.0 us, that of 5.08M particles of honeycombs 700, 691, 689, 686 and 700.
+// Before the sums that nothing reads back became reductions and each path got
+// a kernel of its own, 168 and 752 us (pass 2 117 and 410 us, now 89 and 342).
 template <int BS>
 constexpr int pass2_staged_blocks() {
     constexpr int fit = (228 * 1024) / (Pass2Stage<BS>::SMEM + 1024), want = 1024 / BS;
     return fit < want ? fit : want;
 }
 
-template <int BS>
+template <int BS, bool CONTACT>
 __global__ void __launch_bounds__(BS, pass2_staged_blocks<BS>()) k_pass2_staged(PView<float> P, NView<float> nd, Geom g,
                                                                unsigned* __restrict__ keys,
                                                                unsigned* __restrict__ keys_next,
@@ -1829,18 +1820,13 @@ __global__ void __launch_bounds__(BS, pass2_staged_blocks<BS>()) k_pass2_staged(
     const long long p0 = blockIdx.x * (long long)BS, p = p0 + t;
     float u[3];
     bool queued;
-    step_enter<true>();
-    if (!S::usable(P, keys, p0)) {
-        if (t < 32) pass2_prefetch<float>(P, p0, BS, a.contact);
-        if (p < P.n) pass2_particle<float, 0>(P, nd, g, keys, keys_next, mats, nmat, a, err, p, u, queued);
-        return;
-    }
     const uint32_t bar = shared_addr(smem_raw + S::BYTES);
     if (t == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    step_enter<true>();
     __syncthreads();
     if (t < 32) {
         if (t == 0)
@@ -1848,14 +1834,15 @@ __global__ void __launch_bounds__(BS, pass2_staged_blocks<BS>()) k_pass2_staged(
                          "r"(S::tx_bytes(P))
                          : "memory");
         __syncwarp();
-        for (int i = t; i < S::NSEG; i += 32) S::copy(i, P, keys, p0, smem_raw, bar);
+        if (t < S::NSEG) S::copy(t, P, keys, p0, smem_raw, bar);
     }
     if (!mbar_wait(bar, 0, err)) {
         mbar_wait(bar, 0, err);  // once more (bounded) for copies still in flight, then leave
         return;
     }
-    pass2_particle<float, 0, false, StagedSrc<BS>>(P, nd, g, keys, keys_next, mats, nmat, a, err, p, u, queued,
-                                                   StagedSrc<BS>{smem_raw});
+    if (p >= P.n) return;
+    pass2_particle<float, 0, CONTACT, false, StagedSrc<BS>>(P, nd, g, keys, keys_next, mats, nmat, a, err, p, u, queued,
+                                                            StagedSrc<BS>{smem_raw});
 }
 
 // The large-strain pass 2 (non-contact loop, FP64 form; the reference ships
@@ -1869,7 +1856,7 @@ __global__ void __launch_bounds__(BS) k_pass2_ls(PView<double> P, NView<double> 
     if (p >= P.n) return;
     float u[3];
     bool queued;
-    pass2_particle<double, 0, true>(P, nd, g, keys, keys_next, mats, nmat, a, err, p, u, queued);
+    pass2_particle<double, 0, false, true>(P, nd, g, keys, keys_next, mats, nmat, a, err, p, u, queued);
 }
 
 // ---------------------------------------------------------------------------
