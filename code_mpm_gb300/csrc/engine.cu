@@ -83,7 +83,7 @@ struct mpm_ctx {
         Fe;  // FP64 form: elastic deformation gradient (large-strain pass 2)
     // nodes
     DevBuf g_acc, g_vel, g_ftemp, g_mg, g_state, g_amark, g_fixed, g_friction, g_ratio, g_q, g_owner,
-        g_nowner, g_need, g_list, g_count, rs_chunk;
+        g_nowner, g_need, g_list, g_count;
     int sm_count = 152;
     DevBuf cstart, cend;
     // sort
@@ -155,7 +155,7 @@ struct mpm_ctx {
         DevBuf* list[] = {&xtab, &err_word, &pos, &vel, &fext, &mass, &vol, &vol0, &F, &stress, &strain, &eps_p,
                           &e_strain, &e_strain_max, &e_strain_ti, &e_plastic, &backstress, &mp_mg, &strain_rate,
                           &material, &pflags, &dc_mult, &g_acc, &g_vel, &g_ftemp, &g_mg,
-                          &g_state, &g_fixed, &g_friction, &g_ratio, &g_q, &g_owner, &g_nowner, &g_need, &g_list, &g_count, &rs_chunk, &cstart,
+                          &g_state, &g_fixed, &g_friction, &g_ratio, &g_q, &g_owner, &g_nowner, &g_need, &g_list, &g_count, &cstart,
                           &cend, &keys0, &vals0, &keys1, &vals1, &keys_copy, &counts, &dclist, &mats, &staging, &staging2, &tune_backup, &surf, &mon_mask, &mon_acc, &loc, &geom_tab, &sid, &alist, &acount,
                           &q_in, &q_out, &q_vol, &q_pidx, &q_count, &sg_acc, &hv_count,
                           &dsim, &tl_dev, &orig, &ptmp, &Fe, &work_acc, &fext_any, &g_amark};
@@ -682,33 +682,24 @@ int sort_cells(mpm_ctx* c, const unsigned** skeys_out, const unsigned** perm_out
     const int nblocks = (int)((n + RS_TILE - 1) / RS_TILE);
     unsigned *kin = key_src, *vin = nullptr;
     unsigned *kout = key_other, *vout = (unsigned*)c->vals0.p;
-    const int hist_total = (1 << db) * nblocks;
-    const int nchunks = (hist_total + RS_SCAN_CHUNK - 1) / RS_SCAN_CHUNK;
+    unsigned* counts = (unsigned*)c->counts.p;
     for (int shift = 0; shift < bits; shift += db) {
         if (db == 8)
-            LAUNCH("rs_hist", k_rs_hist<8>, nblocks, RS_THREADS, kin, n, shift, (unsigned*)c->counts.p, nblocks);
+            LAUNCH_STEP("rs_hist", (k_rs_hist<8, RS_ITEMS>), nblocks, RS_THREADS, 0, kin, n, shift, counts, nblocks);
         else if (db == 9)
-            LAUNCH("rs_hist", k_rs_hist<9>, nblocks, RS_THREADS, kin, n, shift, (unsigned*)c->counts.p, nblocks);
+            LAUNCH_STEP("rs_hist", (k_rs_hist<9, RS_ITEMS>), nblocks, RS_THREADS, 0, kin, n, shift, counts, nblocks);
         else
-            LAUNCH("rs_hist", k_rs_hist<10>, nblocks, RS_THREADS, kin, n, shift, (unsigned*)c->counts.p, nblocks);
-        const unsigned* chunk_prefix = nullptr;
-        if (nchunks > 1) {
-            LAUNCH("rs_scan", k_rs_scan_chunks, nchunks, RS_SCAN_THREADS, (unsigned*)c->counts.p, hist_total,
-                   (unsigned*)c->rs_chunk.p);
-            LAUNCH("rs_scan", k_rs_scan, 1, 1024, (unsigned*)c->rs_chunk.p, nchunks);
-            chunk_prefix = (const unsigned*)c->rs_chunk.p;
-        } else {
-            LAUNCH("rs_scan", k_rs_scan, 1, 1024, (unsigned*)c->counts.p, hist_total);
-        }
+            LAUNCH_STEP("rs_hist", (k_rs_hist<10, RS_ITEMS>), nblocks, RS_THREADS, 0, kin, n, shift, counts, nblocks);
+        LAUNCH_STEP("rs_scan", k_rs_scan, 1u << db, RS_SCAN_THREADS, 0, counts, nblocks);
         if (db == 8)
-            LAUNCH("rs_scatter", k_rs_scatter<8>, nblocks, RS_THREADS, kin, (const unsigned*)vin, kout, vout, n, shift,
-                   (const unsigned*)c->counts.p, nblocks, chunk_prefix);
+            LAUNCH_STEP("rs_scatter", (k_rs_scatter<8, RS_ITEMS>), nblocks, RS_THREADS, 0, kin, (const unsigned*)vin, kout, vout, n,
+                        shift, (const unsigned*)counts, nblocks);
         else if (db == 9)
-            LAUNCH("rs_scatter", k_rs_scatter<9>, nblocks, RS_THREADS, kin, (const unsigned*)vin, kout, vout, n, shift,
-                   (const unsigned*)c->counts.p, nblocks, chunk_prefix);
+            LAUNCH_STEP("rs_scatter", (k_rs_scatter<9, RS_ITEMS>), nblocks, RS_THREADS, 0, kin, (const unsigned*)vin, kout, vout, n,
+                        shift, (const unsigned*)counts, nblocks);
         else
-            LAUNCH("rs_scatter", k_rs_scatter<10>, nblocks, RS_THREADS, kin, (const unsigned*)vin, kout, vout, n,
-                   shift, (const unsigned*)c->counts.p, nblocks, chunk_prefix);
+            LAUNCH_STEP("rs_scatter", (k_rs_scatter<10, RS_ITEMS>), nblocks, RS_THREADS, 0, kin, (const unsigned*)vin, kout, vout, n,
+                        shift, (const unsigned*)counts, nblocks);
         std::swap(kin, kout);
         vin = vout;
         vout = (vout == (unsigned*)c->vals0.p) ? (unsigned*)c->vals1.p : (unsigned*)c->vals0.p;
@@ -1407,10 +1398,7 @@ int alloc_particles(mpm_ctx* c, long long n) {
         if (rc) return rc;
     }
     const long long nblocks = std::max<long long>(1, (n + RS_TILE - 1) / RS_TILE);
-    int rc = ensure(c, c->counts, (size_t)1024 * nblocks * 4);
-    if (rc) return rc;
-    const long long nchunks = (1024 * nblocks + RS_SCAN_CHUNK - 1) / RS_SCAN_CHUNK;
-    return ensure(c, c->rs_chunk, (size_t)std::max<long long>(1, nchunks) * 4);
+    return ensure(c, c->counts, (size_t)1024 * (nblocks + 1) * 4);  // digit counts per tile, and totals
 }
 
 }  // namespace

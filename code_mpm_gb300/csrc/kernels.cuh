@@ -83,16 +83,17 @@ __device__ __forceinline__ unsigned particle_key(const Geom& g, const double x[3
     return ok ? g.key_off + (unsigned)((b[0] + 1) + g.kd[0] * ((b[1] + 1) + g.kd[1] * (b[2] + 1))) : g.key_max;
 }
 
-static __global__ void k_cell_keys(const double* __restrict__ pos, long long n, Geom g, unsigned* __restrict__ keys,
-                            unsigned* __restrict__ vals, unsigned* __restrict__ keys_copy, unsigned* err,
+static __global__ void k_cell_keys(const double* __restrict__ pos, long long n, Geom g, unsigned* keys,
+                            unsigned* __restrict__ vals, unsigned* keys_copy, unsigned* err,
                             float* __restrict__ loc, const uint16_t* __restrict__ sid) {
+    step_enter<true>();
     long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (p >= n) return;
     const double x[3] = {pos[p], pos[n + p], pos[2 * n + p]};
     float u[3];
     const unsigned key = particle_key(spec_geom(g, sid, p), x, u, err);
     keys[p] = key;
-    keys_copy[p] = key;
+    if (keys_copy != keys) keys_copy[p] = key;
     if (vals) vals[p] = (unsigned)p;
     if (loc) {
 #pragma unroll

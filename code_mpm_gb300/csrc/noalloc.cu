@@ -28,12 +28,12 @@ using namespace mpm;
 namespace {
 
 constexpr long long NA_MAX = MPM_NOALLOC_MAX_PARTICLES;
-constexpr long long NA_TILES = (NA_MAX + RS_TILE - 1) / RS_TILE;
+constexpr long long NA_TILES = RS_FEW / RS_FEW_TILE > NA_MAX / RS_TILE ? RS_FEW / RS_FEW_TILE : NA_MAX / RS_TILE;
 // layout (32-bit words): keysA, valsA, keysB, valsB (NA_MAX each), digit counts
-// (256 per tile), then one word k_cell_keys may flag a non-finite position in
-// (a write-only sink: such a particle already gets the out-of-grid key, and
-// the word is never read), padded to 64 words.
-constexpr long long NA_WORDS = 4 * NA_MAX + 256 * NA_TILES + 64;
+// (256 per tile) and totals (256), then one word k_cell_keys may flag a
+// non-finite position in (a write-only sink: such a particle already gets the
+// out-of-grid key, and the word is never read), padded to 64 words.
+constexpr long long NA_WORDS = 4 * NA_MAX + 256 * (NA_TILES + 1) + 64;
 
 // The scratch: file scope, static storage on every device that loads the library.
 __device__ __align__(256) unsigned g_noalloc_scratch[NA_WORDS];
@@ -61,6 +61,21 @@ int scratch_for_current_device(unsigned** out) {
     }
     *out = g_scratch_addr[dev];
     return MPM_OK;
+}
+
+// A kernel that begins with step_enter: its launch overlaps the kernel before it.
+template <typename... Ex, typename... Act>
+void launch_after(cudaStream_t st, void (*kernel)(Ex...), unsigned grid, unsigned block, Act&&... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<Act>(args)...);
 }
 
 }  // namespace
@@ -95,32 +110,33 @@ extern "C" int mpm_cell_order_noalloc(const mpm_grid_desc* grid, const double* d
     unsigned* keysB = s + 2 * NA_MAX;
     unsigned* valsB = s + 3 * NA_MAX;
     unsigned* counts = s + 4 * NA_MAX;
-    unsigned* err = counts + 256 * NA_TILES;
+    unsigned* err = counts + 256 * (NA_TILES + 1);
     cudaStream_t st = (cudaStream_t)stream;
-    // every scratch word the sort reads is written first by this call (keys and values by k_cell_keys,
-    // digit counts by each pass's histogram), so the previous call's contents need no clearing
-    const unsigned nb = (unsigned)((n + 255) / 256);
-    k_cell_keys<<<nb, 256, 0, st>>>(d_pos, n, g, keysA, valsA, d_keys, err, nullptr, nullptr);
+    // every scratch word the sort reads is written first by this call (keys by k_cell_keys, digit counts and
+    // totals by each pass), so the previous call's contents need no clearing.  The keys go to the caller's
+    // array and are the first pass's input; its values are the identity, the last pass's the caller's order.
+    launch_after(st, k_cell_keys, (unsigned)((n + 255) / 256), 256, d_pos, n, g, d_keys, (unsigned*)nullptr, d_keys, err,
+                 (float*)nullptr, (const uint16_t*)nullptr);
     if (cudaGetLastError() != cudaSuccess) return MPM_ERR_CUDA;
     int bits = 1;
     while (bits < 32 && ((unsigned long long)1 << bits) <= (unsigned long long)g.key_max) ++bits;
-    const int nblocks = (int)((n + RS_TILE - 1) / RS_TILE);
-    unsigned *kin = keysA, *vin = valsA, *kout = keysB, *vout = valsB;
+    const bool few = n <= RS_FEW;
+    const int tile = few ? RS_FEW_TILE : RS_TILE, nblocks = (int)((n + tile - 1) / tile);
+    const auto hist = few ? k_rs_hist<8, RS_FEW_ITEMS> : k_rs_hist<8, RS_ITEMS>;
+    const auto scatter = few ? k_rs_scatter<8, RS_FEW_ITEMS> : k_rs_scatter<8, RS_ITEMS>;
+    const unsigned *kin = d_keys, *vin = nullptr;
+    unsigned *kout = keysA, *vout = valsA;
     for (int shift = 0; shift < bits; shift += 8) {
-        k_rs_hist<<<nblocks, RS_THREADS, 0, st>>>(kin, n, shift, counts, nblocks);
+        const bool last = shift + 8 >= bits;
+        launch_after(st, hist, nblocks, RS_THREADS, kin, n, shift, counts, nblocks);
+        launch_after(st, k_rs_scan, 256, RS_SCAN_THREADS, counts, nblocks);
+        launch_after(st, scatter, nblocks, RS_THREADS, kin, vin, last ? (unsigned*)nullptr : kout,
+                     last ? d_order : vout, n, shift, (const unsigned*)counts, nblocks);
         if (cudaGetLastError() != cudaSuccess) return MPM_ERR_CUDA;
-        k_rs_scan<<<1, 1024, 0, st>>>(counts, 256 * nblocks);
-        if (cudaGetLastError() != cudaSuccess) return MPM_ERR_CUDA;
-        k_rs_scatter<<<nblocks, RS_THREADS, 0, st>>>(kin, vin, kout, vout, n, shift, counts, nblocks, nullptr);
-        if (cudaGetLastError() != cudaSuccess) return MPM_ERR_CUDA;
-        unsigned* t = kin;
         kin = kout;
-        kout = t;
-        t = vin;
         vin = vout;
-        vout = t;
+        kout = kout == keysA ? keysB : keysA;
+        vout = vout == valsA ? valsB : valsA;
     }
-    if (cudaMemcpyAsync(d_order, vin, (size_t)n * sizeof(unsigned), cudaMemcpyDeviceToDevice, st) != cudaSuccess)
-        return MPM_ERR_CUDA;
     return MPM_OK;
 }

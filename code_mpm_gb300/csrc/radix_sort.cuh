@@ -1,37 +1,47 @@
 // Stable LSD radix sort of (32-bit key, 32-bit value) pairs, DB-bit digits
 // (8 to 10; the caller picks the fewest passes that cover the key bits).
 //
-// Used to order particles by cell key each step.  Stability within a digit
+// Used to order particles by cell key.  Stability within a digit
 // pass comes from ranking every key against the keys before it in its tile
 // (warp match + per-warp digit counters, then a prefix over the warps), so
 // equal keys keep their input order; with values 0..n-1 as input the output
 // is the particle order of a stable CPU sort by key (std::stable_sort).
 //
 // Per pass: k_rs_hist (per-tile digit histogram, digit-major layout),
-// k_rs_scan (one-block exclusive scan of the histogram), k_rs_scatter.
+// k_rs_scan (a block per digit scans that digit's tiles and leaves the digit's
+// total), k_rs_scatter (whose blocks scan the totals themselves).  All three
+// are latency at the sizes they see (700,000 keys in 171 tiles), so the scan
+// is spread over the digits, the tiles are small enough for every SM to have
+// several, and the kernels follow each other by dependent launch.
 #pragma once
 
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "common.cuh"
+
 namespace mpm {
 
 constexpr int RS_THREADS = 256;
 constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int RS_ITEMS = 16;  // keys per thread
-constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
-constexpr int RS_WARP_TILE = 32 * RS_ITEMS;
+// Keys per thread (the kernels' ITEMS): 4 where the keys are few (the order of
+// 700,000 particles took 43 us with 4, 50 with 8, 67 with 16; 192 before, with
+// 16 and a one-block scan), 8 above (1M: 55, 53, 71).
+constexpr int RS_ITEMS = 8, RS_FEW_ITEMS = 4;
+constexpr long long RS_FEW = 3 << 18;  // up to so many keys
+constexpr int RS_TILE = RS_THREADS * RS_ITEMS, RS_FEW_TILE = RS_THREADS * RS_FEW_ITEMS;
 
-template <int DB = 8>
+template <int DB, int ITEMS>
 static __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const unsigned* __restrict__ keys, long long n, int shift,
                                                          unsigned* __restrict__ counts, int nblocks) {
     constexpr unsigned NB = 1u << DB, MASK = NB - 1u;
     __shared__ unsigned h[NB];
     for (int i = threadIdx.x; i < (int)NB; i += RS_THREADS) h[i] = 0;
+    step_enter<true>();
     __syncthreads();
-    long long base = (long long)blockIdx.x * RS_TILE;
+    long long base = (long long)blockIdx.x * (RS_THREADS * ITEMS);
 #pragma unroll 4
-    for (int j = 0; j < RS_ITEMS; ++j) {
+    for (int j = 0; j < ITEMS; ++j) {
         long long idx = base + (long long)j * RS_THREADS + threadIdx.x;
         if (idx < n) atomicAdd(&h[(keys[idx] >> shift) & MASK], 1u);
     }
@@ -39,98 +49,97 @@ static __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const unsigned* _
     for (int i = threadIdx.x; i < (int)NB; i += RS_THREADS) counts[(size_t)i * nblocks + blockIdx.x] = h[i];
 }
 
-// Exclusive scan of counts[0..total) in place, one block of 1024 threads.
-static __global__ void __launch_bounds__(1024) k_rs_scan(unsigned* __restrict__ counts, int total) {
-    __shared__ unsigned part[1024];
-    const int t = threadIdx.x;
-    const int per = (total + 1023) / 1024;
-    const int lo = t * per, hi = min(total, lo + per);
-    unsigned s = 0;
-    for (int i = lo; i < hi; ++i) s += counts[i];
-    part[t] = s;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-        unsigned v = (t >= off) ? part[t - off] : 0u;
-        __syncthreads();
-        part[t] += v;
-        __syncthreads();
-    }
-    unsigned run = part[t] - s;  // exclusive prefix of this thread's chunk
-    for (int i = lo; i < hi; ++i) {
-        unsigned c = counts[i];
-        counts[i] = run;
-        run += c;
-    }
-}
+// Block d: exclusive scan over the tiles of digit d's counts, in place; the
+// digit's total goes to counts[gridDim.x * nblocks + d].
+constexpr int RS_SCAN_THREADS = 256;
+constexpr int RS_SCAN_ITEMS = 4;
 
-// Two-level exclusive scan of the histogram for large inputs: k_rs_scan_chunks
-// scans RS_SCAN_CHUNK entries per block in place and records each chunk's
-// total; k_rs_scan (one block) then scans the chunk totals; the scatter adds
-// the chunk prefix to every offset it reads.
-constexpr int RS_SCAN_THREADS = 1024;
-constexpr int RS_SCAN_PER_THREAD = 4;
-constexpr int RS_SCAN_CHUNK = RS_SCAN_THREADS * RS_SCAN_PER_THREAD;
-
-static __global__ void __launch_bounds__(RS_SCAN_THREADS) k_rs_scan_chunks(unsigned* __restrict__ counts, int total,
-                                                                          unsigned* __restrict__ chunk_totals) {
-    __shared__ unsigned wsum[RS_SCAN_THREADS / 32];
+static __global__ void __launch_bounds__(RS_SCAN_THREADS) k_rs_scan(unsigned* __restrict__ counts, int nblocks) {
+    __shared__ unsigned wsum[2][RS_SCAN_THREADS / 32];
+    step_enter<true>();
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const long long base = (long long)blockIdx.x * RS_SCAN_CHUNK + (long long)t * RS_SCAN_PER_THREAD;
-    unsigned v[RS_SCAN_PER_THREAD], s = 0;
+    unsigned* row = counts + (size_t)blockIdx.x * nblocks;
+    unsigned before = 0;
+    int side = 0;
+    for (int at = 0; at < nblocks; at += RS_SCAN_THREADS * RS_SCAN_ITEMS, side ^= 1) {
+        const int i0 = at + t * RS_SCAN_ITEMS;
+        unsigned v[RS_SCAN_ITEMS], s = 0;
 #pragma unroll
-    for (int j = 0; j < RS_SCAN_PER_THREAD; ++j) {
-        v[j] = (base + j < total) ? counts[base + j] : 0u;
-        s += v[j];
-    }
-    unsigned inc = s;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        unsigned o = __shfl_up_sync(0xffffffffu, inc, d);
-        if (lane >= d) inc += o;
-    }
-    if (lane == 31) wsum[w] = inc;
-    __syncthreads();
-    if (w == 0) {
-        unsigned x = wsum[lane];
+        for (int j = 0; j < RS_SCAN_ITEMS; ++j) {
+            v[j] = i0 + j < nblocks ? row[i0 + j] : 0u;
+            s += v[j];
+        }
+        unsigned inc = s;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            unsigned o = __shfl_up_sync(0xffffffffu, x, d);
-            if (lane >= d) x += o;
+            const unsigned o = __shfl_up_sync(FULL_MASK, inc, d);
+            if (lane >= d) inc += o;
         }
-        wsum[lane] = x;  // inclusive over warps
-    }
-    __syncthreads();
-    unsigned run = inc - s + (w > 0 ? wsum[w - 1] : 0u);
+        if (lane == 31) wsum[side][w] = inc;
+        __syncthreads();  // (the other side's sums are still being read by slower warps)
+        unsigned run = before + inc - s, all = 0;
 #pragma unroll
-    for (int j = 0; j < RS_SCAN_PER_THREAD; ++j) {
-        if (base + j < total) counts[base + j] = run;
-        run += v[j];
+        for (int k = 0; k < RS_SCAN_THREADS / 32; ++k) {
+            const unsigned x = wsum[side][k];
+            if (k < w) run += x;
+            all += x;
+        }
+#pragma unroll
+        for (int j = 0; j < RS_SCAN_ITEMS; ++j) {
+            if (i0 + j < nblocks) row[i0 + j] = run;
+            run += v[j];
+        }
+        before += all;
     }
-    if (t == RS_SCAN_THREADS - 1) chunk_totals[blockIdx.x] = wsum[31];
+    if (t == 0) counts[(size_t)gridDim.x * nblocks + blockIdx.x] = before;
 }
 
-template <int DB = 8>
+template <int DB, int ITEMS>
 static __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const unsigned* __restrict__ kin,
                                                             const unsigned* __restrict__ vin,
                                                             unsigned* __restrict__ kout, unsigned* __restrict__ vout,
                                                             long long n, int shift,
-                                                            const unsigned* __restrict__ offs, int nblocks,
-                                                            const unsigned* __restrict__ chunk_prefix) {
+                                                            const unsigned* __restrict__ offs, int nblocks) {
     constexpr unsigned NB = 1u << DB, MASK = NB - 1u;
     __shared__ unsigned wcnt[RS_WARPS][NB];
     __shared__ unsigned gofs[NB];
+    __shared__ unsigned wtot[RS_WARPS];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < RS_WARPS * (int)NB; i += RS_THREADS) (&wcnt[0][0])[i] = 0;
-    for (int i = threadIdx.x; i < (int)NB; i += RS_THREADS) {
-        size_t j = (size_t)i * nblocks + blockIdx.x;
-        gofs[i] = offs[j] + (chunk_prefix ? chunk_prefix[j / RS_SCAN_CHUNK] : 0u);
+    step_enter<true>();
+    {  // where each digit's keys of this tile go: the digits before it, then its keys in earlier tiles
+        constexpr int PER = (int)NB / RS_THREADS;
+        unsigned v[PER], s = 0;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            v[j] = offs[(size_t)NB * nblocks + threadIdx.x * PER + j];
+            s += v[j];
+        }
+        unsigned inc = s;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned o = __shfl_up_sync(FULL_MASK, inc, d);
+            if (lane >= d) inc += o;
+        }
+        if (lane == 31) wtot[w] = inc;
+        __syncthreads();
+        unsigned run = inc - s;
+#pragma unroll
+        for (int k = 0; k < RS_WARPS; ++k)
+            if (k < w) run += wtot[k];
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            const int d = threadIdx.x * PER + j;
+            gofs[d] = run + offs[(size_t)d * nblocks + blockIdx.x];
+            run += v[j];
+        }
     }
     __syncthreads();
-    const long long base = (long long)blockIdx.x * RS_TILE + (long long)w * RS_WARP_TILE;
+    const long long base = (long long)blockIdx.x * (RS_THREADS * ITEMS) + (long long)w * (32 * ITEMS);
     const unsigned lt = (1u << lane) - 1u;
-    unsigned k[RS_ITEMS], v[RS_ITEMS], r[RS_ITEMS];
+    unsigned k[ITEMS], v[ITEMS], r[ITEMS];
 #pragma unroll
-    for (int c = 0; c < RS_ITEMS; ++c) {
+    for (int c = 0; c < ITEMS; ++c) {
         long long idx = base + c * 32 + lane;
         bool ok = idx < n;
         unsigned key = ok ? kin[idx] : 0u;
@@ -157,12 +166,12 @@ static __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const unsigned
     }
     __syncthreads();
 #pragma unroll
-    for (int c = 0; c < RS_ITEMS; ++c) {
+    for (int c = 0; c < ITEMS; ++c) {
         long long idx = base + c * 32 + lane;
         if (idx < n) {
             unsigned d = (k[c] >> shift) & MASK;
             unsigned dst = gofs[d] + wcnt[w][d] + r[c];
-            kout[dst] = k[c];
+            if (kout) kout[dst] = k[c];  // (the last pass of a caller that wants the order alone)
             vout[dst] = v[c];
         }
     }

@@ -248,7 +248,7 @@ int mpm_cell_order(mpm_ctx* ctx, uint32_t* keys, uint32_t* sorted_order, int64_t
  * device arrays of n uint32), exactly as mpm_cell_order() reports them.
  * No memory is allocated, by this call or by any routine it calls: the
  * working memory is one fixed array of static device storage inside the
- * library (about 16.3 MiB, sized for MPM_NOALLOC_MAX_PARTICLES), which every
+ * library (about 16.8 MiB, sized for MPM_NOALLOC_MAX_PARTICLES), which every
  * GPU that loads the library holds until the process exits.
  *   - n > MPM_NOALLOC_MAX_PARTICLES returns MPM_ERR_TOO_LARGE and does nothing.
  *   - Work is queued on `stream` (a cudaStream_t, NULL for the default
