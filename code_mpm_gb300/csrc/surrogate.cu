@@ -209,139 +209,321 @@ __global__ void k_normalise_targets(long long n, const float* __restrict__ t, co
 }
 
 // ---------------------------------------------------------------------------
-// FP32 GEMM for training: C[M x N] = op(A)[M x K] op(B)[K x N], 64 x 64 tiles,
-// 16-deep k slices, 4 x 4 outputs per thread.  op(A) = A (row-major, lda) or
-// A^T (A stored K x M); op(B) = B (row-major K x N) or B^T (B stored N x K,
-// the layer weights W[out][in]).  Epilogues: store (+bias), bias + ReLU
-// (keeps the pre-activation in aux), times ReLU'(aux) (backward), and atomic
-// accumulation of split-K partial sums (weight gradients; blockIdx.z picks
-// the k range).
+// FP32 training kernels.  A batch of n rows goes through
+//   forward   h = relu(x W^T + b), three layers          k_layer<true>
+//   head      y = h3 W4^T + b4, the loss, dL/dy, and back through layer 4:
+//             d3 = (dy W4) relu'(h3), the gradients of W4, b4 and b3   k_head
+//   backward  d = (d W) relu'(h), two layers, and the bias gradient of each
+//             (the column sums of d, from the tile in registers)  k_layer<false>
+//   weights   dW += d^T h, split over the rows                      k_weight_grad
+// relu'(z) is taken from h (z > 0 exactly where h = relu(z) > 0), so the
+// pre-activations are not stored.
+//
+// The GEMMs are bound by the FP32 FMAs: a block of 256 threads forms a 128 x
+// 128 tile, 8 x 8 outputs per thread in four 4 x 4 quarters (each thread's 16
+// operand values per k are four 16-byte shared loads for 64 FMAs), the next
+// 16-deep slice on its way to registers while the current one is used.  Before,
+// with 64 x 64 tiles, 4 x 4 outputs, no overlap, stored pre-activations and
+// separate kernels for layer 4, the loss and the column sums, a batch of 65,536
+// took 928 us through mpm_net_loss_grad, 1,000 rows 340 us; now 476 and 146.
 // ---------------------------------------------------------------------------
-enum { EPI_STORE = 0, EPI_RELU = 1, EPI_DRELU = 2, EPI_ATOMIC = 3 };
+constexpr int GT = 256;       // threads
+constexpr int GK = 16;        // slice depth
+constexpr int GS = HID + 4;   // shared row stride
 
-template <bool TA, bool TB, int EPI>
-__global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float* __restrict__ A, int lda,
-                                               const float* __restrict__ B, int ldb, float* __restrict__ C, int ldc,
-                                               const float* __restrict__ bias, float* __restrict__ aux, int kchunk) {
-    __shared__ __align__(16) float As[16][68];
-    __shared__ __align__(16) float Bs[16][68];
-    const int tid = threadIdx.x;
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    const int kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
-    const int tm = (tid >> 4) * 4, tn = (tid & 15) * 4;
-    float acc[4][4];
+struct GemmTile {
+    float a[2][GK][GS], b[2][GK][GS];
+};
+
+// acc[i][j]: rows ty * 4 + (i & 3) + 64 (i >> 2), columns tx * 4 + (j & 3) + 64 (j >> 2)
+__device__ __forceinline__ void tile_fma(const GemmTile& s, int buf, int ty, int tx, float acc[8][8]) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int k = 0; k < GK; ++k) {
+        float a[8], b[8];
+        *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&s.a[buf][k][4 * ty]);
+        *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&s.a[buf][k][64 + 4 * ty]);
+        *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(&s.b[buf][k][4 * tx]);
+        *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(&s.b[buf][k][64 + 4 * tx]);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-    for (int k0 = kbeg; k0 < kend; k0 += 16) {
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int e = tid + r * 256;
-            int mm, kk;
-            if (!TA) {
-                mm = e >> 4;
-                kk = e & 15;
-            } else {
-                kk = e >> 6;
-                mm = e & 63;
-            }
-            const int gm = m0 + mm, gk = k0 + kk;
-            float v = 0.0f;
-            if (gm < M && gk < kend) v = TA ? A[(long long)gk * lda + gm] : A[(long long)gm * lda + gk];
-            As[kk][mm] = v;
+            for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+    }
+}
+
+// FWD: C = relu(A W^T + bias), A n x K, W 128 x K.
+// else: C = (A W) where H > 0 (else 0), A n x 128, W 128 x 128; the column sums of C added to gbias.
+template <bool FWD, int K>
+__global__ void __launch_bounds__(GT, 2) k_layer(int n, const float* __restrict__ A, const float* __restrict__ W,
+                                                 const float* __restrict__ bias, const float* __restrict__ H,
+                                                 float* __restrict__ C, float* __restrict__ gbias) {
+    extern __shared__ __align__(16) unsigned char net_smem[];
+    GemmTile& s = *reinterpret_cast<GemmTile*>(net_smem);
+    step_enter<true>();
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    const int m0 = blockIdx.x * 128;
+    // a slice: rows r and r + 64, four k each (stored transposed); W the same, or (backward) k rows of 128
+    const int lr = tid >> 2, lk = (tid & 3) * 4, br = tid >> 5, bc = (tid & 31) * 4;
+    float4 ra[2], rb[2];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = lr + 64 * h;
+            ra[h] = m0 + r < n ? *reinterpret_cast<const float4*>(A + (long long)(m0 + r) * K + k0 + lk)
+                               : make_float4(0.f, 0.f, 0.f, 0.f);
+            rb[h] = FWD ? *reinterpret_cast<const float4*>(W + r * K + k0 + lk)
+                        : *reinterpret_cast<const float4*>(W + (k0 + br + 8 * h) * HID + bc);
         }
+    };
+    auto store = [&](int buf) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int e = tid + r * 256;
-            int kk, nn;
-            if (!TB) {
-                kk = e >> 6;
-                nn = e & 63;
+        for (int h = 0; h < 2; ++h) {
+            const int r = lr + 64 * h;
+            const float va[4] = {ra[h].x, ra[h].y, ra[h].z, ra[h].w}, vb[4] = {rb[h].x, rb[h].y, rb[h].z, rb[h].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s.a[buf][lk + j][r] = va[j];
+            if (FWD) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s.b[buf][lk + j][r] = vb[j];
             } else {
-                nn = e >> 4;
-                kk = e & 15;
+                *reinterpret_cast<float4*>(&s.b[buf][br + 8 * h][bc]) = rb[h];
             }
-            const int gn = n0 + nn, gk = k0 + kk;
-            float v = 0.0f;
-            if (gn < N && gk < kend) v = TB ? B[(long long)gn * ldb + gk] : B[(long long)gk * ldb + gn];
-            Bs[kk][nn] = v;
         }
+    };
+    float acc[8][8] = {};
+    load(0);
+    store(0);
+    __syncthreads();
+#pragma unroll 1
+    for (int k0 = 0; k0 < K; k0 += GK) {
+        const int buf = (k0 / GK) & 1;
+        if (k0 + GK < K) load(k0 + GK);
+        tile_fma(s, buf, ty, tx, acc);
+        if (k0 + GK < K) store(buf ^ 1);
         __syncthreads();
+    }
+    float cs[8] = {};
 #pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            const float4 a = *reinterpret_cast<const float4*>(&As[kk][tm]);
-            const float4 b = *reinterpret_cast<const float4*>(&Bs[kk][tn]);
-            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+    for (int i = 0; i < 8; ++i) {
+        const int m = m0 + 4 * ty + (i & 3) + 64 * (i >> 2);
+        if (m >= n) continue;
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+        for (int q = 0; q < 2; ++q) {
+            const int c = 4 * tx + 64 * q;
+            const long long o = (long long)m * HID + c;
+            float v[4];
+            if (FWD) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+                for (int j = 0; j < 4; ++j) v[j] = fmaxf(acc[i][4 * q + j] + bias[c + j], 0.0f);
+            } else {
+                const float4 h = *reinterpret_cast<const float4*>(H + o);
+                const float hv[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    v[j] = hv[j] > 0.0f ? acc[i][4 * q + j] : 0.0f;
+                    cs[4 * q + j] += v[j];
+                }
+            }
+            *reinterpret_cast<float4*>(C + o) = make_float4(v[0], v[1], v[2], v[3]);
         }
+    }
+    if (!FWD) {  // the tile's column sums: over ty in shared memory, then one atomic per column
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s.a[0][ty][4 * tx + (j & 3) + 64 * (j >> 2)] = cs[j];
+        __syncthreads();
+        if (tid < HID) {
+            float v = 0.0f;
+#pragma unroll
+            for (int r = 0; r < 16; ++r) v += s.a[0][r][tid];
+            atomicAdd(&gbias[tid], v);
+        }
+    }
+}
+
+// gW[128 x N] += D^T X over this block's rows (D n x 128, X n x N), N = 128 or 16.
+template <int N>
+__global__ void __launch_bounds__(GT, 2) k_weight_grad(int n, int rows, const float* __restrict__ D,
+                                                       const float* __restrict__ X, float* __restrict__ gW) {
+    static_assert(N == HID || N == IN, "layer widths");
+    extern __shared__ __align__(16) unsigned char net_smem[];
+    GemmTile& s = *reinterpret_cast<GemmTile*>(net_smem);
+    step_enter<true>();
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15, br = tid >> 5, bc = (tid & 31) * 4;
+    const int beg = blockIdx.x * rows, end = min(n, beg + rows);
+    float4 rd[2], rx[2];
+    auto load = [&](int r0) {
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = r0 + br + 8 * h;
+            rd[h] = r < end ? *reinterpret_cast<const float4*>(D + (long long)r * HID + bc) : z;
+            if (N == HID) rx[h] = r < end ? *reinterpret_cast<const float4*>(X + (long long)r * HID + bc) : z;
+        }
+        if (N == IN) {  // 16 rows of 16: the first 64 threads
+            const int r = r0 + (tid >> 2);
+            rx[0] = tid < 64 && r < end ? *reinterpret_cast<const float4*>(X + (long long)r * IN + (tid & 3) * 4) : z;
+        }
+    };
+    auto store = [&](int buf) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            *reinterpret_cast<float4*>(&s.a[buf][br + 8 * h][bc]) = rd[h];
+            if (N == HID) *reinterpret_cast<float4*>(&s.b[buf][br + 8 * h][bc]) = rx[h];
+        }
+        if (N == IN && tid < 64) *reinterpret_cast<float4*>(&s.b[buf][tid >> 2][(tid & 3) * 4]) = rx[0];
+    };
+    float acc[8][8] = {};  // N = 16: acc[i][0] of column tx
+    load(beg);
+    store(0);
+    __syncthreads();
+    int buf = 0;
+#pragma unroll 1
+    for (int r0 = beg; r0 < end; r0 += GK, buf ^= 1) {
+        if (r0 + GK < end) load(r0 + GK);
+        if constexpr (N == HID) {
+            tile_fma(s, buf, ty, tx, acc);
+        } else {
+#pragma unroll
+            for (int k = 0; k < GK; ++k) {
+                const float b = s.b[buf][k][tx];
+                const float4 a0 = *reinterpret_cast<const float4*>(&s.a[buf][k][4 * ty]);
+                const float4 a1 = *reinterpret_cast<const float4*>(&s.a[buf][k][64 + 4 * ty]);
+                const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[i][0] = fmaf(a[i], b, acc[i][0]);
+            }
+        }
+        if (r0 + GK < end) store(buf ^ 1);
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 8; ++i) {
+        float* g = gW + (4 * ty + (i & 3) + 64 * (i >> 2)) * N;
+        if constexpr (N == HID) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                atomicAdd(reinterpret_cast<float4*>(g + 4 * tx + 64 * q),
+                          make_float4(acc[i][4 * q], acc[i][4 * q + 1], acc[i][4 * q + 2], acc[i][4 * q + 3]));
+        } else {
+            atomicAdd(g + tx, acc[i][0]);
+        }
+    }
+}
+
+// The output layer, a warp per row (lane l holds columns 4l .. 4l + 3).
+// GRAD: also the loss (mean over the batch and the 7 used outputs), dL/dy and
+// layer 4's backward pass: d = (dy W4) where h > 0, gradients of W4, b4 and,
+// as the column sums of d, of layer 3's bias; without it y is written.
+constexpr int HEAD_WARPS = 16;
+template <bool GRAD>
+__global__ void __launch_bounds__(HEAD_WARPS * 32) k_head(long long n, const float* __restrict__ h,
+                                                          const float* __restrict__ W4, const float* __restrict__ b4,
+                                                          const float* __restrict__ t, float* __restrict__ y,
+                                                          float* __restrict__ d, float* __restrict__ gW4,
+                                                          float* __restrict__ gb4, float* __restrict__ gb3,
+                                                          double* __restrict__ loss) {
+    __shared__ float sg[OUT * HID + HID + OUT];
+    step_enter<true>();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (GRAD) {
+        for (int i = threadIdx.x; i < OUT * HID + HID + OUT; i += blockDim.x) sg[i] = 0.0f;
+        __syncthreads();
+    }
+    float w[OUT][4], gw[OUT][4] = {}, gs[4] = {}, gb = 0.0f;
+#pragma unroll
+    for (int c = 0; c < OUT; ++c) *reinterpret_cast<float4*>(w[c]) = *reinterpret_cast<const float4*>(W4 + c * HID + 4 * lane);
+    // after the halving exchange below a lane holds output c
+    const int c = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+    const float bc = b4[c], sc = 2.0f / (float)(n * NOUT);
+    double l = 0.0;
+    // two rows' loads ahead of the row in hand
+    const long long step = (long long)gridDim.x * HEAD_WARPS, r0 = blockIdx.x * (long long)HEAD_WARPS + warp;
+    float4 hn[2];
+    float tn[2];
+    auto fetch = [&](int q, long long r) {
+        hn[q] = r < n ? *reinterpret_cast<const float4*>(h + r * HID + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+        tn[q] = GRAD && r < n ? t[r * OUT + c] : 0.0f;
+    };
+    fetch(0, r0);
+    fetch(1, r0 + step);
+    for (long long r = r0; r < n; r += step) {
+        const float hv[4] = {hn[0].x, hn[0].y, hn[0].z, hn[0].w}, tv = tn[0];
+        hn[0] = hn[1];
+        tn[0] = tn[1];
+        fetch(1, r + 2 * step);
+        float p[OUT];
+#pragma unroll
+        for (int k = 0; k < OUT; ++k) p[k] = w[k][0] * hv[0] + w[k][1] * hv[1] + w[k][2] * hv[2] + w[k][3] * hv[3];
+        // eight sums over the warp: halve the outputs a lane keeps with each exchange
+#pragma unroll
+        for (int half = 4, off = 16; half; half >>= 1, off >>= 1) {
+            const bool up = lane & off;
+#pragma unroll
+            for (int k = 0; k < half; ++k) {
+                const float send = up ? p[k] : p[half + k], keep = up ? p[half + k] : p[k];
+                p[k] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+            }
+        }
+        float v = p[0];
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += bc;
+        if (!GRAD) {
+            if ((lane & 3) == 0) y[r * OUT + c] = v;
+            continue;
+        }
+        const float diff = c < NOUT ? v - tv : 0.0f, dy = sc * diff;
+        l += (double)diff * diff;
+        gb += dy;
+        float o[4] = {};
+#pragma unroll
+        for (int k = 0; k < OUT; ++k) {
+            const float g = __shfl_sync(0xffffffffu, dy, ((k & 4) ? 16 : 0) | ((k & 2) ? 8 : 0) | ((k & 1) ? 4 : 0));
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                o[j] = fmaf(g, w[k][j], o[j]);
+                gw[k][j] = fmaf(g, hv[j], gw[k][j]);
+            }
+        }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int m = m0 + tm + i, n = n0 + tn + j;
-            if (m >= M || n >= N) continue;
-            float v = acc[i][j];
-            const long long o = (long long)m * ldc + n;
-            if constexpr (EPI == EPI_STORE) {
-                if (bias) v += bias[n];
-                C[o] = v;
-            } else if constexpr (EPI == EPI_RELU) {
-                v += bias[n];
-                aux[o] = v;
-                C[o] = fmaxf(v, 0.0f);
-            } else if constexpr (EPI == EPI_DRELU) {
-                C[o] = aux[o] > 0.0f ? v : 0.0f;
-            } else {
-                atomicAdd(&C[o], v);
-            }
+            o[j] = hv[j] > 0.0f ? o[j] : 0.0f;
+            gs[j] += o[j];
         }
-}
-
-template <bool TA, bool TB, int EPI>
-static void sgemm(cudaStream_t s, int M, int N, int K, const float* A, int lda, const float* B, int ldb, float* C,
-                  int ldc, const float* bias = nullptr, float* aux = nullptr, int splits = 1) {
-    const int kchunk = ((K + splits - 1) / splits + 15) / 16 * 16;
-    splits = (K + kchunk - 1) / kchunk;
-    dim3 grid((N + 63) / 64, (M + 63) / 64, splits);
-    k_sgemm<TA, TB, EPI><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, aux, kchunk);
-}
-
-// column sums of an n x N row-major matrix into g (atomic; N divides 256)
-template <int N>
-__global__ void k_colsum(long long n, const float* __restrict__ d, float* __restrict__ g) {
-    static_assert(256 % N == 0, "N must divide 256");
-    constexpr int RPI = 256 / N;
-    const int col = threadIdx.x % N, r0 = threadIdx.x / N;
-    const long long base = blockIdx.x * 1024LL;
-    float s = 0.0f;
-    for (int r = r0; r < 1024; r += RPI) {
-        const long long i = base + r;
-        if (i < n) s += d[i * N + col];
+        *reinterpret_cast<float4*>(d + r * HID + 4 * lane) = make_float4(o[0], o[1], o[2], o[3]);
     }
-    atomicAdd(&g[col], s);
-}
-
-// loss (mean over samples and the 7 used outputs) and its gradient
-__global__ void k_loss(long long n, const float* __restrict__ y, const float* __restrict__ t, float* __restrict__ dy,
-                       double* __restrict__ loss) {
-    long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    double l = 0.0;
-    if (i < n) {
-        const float sc = 2.0f / (float)(n * NOUT);
-        for (int c = 0; c < OUT; ++c) {
-            const float d = c < NOUT ? y[i * OUT + c] - t[i * OUT + c] : 0.0f;
-            dy[i * OUT + c] = sc * d;
-            l += (double)d * d;
-        }
-    }
+    if (!GRAD) return;
+    // the block's sums, then one atomic per parameter
+#pragma unroll
+    for (int k = 0; k < OUT; ++k)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) atomicAdd(&sg[k * HID + 4 * lane + j], gw[k][j]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) atomicAdd(&sg[OUT * HID + 4 * lane + j], gs[j]);
+    if ((lane & 3) == 0) atomicAdd(&sg[OUT * HID + HID + c], gb);
+    l = (lane & 3) == 0 ? l : 0.0;
     for (int o = 16; o; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, l / (double)(n * NOUT));
+    if (lane == 0) atomicAdd(loss, l / (double)(n * NOUT));
+    __syncthreads();
+    for (int i = threadIdx.x; i < OUT * HID; i += blockDim.x) atomicAdd(&gW4[i], sg[i]);
+    if (threadIdx.x < HID) atomicAdd(&gb3[threadIdx.x], sg[OUT * HID + threadIdx.x]);
+    if (threadIdx.x < OUT) atomicAdd(&gb4[threadIdx.x], sg[OUT * HID + HID + threadIdx.x]);
+}
+
+// A training kernel (they begin with step_enter): its launch overlaps the kernel before it.
+template <typename... Ex, typename... Act>
+static void launch_net(cudaStream_t s, void (*kernel)(Ex...), long long grid, unsigned block, size_t smem, Act&&... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<Act>(args)...);
 }
 
 __global__ void k_adam(long long n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
@@ -919,6 +1101,7 @@ struct mpm_net {
     float* scratch = nullptr;
     size_t scratch_bytes = 0;
     unsigned* err = nullptr;
+    void* h_result = nullptr;  // pinned: mpm_net_loss_grad's gradient and loss
     float in_inv_scale[NIN];
     float out_scale[NOUT], out_shift[NOUT];
     bool packed = false;
@@ -1005,40 +1188,54 @@ static int pack_weights(mpm_net* net) {
     return MPM_OK;
 }
 
-// forward pass on normalised rows x (n x 16) with the FP32 kernels; y (n x 8);
-// z1..z3/h1..h3 scratch (n x 128 each)
-static void forward_fp32(mpm_net* net, cudaStream_t s, long long n, const float* x, float* z1, float* h1, float* z2,
-                         float* h2, float* z3, float* h3, float* y) {
+// the hidden layers on normalised rows x (n x 16): h1..h3 (n x 128 each)
+static void hidden_fp32(mpm_net* net, cudaStream_t s, long long n, const float* x, float* h1, float* h2, float* h3) {
     const float* p = net->p;
-    sgemm<false, true, EPI_RELU>(s, (int)n, HID, IN, x, IN, p + OW1, IN, h1, HID, p + OB1, z1);
-    sgemm<false, true, EPI_RELU>(s, (int)n, HID, HID, h1, HID, p + OW2, HID, h2, HID, p + OB2, z2);
-    sgemm<false, true, EPI_RELU>(s, (int)n, HID, HID, h2, HID, p + OW3, HID, h3, HID, p + OB3, z3);
-    sgemm<false, true, EPI_STORE>(s, (int)n, OUT, HID, h3, HID, p + OW4, HID, y, OUT, p + OB4);
+    const float* none = nullptr;
+    float* no_sums = nullptr;
+    const long long tiles = (n + 127) / 128;
+    launch_net(s, k_layer<true, IN>, tiles, GT, sizeof(GemmTile), (int)n, x, p + OW1, p + OB1, none, h1, no_sums);
+    launch_net(s, k_layer<true, HID>, tiles, GT, sizeof(GemmTile), (int)n, (const float*)h1, p + OW2, p + OB2, none, h2,
+               no_sums);
+    launch_net(s, k_layer<true, HID>, tiles, GT, sizeof(GemmTile), (int)n, (const float*)h2, p + OW3, p + OB3, none, h3,
+               no_sums);
 }
 
-// gradient of the loss into g (NPARAM, zeroed here); dy already holds dL/dy
-static void backward_fp32(mpm_net* net, cudaStream_t s, long long n, const float* x, const float* z1,
-                          const float* h1, const float* z2, const float* h2, const float* z3, const float* h3,
-                          const float* dy, float* d1, float* d2, float* g) {
+static long long head_blocks(const mpm_net* net, long long n) {
+    return std::max(1LL, std::min<long long>(net->sm_count, (n + HEAD_WARPS - 1) / HEAD_WARPS));
+}
+
+// forward pass on normalised rows x; y (n x 8)
+static void forward_fp32(mpm_net* net, cudaStream_t s, long long n, const float* x, float* h1, float* h2, float* h3,
+                         float* y) {
+    hidden_fp32(net, s, n, x, h1, h2, h3);
     const float* p = net->p;
+    launch_net(s, k_head<false>, head_blocks(net, n) * 2, HEAD_WARPS * 32, 0, n, (const float*)h3, p + OW4, p + OB4,
+               (const float*)nullptr, y, (float*)nullptr, (float*)nullptr, (float*)nullptr, (float*)nullptr,
+               (double*)nullptr);
+}
+
+// loss (added to *loss) and its gradient into g (NPARAM, zeroed here) on rows x, t; h1..h3, da, db scratch (n x 128)
+static void loss_grad_fp32(mpm_net* net, cudaStream_t s, long long n, const float* x, const float* t, float* h1,
+                           float* h2, float* h3, float* da, float* db, float* g, double* loss) {
+    const float* p = net->p;
+    const float* none = nullptr;
     cudaMemsetAsync(g, 0, NPARAM * 4, s);
-    const int splits = (int)std::max(1LL, std::min(256LL, n / 256));
-    const unsigned cb = (unsigned)((n + 1023) / 1024);
-    // layer 4
-    sgemm<true, false, EPI_ATOMIC>(s, OUT, HID, (int)n, dy, OUT, h3, HID, g + OW4, HID, nullptr, nullptr, splits);
-    k_colsum<OUT><<<cb, 256, 0, s>>>(n, dy, g + OB4);
-    sgemm<false, false, EPI_DRELU>(s, (int)n, HID, OUT, dy, OUT, p + OW4, HID, d1, HID, nullptr, (float*)z3);
-    // layer 3
-    sgemm<true, false, EPI_ATOMIC>(s, HID, HID, (int)n, d1, HID, h2, HID, g + OW3, HID, nullptr, nullptr, splits);
-    k_colsum<HID><<<cb, 256, 0, s>>>(n, d1, g + OB3);
-    sgemm<false, false, EPI_DRELU>(s, (int)n, HID, HID, d1, HID, p + OW3, HID, d2, HID, nullptr, (float*)z2);
-    // layer 2
-    sgemm<true, false, EPI_ATOMIC>(s, HID, HID, (int)n, d2, HID, h1, HID, g + OW2, HID, nullptr, nullptr, splits);
-    k_colsum<HID><<<cb, 256, 0, s>>>(n, d2, g + OB2);
-    sgemm<false, false, EPI_DRELU>(s, (int)n, HID, HID, d2, HID, p + OW2, HID, d1, HID, nullptr, (float*)z1);
-    // layer 1
-    sgemm<true, false, EPI_ATOMIC>(s, HID, IN, (int)n, d1, HID, x, IN, g + OW1, IN, nullptr, nullptr, splits);
-    k_colsum<HID><<<cb, 256, 0, s>>>(n, d1, g + OB1);
+    hidden_fp32(net, s, n, x, h1, h2, h3);
+    launch_net(s, k_head<true>, head_blocks(net, n), HEAD_WARPS * 32, 0, n, (const float*)h3, p + OW4, p + OB4, t,
+               (float*)nullptr, da, g + OW4, g + OB4, g + OB3, loss);
+    // the weight gradients' rows over two blocks per SM, whole slices each
+    const long long blocks = 2LL * net->sm_count;
+    const int rows = (int)(((n + blocks - 1) / blocks + GK - 1) / GK * GK);
+    const long long wb = (n + rows - 1) / rows, tiles = (n + 127) / 128;
+    const size_t sm = sizeof(GemmTile);
+    launch_net(s, k_weight_grad<HID>, wb, GT, sm, (int)n, rows, (const float*)da, (const float*)h2, g + OW3);
+    launch_net(s, k_layer<false, HID>, tiles, GT, sm, (int)n, (const float*)da, p + OW3, none, (const float*)h2, db,
+               g + OB2);
+    launch_net(s, k_weight_grad<HID>, wb, GT, sm, (int)n, rows, (const float*)db, (const float*)h1, g + OW2);
+    launch_net(s, k_layer<false, HID>, tiles, GT, sm, (int)n, (const float*)db, p + OW2, none, (const float*)h1, da,
+               g + OB1);
+    launch_net(s, k_weight_grad<IN>, wb, GT, sm, (int)n, rows, (const float*)da, x, g + OW1);
 }
 
 extern "C" {
@@ -1115,6 +1312,7 @@ void mpm_net_destroy(mpm_net* net) {
     if (net->wpack) cudaFree(net->wpack);
     if (net->scratch) cudaFree(net->scratch);
     if (net->err) cudaFree(net->err);
+    if (net->h_result) cudaFreeHost(net->h_result);
     delete net;
 }
 
@@ -1143,34 +1341,35 @@ int mpm_net_scales(mpm_net* net, double in_scale[13], double out_scale[7], doubl
 
 int mpm_net_loss_grad(mpm_net* net, const float* x, const float* t, int64_t n, float* grad, double* loss) {
     if (!net || !x || !t || !grad || n < 1) return MPM_ERR_ARG;
-    const size_t fb = 4;
-    const size_t need = fb * ((size_t)n * (IN + OUT + OUT + OUT) + (size_t)n * HID * 8 + NPARAM) + 64;
+    const size_t need = 4 * ((size_t)n * (IN + OUT) + (size_t)n * HID * 5 + NPARAM) + 64;
     int rc = ensure_scratch(net, need);
     if (rc) return rc;
+    // gradient and loss come back in one copy, through a pinned buffer
+    constexpr size_t RESULT = (NPARAM * 4 + 15) / 16 * 16 + 8;
+    if (!net->h_result && cudaMallocHost(&net->h_result, RESULT) != cudaSuccess) {
+        cudaGetLastError();
+        net->h_result = nullptr;
+        return MPM_ERR_NOMEM;
+    }
     float* xs = net->scratch;
     float* ts = xs + n * IN;
-    float* y = ts + n * OUT;
-    float* dy = y + n * OUT;
-    float* z1 = dy + n * OUT;
-    float* h1 = z1 + n * HID;
-    float* z2 = h1 + n * HID;
-    float* h2 = z2 + n * HID;
-    float* z3 = h2 + n * HID;
-    float* h3 = z3 + n * HID;
+    float* h1 = ts + n * OUT;
+    float* h2 = h1 + n * HID;
+    float* h3 = h2 + n * HID;
     float* d1 = h3 + n * HID;
     float* d2 = d1 + n * HID;
     float* g = d2 + n * HID;
-    double* dl = reinterpret_cast<double*>(((uintptr_t)(g + NPARAM) + 7) & ~(uintptr_t)7);
+    double* dl = reinterpret_cast<double*>(g + (RESULT - 8) / 4);
     cudaStream_t s = 0;
     NCK(cudaMemcpy(xs, x, (size_t)n * IN * 4, cudaMemcpyHostToDevice));
     NCK(cudaMemcpy(ts, t, (size_t)n * OUT * 4, cudaMemcpyHostToDevice));
-    NCK(cudaMemset(dl, 0, 8));
-    forward_fp32(net, s, n, xs, z1, h1, z2, h2, z3, h3, y);
-    k_loss<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, y, ts, dy, dl);
-    backward_fp32(net, s, n, xs, z1, h1, z2, h2, z3, h3, dy, d1, d2, g);
+    NCK(cudaMemsetAsync(dl, 0, 8, s));
+    loss_grad_fp32(net, s, n, xs, ts, h1, h2, h3, d1, d2, g, dl);
     NCK(cudaGetLastError());
-    NCK(cudaMemcpy(grad, g, NPARAM * 4, cudaMemcpyDeviceToHost));
-    if (loss) NCK(cudaMemcpy(loss, dl, 8, cudaMemcpyDeviceToHost));
+    NCK(cudaMemcpyAsync(net->h_result, g, RESULT, cudaMemcpyDeviceToHost, s));
+    NCK(cudaStreamSynchronize(s));
+    memcpy(grad, net->h_result, NPARAM * 4);
+    if (loss) memcpy(loss, (const char*)net->h_result + RESULT - 8, 8);
     return MPM_OK;
 }
 
@@ -1252,7 +1451,7 @@ static int train_impl(mpm_net* net, const float* d_rows, long long n_rows, mpm_n
     auto t1 = std::chrono::steady_clock::now();
     r.seconds_generate = std::chrono::duration<double>(t1 - t0).count();
     // training buffers
-    const size_t need = 4 * ((size_t)B * (IN + 3 * OUT) + (size_t)B * HID * 8 + 3 * NPARAM) + 1024;
+    const size_t need = 4 * ((size_t)B * (IN + 2 * OUT) + (size_t)B * HID * 5 + 3 * NPARAM) + 1024;
     int rc = ensure_scratch(net, need);
     if (rc) {
         freeall();
@@ -1263,13 +1462,9 @@ static int train_impl(mpm_net* net, const float* d_rows, long long n_rows, mpm_n
     float* xb = net->scratch;
     float* tb = xb + B * IN;
     float* y = tb + B * OUT;
-    float* dy = y + B * OUT;
-    float* z1 = dy + B * OUT;
-    float* h1 = z1 + B * HID;
-    float* z2 = h1 + B * HID;
-    float* h2 = z2 + B * HID;
-    float* z3 = h2 + B * HID;
-    float* h3 = z3 + B * HID;
+    float* h1 = y + B * OUT;
+    float* h2 = h1 + B * HID;
+    float* h3 = h2 + B * HID;
     float* d1 = h3 + B * HID;
     float* d2 = d1 + B * HID;
     float* g = d2 + B * HID;
@@ -1289,9 +1484,7 @@ static int train_impl(mpm_net* net, const float* d_rows, long long n_rows, mpm_n
         cudaMemsetAsync(acc + 32, 0, 8, s);
         for (long long b = 0; b < per_epoch; ++b, ++step) {
             k_gather<<<(unsigned)((B + 255) / 256), 256, 0, s>>>(n, x, tn, a, cc, b * B, (int)B, xb, tb);
-            forward_fp32(net, s, B, xb, z1, h1, z2, h2, z3, h3, y);
-            k_loss<<<(unsigned)((B + 255) / 256), 256, 0, s>>>(B, y, tb, dy, acc + 32);
-            backward_fp32(net, s, B, xb, z1, h1, z2, h2, z3, h3, dy, d1, d2, g);
+            loss_grad_fp32(net, s, B, xb, tb, h1, h2, h3, d1, d2, g, acc + 32);
             // Adam, cosine-decayed step size after a short warm-up
             const double tt = (double)(step + 1);
             const double warm = std::min(1.0, tt / (double)std::max(1LL, std::min(200LL, total / 10)));
@@ -1330,7 +1523,7 @@ static int train_impl(mpm_net* net, const float* d_rows, long long n_rows, mpm_n
         unsigned* maxbits = reinterpret_cast<unsigned*>(acc + 8);
         for (long long o = 0; o < nval; o += chunk) {
             const long long m = std::min(chunk, nval - o);
-            forward_fp32(net, s, m, xv + o * IN, z1, h1, z2, h2, z3, h3, y);
+            forward_fp32(net, s, m, xv + o * IN, h1, h2, h3, y);
             k_val_errors<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(m, y, tv + o * OUT, dvec, dvec + NOUT,
                                                                     (float)(1.0 / c.yield), 0.02f, acc, maxbits);
         }
@@ -1411,17 +1604,14 @@ int mpm_net_infer(mpm_net* net, const float* d_in, float* d_out, int64_t n, int 
     }
     // FP32 reference: normalise, the training forward pass in chunks, de-normalise
     const long long chunk = std::min<long long>(n, 1 << 20);
-    const size_t need = 4 * ((size_t)chunk * (IN + OUT) + (size_t)chunk * HID * 6 + 2 * NIN + 2 * NOUT) + 256;
+    const size_t need = 4 * ((size_t)chunk * (IN + OUT) + (size_t)chunk * HID * 3 + 2 * NIN + 2 * NOUT) + 256;
     int rc = ensure_scratch(net, need);
     if (rc) return rc;
     float* x = net->scratch;
     float* y = x + chunk * IN;
-    float* z1 = y + chunk * OUT;
-    float* h1 = z1 + chunk * HID;
-    float* z2 = h1 + chunk * HID;
-    float* h2 = z2 + chunk * HID;
-    float* z3 = h2 + chunk * HID;
-    float* h3 = z3 + chunk * HID;
+    float* h1 = y + chunk * OUT;
+    float* h2 = h1 + chunk * HID;
+    float* h3 = h2 + chunk * HID;
     float* sc = h3 + chunk * HID;
     float hs[NIN + 2 * NOUT];
     for (int c = 0; c < NIN; ++c) hs[c] = net->in_inv_scale[c];
@@ -1433,7 +1623,7 @@ int mpm_net_infer(mpm_net* net, const float* d_in, float* d_out, int64_t n, int 
     for (long long o = 0; o < n; o += chunk) {
         const long long m = std::min(chunk, n - o);
         k_norm_inputs<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(m, d_in + o * NIN, sc, x);
-        forward_fp32(net, s, m, x, z1, h1, z2, h2, z3, h3, y);
+        forward_fp32(net, s, m, x, h1, h2, h3, y);
         k_denorm_outputs<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(m, y, sc + NIN, sc + NIN + NOUT,
                                                                      d_in + o * NIN, net->mat, d_out + o * NOUT);
     }
