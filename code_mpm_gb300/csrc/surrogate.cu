@@ -225,7 +225,7 @@ __global__ void k_normalise_targets(long long n, const float* __restrict__ t, co
 // 16-deep slice on its way to registers while the current one is used.  Before,
 // with 64 x 64 tiles, 4 x 4 outputs, no overlap, stored pre-activations and
 // separate kernels for layer 4, the loss and the column sums, a batch of 65,536
-// took 928 us through mpm_net_loss_grad, 1,000 rows 340 us; now 476 and 146.
+// took 928 us through mpm_net_loss_grad, 1,000 rows 340 us; now 449 and 140.
 // ---------------------------------------------------------------------------
 constexpr int GT = 256;       // threads
 constexpr int GK = 16;        // slice depth
@@ -235,19 +235,26 @@ struct GemmTile {
     float a[2][GK][GS], b[2][GK][GS];
 };
 
-// acc[i][j]: rows ty * 4 + (i & 3) + 64 (i >> 2), columns tx * 4 + (j & 3) + 64 (j >> 2)
+// acc[i][j]: rows ty * 4 + (i & 3) + 64 (i >> 2), columns tx * 4 + (j & 3) + 64 (j >> 2).  Two columns per
+// instruction (fma.rn.f32x2, the same roundings as two fmaf): half the issue slots beside the shared loads.
 __device__ __forceinline__ void tile_fma(const GemmTile& s, int buf, int ty, int tx, float acc[8][8]) {
+    unsigned long long (*acc2)[4] = reinterpret_cast<unsigned long long (*)[4]>(acc);
 #pragma unroll
     for (int k = 0; k < GK; ++k) {
-        float a[8], b[8];
+        float a[8];
+        unsigned long long b[4];
         *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&s.a[buf][k][4 * ty]);
         *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&s.a[buf][k][64 + 4 * ty]);
-        *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(&s.b[buf][k][4 * tx]);
-        *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(&s.b[buf][k][64 + 4 * tx]);
+        const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&s.b[buf][k][4 * tx]);
+        const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(&s.b[buf][k][64 + 4 * tx]);
+        b[0] = b0.x, b[1] = b0.y, b[2] = b1.x, b[3] = b1.y;
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < 8; ++i) {
+            unsigned long long aa;
+            asm("mov.b64 %0, {%1, %1};" : "=l"(aa) : "f"(a[i]));
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+            for (int j = 0; j < 4; ++j) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc2[i][j]) : "l"(aa), "l"(b[j]));
+        }
     }
 }
 
@@ -290,7 +297,7 @@ __global__ void __launch_bounds__(GT, 2) k_layer(int n, const float* __restrict_
             }
         }
     };
-    float acc[8][8] = {};
+    __align__(8) float acc[8][8] = {};
     load(0);
     store(0);
     __syncthreads();
@@ -372,7 +379,7 @@ __global__ void __launch_bounds__(GT, 2) k_weight_grad(int n, int rows, const fl
         }
         if (N == IN && tid < 64) *reinterpret_cast<float4*>(&s.b[buf][tid >> 2][(tid & 3) * 4]) = rx[0];
     };
-    float acc[8][8] = {};  // N = 16: acc[i][0] of column tx
+    __align__(8) float acc[8][8] = {};  // N = 16: acc[i][0] of column tx
     load(beg);
     store(0);
     __syncthreads();
