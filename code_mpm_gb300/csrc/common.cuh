@@ -159,6 +159,7 @@ struct MatConst {
     double C;      // E/(1+nu)/(1-2nu)
     double one_m_nu, half_m_nu;
     double G;      // 0.5*E/(1+nu)
+    double lam, two_G;  // C nu, 2 G
     double k0;     // Y/sqrt(3)
     double s23C1;  // sqrt(2/3)*C1
     double inv_E, nu_over_E, inv_G;
@@ -168,6 +169,8 @@ struct MatConst {
 };
 
 inline void set_float_constants(MatConst& k) {
+    k.lam = k.C * k.nu;
+    k.two_G = 2.0 * k.G;
     k.fC = (float)k.C;
     k.fone_m_nu = (float)k.one_m_nu;
     k.fnu = (float)k.nu;

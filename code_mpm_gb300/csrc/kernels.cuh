@@ -508,8 +508,9 @@ struct P2GBlock {
             for (int c = 0; c < 3; ++c) {
                 const T X0 = quad_shfl(fx[c], quad + 2 * b), X1 = quad_shfl(fx[c], quad + 2 * b + 1);
                 const T Y0 = quad_shfl(fy[c], quad + 2 * a), Y1 = quad_shfl(fy[c], quad + 2 * a + 1);
-                p0[c] = e0[c] + (hx * X0 + hy * Y0 - hz * fz[c]);
-                p1[c] = e1[c] + (hx * X1 + hy * Y1 + hz * fz[c]);
+                p0[c] = hx * X0 + hy * Y0 - hz * fz[c];
+                p1[c] = hx * X1 + hy * Y1 + hz * fz[c];
+                if constexpr (FE) p0[c] += e0[c], p1[c] += e1[c];
             }
             if constexpr (MG) {
                 g0[0] = hx * quad_shfl(mx, quad + 2 * b), g1[0] = hx * quad_shfl(mx, quad + 2 * b + 1);
@@ -747,8 +748,7 @@ __device__ __forceinline__ void grid_update_regs(const NView<T>& nd, long long i
 template <typename T, int BATCH>
 __global__ void __launch_bounds__(256) k_pass1_remap(PView<T> P, NView<T> nd, Geom g,
                                                      const unsigned* __restrict__ skeys,
-                                                     const unsigned* __restrict__ perm, long long n, T dt,
-                                                     T mass_min, int contact) {
+                                                     const unsigned* __restrict__ perm, long long n, int contact) {
     step_enter<sizeof(T) == 4>();
     long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     unsigned key = (s < n) ? skeys[s] : 0xffffffffu;
@@ -790,9 +790,9 @@ __global__ void __launch_bounds__(256) k_pass1_remap(PView<T> P, NView<T> nd, Ge
                 if (!(r[k].w != (T)0)) continue;  // out of range or m <= mass_min
                 T N, G[3];
                 B.corner(k, N, G);
-                v[0] = v[0] + N * r[k].x * dt;
-                v[1] = v[1] + N * r[k].y * dt;
-                v[2] = v[2] + N * r[k].z * dt;
+                v[0] = v[0] + N * r[k].x;
+                v[1] = v[1] + N * r[k].y;
+                v[2] = v[2] + N * r[k].z;
             }
         } else {
 #pragma unroll 1
@@ -803,9 +803,9 @@ __global__ void __launch_bounds__(256) k_pass1_remap(PView<T> P, NView<T> nd, Ge
                 if (!(r.w != (T)0)) continue;
                 T N, G[3];
                 B.corner(k, N, G);
-                v[0] = v[0] + N * r.x * dt;
-                v[1] = v[1] + N * r.y * dt;
-                v[2] = v[2] + N * r.z * dt;
+                v[0] = v[0] + N * r.x;
+                v[1] = v[1] + N * r.y;
+                v[2] = v[2] + N * r.z;
             }
         }
 #pragma unroll
@@ -855,7 +855,7 @@ __host__ __device__ constexpr size_t pass1_cells_smem(int bs) {
 template <typename T, int CPT, int BS>
 __global__ void __launch_bounds__(BS, sizeof(T) == 4 && CPT < 4 ? 1536 / BS : 1) k_pass1_cells(PView<T> P, NView<T> nd, Geom g,
                                                      const unsigned* __restrict__ skeys,
-                                                     const unsigned* __restrict__ perm, long long n, T dt, int contact) {
+                                                     const unsigned* __restrict__ perm, long long n, int contact) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int bs = BS;
     const int t = threadIdx.x;
@@ -885,7 +885,6 @@ __global__ void __launch_bounds__(BS, sizeof(T) == 4 && CPT < 4 ? 1536 / BS : 1)
             particle_bases<T>(P, gs, p, b, B);
             const T m = P.mass[p];
             T v[3] = {P.vel[p], P.vel[np + p], P.vel[2 * np + p]};
-            T dv[3] = {0, 0, 0};
             // four corners' records requested before any is used; summed in corner order
 #pragma unroll(F32 ? 2 : 1)
             for (int h = 0; h < 2; ++h) {
@@ -900,14 +899,13 @@ __global__ void __launch_bounds__(BS, sizeof(T) == 4 && CPT < 4 ? 1536 / BS : 1)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const T N = nx * ((j & 2) ? B.Ny[1] : B.Ny[0]) * ((j & 1) ? B.Nz[1] : B.Nz[0]);
-                    dv[0] += N * rq[j].x;
-                    dv[1] += N * rq[j].y;
-                    dv[2] += N * rq[j].z;
+                    v[0] += N * rq[j].x;
+                    v[1] += N * rq[j].y;
+                    v[2] += N * rq[j].z;
                 }
             }
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                v[c] += dv[c] * dt;
                 P.vel[c * np + p] = v[c];
                 mv[c] = m * v[c];
             }
@@ -999,7 +997,8 @@ __device__ __forceinline__ void node_dc_regs(const unsigned own[3], const unsign
 // the node's values in registers: displacement control (non-contact: before
 // the update, …MPLocks.cpp:143-174), the grid update (IntegrateGrid, :90-142;
 // contact :242-277), displacement control (contact: after it), then the
-// record (f/m, m > m_min), the divisor of G2P pass 1 (:508).  The updated
+// record (dt f/m, m > m_min), G2P pass 1's increment (:508; the factor dt is
+// taken here once per node instead of in every particle).  The updated
 // momentum and the mass also go to the record's second half for phase B
 // (which overwrites it with p/m and v); clean (not an output step): the
 // node's mass, momentum and force are zeroed here, for the next step's P2G.
@@ -1097,9 +1096,9 @@ __global__ void __launch_bounds__(256, 4) k_node_phase_a(NView<T> nd, T dt, doub
         if (fx & 2u) nd.ftemp[nn + i] += ft_y;
         const bool has = m > mass_min;
         Quad<T> r, pm;
-        r.x = has ? f[0] / m : (T)0;
-        r.y = has ? f[1] / m : (T)0;
-        r.z = has ? f[2] / m : (T)0;
+        r.x = has ? f[0] / m * dt : (T)0;
+        r.y = has ? f[1] / m * dt : (T)0;
+        r.z = has ? f[2] / m * dt : (T)0;
         r.w = has ? (T)1 : (T)0;
         pm.x = p[0];
         pm.y = p[1];
@@ -1114,14 +1113,15 @@ __global__ void __launch_bounds__(256, 4) k_node_phase_a(NView<T> nd, T dt, doub
 
 // The node work between pass 1 and pass 2, in registers: the remap v += q/m
 // (:559-560; phase A cleared q before pass 1 summed it), displacement
-// control and BC (:573-599) in the path's order, then the record (p/m,
-// m > m_min, v).  The claims are cleared after this last use (every claimed
+// control and BC (:573-599) in the path's order, then the record (dt p/m,
+// m > m_min, dt v: the displacement and the velocity gradient that pass 2
+// gathers carry the factor dt).  The claims are cleared after this last use (every claimed
 // node is active: platen particles take part in P2G).  clean: a step whose
 // node values nobody sees (not the last of an advance; pass 2 reads only the
 // records) leaves the node zeroed as the next step's grid reset would
 // (ResetGrid, …MPLocks.cpp:4-22), so that step needs no reset pass.
 template <typename T>
-__global__ void __launch_bounds__(256, 4) k_node_phase_b(NView<T> nd, int contact, const unsigned* __restrict__ dclist, int ndc,
+__global__ void __launch_bounds__(256, 4) k_node_phase_b(NView<T> nd, T dt, int contact, const unsigned* __restrict__ dclist, int ndc,
                                const T* __restrict__ pvel, long long np, T mass_min, int clean, int vel_zero) {
     step_enter<sizeof(T) == 4>();
     const long long nn = nd.nn;
@@ -1168,13 +1168,13 @@ __global__ void __launch_bounds__(256, 4) k_node_phase_b(NView<T> nd, int contac
         }
         if (contact) node_dc_regs<T>(own, dclist, pvel, np, m, v, vset, p, fz);
         Quad<T> r, vq;
-        r.x = has ? p[0] / m : (T)0;
-        r.y = has ? p[1] / m : (T)0;
-        r.z = has ? p[2] / m : (T)0;
+        r.x = has ? p[0] / m * dt : (T)0;
+        r.y = has ? p[1] / m * dt : (T)0;
+        r.z = has ? p[2] / m * dt : (T)0;
         r.w = has ? (T)1 : (T)0;
-        vq.x = v[0];
-        vq.y = v[1];
-        vq.z = v[2];
+        vq.x = v[0] * dt;
+        vq.y = v[1] * dt;
+        vq.z = v[2] * dt;
         vq.w = (T)0;
         *reinterpret_cast<Quad<T>*>(nd.rec + 8 * i) = r;
         *reinterpret_cast<Quad<T>*>(nd.rec + 8 * i + 4) = vq;
@@ -1493,7 +1493,7 @@ __device__ __forceinline__ void pass2_prefetch(const PView<T>& P, long long p0, 
 // F = F dF, and stress = Kirchhoff / det F.  Energies add stress x increment x
 // V component by component, as the reference does.
 template <typename T>
-__device__ __forceinline__ void large_strain_update(const PView<T>& P, long long p, const T Lt[9], double dt,
+__device__ __forceinline__ void large_strain_update(const PView<T>& P, long long p, const T Ldt[9],
                                                     const MatConst* __restrict__ mats, int nmat, unsigned* err) {
     if constexpr (sizeof(T) == 8) {
         const long long np = P.n;
@@ -1503,7 +1503,7 @@ __device__ __forceinline__ void large_strain_update(const PView<T>& P, long long
 #pragma unroll
         for (int c = 0; c < 3; ++c)
 #pragma unroll
-            for (int r = 0; r < 3; ++r) dF[3 * c + r] = (c == r ? 1.0 : 0.0) + (double)Lt[3 * c + r] * dt;
+            for (int r = 0; r < 3; ++r) dF[3 * c + r] = (c == r ? 1.0 : 0.0) + (double)Ldt[3 * c + r];
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
             F[k] = P.F[k * np + p];
@@ -1576,9 +1576,9 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
     double x[3] = {src.pos(P, 0, p), src.pos(P, 1, p), src.pos(P, 2, p)};
     if (!skip) {
         const unsigned key = src.key(keys, p);
-        T L[9];
+        T Ldt[9];  // velocity gradient times dt
 #pragma unroll
-        for (int k = 0; k < 9; ++k) L[k] = 0;
+        for (int k = 0; k < 9; ++k) Ldt[k] = 0;
         if (key < g.key_max) {
             int b[3];
             key_to_base(key, gs, b);
@@ -1595,7 +1595,7 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
             // -(Bx Nz, By Nz, A gz), so
             //   disp += A (Nz r), L_x -= Bx (Nz v), L_y -= By (Nz v), L_z -= A (gz v):
             // 132 products and sums per particle instead of 168 corner by
-            // corner.  FP32 form: the displacement sum is formed in FP32 and
+            // corner.  The records carry the factor dt.  FP32 form: the displacement sum is formed in FP32 and
             // added to the FP64 position once.  FP64 form (bound by its FP64
             // pipe): added per corner in the reference's order
             // (…MPLocks.cpp:197-198), so positions keep its last bits, on
@@ -1623,28 +1623,25 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
                     if constexpr (sizeof(T) == 4) {
                         disp[c] += A * (B.Nz[0] * r0[c] + B.Nz[1] * r1[c]);
                     } else {
-                        x[c] = x[c] + (A * B.Nz[0] * r0[c]) * a.dt;
-                        x[c] = x[c] + (A * B.Nz[1] * r1[c]) * a.dt;
+                        x[c] = x[c] + A * B.Nz[0] * r0[c];
+                        x[c] = x[c] + A * B.Nz[1] * r1[c];
                     }
                     // outerProduct(v_i, grad N): column c, row r = v_i[r] * G[c]
-                    L[c] -= Bx * w;
-                    L[3 + c] -= By * w;
-                    L[6 + c] -= A * d;
+                    Ldt[c] -= Bx * w;
+                    Ldt[3 + c] -= By * w;
+                    Ldt[6 + c] -= A * d;
                 }
             }
             if constexpr (sizeof(T) == 4) {
 #pragma unroll
-                for (int c = 0; c < 3; ++c) x[c] += fps_f2d(disp[c] * dt);
+                for (int c = 0; c < 3; ++c) x[c] += fps_f2d(disp[c]);
             }
         }
         if constexpr (LS) {
-            large_strain_update(P, p, L, (double)dt, mats, nmat, err);
+            large_strain_update(P, p, Ldt, mats, nmat, err);
         } else {
         // strain increment: diagonal from dF = I + L dt (form-specific, see
         // Kinematics), off-diagonal (L_ij + L_ji) dt in Voigt engineering shear
-        T Ldt[9];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) Ldt[k] = L[k] * dt;
         T e[6];
         e[0] = Kinematics<T>::strain_diag(Ldt[0]);
         e[1] = Kinematics<T>::strain_diag(Ldt[4]);

@@ -251,7 +251,15 @@ struct CrTrial {
 
 template <typename T>
 __device__ __forceinline__ void cr_trial(const MatConst& m, T R, const T sig[6], const T e[6], CrTrial<T>& t) {
-    trial_increment<T>(m, e, t.dtr);
+    if constexpr (sizeof(T) == 8) {  // D de as lambda tr + 2G de: 9 operations on the FP64 pipe instead of 18
+        const T l = m.lam * (e[0] + e[1] + e[2]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) t.dtr[i] = m.two_G * e[i] + l;
+#pragma unroll
+        for (int i = 3; i < 6; ++i) t.dtr[i] = m.G * e[i];
+    } else {
+        trial_increment<T>(m, e, t.dtr);
+    }
     if (m.type == 0) return;
 #pragma unroll
     for (int i = 0; i < 6; ++i) t.tr[i] = sig[i] + t.dtr[i];
