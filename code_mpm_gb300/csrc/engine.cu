@@ -1069,9 +1069,11 @@ int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
                            ns);
                 LAUNCH("contact_compact", k_contact_compact, blocks_for(nn), NTHREADS, (const unsigned*)c->g_need.p,
                        nn, (unsigned*)c->g_list.p, (unsigned*)c->g_count.p);
-                LAUNCH("contact_mass_gradient", k_contact_mass_gradient<T>, (unsigned)c->sm_count * 8, CG_WARPS * 32,
-                       P, N, g, (const unsigned*)c->g_list.p, (const unsigned*)c->g_count.p, perm,
-                       (const unsigned*)c->cstart.p, (const unsigned*)c->cend.p);
+                if constexpr (sizeof(T) == 8)
+                    LAUNCH_SMEM("contact_mass_gradient", k_contact_mass_gradient<T>, (unsigned)c->sm_count * 8,
+                                CG_WARPS * 32, sizeof(ContactScratch), P, N, g, (const unsigned*)c->g_list.p,
+                                (const unsigned*)c->g_count.p, perm, (const unsigned*)c->cstart.p,
+                                (const unsigned*)c->cend.p);
             }
             if (ns > 0)
                 LAUNCH("contact_mp_gradient", k_contact_mp_gradient<T>, sb, NTHREADS, P, N, g, keys, surf, ns);
@@ -1496,7 +1498,9 @@ int mpm_create_batch(const mpm_grid_desc* grids, int32_t nspec, int form, mpm_ct
     cudaGetDevice(&c->device);
     cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device);
     if (c->sm_count <= 0) c->sm_count = 152;
-    if (!cells_attrs<double>() || !cells_attrs<float>() || !pass2_staged_attr<128>() || !pass2_staged_attr<256>() || !pass2_staged_attr<512>() || !pairs_attr<128>() ||
+    if (cudaFuncSetAttribute(k_contact_mass_gradient<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(ContactScratch)) != cudaSuccess ||
+        !cells_attrs<double>() || !cells_attrs<float>() || !pass2_staged_attr<128>() || !pass2_staged_attr<256>() || !pass2_staged_attr<512>() || !pairs_attr<128>() ||
         !pairs_attr<256>() || !pairs_attr<512>()) {
         cudaGetLastError();
         delete c;

@@ -1899,11 +1899,16 @@ static __global__ void k_contact_compact(const unsigned* __restrict__ need, long
 
 // One warp per needed node: gather the slots of the eight surrounding cells'
 // particles into shared memory, rank them by the caller's particle index (the
-// slot itself when particles are not stored in cell order), compute each
-// pair's exact grad N * m in parallel, then add them in index order on one
-// lane.  Nodes with more than CG_CAP contributors take the selection below:
+// slot itself when particles are not stored in cell order), and compute each
+// pair's exact grad N * m in parallel.  The sums in index order are serial
+// chains of FP64 additions, each costing the pipe a whole warp's slot however
+// few its lanes: the block's first warp adds all of the block's nodes' chains
+// together, three lanes per node (one node's chain per warp before: 884 us for
+// the 406k-particle honeycombs, now 439, with exact_gradient's comparisons off the pipe).
+// Nodes with more than CG_CAP contributors take the selection below:
 // the warp looks for the next larger index among all of them, one at a time.
-constexpr int CG_WARPS = 4;
+constexpr int CG_WARPS = 8;
+static_assert(3 * CG_WARPS <= 32, "one warp adds the block's chains");
 constexpr int CG_CAP = 256;
 
 template <typename T>
@@ -1943,6 +1948,13 @@ __device__ __noinline__ void mass_gradient_select(const PView<T>& P, const Geom&
     }
 }
 
+struct ContactScratch {
+    double c[CG_WARPS][CG_CAP][3];    // contributions by rank
+    unsigned id[CG_WARPS][CG_CAP];    // the caller's index
+    unsigned total[CG_WARPS];         // ranked contributors
+    long long node[CG_WARPS];         // -1: the warp has no node, or has summed it itself
+};
+
 template <typename T>
 __global__ void __launch_bounds__(CG_WARPS * 32) k_contact_mass_gradient(PView<T> P, NView<T> nd, Geom g,
                                                                          const unsigned* __restrict__ list,
@@ -1950,88 +1962,89 @@ __global__ void __launch_bounds__(CG_WARPS * 32) k_contact_mass_gradient(PView<T
                                                                          const unsigned* __restrict__ perm,
                                                                          const unsigned* __restrict__ cstart,
                                                                          const unsigned* __restrict__ cend) {
-    __shared__ unsigned s_id[CG_WARPS][CG_CAP];  // the caller's index
-    __shared__ double s_c[CG_WARPS][CG_CAP][3];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ContactScratch& S = *reinterpret_cast<ContactScratch*>(smem_raw);
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long np = P.n, nn = nd.nn;
     const unsigned total_nodes = *count;
-    for (unsigned item = blockIdx.x * CG_WARPS + w; item < total_nodes; item += gridDim.x * CG_WARPS) {
-        const long long i = list[item];
-        const Geom& gs = node_geom(g, i);
-        const long long il = i - gs.node_off;
-        int node[3];
-        node[0] = (int)(il % gs.nn[0]);
-        node[1] = (int)((il / gs.nn[0]) % gs.nn[1]);
-        node[2] = (int)(il / ((long long)gs.nn[0] * gs.nn[1]));
-        // lanes 0..7: the eight surrounding cells (cell = node - {0,1}^3)
-        unsigned s0 = 0, len = 0;
-        if (lane < 8) {
-            int cb[3] = {node[0] - ((lane >> 2) & 1), node[1] - ((lane >> 1) & 1), node[2] - (lane & 1)};
-            unsigned key = gs.key_off + (unsigned)((cb[0] + 1) + gs.kd[0] * ((cb[1] + 1) + gs.kd[1] * (cb[2] + 1)));
-            s0 = cstart[key];
-            unsigned s1 = cend[key];
-            len = s1 > s0 ? s1 - s0 : 0u;
-        }
-        // exclusive offsets of the segments
-        unsigned off = len;
-#pragma unroll
-        for (int d = 1; d < 8; d <<= 1) {
-            unsigned o = __shfl_up_sync(FULL_MASK, off, d);
-            if (lane >= d) off += o;
-        }
-        const unsigned total = __shfl_sync(FULL_MASK, off, 7);
-        off -= len;
-        unsigned segs[8], offs[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            segs[k] = __shfl_sync(FULL_MASK, s0, k);
-            offs[k] = __shfl_sync(FULL_MASK, off, k);
-        }
-        double gsum[3] = {0.0, 0.0, 0.0};
-        if (total > (unsigned)CG_CAP) {
-            mass_gradient_select<T>(P, gs, node, perm, segs, offs, total, gsum);
-        } else {
-            for (unsigned e = lane; e < total; e += 32) {
-                int k = 0;
-#pragma unroll
-                for (int kk = 1; kk < 8; ++kk)
-                    if (e >= offs[kk]) k = kk;
-                s_id[w][e] = caller_index(P, perm[segs[k] + (e - offs[k])]);
+    for (unsigned first = blockIdx.x * CG_WARPS; first < total_nodes; first += gridDim.x * CG_WARPS) {
+        const unsigned item = first + w;
+        if (lane == 0) S.node[w] = -1;
+        if (item < total_nodes) {
+            const long long i = list[item];
+            const Geom& gs = node_geom(g, i);
+            const long long il = i - gs.node_off;
+            int node[3];
+            node[0] = (int)(il % gs.nn[0]);
+            node[1] = (int)((il / gs.nn[0]) % gs.nn[1]);
+            node[2] = (int)(il / ((long long)gs.nn[0] * gs.nn[1]));
+            // lanes 0..7: the eight surrounding cells (cell = node - {0,1}^3)
+            unsigned s0 = 0, len = 0;
+            if (lane < 8) {
+                int cb[3] = {node[0] - ((lane >> 2) & 1), node[1] - ((lane >> 1) & 1), node[2] - (lane & 1)};
+                unsigned key = gs.key_off + (unsigned)((cb[0] + 1) + gs.kd[0] * ((cb[1] + 1) + gs.kd[1] * (cb[2] + 1)));
+                s0 = cstart[key];
+                unsigned s1 = cend[key];
+                len = s1 > s0 ? s1 - s0 : 0u;
             }
-            __syncwarp();
-            for (unsigned e = lane; e < total; e += 32) {
-                const unsigned key = s_id[w][e];
-                int k = 0;
+            // exclusive offsets of the segments
+            unsigned off = len;
 #pragma unroll
-                for (int kk = 1; kk < 8; ++kk)
-                    if (e >= offs[kk]) k = kk;
-                const unsigned id = perm[segs[k] + (e - offs[k])];
-                unsigned rank = 0;
-                for (unsigned j = 0; j < total; ++j) rank += s_id[w][j] < key ? 1u : 0u;
-                double x[3] = {P.pos[id], P.pos[np + id], P.pos[2 * np + id]};
-                double G[3];
-                exact_gradient(gs, x, node, G);
-                const double m = (double)P.mass[id];
-                s_c[w][rank][0] = __dmul_rn(G[0], m);
-                s_c[w][rank][1] = __dmul_rn(G[1], m);
-                s_c[w][rank][2] = __dmul_rn(G[2], m);
+            for (int d = 1; d < 8; d <<= 1) {
+                unsigned o = __shfl_up_sync(FULL_MASK, off, d);
+                if (lane >= d) off += o;
             }
-            __syncwarp();
-            if (lane < 3) {
-                double acc = 0.0;
-                for (unsigned e = 0; e < total; ++e) acc = __dadd_rn(acc, s_c[w][e][lane]);
-                gsum[lane] = acc;
+            const unsigned total = __shfl_sync(FULL_MASK, off, 7);
+            off -= len;
+            unsigned segs[8], offs[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                segs[k] = __shfl_sync(FULL_MASK, s0, k);
+                offs[k] = __shfl_sync(FULL_MASK, off, k);
+            }
+            if (total > (unsigned)CG_CAP) {
+                double gsum[3] = {0.0, 0.0, 0.0};
+                mass_gradient_select<T>(P, gs, node, perm, segs, offs, total, gsum);
+                if (lane == 0) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) nd.mg[c * nn + i] = gsum[c];
+                }
+            } else {
+                auto slot_of = [&](unsigned e) {
+                    int k = 0;
+#pragma unroll
+                    for (int kk = 1; kk < 8; ++kk)
+                        if (e >= offs[kk]) k = kk;
+                    return perm[segs[k] + (e - offs[k])];
+                };
+                for (unsigned e = lane; e < total; e += 32) S.id[w][e] = caller_index(P, slot_of(e));
+                __syncwarp();
+                for (unsigned e = lane; e < total; e += 32) {
+                    const unsigned key = S.id[w][e], id = slot_of(e);
+                    unsigned rank = 0;
+                    for (unsigned j = 0; j < total; ++j) rank += S.id[w][j] < key ? 1u : 0u;
+                    double x[3] = {P.pos[id], P.pos[np + id], P.pos[2 * np + id]};
+                    double G[3];
+                    exact_gradient(gs, x, node, G);
+                    const double m = (double)P.mass[id];
+                    S.c[w][rank][0] = __dmul_rn(G[0], m);
+                    S.c[w][rank][1] = __dmul_rn(G[1], m);
+                    S.c[w][rank][2] = __dmul_rn(G[2], m);
+                }
+                if (lane == 0) {
+                    S.node[w] = i;
+                    S.total[w] = total;
+                }
             }
         }
-        if (total > (unsigned)CG_CAP) {
-            if (lane == 0) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) nd.mg[c * nn + i] = gsum[c];
-            }
-        } else if (lane < 3) {
-            nd.mg[lane * nn + i] = gsum[lane];
+        __syncthreads();
+        if (w == 0 && lane < 3 * CG_WARPS && S.node[lane / 3] >= 0) {
+            const int q = lane / 3, c = lane % 3;
+            double acc = 0.0;
+            for (unsigned e = 0; e < S.total[q]; ++e) acc = __dadd_rn(acc, S.c[q][e][c]);
+            nd.mg[c * nn + S.node[q]] = acc;
         }
-        __syncwarp();
+        __syncthreads();
     }
 }
 

@@ -120,24 +120,27 @@ __device__ __forceinline__ bool cell_and_local(const Geom& g, int a, double x, d
 // bit (contact mass gradients): correctly rounded d/h and the reference's
 // association order, with the _rn intrinsics so nothing is contracted.
 // ---------------------------------------------------------------------------
+// The comparisons and signs are taken on the bit patterns (non-negative
+// doubles order as their bits, a product by +-1 is a sign flip), which keeps
+// them off the FP64 pipe: 30 operations there instead of 54.
 __device__ __forceinline__ void exact_gradient(const Geom& g, const double x[3], const int node[3], double G[3]) {
-    double Nv[3], d[3], r[3];
+    const unsigned long long lo = fps_d2u(1.0e-12), hi = fps_d2u(1.0 - 1.0e-12), sign = 0x8000000000000000ull;
+    double Nv[3], d[3];
+    unsigned long long ar[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         d[a] = __dadd_rn(x[a], -node_coord(g, a, node[a]));
-        r[a] = div_rn_by(d[a], g.h[a], g.inv_h[a]);
-        double ar = r[a] >= 0.0 ? r[a] : -r[a];
-        Nv[a] = __dadd_rn(1.0, -ar);
-        if (Nv[a] < 0.0 || Nv[a] > 1.0) Nv[a] = 0.0;
+        ar[a] = fps_d2u(div_rn_by(d[a], g.h[a], g.inv_h[a])) & ~sign;
+        const double nv = __dadd_rn(1.0, -fps_u2d(ar[a]));
+        Nv[a] = (long long)fps_d2u(nv) < 0 ? 0.0 : nv;
     }
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        double ar = r[a] >= 0.0 ? r[a] : -r[a];
         G[a] = 0.0;
-        if (ar > 1.0e-12 && ar < 1.0 - 1.0e-12) {
-            double o1 = Nv[a == 0 ? 1 : 0], o2 = Nv[a == 2 ? 1 : 2];
-            double sg = (double)((d[a] > 0.0) - (d[a] < 0.0));
-            G[a] = div_rn_by(__dmul_rn(__dmul_rn(-o1, o2), sg), g.h[a], g.inv_h[a]);
+        if (ar[a] > lo && ar[a] < hi) {  // (so d is not zero)
+            const double o1 = Nv[a == 0 ? 1 : 0], o2 = Nv[a == 2 ? 1 : 2];
+            const unsigned long long w = fps_d2u(__dmul_rn(-o1, o2)) ^ (fps_d2u(d[a]) & sign);
+            G[a] = div_rn_by(fps_u2d(w), g.h[a], g.inv_h[a]);
         }
     }
 }
