@@ -109,7 +109,8 @@ struct mpm_ctx {
     long long launches = 0;
     const unsigned* last_perm = nullptr;
     const unsigned* last_skeys = nullptr;
-    bool keys_valid = false;  // keys_copy / keys[key_buf] / loc hold the keys of the current positions
+    bool keys_valid = false;  // keys[key_buf] / loc hold the keys of the current positions
+    bool copy_valid = false;  // and keys_copy, too
     int key_buf = 0;
     DevBuf loc;
     // return-map network (FP32 form)
@@ -667,6 +668,9 @@ int sort_cells(mpm_ctx* c, const unsigned** skeys_out, const unsigned** perm_out
         LAUNCH("cell_keys", k_cell_keys, blocks_for(n), NTHREADS, (const double*)c->pos.p, n, g, key_src,
                (unsigned*)nullptr, (unsigned*)c->keys_copy.p, err,
                c->form == MPM_FORM_FP32 ? (float*)c->loc.p : (float*)nullptr, sid);
+    else if (sort && !c->copy_valid)  // the last step took the storage order
+        CK(cudaMemcpyAsync(c->keys_copy.p, key_src, (size_t)n * 4, cudaMemcpyDeviceToDevice, c->stream));
+    c->copy_valid = c->copy_valid || sort || !c->keys_valid;
     if (!sort) {  // the slots in storage order with their keys (identity permutation)
         c->last_perm = nullptr;
         c->last_skeys = key_src;
@@ -745,7 +749,7 @@ int reorder(mpm_ctx* c) {
                   {&c->strain, 6, t},      {&c->eps_p, 6, t},     {&c->e_strain, 1, 8},   {&c->e_strain_max, 1, 8},
                   {&c->e_strain_ti, 1, 8}, {&c->e_plastic, 1, 8}, {&c->backstress, 1, t}, {&c->mp_mg, 3, t},
                   {&c->strain_rate, 6, t}, {&c->material, 1, 4},  {&c->pflags, 1, 1},     {&c->dc_mult, 1, 4},
-                  {&c->loc, 3, 4},         {&c->Fe, 9, 8},        {&c->keys_copy, 1, 4},  {&c->orig, 1, 4},
+                  {&c->loc, 3, 4},         {&c->Fe, 9, 8},        {&c->orig, 1, 4},
                   {&c->sid, 1, 2},         {&c->mon_mask, 1, 1}};
     const unsigned grid = (unsigned)std::min<long long>(blocks_for(n * 3), (long long)c->sm_count * 32);
     for (auto& f : fields) {
@@ -775,7 +779,9 @@ int reorder(mpm_ctx* c) {
     LAUNCH("reorder", k_iota, blocks_for(n), NTHREADS, ident, n);
     c->last_perm = ident;
     c->last_skeys = skeys;
+    CK(cudaMemcpyAsync(c->keys_copy.p, skeys, (size_t)n * 4, cudaMemcpyDeviceToDevice, c->stream));
     c->keys_valid = true;
+    c->copy_valid = true;
     CK(cudaGetLastError());
     return MPM_OK;
 }
@@ -967,7 +973,9 @@ int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
         // pass 2 writes the next step's sort input into the buffer not holding skeys
         unsigned* keys_next = (skeys == (unsigned*)c->keys0.p) ? (unsigned*)c->keys1.p : (unsigned*)c->keys0.p;
         c->key_buf = (keys_next == (unsigned*)c->keys1.p) ? 1 : 0;
-        const unsigned* keys = (const unsigned*)c->keys_copy.p;
+        // this step's keys by slot: in storage order the sort's input, which a sort would overwrite
+        unsigned* copy = sort ? (unsigned*)c->keys_copy.p : nullptr;
+        const unsigned* keys = sort ? copy : skeys;
         // P2G marks the active nodes.  FP32 form: the contact mass gradient is
         // accumulated by P2G itself; the FP64 form records the per-cell ranges
         // its bit-exact ordered gather reads.
@@ -1170,30 +1178,30 @@ int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
         {
             const int b2 = auto_block(c, c->pass_block);
             const unsigned pb = blocks_for(n, b2);
-            unsigned* kc = (unsigned*)c->keys_copy.p;
+            const PassKeys pk{keys, keys_next, copy};
             const MatConst* mats = (const MatConst*)c->mats.p;
             // FP32: the corner pairs' loads are issued together either way
 #define PASS2(B, S)                                                                                              \
     do {                                                                                                         \
         constexpr int B_ = sizeof(T) == 4 ? 0 : (B);                                                             \
         if (contact)                                                                                             \
-            LAUNCH_STEP("pass2", (k_pass2<T, B_, S, true>), pb, S, 0, P, N, g, kc, keys_next, mats, c->nmat, a, err); \
+            LAUNCH_STEP("pass2", (k_pass2<T, B_, S, true>), pb, S, 0, P, N, g, pk, mats, c->nmat, a, err); \
         else                                                                                                     \
-            LAUNCH_STEP("pass2", (k_pass2<T, B_, S, false>), pb, S, 0, P, N, g, kc, keys_next, mats, c->nmat, a, err); \
+            LAUNCH_STEP("pass2", (k_pass2<T, B_, S, false>), pb, S, 0, P, N, g, pk, mats, c->nmat, a, err); \
     } while (0)
 #define PASS2_STAGED(S)                                                                                          \
     do {                                                                                                         \
         if (contact)                                                                                             \
-            LAUNCH_STEP("pass2", (k_pass2_staged<S, true>), pb, S, Pass2Stage<S>::SMEM, P, N, g, kc, keys_next, mats, \
+            LAUNCH_STEP("pass2", (k_pass2_staged<S, true>), pb, S, Pass2Stage<S>::SMEM, P, N, g, pk, mats, \
                         c->nmat, a, err);                                                                        \
         else                                                                                                     \
-            LAUNCH_STEP("pass2", (k_pass2_staged<S, false>), pb, S, Pass2Stage<S>::SMEM, P, N, g, kc, keys_next, mats, \
+            LAUNCH_STEP("pass2", (k_pass2_staged<S, false>), pb, S, Pass2Stage<S>::SMEM, P, N, g, pk, mats, \
                         c->nmat, a, err);                                                                        \
     } while (0)
             bool large = false;
             if constexpr (sizeof(T) == 8) {
                 if (c->large_strain && !contact) {  // non-contact loop only, as in the reference
-                    LAUNCH_STEP("pass2", k_pass2_ls<128>, blocks_for(n, 128), 128, 0, P, N, g, kc, keys_next, mats, c->nmat,
+                    LAUNCH_STEP("pass2", k_pass2_ls<128>, blocks_for(n, 128), 128, 0, P, N, g, pk, mats, c->nmat,
                            a, err);
                     large = true;
                 }
@@ -1232,6 +1240,7 @@ int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
             }
         }
         c->keys_valid = true;
+        c->copy_valid = sort;
     }
     c->steps_since_reorder += 1;
     CK(cudaGetLastError());

@@ -276,32 +276,34 @@ __global__ void __launch_bounds__(512) k_p2g(PView<T> P, NView<T> nd, Geom g, co
 // cell-local coordinate below 3e-8), the staging thread adds that factor's
 // share to the nodes itself (rare: one particle in some ten million).
 // ---------------------------------------------------------------------------
-// Runs of equal cell keys among the block's first nslots slots (keys staged
-// in shared memory, a __syncthreads after the staging): run r covers slots
-// run_start[r] .. run_start[r + 1] - 1.  Returns the run count.  The slots
-// need not be sorted (a cell met twice is two runs) and slots whose key is out
-// of range form runs of their own, which the callers skip.
-__device__ __forceinline__ int block_runs(const unsigned* skey, int nslots, int* run_start, int* wsum) {
+// Runs of equal cell keys among a block's slots: run r covers slots
+// run_start[r] .. run_start[r + 1] - 1.  The slots need not be sorted (a cell met
+// twice is two runs) and slots whose key is out of range form runs of their own,
+// which the callers skip.  In two halves around the callers' staging, so that
+// the block waits twice in all: run_heads (before) marks the warp's run heads
+// from the keys, whose neighbours come by shuffle, and counts them; run_starts
+// (after a __syncthreads) numbers them and ends with a __syncthreads (four waits
+// before: P2G 135 -> 131 us on the 5.08M-particle batch, 33.1 -> 31.6 on the 1.07M block).
+__device__ __forceinline__ unsigned run_heads(unsigned key, const unsigned* __restrict__ skeys, long long s, long long n,
+                                              int* wsum) {
+    const int t = threadIdx.x, lane = t & 31;
+    unsigned prev = __shfl_up_sync(FULL_MASK, key, 1);
+    if (lane == 0 && t > 0 && s < n) prev = skeys[s - 1];
+    const unsigned heads = __ballot_sync(FULL_MASK, s < n && (t == 0 || prev != key));
+    if (lane == 0) wsum[t >> 5] = __popc(heads);
+    return heads;
+}
+template <int BS>
+__device__ __forceinline__ int run_starts(unsigned heads, int nslots, int* run_start, const int* wsum) {
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const bool head = t < nslots && (t == 0 || skey[t - 1] != skey[t]);
-    const unsigned bal = __ballot_sync(FULL_MASK, head);
-    if (lane == 0) wsum[w] = __popc(bal);
-    __syncthreads();
-    if (t < 32) {
-        const int nw = blockDim.x >> 5;
-        int v = (t < nw) ? wsum[t] : 0;
-        int incl = v;
+    int before = 0, R = 0;
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            int o = __shfl_up_sync(FULL_MASK, incl, off);
-            if (t >= off) incl += o;
-        }
-        if (t < nw) wsum[t] = incl - v;
-        if (t == 31) wsum[32] = incl;
+    for (int k = 0; k < BS / 32; ++k) {
+        const int x = wsum[k];
+        if (k < w) before += x;
+        R += x;
     }
-    __syncthreads();
-    if (head) run_start[wsum[w] + __popc(bal & ((1u << lane) - 1u))] = t;
-    const int R = wsum[32];
+    if ((heads >> lane) & 1u) run_start[before + __popc(heads & ((1u << lane) - 1u))] = t;
     if (t == 0) run_start[R] = nslots;
     __syncthreads();
     return R;
@@ -316,7 +318,7 @@ __device__ __forceinline__ int block_runs(const unsigned* skey, int nslots, int*
 __device__ __forceinline__ int slot_swz(int s) { return s ^ ((s >> 3) & 7); }
 
 // The run arrays that follow the values: the slots' cell keys, the run starts
-// (bs + 1) and 32 warp counts with their total.
+// (bs + 1) and the warps' run counts.
 struct CellSlots {
     unsigned* key;
     int *run_start, *wsum;
@@ -426,7 +428,7 @@ struct P2GBlock {
     }
 
     // After the staging and a __syncthreads (keys in cs.key for the first nslots
-    // slots, out of range where nothing was staged): the runs' sums and their
+    // slots, out of range where nothing was staged; heads from run_heads): the runs' sums and their
     // atomics, which also mark the corners active.  MG: also the node
     // mass gradients.  sid: the slots' specimens from the block's first slot on
     // (perm: through the sort order), for the runs' geometry.
@@ -438,11 +440,12 @@ struct P2GBlock {
     // honeycomb batch about three runs in four have such a neighbour, so a
     // third of the corner atomics go).
     __device__ __forceinline__ void scatter(const NView<T>& nd, const Geom& g, const uint16_t* __restrict__ sid,
-                                            const unsigned* __restrict__ perm, long long s0, int nslots) const {
+                                            const unsigned* __restrict__ perm, long long s0, int nslots,
+                                            unsigned heads) const {
         const int t = threadIdx.x, lane = t & 31;
         const long long nn = nd.nn;
         const unsigned* skey = cs.key;
-        const int R = block_runs(skey, nslots, cs.run_start, cs.wsum);
+        const int R = run_starts<BS>(heads, nslots, cs.run_start, cs.wsum);
         const int nitems = R * 4;
         const int quad = lane & ~3, a = (t >> 1) & 1, b = t & 1;
         // whole warps take the loop together (the shuffles)
@@ -575,6 +578,7 @@ __device__ __forceinline__ void p2g_cells_run(const PView<T>& P, const NView<T>&
     if (blockIdx.x == 0 && t == 0) *nd.acount = 0u;
     const long long s0 = blockIdx.x * (long long)BS, s = s0 + t;
     const unsigned key = (s < n) ? skeys[s] : 0xffffffffu;
+    const unsigned heads = run_heads(key, skeys, s, n, blk.cs.wsum);
     const long long np = P.n;
     if (key < g.key_max) {
         const long long p = perm ? perm[s] : s;
@@ -596,7 +600,7 @@ __device__ __forceinline__ void p2g_cells_run(const PView<T>& P, const NView<T>&
     }
     blk.cs.key[t] = key;
     __syncthreads();
-    blk.scatter(nd, g, P.sid, perm, s0, (int)min((long long)BS, n - s0));
+    blk.scatter(nd, g, P.sid, perm, s0, (int)min((long long)BS, n - s0), heads);
 }
 
 // Threads resident per SM that the FP32 kernels are built for (P2G: 1280 at 48
@@ -870,6 +874,7 @@ __global__ void __launch_bounds__(BS, sizeof(T) == 4 && CPT < 4 ? 1536 / BS : 1)
     step_enter<sizeof(T) == 4>();
     const long long s = blockIdx.x * (long long)bs + t;
     const unsigned key = (s < n) ? skeys[s] : 0xffffffffu;
+    const unsigned heads = run_heads(key, skeys, s, n, cs.wsum);
     const long long np = P.n;
     if (key < g.key_max) {
         const long long p = perm ? perm[s] : s;
@@ -933,7 +938,7 @@ __global__ void __launch_bounds__(BS, sizeof(T) == 4 && CPT < 4 ? 1536 / BS : 1)
     }
     skey[t] = key;
     __syncthreads();
-    const int R = block_runs(skey, (int)min((long long)bs, n - blockIdx.x * (long long)bs), cs.run_start, cs.wsum);
+    const int R = run_starts<BS>(heads, (int)min((long long)bs, n - blockIdx.x * (long long)bs), cs.run_start, cs.wsum);
     constexpr int TPR = 8 / CPT;  // threads per run; each sums CPT corners sharing its x (and y) bases
     for (int item = t; item < R * TPR; item += bs) {
         const int r = item / TPR, k0 = (item % TPR) * CPT;
@@ -1236,6 +1241,16 @@ struct StepArgs {
     int outputs;
 };
 
+// The cell keys pass 2 reads and writes, by slot: this step's, the next step's
+// (its sort's input, or in storage order its keys) and, on sorted steps, whose
+// sort overwrites its input, a copy in slot order (`now` may be that copy;
+// writing it in storage order, too, cost 20 MB a step at 5.08M particles).
+struct PassKeys {
+    const unsigned* now;
+    unsigned* next;
+    unsigned* copy;
+};
+
 // Where pass 2 reads a particle's fields from: its arrays in global memory
 // (DirectSrc), or the block's copies in shared memory (StagedSrc below).
 // Values written by the same step are always read back from global memory.
@@ -1481,8 +1496,7 @@ __device__ __forceinline__ void pass2_prefetch(const PView<T>& P, long long p0, 
 // One thread per particle in index order (coalesced particle streams).  At
 // the end each particle also computes the cell key (and, in the FP32 form,
 // the cell-local coordinate) of its new position for the next step, so the
-// next step needs no separate key pass: `keys` is read (this step) and
-// rewritten (next step), `keys_next` receives the next step's sort input.
+// next step needs no separate key pass.
 // ---------------------------------------------------------------------------
 // The large-strain pass 2's update of one particle after its gather
 // (G2P_P2_LargeStrain, …MPLocks.cpp:311-435; FP64 form): the stress is reset,
@@ -1562,10 +1576,9 @@ __device__ __forceinline__ void large_strain_update(const PView<T>& P, long long
 // coordinate; queued: its stress increment waits for the network).
 template <typename T, int BATCH, bool CONTACT, bool LS = false, class SRC = DirectSrc<T>>
 __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NView<T>& nd, const Geom& g,
-                                                   unsigned* __restrict__ keys, unsigned* __restrict__ keys_next,
-                                                   const MatConst* __restrict__ mats, int nmat, const StepArgs& a,
-                                                   unsigned* err, long long p, float u[3], bool& queued,
-                                                   const SRC& src = SRC{}) {
+                                                   const PassKeys& keys, const MatConst* __restrict__ mats, int nmat,
+                                                   const StepArgs& a, unsigned* err, long long p, float u[3],
+                                                   bool& queued, const SRC& src = SRC{}) {
     const long long np = P.n;
     queued = false;
     const unsigned fl = src.pflags(P, p);
@@ -1575,7 +1588,7 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
     // the position stays in registers until the new cell key is formed
     double x[3] = {src.pos(P, 0, p), src.pos(P, 1, p), src.pos(P, 2, p)};
     if (!skip) {
-        const unsigned key = src.key(keys, p);
+        const unsigned key = src.key(keys.now, p);
         T Ldt[9];  // velocity gradient times dt
 #pragma unroll
         for (int k = 0; k < 9; ++k) Ldt[k] = 0;
@@ -1763,8 +1776,8 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
     for (int c = 0; c < 3; ++c) P.pos[c * np + p] = x[c];
     // the next step's cell key (and FP32 cell-local coordinate) from the new position
     const unsigned nk = particle_key(gs, x, u, err);
-    keys[p] = nk;
-    if (keys_next) keys_next[p] = nk;
+    keys.next[p] = nk;
+    if (keys.copy) keys.copy[p] = nk;
     if constexpr (sizeof(T) == 4) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) P.loc[c * np + p] = u[c];
@@ -1777,16 +1790,15 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
 // gathers' latency).  CONTACT: the loop's path, apart so that each kernel holds
 // one path's code (pass 2's warps also wait for instructions).
 template <typename T, int BATCH, int BS, bool CONTACT>
-__global__ void __launch_bounds__(BS, sizeof(T) == 4 ? 1280 / BS : 1) k_pass2(PView<T> P, NView<T> nd, Geom g, unsigned* __restrict__ keys,
-                                               unsigned* __restrict__ keys_next, const MatConst* __restrict__ mats,
-                                               int nmat, StepArgs a, unsigned* err) {
+__global__ void __launch_bounds__(BS, sizeof(T) == 4 ? 1280 / BS : 1) k_pass2(PView<T> P, NView<T> nd, Geom g, PassKeys keys,
+                                               const MatConst* __restrict__ mats, int nmat, StepArgs a, unsigned* err) {
     step_enter<sizeof(T) == 4>();
     const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (threadIdx.x < 32) pass2_prefetch<T>(P, blockIdx.x * (long long)blockDim.x, blockDim.x, CONTACT);
     if (p >= P.n) return;
     float u[3];
     bool queued;
-    pass2_particle<T, BATCH, CONTACT>(P, nd, g, keys, keys_next, mats, nmat, a, err, p, u, queued);
+    pass2_particle<T, BATCH, CONTACT>(P, nd, g, keys, mats, nmat, a, err, p, u, queued);
 }
 
 // FP32 pass 2 with the block's particle fields staged in shared memory
@@ -1808,10 +1820,8 @@ constexpr int pass2_staged_blocks() {
 
 template <int BS, bool CONTACT>
 __global__ void __launch_bounds__(BS, pass2_staged_blocks<BS>()) k_pass2_staged(PView<float> P, NView<float> nd, Geom g,
-                                                               unsigned* __restrict__ keys,
-                                                               unsigned* __restrict__ keys_next,
-                                                               const MatConst* __restrict__ mats, int nmat,
-                                                               StepArgs a, unsigned* err) {
+                                                               PassKeys keys, const MatConst* __restrict__ mats,
+                                                               int nmat, StepArgs a, unsigned* err) {
     using S = Pass2Stage<BS>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int t = threadIdx.x;
@@ -1832,29 +1842,28 @@ __global__ void __launch_bounds__(BS, pass2_staged_blocks<BS>()) k_pass2_staged(
                          "r"(S::tx_bytes(P))
                          : "memory");
         __syncwarp();
-        if (t < S::NSEG) S::copy(t, P, keys, p0, smem_raw, bar);
+        if (t < S::NSEG) S::copy(t, P, keys.now, p0, smem_raw, bar);
     }
     if (!mbar_wait(bar, 0, err)) {
         mbar_wait(bar, 0, err);  // once more (bounded) for copies still in flight, then leave
         return;
     }
     if (p >= P.n) return;
-    pass2_particle<float, 0, CONTACT, false, StagedSrc<BS>>(P, nd, g, keys, keys_next, mats, nmat, a, err, p, u, queued,
+    pass2_particle<float, 0, CONTACT, false, StagedSrc<BS>>(P, nd, g, keys, mats, nmat, a, err, p, u, queued,
                                                             StagedSrc<BS>{smem_raw});
 }
 
 // The large-strain pass 2 (non-contact loop, FP64 form; the reference ships
 // it disabled, …MPLocks.cpp:605, and MPM_OPT_LARGE_STRAIN switches it on).
 template <int BS>
-__global__ void __launch_bounds__(BS) k_pass2_ls(PView<double> P, NView<double> nd, Geom g, unsigned* __restrict__ keys,
-                                                 unsigned* __restrict__ keys_next, const MatConst* __restrict__ mats,
-                                                 int nmat, StepArgs a, unsigned* err) {
+__global__ void __launch_bounds__(BS) k_pass2_ls(PView<double> P, NView<double> nd, Geom g, PassKeys keys,
+                                                 const MatConst* __restrict__ mats, int nmat, StepArgs a, unsigned* err) {
     step_enter<false>();
     const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (p >= P.n) return;
     float u[3];
     bool queued;
-    pass2_particle<double, 0, false, true>(P, nd, g, keys, keys_next, mats, nmat, a, err, p, u, queued);
+    pass2_particle<double, 0, false, true>(P, nd, g, keys, mats, nmat, a, err, p, u, queued);
 }
 
 // ---------------------------------------------------------------------------
