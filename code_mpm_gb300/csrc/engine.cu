@@ -856,7 +856,7 @@ __global__ void __launch_bounds__(CS_THREADS) k_step_lists(uint8_t* amark, unsig
     if (clock && blockIdx.x == gridDim.x - 1 && t == 0) clock->now = clock->ahead;
     if (blockIdx.x >= ncompact) {
         const int k = (int)(blockIdx.x - ncompact) * CS_THREADS + t;
-        if (k < dc.ndc) dc_claim(k, dc.dclist, dc.keys, dc.pflags, g, dc.owner, nn, dc.contact, dc.sid, state);
+        dc_claim(k, dc.ndc, dc.dclist, dc.keys, dc.pflags, g, dc.owner, nn, dc.contact, dc.sid, state);
         return;
     }
     const long long at = (blockIdx.x * (long long)CS_THREADS + t) * 16;

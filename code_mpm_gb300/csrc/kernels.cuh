@@ -631,16 +631,22 @@ __global__ void __launch_bounds__(BS) k_p2g_cells_mg(PView<float> P, NView<float
 // particle write.  contact: every particle claims all three axes, so the axis-0
 // claim word stands for the three (one atomic per corner instead of three).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void dc_claim(int k, const unsigned* __restrict__ dclist, const unsigned* __restrict__ keys,
-                                         const uint8_t* __restrict__ pflags, const Geom& g, unsigned* owner,
-                                         long long nn, int contact, const uint16_t* __restrict__ sid,
-                                         unsigned* state) {
-    const unsigned p = dclist[k];
-    const unsigned key = keys[p];
-    if (key >= g.key_max) return;
+// Called by whole warps, lane by lane along the list (k < ndc: this lane has an
+// entry).  A claim is lost where the next entry claims the same nodes and axes,
+// as neighbours in a platen's list mostly do, two to a cell: it is not made (the
+// atomics of one cell queue: 24.4 -> 17.4 us on the 5.08M-particle batch).
+__device__ __forceinline__ void dc_claim(int k, int ndc, const unsigned* __restrict__ dclist,
+                                         const unsigned* __restrict__ keys, const uint8_t* __restrict__ pflags,
+                                         const Geom& g, unsigned* owner, long long nn, int contact,
+                                         const uint16_t* __restrict__ sid, unsigned* state) {
+    const bool have = k < ndc;
+    const unsigned p = have ? dclist[k] : 0u;
+    const unsigned key = have ? keys[p] : 0xffffffffu;
+    const unsigned axes = contact ? 7u : have ? pflags[p] & 7u : 0u;
+    const unsigned next_key = __shfl_down_sync(FULL_MASK, key, 1), next_axes = __shfl_down_sync(FULL_MASK, axes, 1);
+    if (!(key < g.key_max) || !axes) return;
+    if ((threadIdx.x & 31) < 31 && next_key == key && next_axes == axes) return;
     const Geom& gs = spec_geom(g, sid, p);
-    const unsigned axes = contact ? 7u : (pflags[p] & 7u);
-    if (!axes) return;
     int b[3];
     key_to_base(key, gs, b);
     const CellNodes cn = cell_nodes(gs, b);
