@@ -1047,8 +1047,13 @@ __device__ __forceinline__ double dc_power(const T f[3], const T v[3], const boo
     return fps_f2d_form(s);
 }
 
+// FP32, five blocks per SM (phase b six; four before): the nodes' gathers and
+// records are latency and traffic, so resident warps count until registers
+// spill.  5.08M-particle batch: 45.4 / 45.0 / 47.8 / 65.5 us with 4 / 5 / 6 / 8
+// blocks, phase b 40.9 / 37.9 / 35.6 / 47.3; foam 18.4 / 17.2 / 19.5 / 24.7 and
+// 17.7 / 16.1 / 15.9 / 21.6.  FP64 is bound by its pipe.
 template <typename T>
-__global__ void __launch_bounds__(256, 4) k_node_phase_a(NView<T> nd, T dt, double damping, int contact, int floor_friction,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) k_node_phase_a(NView<T> nd, T dt, double damping, int contact, int floor_friction,
                                const unsigned* __restrict__ dclist, int ndc, const T* __restrict__ pvel, long long np,
                                T mass_min, int clean, double* work, double dtd) {
     step_enter<sizeof(T) == 4>();
@@ -1132,7 +1137,7 @@ __global__ void __launch_bounds__(256, 4) k_node_phase_a(NView<T> nd, T dt, doub
 // records) leaves the node zeroed as the next step's grid reset would
 // (ResetGrid, …MPLocks.cpp:4-22), so that step needs no reset pass.
 template <typename T>
-__global__ void __launch_bounds__(256, 4) k_node_phase_b(NView<T> nd, T dt, int contact, const unsigned* __restrict__ dclist, int ndc,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_node_phase_b(NView<T> nd, T dt, int contact, const unsigned* __restrict__ dclist, int ndc,
                                const T* __restrict__ pvel, long long np, T mass_min, int clean, int vel_zero) {
     step_enter<sizeof(T) == 4>();
     const long long nn = nd.nn;
