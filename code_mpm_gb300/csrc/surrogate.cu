@@ -713,15 +713,15 @@ constexpr uint32_t SW1 = 0, SW2 = SW1 + HID * IN * 2, SW3 = SW2 + HID * KH * 2, 
 constexpr uint32_t NBIAS = 3 * HID + 16;
 // kernel shared memory: weights, biases (FP32; the output bias is used), then
 // per tile slot (NSLOT) the inputs A0 (128 x 16), the mbarriers (MMA done and
-// operand ready per slot, the final drain), the TMEM address.  Tensor memory
-// per slot (256 columns): the accumulator D (128 columns) and the hidden
-// activations, the A operand of layers 2-4 (128 x 144 BF16 = 72 columns, the
-// last 8 the constant bias column), so the MMAs read only the weights from
-// shared memory.
+// final drain per slot), the TMEM address.  Tensor memory per slot (256
+// columns): the accumulator D (128 columns), the hidden activations, the A
+// operand of layers 2-4 (128 x 144 BF16 = 72 columns, the last 8 the constant
+// bias column), so the MMAs read only the weights from shared memory, and the
+// last layer's accumulator (16 columns).
 constexpr int NSLOT = 2;
-constexpr uint32_t SLOT_COLS = 256, TMEM_COLS = SLOT_COLS * NSLOT, ACT_COL = 128;
+constexpr uint32_t SLOT_COLS = 256, TMEM_COLS = SLOT_COLS * NSLOT, ACT_COL = 128, OUT_COL = 208;
 constexpr uint32_t S_BIAS = WBYTES, S_A0 = (S_BIAS + NBIAS * 4 + 1023) / 1024 * 1024, A0_BYTES = 128 * IN * 2,
-                   S_BAR = S_A0 + NSLOT * A0_BYTES, S_TADDR = S_BAR + 8 * (2 * NSLOT + 1),
+                   S_BAR = S_A0 + NSLOT * A0_BYTES, S_TADDR = S_BAR + 8 * 2 * NSLOT,
                    SMEM_TC = S_TADDR + 8 + 1024;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -736,6 +736,13 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b
 
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+// one lane of a converged warp (the compiler knows that it is one)
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
 }
 
 // bounded wait on an mbarrier phase; false (and the error bit) on timeout
@@ -765,25 +772,25 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// the 64 columns at taddr of this warp's lanes into u: two loads in flight,
-// then the wait, in one statement so no use of u precedes the wait
-__device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t* u) {
+// the 32 columns at taddr of this warp's lanes into u, which nothing may use
+// before tmem_wait_ld(u)
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* u) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,"
-        "%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%64];\n"
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,"
-        "%44,%45,%46,%47,%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%65];\n"
-        "tcgen05.wait::ld.sync.aligned;"
+        "%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
         : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]),
           "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15]),
           "=r"(u[16]), "=r"(u[17]), "=r"(u[18]), "=r"(u[19]), "=r"(u[20]), "=r"(u[21]), "=r"(u[22]), "=r"(u[23]),
-          "=r"(u[24]), "=r"(u[25]), "=r"(u[26]), "=r"(u[27]), "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31]),
-          "=r"(u[32]), "=r"(u[33]), "=r"(u[34]), "=r"(u[35]), "=r"(u[36]), "=r"(u[37]), "=r"(u[38]), "=r"(u[39]),
-          "=r"(u[40]), "=r"(u[41]), "=r"(u[42]), "=r"(u[43]), "=r"(u[44]), "=r"(u[45]), "=r"(u[46]), "=r"(u[47]),
-          "=r"(u[48]), "=r"(u[49]), "=r"(u[50]), "=r"(u[51]), "=r"(u[52]), "=r"(u[53]), "=r"(u[54]), "=r"(u[55]),
-          "=r"(u[56]), "=r"(u[57]), "=r"(u[58]), "=r"(u[59]), "=r"(u[60]), "=r"(u[61]), "=r"(u[62]), "=r"(u[63])
-        : "r"(taddr), "r"(taddr + 32u)
+          "=r"(u[24]), "=r"(u[25]), "=r"(u[26]), "=r"(u[27]), "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31])
+        : "r"(taddr)
         : "memory");
+}
+
+// the load into u (32 words) is done; u passes through, so that no use of it comes before
+__device__ __forceinline__ void tmem_wait_ld(uint32_t* u) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int k = 0; k < 32; ++k) asm volatile("" : "+r"(u[k]));
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
@@ -791,16 +798,14 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// 32 words of this warp's lanes to TMEM columns taddr .. taddr + 31 (the
+// 16 words of this warp's lanes to TMEM columns taddr .. taddr + 15 (the
 // caller waits with tcgen05.wait::st before the columns are read)
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* w) {
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* w) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-        "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
+            taddr),
         "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(w[8]), "r"(w[9]),
-        "r"(w[10]), "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15]), "r"(w[16]), "r"(w[17]), "r"(w[18]),
-        "r"(w[19]), "r"(w[20]), "r"(w[21]), "r"(w[22]), "r"(w[23]), "r"(w[24]), "r"(w[25]), "r"(w[26]), "r"(w[27]),
-        "r"(w[28]), "r"(w[29]), "r"(w[30]), "r"(w[31])
+        "r"(w[10]), "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15])
         : "memory");
 }
 
@@ -859,22 +864,33 @@ __device__ __forceinline__ void issue_layer(uint32_t tmem, uint32_t a_addr, uint
 }
 
 // hidden-layer epilogue of one tile by its group of WPS warps: thread t of
-// group warp j (TMEM lane quarter j % 4) owns sample r = 32 (j % 4) + t and
-// columns c0 .. c0 + SPAN - 1; 64 accumulator columns at a time it reads
-// them (one wait; the bias is in the sums), applies ReLU and stores the 32
-// BF16 pairs to the activation columns (c0 / 2 ...) of its lane
-constexpr int WPS = 4;               // epilogue warps per tile slot: 4 (all 128 columns each) or 8 (64 each)
-constexpr int SPAN = HID * 4 / WPS;  // columns per epilogue warp
+// group warp j (TMEM lane quarter j) owns sample r = 32 j + t; 32 accumulator
+// columns at a time it reads them (the bias is in the sums), applies ReLU and
+// stores the 16 BF16 pairs to the activation columns of its lane; each load
+// runs under the conversions before it
+constexpr int WPS = 4;  // epilogue warps per tile slot
 
-__device__ __forceinline__ void hidden_epilogue(uint32_t d_row, uint32_t act_row, int c0) {
+__device__ __forceinline__ void relu_store16(uint32_t act_row, const uint32_t* u) {
+    uint32_t y[16];
 #pragma unroll
-    for (int h = c0; h < c0 + SPAN; h += 64) {
-        uint32_t u[64], y[32];
-        tmem_ld64(d_row + (uint32_t)h, u);
-#pragma unroll
-        for (int k = 0; k < 32; ++k) y[k] = relu_bf16x2(__uint_as_float(u[2 * k]), __uint_as_float(u[2 * k + 1]));
-        tmem_st32(act_row + (uint32_t)(h / 2), y);
-    }
+    for (int k = 0; k < 16; ++k) y[k] = relu_bf16x2(__uint_as_float(u[2 * k]), __uint_as_float(u[2 * k + 1]));
+    tmem_st16(act_row, y);
+}
+
+__device__ __forceinline__ void hidden_epilogue(uint32_t d_row, uint32_t act_row) {
+    uint32_t u[32], v[32];
+    tmem_ld32(d_row, u);
+    tmem_wait_ld(u);
+    tmem_ld32(d_row + 32u, v);
+    relu_store16(act_row, u);
+    tmem_wait_ld(v);
+    tmem_ld32(d_row + 64u, u);
+    relu_store16(act_row + 16u, v);
+    tmem_wait_ld(u);
+    tmem_ld32(d_row + 96u, v);
+    relu_store16(act_row + 32u, u);
+    tmem_wait_ld(v);
+    relu_store16(act_row + 48u, v);
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
@@ -884,35 +900,32 @@ __device__ __forceinline__ void load_inputs(const float* __restrict__ in, long l
     for (int c = 0; c < NIN; ++c) x[c] = i < n ? in[i * NIN + c] : 0.0f;
 }
 
-// a warp's lanes have finished writing an operand: lane 0 arrives on the
-// slot's ready barrier (one arrival per warp) once the whole warp's shared
-// stores are visible to the tensor core's (async) proxy
-__device__ __forceinline__ void warp_arrive_ready(uint32_t bar) {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncwarp();
-    if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-// a warp waits for a barrier phase: lane 0 polls (bounded), the warp follows;
-// false on a timeout (same answer in every lane)
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, unsigned* err) {
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = bar_wait(bar, parity, err) ? 1 : 0;
-    ok = __shfl_sync(FULL_MASK, ok, 0);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    return ok != 0;
-}
-
-// non-blocking test of an mbarrier phase
-__device__ __forceinline__ bool bar_test(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
+// A slot's group and its MMA warp meet when the operand is written and the
+// accumulators are read.  True when every thread brings ok, the same answer for
+// all, so that after a timeout all of them leave together.
+__device__ __forceinline__ bool slot_ready(int slot, bool ok) {
+    uint32_t all;
     asm volatile(
-        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
+        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.and.pred.aligned q, %2, %3, p;\n"
+        " selp.u32 %0, 1, 0, q;\n}\n"
+        : "=r"(all)
+        : "r"((uint32_t)ok), "r"(1 + slot), "n"(32 * (WPS + 1))
         : "memory");
-    return ok != 0;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    return all != 0u;
+}
+// the group's side (in_shared: an operand in shared memory, too)
+__device__ __forceinline__ bool operand_ready(int slot, bool ok, bool in_shared) {
+    if (in_shared) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    return slot_ready(slot, ok);
+}
+
+// a warp waits (bounded) for its slot's MMAs; false on a timeout (same answer in every lane)
+__device__ __forceinline__ bool group_wait(uint32_t bar, uint32_t parity, unsigned* err) {
+    const bool ok = __all_sync(FULL_MASK, bar_wait(bar, parity, err));
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    return ok;
 }
 
 struct TcArgs {
@@ -928,21 +941,64 @@ struct TcArgs {
     MatConst mat;              // for the elastic predictor D de
 };
 
+// row r of a tile's first operand (128 x 16 BF16): the inputs normalised, a 1 in
+// column 13 (the bias)
+__device__ __forceinline__ void store_inputs(const TcArgs& a, unsigned char* a0, int r, const float x[NIN]) {
+    float xn[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) xn[c] = c < NIN ? x[c] * a.in_inv_scale[c] : (c == NIN ? 1.0f : 0.0f);
+    uint4 p0, p1;
+    p0.x = pack_bf16(xn[0], xn[1]);
+    p0.y = pack_bf16(xn[2], xn[3]);
+    p0.z = pack_bf16(xn[4], xn[5]);
+    p0.w = pack_bf16(xn[6], xn[7]);
+    p1.x = pack_bf16(xn[8], xn[9]);
+    p1.y = pack_bf16(xn[10], xn[11]);
+    p1.z = pack_bf16(xn[12], xn[13]);
+    p1.w = pack_bf16(xn[14], xn[15]);
+    *reinterpret_cast<uint4*>(a0 + kmajor_off(r, 0, 128)) = p0;
+    *reinterpret_cast<uint4*>(a0 + kmajor_off(r, 8, 128)) = p1;
+}
+
+// sample i's outputs from its lane's 16 output columns: the network's correction
+// plus the elastic predictor D de, and dR
+__device__ __forceinline__ void write_outputs(const TcArgs& a, uint32_t out_row, const float* bias, const float de[6],
+                                              long long i, long long n) {
+    float v[16];
+    tmem_ld16(out_row, v);
+    if (i >= n) return;
+    float d[6];
+    trial_increment<float>(a.mat, de, d);
+#pragma unroll
+    for (int c = 0; c < NOUT; ++c)
+        a.out[i * NOUT + c] = (v[c] + bias[3 * HID + c]) * a.out_scale[c] + a.out_shift[c] + (c < 6 ? d[c] : 0.0f);
+}
+
 // NSLOT epilogue groups of WPS warps (one per tile slot; warp j of a group
-// reads TMEM lane quarter j % 4) and the MMA warp
-constexpr int TC_THREADS = 32 * (WPS * NSLOT + 1);
+// reads TMEM lane quarter j) and an MMA warp per slot
+constexpr int TC_THREADS = 32 * (WPS + 1) * NSLOT;
 
 // One CTA per SM takes groups of NSLOT 128-sample tiles, one per slot, and
 // runs the slots as independent pipelines that share the tensor core.  A
 // slot's epilogue group writes the operand (the inputs into shared memory,
-// or the previous layer's activations into tensor memory) and arrives on the
-// slot's `ready` mbarrier (one arrival per warp); the MMA warp issues the
-// layer of whichever slot is ready and commits to that slot's `full`
+// the activations into tensor memory) and meets the slot's MMA warp
+// (slot_ready), which issues the layer and commits it to the slot's `full`
 // mbarrier; the group waits on `full`, turns the accumulators into the next
-// operand, and so on.  The group loads its next tile's inputs while the
-// current tile runs.
+// operand, and so on.  A tile has three hand-offs, not four: its fourth layer
+// goes with the next tile's first, whose operand is written, and the last
+// tile's outputs and the next tile's inputs are dealt with, while the second
+// layer runs.
+//
+// Bound by the MMAs of the two slots, which take turns: 1,432 clocks per tile
+// (nine of 64 in each hidden layer, eight of 27 in the last), 2,860 of the
+// 3,470 a pair of tiles takes.  8M samples: 372 us, 1.52 PFLOP/s (654 us with
+// one MMA warp that issued under a test of its lane number: an MMA takes
+// uniform operands, and each one went round a loop over the lanes, 64 to 79
+// clocks; elected lanes issue one in 16).  300k samples 33 -> 23.5 us.  Tried:
+// the group's first warp issuing (437 us; its own epilogue waits meanwhile), an
+// mbarrier in place of slot_ready (376).
 // Waits are bounded: on a timeout the error word is set and the roles stop;
-// the MMA thread then waits (bounded) for its last MMAs before the TMEM is
+// the MMA warps then wait (bounded) for their last MMAs before the TMEM is
 // freed.
 __global__ void __launch_bounds__(TC_THREADS, 1) k_mlp_tc(TcArgs a) {
     extern __shared__ __align__(1024) unsigned char sm[];
@@ -955,13 +1011,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_mlp_tc(TcArgs a) {
     for (uint32_t i = t; i < NBIAS; i += TC_THREADS) bias[i] = a.bias[i];
     uint32_t* taddr_slot = reinterpret_cast<uint32_t*>(s + S_TADDR);
     // mbarriers: slot sl's MMA-done at full0 + 8 sl, its operand-ready at ready0 + 8 sl
-    const uint32_t full0 = sbase + S_BAR, ready0 = full0 + 8 * NSLOT, drain = ready0 + 8 * NSLOT;
+    const uint32_t full0 = sbase + S_BAR, drain0 = full0 + 8 * NSLOT;
     if (t == 0) {
         for (uint32_t sl = 0; sl < NSLOT; ++sl) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full0 + 8 * sl) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ready0 + 8 * sl), "n"(WPS) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(drain0 + 8 * sl) : "memory");
         }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(drain) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (w == 0) {
@@ -979,110 +1034,93 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_mlp_tc(TcArgs a) {
     const long long ngroups = (n + 128 * NSLOT - 1) / (128 * NSLOT);
     // tile groups of this CTA: blockIdx.x, blockIdx.x + gridDim.x, ...
     const long long mine = blockIdx.x < ngroups ? (ngroups - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-    if (w == WPS * NSLOT) {
-        // the MMA warp: lane 0 issues the next layer of any slot whose operand is ready
-        if ((t & 31) == 0) {
-            const unsigned total = 4u * (unsigned)mine;  // layers per slot
-            unsigned issued[NSLOT];
-#pragma unroll
-            for (int sl = 0; sl < NSLOT; ++sl) issued[sl] = 0u;
-            uint32_t ph = 0u;  // bit sl: slot sl's ready parity
-            bool ok = true;
-            unsigned idle = 0u;
-            for (unsigned left = NSLOT * total; left > 0 && ok;) {
-                bool progress = false;
-#pragma unroll
-                for (int sl = 0; sl < NSLOT; ++sl) {
-                    if (issued[sl] < total && bar_test(ready0 + 8u * sl, (ph >> sl) & 1u)) {
-                        ph ^= 1u << sl;
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        const int layer = (int)(issued[sl] & 3u);
-                        const uint32_t d = tmem + SLOT_COLS * sl, act = d + ACT_COL;
-                        if (layer == 0)
-                            issue_layer<IN, HID>(d, sbase + S_A0 + sl * A0_BYTES, sbase + SW1);
-                        else if (layer < 3)
-                            issue_layer_ts<KH, HID>(d, act, sbase + (layer == 1 ? SW2 : SW3));
-                        else
-                            issue_layer_ts<HID, 16>(d, act, sbase + SW4);
-                        mma_commit(full0 + 8u * sl);
-                        ++issued[sl];
-                        --left;
-                        progress = true;
-                    }
-                }
-                if (progress) {
-                    idle = 0u;
-                } else if (++idle > (1u << 26)) {
-                    atomicOr(a.err, ERR_WAIT_TIMEOUT);
-                    ok = false;
-                }
+    if (w >= WPS * NSLOT) {
+        // slot sl's MMA warp: issues a layer whenever its group has the operand ready
+        const int sl = w - WPS * NSLOT;
+        const uint32_t full = full0 + 8u * sl;
+        const uint32_t d = tmem + SLOT_COLS * sl, act = d + ACT_COL;
+        bool ok = mine > 0;
+        for (long long k = 0; k < mine; ++k) {
+            if (!(ok = slot_ready(sl, true))) break;
+            if (elect_one()) {
+                if (k > 0) issue_layer_ts<HID, 16>(d + OUT_COL, act, sbase + SW4);  // of the last tile
+                issue_layer<IN, HID>(d, sbase + S_A0 + sl * A0_BYTES, sbase + SW1);
+                mma_commit(full);
             }
-            // every MMA issued has completed before the TMEM is freed
-            mma_commit(drain);
-            bar_wait(drain, 0u, a.err);
+            __syncwarp();
+            if (!(ok = slot_ready(sl, true))) break;
+            if (elect_one()) {
+                issue_layer_ts<KH, HID>(d, act, sbase + SW2);
+                mma_commit(full);
+            }
+            __syncwarp();
+            if (!(ok = slot_ready(sl, true))) break;
+            if (elect_one()) {
+                issue_layer_ts<KH, HID>(d, act, sbase + SW3);
+                mma_commit(full);
+            }
+            __syncwarp();
         }
+        if (ok && slot_ready(sl, true)) {
+            if (elect_one()) {
+                issue_layer_ts<HID, 16>(d + OUT_COL, act, sbase + SW4);
+                mma_commit(full);
+            }
+            __syncwarp();
+        }
+        // every MMA issued has completed before the TMEM is freed
+        if (elect_one()) {
+            mma_commit(drain0 + 8u * sl);
+            bar_wait(drain0 + 8u * sl, 0u, a.err);
+        }
+        __syncwarp();
     } else {
-        // epilogue group = slot sl; its warp j reads lanes 32 (j % 4) .. + 31, columns c0 .. c0 + SPAN - 1;
-        // the warps of columns from 0 own the samples' inputs and outputs
-        const int sl = w / WPS, j = w % WPS, r = 32 * (j & 3) + (t & 31), c0 = (j >> 2) * SPAN;
-        const bool owner = c0 == 0;
-        const uint32_t trow = tmem + SLOT_COLS * (uint32_t)sl + ((uint32_t)(32 * (j & 3)) << 16);
+        // epilogue group = slot sl; its warp j reads lanes 32 j .. + 31, one sample per lane
+        const int sl = w / WPS, j = w % WPS, r = 32 * j + (t & 31);
+        const uint32_t full = full0 + 8u * sl;
+        const uint32_t trow = tmem + SLOT_COLS * (uint32_t)sl + ((uint32_t)(32 * j) << 16);
         unsigned char* a0 = s + S_A0 + sl * A0_BYTES;
-        if (owner) {
+        {
             // the activations' constant K columns 128 .. 143: 1, 0, ..., 0 (the bias column)
             uint32_t one[8] = {0x3F80u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
             tmem_st8(trow + ACT_COL + HID / 2, one);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         }
+        const long long stride = (long long)gridDim.x * NSLOT * 128;
+        long long i = ((long long)blockIdx.x * NSLOT + sl) * 128 + r;  // this tile's sample
         uint32_t ph = 0u;
-        bool ok = true;
-        float x[NIN];  // the next tile's physical inputs, loaded one tile ahead
-        load_inputs(a.in, ((long long)blockIdx.x * NSLOT + sl) * 128 + r, owner ? n : 0, x);
+        bool ok = mine > 0;
+        float x[NIN], de[6], de_out[6];  // the next tile's physical inputs; strain increments of this tile and the last
+        load_inputs(a.in, i, n, x);
+        store_inputs(a, a0, r, x);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) de[c] = de_out[c] = x[7 + c];
+        if (ok) ok = operand_ready(sl, true, true);
+        load_inputs(a.in, i + stride, n, x);
         for (long long k = 0; k < mine && ok; ++k) {
-            const long long i = (((long long)blockIdx.x + k * gridDim.x) * NSLOT + sl) * 128 + r;
-            // inputs -> A0 (128 x 16 BF16), then the next tile's inputs are requested
-            float xn[16];
+            // first layer done (and the last tile's outputs)
+            ok = group_wait(full, ph, a.err);
+            if (ok) hidden_epilogue(trow, trow + ACT_COL);
+            if (!(ok = operand_ready(sl, ok, false))) break;
+            // while the second runs: the last tile's outputs, the next tile's operand
+            if (k > 0) write_outputs(a, trow + OUT_COL, bias, de_out, i - stride, n);
+            store_inputs(a, a0, r, x);
 #pragma unroll
-            for (int c = 0; c < 16; ++c) xn[c] = c < NIN ? x[c] * a.in_inv_scale[c] : (c == NIN ? 1.0f : 0.0f);
-            float de[6];  // this tile's strain increment, for the elastic predictor
-#pragma unroll
-            for (int c = 0; c < 6; ++c) de[c] = x[7 + c];
-            uint4 p0, p1;
-            p0.x = pack_bf16(xn[0], xn[1]);
-            p0.y = pack_bf16(xn[2], xn[3]);
-            p0.z = pack_bf16(xn[4], xn[5]);
-            p0.w = pack_bf16(xn[6], xn[7]);
-            p1.x = pack_bf16(xn[8], xn[9]);
-            p1.y = pack_bf16(xn[10], xn[11]);
-            p1.z = pack_bf16(xn[12], xn[13]);
-            p1.w = pack_bf16(xn[14], xn[15]);
-            if (owner) {
-                *reinterpret_cast<uint4*>(a0 + kmajor_off(r, 0, 128)) = p0;
-                *reinterpret_cast<uint4*>(a0 + kmajor_off(r, 8, 128)) = p1;
-                load_inputs(a.in, i + (long long)gridDim.x * NSLOT * 128, n, x);
+            for (int c = 0; c < 6; ++c) {
+                de_out[c] = de[c];
+                de[c] = x[7 + c];
             }
-            for (int layer = 0; layer < 4 && ok; ++layer) {
-                // the operand (inputs, or the previous layer's activations) is ready
-                warp_arrive_ready(ready0 + 8 * sl);
-                ok = warp_wait(full0 + 8 * sl, ph, a.err);
-                if (!ok) break;
-                ph ^= 1u;
-                if (layer < 3) {
-                    hidden_epilogue(trow, trow + ACT_COL, c0);
-                } else if (owner) {
-                    float v[16];
-                    tmem_ld16(trow, v);
-                    if (i < n) {
-                        float d[6];
-                        trial_increment<float>(a.mat, de, d);  // the elastic predictor D de
-#pragma unroll
-                        for (int c = 0; c < NOUT; ++c)
-                            a.out[i * NOUT + c] =
-                                (v[c] + bias[3 * HID + c]) * a.out_scale[c] + a.out_shift[c] + (c < 6 ? d[c] : 0.0f);
-                    }
-                }
-            }
+            load_inputs(a.in, i + 2 * stride, n, x);
+            ok = group_wait(full, ph ^ 1u, a.err);
+            if (ok) hidden_epilogue(trow, trow + ACT_COL);
+            if (!(ok = operand_ready(sl, ok, false))) break;
+            ok = group_wait(full, ph, a.err);
+            if (ok) hidden_epilogue(trow, trow + ACT_COL);
+            ok = operand_ready(sl, ok, true);  // and the next tile's inputs
+            ph ^= 1u;
+            i += stride;
         }
+        if (ok && group_wait(full, ph, a.err)) write_outputs(a, trow + OUT_COL, bias, de_out, i - stride, n);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
