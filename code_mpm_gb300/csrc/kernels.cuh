@@ -145,16 +145,28 @@ struct Runs {
 // Bases of particle p: FP64 form from the position, FP32 form from the
 // cell-local coordinate the previous step stored (no FP64 instructions).
 template <typename T>
+__device__ __forceinline__ void load_place(const PView<T>& P, long long p, T x[3]) {
+    const T* at;
+    if constexpr (sizeof(T) == 4)
+        at = P.loc;
+    else
+        at = P.pos;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) x[c] = at[c * P.n + p];
+}
+template <typename T>
+__device__ __forceinline__ void place_bases(const Geom& g, const T x[3], const int b[3], Bases<T>& B) {
+    if constexpr (sizeof(T) == 4)
+        B.init_local(g, x);
+    else
+        B.init(g, x, b);
+}
+template <typename T>
 __device__ __forceinline__ void particle_bases(const PView<T>& P, const Geom& g, long long p, const int b[3],
                                                Bases<T>& B) {
-    const long long np = P.n;
-    if constexpr (sizeof(T) == 4) {
-        const float u[3] = {P.loc[p], P.loc[np + p], P.loc[2 * np + p]};
-        B.init_local(g, u);
-    } else {
-        const double x[3] = {P.pos[p], P.pos[np + p], P.pos[2 * np + p]};
-        B.init(g, x, b);
-    }
+    T x[3];
+    load_place(P, p, x);
+    place_bases(g, x, b, B);
 }
 
 // Prefetch into L2 the bytes of elements [p0, p0 + cnt) of an array of n
@@ -861,7 +873,10 @@ __host__ __device__ constexpr size_t pass1_cells_smem(int bs) {
 // FP32 with 1 or 2 corners per thread: registers capped for 1536 resident
 // threads per SM (40 registers), about 10% faster than 56 registers at 1152
 // threads: the kernel waits on its record gathers, and more resident warps
-// keep more of them in flight.
+// keep more of them in flight (1280 and 1024 threads with all eight records
+// requested at once: 135 us against 118 on the 5.08M-particle batch).  A
+// slot's particle fields are requested with its key rather than after it: 129
+// -> 118 us there, 48.1 -> 44.7 on 1.89M particles, 26.9 -> 26.0 on 1.07M.
 template <typename T, int CPT, int BS>
 __global__ void __launch_bounds__(BS, sizeof(T) == 4 && CPT < 4 ? 1536 / BS : 1) k_pass1_cells(PView<T> P, NView<T> nd, Geom g,
                                                      const unsigned* __restrict__ skeys,
@@ -879,23 +894,29 @@ __global__ void __launch_bounds__(BS, sizeof(T) == 4 && CPT < 4 ? 1536 / BS : 1)
     unsigned* skey = cs.key;
     step_enter<sizeof(T) == 4>();
     const long long s = blockIdx.x * (long long)bs + t;
-    const unsigned key = (s < n) ? skeys[s] : 0xffffffffu;
-    const unsigned heads = run_heads(key, skeys, s, n, cs.wsum);
     const long long np = P.n;
+    const unsigned key = (s < n) ? skeys[s] : 0xffffffffu;
+    const long long p = s < n ? (perm ? perm[s] : s) : 0;
+    T x[3] = {0, 0, 0}, v[3] = {0, 0, 0}, m = 0;
+    bool valid = true;
+    if (s < n) {
+        load_place(P, p, x);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[c] = P.vel[c * np + p];
+        m = P.mass[p];
+        valid = !(contact && (P.pflags[p] & 8u));
+    }
+    const unsigned heads = run_heads(key, skeys, s, n, cs.wsum);
     if (key < g.key_max) {
-        const long long p = perm ? perm[s] : s;
         const Geom& gs = spec_geom(g, P.sid, p);
         int b[3];
         key_to_base(key, gs, b);
         const CellNodes cn = cell_nodes(gs, b);
         scn[t] = cn;
-        const bool valid = !(contact && (P.pflags[p] & 8u));
         T N6[6] = {0, 0, 0, 0, 0, 0}, mv[3] = {0, 0, 0};
         if (valid) {
             Bases<T> B;
-            particle_bases<T>(P, gs, p, b, B);
-            const T m = P.mass[p];
-            T v[3] = {P.vel[p], P.vel[np + p], P.vel[2 * np + p]};
+            place_bases<T>(gs, x, b, B);
             // four corners' records requested before any is used; summed in corner order
 #pragma unroll(F32 ? 2 : 1)
             for (int h = 0; h < 2; ++h) {
