@@ -1095,7 +1095,9 @@ int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
         // the mass threshold in the form's type (FP32: rounded down, so float masses compare exactly)
         const T mm = sizeof(T) == 4 ? (T)fps_float_threshold(c->sim.mass_min) : (T)c->sim.mass_min;
         // displacement control, grid update, displacement control, f/m: one pass over the active nodes
-        LAUNCH_STEP("node_phase_a", k_node_phase_a<T>, nodeblocks, NTHREADS, 0, N, (T)dt, c->sim.damping, contact,
+        constexpr int nt = NODE_THREADS<T>;
+        const unsigned phaseblocks = (unsigned)std::min<long long>(blocks_for(nn, nt), (long long)c->sm_count * (4096 / nt));
+        LAUNCH_STEP("node_phase_a", k_node_phase_a<T>, phaseblocks, nt, 0, N, (T)dt, c->sim.damping, contact,
                c->floor_friction, (const unsigned*)c->dclist.p, c->ndc, (const T*)c->vel.p, n, mm, output ? 0 : 1,
                (double*)c->work_acc.p, dt);
         if (sizeof(T) == 4 && c->p2g_reduce >= 5) {  // the same runs as P2G, reduced by lane pairs
@@ -1133,7 +1135,7 @@ int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
             LAUNCH_STEP("pass1_remap", (k_pass1_remap<T, 0>), blocks_for(n), NTHREADS, 0, P, N, g, skeys, perm, n,
                         contact);
         // remap, displacement control and BC in the path's order, p/m and v: one pass
-        LAUNCH_STEP("node_phase_b", k_node_phase_b<T>, nodeblocks, NTHREADS, 0, N, (T)dt, contact, (const unsigned*)c->dclist.p,
+        LAUNCH_STEP("node_phase_b", k_node_phase_b<T>, phaseblocks, nt, 0, N, (T)dt, contact, (const unsigned*)c->dclist.p,
                c->ndc, (const T*)c->vel.p, n, mm, output ? 0 : 1, vel_zero);
         if (output) c->grid_dirty = true;  // the last step of an advance keeps its node values for the caller
         if (c->ndc > 0) c->owner_clean = true;

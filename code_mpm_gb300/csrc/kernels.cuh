@@ -1068,11 +1068,19 @@ __device__ __forceinline__ double dc_power(const T f[3], const T v[3], const boo
     return fps_f2d_form(s);
 }
 
-// FP32, five blocks per SM (phase b six; four before): the nodes' gathers and
+// FP64: small blocks, as the phases are bound by the FP64 pipe of each SM and what
+// counts is that every SM gets its share of the warps.  256 / 128 / 64 / 32
+// threads: 26.4 / 24.8 / 23.9 / 23.2 us (phase b 26.4 / 23.5 / 22.9 / 23.4) on
+// 406k particles of honeycombs; 40k and 1k particles, whose nodes fill 35 and 3
+// blocks of 256 threads, 70 -> 67 and 70 -> 65 us per step.  FP32: with 64
+// threads phase b takes 16.5 us for 14.9 on the 1.89M-particle foam.
+// FP32, 1280 threads per SM (phase b 1536; 1024 before): the nodes' gathers and
 // records are latency and traffic, so resident warps count until registers
-// spill.  5.08M-particle batch: 45.4 / 45.0 / 47.8 / 65.5 us with 4 / 5 / 6 / 8
-// blocks, phase b 40.9 / 37.9 / 35.6 / 47.3; foam 18.4 / 17.2 / 19.5 / 24.7 and
-// 17.7 / 16.1 / 15.9 / 21.6.  FP64 is bound by its pipe.
+// spill.  5.08M-particle batch: 45.4 / 45.0 / 47.8 / 65.5 us with 1024 / 1280 /
+// 1536 / 2048, phase b 40.9 / 37.9 / 35.6 / 47.3; foam 18.4 / 17.2 / 19.5 / 24.7
+// and 17.7 / 16.1 / 15.9 / 21.6.
+template <typename T>
+constexpr int NODE_THREADS = sizeof(T) == 8 ? 64 : 256;
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) k_node_phase_a(NView<T> nd, T dt, double damping, int contact, int floor_friction,
                                const unsigned* __restrict__ dclist, int ndc, const T* __restrict__ pvel, long long np,
