@@ -823,13 +823,15 @@ __global__ void k_step_end(DevSim* d) {
 // What a step needs between P2G and the node phases, in one launch (two
 // kernels and the counter's memset before, each a launch's latency on a small
 // scene):
-//  * blocks [0, ncompact): the active-node list from P2G's marks, 16 nodes per
-//    thread (a byte per node; the state words cost four: on a grid of 32M nodes,
-//    6% of them active, list and claims took 39-48 us from the state words,
-//    21 from the marks).  A block
+//  * blocks [0, ncompact): the active-node list from P2G's marks, NPT nodes per
+//    thread: 16, or 4 on grids that 16 would not spread over a block per SM (8.1
+//    and 6.7 us with 9,000 nodes, a 40,000-particle step 26.7 and 25.7; 8.4 and
+//    7.8 with 65,000; but 17 and 23 with 7.7M, 18 and 41 with 32M).  A mark is a
+//    byte; the state words cost four: on a grid of 32M nodes, 6% of them active,
+//    list and claims took 39-48 us from the state words, 21 from the marks.  A block
 //    reserves its range with one atomic (a counter shared by every warp would
 //    serialise tens of thousands of atomics at one L2 address), so the list is
-//    in node order within each 4,096 nodes.  The marks are cleared for the next
+//    in node order within each block's nodes.  The marks are cleared for the next
 //    step; an output step also sets the nodes' state bits, which its caller sees;
 //  * the blocks after them: the displacement-control claims, one particle of
 //    the list per thread (they set another bit of the state words);
@@ -844,7 +846,7 @@ struct ClaimArgs {
     int contact;
     const uint16_t* sid;
 };
-template <bool EARLY>
+template <bool EARLY, int NPT>
 __global__ void __launch_bounds__(CS_THREADS) k_step_lists(uint8_t* amark, unsigned* state, long long nn,
                                                            unsigned ncompact, unsigned* __restrict__ list,
                                                            unsigned* count, int output, ClaimArgs dc, Geom g,
@@ -859,16 +861,24 @@ __global__ void __launch_bounds__(CS_THREADS) k_step_lists(uint8_t* amark, unsig
         dc_claim(k, dc.ndc, dc.dclist, dc.keys, dc.pflags, g, dc.owner, nn, dc.contact, dc.sid, state);
         return;
     }
-    const long long at = (blockIdx.x * (long long)CS_THREADS + t) * 16;
+    static_assert(NPT == 16 || NPT == 4, "nodes per thread");
+    const long long at = (blockIdx.x * (long long)CS_THREADS + t) * NPT;
     unsigned bits = 0u;  // this thread's marked nodes
     if (at < nn) {       // (the marks are padded to whole groups of 16)
-        uint4* p = reinterpret_cast<uint4*>(amark + at);
-        const uint4 m = *p;
-        if (m.x | m.y | m.z | m.w) {
-            *p = make_uint4(0u, 0u, 0u, 0u);
-            // bytes of value 0 or 1: the product gathers a word's four into its top nibble
-            bits = ((m.x * 0x10204080u) >> 28) | ((m.y * 0x10204080u) >> 28) << 4 |
-                   ((m.z * 0x10204080u) >> 28) << 8 | ((m.w * 0x10204080u) >> 28) << 12;
+        // bytes of value 0 or 1: the product gathers a word's four into its top nibble
+        if constexpr (NPT == 16) {
+            uint4* p = reinterpret_cast<uint4*>(amark + at);
+            const uint4 m = *p;
+            if (m.x | m.y | m.z | m.w) {
+                *p = make_uint4(0u, 0u, 0u, 0u);
+                bits = ((m.x * 0x10204080u) >> 28) | ((m.y * 0x10204080u) >> 28) << 4 |
+                       ((m.z * 0x10204080u) >> 28) << 8 | ((m.w * 0x10204080u) >> 28) << 12;
+            }
+        } else {
+            unsigned* p = reinterpret_cast<unsigned*>(amark + at);
+            const unsigned m = *p;
+            if (m) *p = 0u;
+            bits = (m * 0x10204080u) >> 28;
         }
     }
     // entries of this warp's threads before this one
@@ -892,16 +902,19 @@ __global__ void __launch_bounds__(CS_THREADS) k_step_lists(uint8_t* amark, unsig
     }
     __syncthreads();
     const unsigned off = base + woff[w] + incl - cnt;
-    // the warp writes the nodes of two threads at a time
-    const unsigned first = (unsigned)((blockIdx.x * (long long)CS_THREADS + (t - lane)) * 16);
-    const int half = lane >> 4, l16 = lane & 15;
-    const unsigned have = __ballot_sync(FULL_MASK, bits != 0u);
-    for (unsigned pairs = (have | have >> 1) & 0x55555555u; pairs; pairs &= pairs - 1u) {
-        const int src = __ffs(pairs) - 1 + half;
+    // the warp writes the nodes of 32 / NPT threads at a time
+    constexpr int GRP = 32 / NPT;
+    const unsigned first = (unsigned)((blockIdx.x * (long long)CS_THREADS + (t - lane)) * NPT);
+    const int sub = lane / NPT, ln = lane % NPT;
+    unsigned have = __ballot_sync(FULL_MASK, bits != 0u);
+#pragma unroll
+    for (int d = 1; d < GRP; d <<= 1) have |= have >> d;  // bit g GRP: any thread of group g
+    for (have &= GRP == 2 ? 0x55555555u : 0x01010101u; have; have &= have - 1u) {
+        const int src = __ffs(have) - 1 + sub;
         const unsigned b = __shfl_sync(FULL_MASK, bits, src), o = __shfl_sync(FULL_MASK, off, src);
-        if ((b >> l16) & 1u) {
-            const unsigned node = first + 16u * src + l16;
-            list[o + __popc(b & ((1u << l16) - 1u))] = node;
+        if ((b >> ln) & 1u) {
+            const unsigned node = first + (unsigned)NPT * src + ln;
+            list[o + __popc(b & ((1u << ln) - 1u))] = node;
             if (output) atomicOr(&state[node], 1u);
         }
     }
@@ -1044,13 +1057,18 @@ int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
             if (!c->owner_clean) CK(cudaMemsetAsync(c->g_owner.p, 0, (size_t)3 * nn * 4, c->stream));
             c->owner_clean = false;  // claims in use until phase B clears them
         }
-        const unsigned ncompact = (unsigned)((nn + 16 * CS_THREADS - 1) / (16 * CS_THREADS));
+        const int npt = nn < 16LL * CS_THREADS * c->sm_count ? 4 : 16;
+        const unsigned ncompact = (unsigned)((nn + npt * CS_THREADS - 1) / (npt * CS_THREADS));
         const unsigned nclaim = (unsigned)((c->ndc + CS_THREADS - 1) / CS_THREADS);
         const ClaimArgs dc{(const unsigned*)c->dclist.p, c->ndc, keys, (const uint8_t*)c->pflags.p,
                            (unsigned*)c->g_owner.p, contact, P.sid};
-        LAUNCH_STEP("step_lists", k_step_lists<sizeof(T) == 4>, ncompact + nclaim, CS_THREADS, 0, N.amark, N.state,
-                    nn, ncompact, (unsigned*)c->alist.p, N.acount, output ? 1 : 0, dc, g,
-                    graph == 1 ? dsim : (DevSim*)nullptr);
+        DevSim* clock = graph == 1 ? dsim : nullptr;
+        if (npt == 4)
+            LAUNCH_STEP("step_lists", (k_step_lists<sizeof(T) == 4, 4>), ncompact + nclaim, CS_THREADS, 0, N.amark, N.state,
+                        nn, ncompact, (unsigned*)c->alist.p, N.acount, output ? 1 : 0, dc, g, clock);
+        else
+            LAUNCH_STEP("step_lists", (k_step_lists<sizeof(T) == 4, 16>), ncompact + nclaim, CS_THREADS, 0, N.amark, N.state,
+                        nn, ncompact, (unsigned*)c->alist.p, N.acount, output ? 1 : 0, dc, g, clock);
         if (graph == 1) {  // the next replay's clock, on a branch beside the two steps
             const double* tl = (const double*)c->tl_dev.p;
             const int nt = (int)c->tl_t.size();
