@@ -944,6 +944,25 @@ int auto_block(const mpm_ctx* c, int chosen) {
     return b;
 }
 
+// Pass 2's mode: the caller's (or the autotuner's), else, in the FP32 form,
+// staged (2) for particles that fill less than half a wave of it (1024 threads
+// per SM), where each block's copies are all there is in flight, and direct (0)
+// beyond, where the staging only delays a block's first gathers.  Staged /
+// direct, us per step: 40,000 particles 25.7 / 26.7, 43,500 32.1 / 32.1, 89,000
+// 38.9 / 38.3, 209,000 46.4 / 45.1, 383,000 73.1 / 70.6, 1.07M 143.5 / 138.0,
+// 1.89M 255 / 247, 5.08M 669 / 657.
+int gather_mode(const mpm_ctx* c) {
+    if (c->gather_batch >= 0) return c->gather_batch;
+    return c->n < 512LL * c->sm_count ? 2 : 0;
+}
+// And its block: 256 threads where nobody chose and it runs direct (128: 138.4
+// against 138.0 us with 1.07M particles, 71.2 against 70.6 with 383,000; 512: 666
+// against 658 with 5.08M).
+int pass2_block(const mpm_ctx* c) {
+    if (!c->pass_block && c->gather_batch < 0 && gather_mode(c) == 0) return 256;
+    return auto_block(c, c->pass_block);
+}
+
 // graph: 0, or which of the two captured steps this is (1, 2).
 // output: the step is an output step, the last of an advance, whose results
 // the caller can see.  Only an output step runs the contact path's contact
@@ -1196,7 +1215,7 @@ int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
             a.sg_acc = (SurrogateAcc*)c->sg_acc.p;
         }
         {
-            const int b2 = auto_block(c, c->pass_block);
+            const int b2 = pass2_block(c);
             const unsigned pb = blocks_for(n, b2);
             const PassKeys pk{keys, keys_next, copy};
             const MatConst* mats = (const MatConst*)c->mats.p;
@@ -1227,7 +1246,7 @@ int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
                 }
             }
             if (large) {
-            } else if (c->gather_batch == 2 && sizeof(T) == 4) {
+            } else if (gather_mode(c) == 2 && sizeof(T) == 4) {
                 if constexpr (sizeof(T) == 4) {
                     if (b2 == 128) PASS2_STAGED(128);
                     else if (b2 == 256) PASS2_STAGED(256);
@@ -1520,9 +1539,7 @@ int mpm_create_batch(const mpm_grid_desc* grids, int32_t nspec, int form, mpm_ct
     mpm_ctx* c = new mpm_ctx();
     c->form = form;
     c->tsize = form == MPM_FORM_FP64 ? 8 : 4;
-    if (form == MPM_FORM_FP32) {  // the autotuner's choice on the honeycomb batch
-        c->gather_batch = 2;
-    }
+    if (form == MPM_FORM_FP32) c->gather_batch = -1;  // gather_mode's choice
     c->nspec = nspec;
     cudaGetDevice(&c->device);
     cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device);
@@ -2359,8 +2376,8 @@ int mpm_autotune(mpm_ctx* c, int32_t steps, double dt, int contact, mpm_tune_res
         out->p2g_block = best[1] ? best[1] : 128;
         out->pass1_corners = best[2];
         out->pass1_block = best[3] ? best[3] : 128;
-        out->pass_block = best[4] ? best[4] : 128;
-        out->gather_batch = best[5];
+        out->pass_block = std::max(128, pass2_block(c));
+        out->gather_batch = gather_mode(c);
         out->candidates = ncand;
         out->best_ms_per_step = best_ms;
         out->worst_ms_per_step = worst_ms;

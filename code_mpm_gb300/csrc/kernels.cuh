@@ -1825,12 +1825,14 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
     return nk;
 }
 
-// BS: the block size; the FP32 form asks for 1280 / BS blocks per SM (48
-// registers: a few spill, and the extra resident warps hide more of the
-// gathers' latency).  CONTACT: the loop's path, apart so that each kernel holds
+// BS: the block size; the FP32 form asks for 1024 / BS blocks per SM (64
+// registers).  Blocks of 128, us per step of a 1.07M-particle block and of 5.08M
+// particles of honeycombs: 142.9 and 677 with 768 threads per SM, 140.3 and 665
+// with 896, 138.4 and 657 with 1024, 140.0 and 660 with 1152; 144.6 and 679 with
+// 1280 (256 threads per block; 48 registers and spills).  CONTACT: the loop's path, apart so that each kernel holds
 // one path's code (pass 2's warps also wait for instructions).
 template <typename T, int BATCH, int BS, bool CONTACT>
-__global__ void __launch_bounds__(BS, sizeof(T) == 4 ? 1280 / BS : 1) k_pass2(PView<T> P, NView<T> nd, Geom g, PassKeys keys,
+__global__ void __launch_bounds__(BS, sizeof(T) == 4 ? 1024 / BS : 1) k_pass2(PView<T> P, NView<T> nd, Geom g, PassKeys keys,
                                                const MatConst* __restrict__ mats, int nmat, StepArgs a, unsigned* err) {
     step_enter<sizeof(T) == 4>();
     const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;

@@ -75,7 +75,8 @@ extern "C" {
 #define MPM_OPT_PASS_BLOCK 5     /* G2P pass-2 threads per block: 128 (default), 256 or 512; by default the FP64 form takes 64 or 32 where the particles are few */
 #define MPM_OPT_GATHER 6         /* pass-2 (G2P) mode: 0 = node gathers one (x, y) pair of corners at a time, 1 = several
                                     pairs' loads issued together, 2 = (FP32 form) as 0 with the block's particle fields
-                                    brought into shared memory by bulk copies first */
+                                    brought into shared memory by bulk copies first.  Until set: FP64 form 0, FP32 form 2
+                                    for few particles (under 512 per SM), else 0 */
 #define MPM_OPT_GRAPH 7          /* 1 (default): mpm_advance replays a captured two-step CUDA graph in the steady state; 0: launch every kernel */
 #define MPM_OPT_REORDER 8        /* store particles in cell order after each particle upload (0, default; FP64 form: once 8 steps have been asked for), also every N steps (N > 0), or never (-1); results stay in the caller's order */
 #define MPM_OPT_PASS1_CORNERS 10 /* cell-run G2P pass 1 (P2G modes 2-4): corners per thread, 1, 2 (default) or 4 */
