@@ -117,7 +117,7 @@ struct mpm_ctx {
     mpm_net* net = nullptr;
     float sg_band = 0.02f, sg_recheck = 0.01f;  // the network takes trial states at least sg_band k0 past the surface
     float sg_guard = 0.001f;  // tolerance of the guard on the network's results, a fraction of k0 (0: off)
-    int fp64_fallback = 1;  // FP32 form: the exact map in FP64 for von Mises hardening particles near or past the surface
+    int fp64_fallback = 1;  // FP32 form: the exact map (in pairs of floats) for von Mises hardening particles near or past the surface
     unsigned sg_mats = 0;
     std::vector<MatConst> mats_host;
     DevBuf q_in, q_out, q_vol, q_pidx, q_count, sg_acc;
@@ -1178,9 +1178,7 @@ int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
         if (c->ndc > 0) c->owner_clean = true;
         StepArgs a;
         a.dt = dt;
-        a.mass_min = c->sim.mass_min;
         a.dt_f = (float)dt;
-        a.mass_min_f = fps_float_threshold(c->sim.mass_min);
         timeline_velocity(c, c->sim.time, a.tv);
         a.tv_dev = graph ? dsim->now.tv[graph - 1] : nullptr;
         a.has_timeline = c->tl_t.empty() ? 0 : 1;

@@ -618,8 +618,8 @@ __device__ __forceinline__ void p2g_cells_run(const PView<T>& P, const NView<T>&
 // Threads resident per SM that the FP32 kernels are built for (P2G: 1280 at 48
 // registers; 5.08M particles of honeycombs, 138 us, against 140 us for 1536 at
 // 40 registers with spills and 176 us for 1024).  Before the moments P2G took
-// 154 us there, 39.1 us (now 33.7) on a solid block of 1.07M particles; FP64
-// form, a solid block of 286k particles: 233 us before, 115 now.
+// 154 us there (now 131), 39.1 us (now 31.6) on a solid block of 1.07M particles; FP64
+// form, a solid block of 286k particles: 233 us before, 112 now.
 template <typename T, int BS, bool FE>
 __global__ void __launch_bounds__(BS, sizeof(T) == 4 ? 1280 / BS : 1) k_p2g_cells(
     PView<T> P, NView<T> nd, Geom g, const unsigned* __restrict__ skeys, const unsigned* __restrict__ perm, long long n) {
@@ -1245,9 +1245,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_node_phase_b(NV
 // and passed in as tv.
 struct StepArgs {
     double dt;
-    double mass_min;
-    float dt_f;        // RN32(dt)
-    float mass_min_f;  // mass_min rounded down to float (fps_float_threshold)
+    float dt_f;  // RN32(dt)
     double tv[3];
     const double* tv_dev;  // graph replay: the timeline velocity computed on the device (else tv)
     int has_timeline;
