@@ -239,7 +239,8 @@ struct NView {
     uint8_t* fixed;
     double* friction;
     T* rec;            // scratch: per node 8 values {r, has, v, 0}: r = f/m before pass 1, p/m before
-                       // pass 2; has = 1 when m > mass_min; v = node velocity (pass 2 only)
+                       // pass 2; has = 1 when m > mass_min; v = node velocity (pass 2 only);
+                       // FP64 form: r and v times dt
     T* q;              // scratch: remap accumulator sum N m_p v_p, 4 values per node {q[3], 0}
     unsigned* owner;   // scratch: displacement-control last-writer claims, 3 x nn
     unsigned* nowner;  // scratch: contact-normal last-writer claims, nn

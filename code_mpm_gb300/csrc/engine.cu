@@ -357,7 +357,7 @@ void launch_step(mpm_ctx* c, void (*kernel)(Ex...), unsigned grid, unsigned bloc
         }                                                                               \
     } while (0)
 template <typename T, int BS>
-using Pass1Kernel = void (*)(PView<T>, NView<T>, Geom, const unsigned*, const unsigned*, long long, int);
+using Pass1Kernel = void (*)(PView<T>, NView<T>, Geom, const unsigned*, const unsigned*, long long, T, int);
 // pass 1 with the option's corners per thread (1, 2 or 4)
 template <typename T, int BS>
 Pass1Kernel<T, BS> pass1_kernel(int cpt) {
@@ -1142,35 +1142,35 @@ int step_impl(mpm_ctx* c, double dt, int contact, int graph, bool output) {
                 const int b1 = auto_block(c, c->pass1_block);
                 const unsigned pg = (unsigned)((n + 4LL * b1 - 1) / (4LL * b1));
                 if (b1 == 128)
-                    LAUNCH_STEP("pass1_remap", k_pass1_pairs<128>, pg, 128, 0, P, N, g, skeys, perm, n, contact);
+                    LAUNCH_STEP("pass1_remap", k_pass1_pairs<128>, pg, 128, 0, P, N, g, skeys, perm, n, (T)dt, contact);
                 else if (b1 == 256)
-                    LAUNCH_STEP("pass1_remap", k_pass1_pairs<256>, pg, 256, 0, P, N, g, skeys, perm, n, contact);
+                    LAUNCH_STEP("pass1_remap", k_pass1_pairs<256>, pg, 256, 0, P, N, g, skeys, perm, n, (T)dt, contact);
                 else
-                    LAUNCH_STEP("pass1_remap", k_pass1_pairs<512>, pg, 512, 0, P, N, g, skeys, perm, n, contact);
+                    LAUNCH_STEP("pass1_remap", k_pass1_pairs<512>, pg, 512, 0, P, N, g, skeys, perm, n, (T)dt, contact);
             }
         } else if (c->p2g_reduce >= 2) {  // the same reduction as P2G: shared-memory cell runs
             const int cpt = c->pass1_corners, b1 = std::max(auto_block(c, c->pass1_block), cpt == 2 ? 32 : 128);
             const unsigned gb = blocks_for(n, b1);
             const size_t sm = pass1_cells_smem<T>(b1);
             if (b1 == 128)
-                LAUNCH_STEP("pass1_remap", (pass1_kernel<T, 128>(cpt)), gb, 128, sm, P, N, g, skeys, perm, n, contact);
+                LAUNCH_STEP("pass1_remap", (pass1_kernel<T, 128>(cpt)), gb, 128, sm, P, N, g, skeys, perm, n, (T)dt, contact);
             else if (b1 == 256)
-                LAUNCH_STEP("pass1_remap", (pass1_kernel<T, 256>(cpt)), gb, 256, sm, P, N, g, skeys, perm, n, contact);
+                LAUNCH_STEP("pass1_remap", (pass1_kernel<T, 256>(cpt)), gb, 256, sm, P, N, g, skeys, perm, n, (T)dt, contact);
             else if (b1 == 512)
-                LAUNCH_STEP("pass1_remap", (pass1_kernel<T, 512>(cpt)), gb, 512, sm, P, N, g, skeys, perm, n, contact);
+                LAUNCH_STEP("pass1_remap", (pass1_kernel<T, 512>(cpt)), gb, 512, sm, P, N, g, skeys, perm, n, (T)dt, contact);
             else if constexpr (sizeof(T) == 8) {
                 if (b1 == 64)
-                    LAUNCH_STEP("pass1_remap", (k_pass1_cells<T, 2, 64>), gb, 64, sm, P, N, g, skeys, perm, n, contact);
+                    LAUNCH_STEP("pass1_remap", (k_pass1_cells<T, 2, 64>), gb, 64, sm, P, N, g, skeys, perm, n, (T)dt, contact);
                 else
-                    LAUNCH_STEP("pass1_remap", (k_pass1_cells<T, 2, 32>), gb, 32, sm, P, N, g, skeys, perm, n, contact);
+                    LAUNCH_STEP("pass1_remap", (k_pass1_cells<T, 2, 32>), gb, 32, sm, P, N, g, skeys, perm, n, (T)dt, contact);
             }
         }
         else if (c->gather_batch)
             LAUNCH_STEP("pass1_remap", (k_pass1_remap<T, 1>), blocks_for(n), NTHREADS, 0, P, N, g, skeys, perm, n,
-                        contact);
+                        (T)dt, contact);
         else
             LAUNCH_STEP("pass1_remap", (k_pass1_remap<T, 0>), blocks_for(n), NTHREADS, 0, P, N, g, skeys, perm, n,
-                        contact);
+                        (T)dt, contact);
         // remap, displacement control and BC in the path's order, p/m and v: one pass
         LAUNCH_STEP("node_phase_b", k_node_phase_b<T>, phaseblocks, nt, 0, N, (T)dt, contact, (const unsigned*)c->dclist.p,
                c->ndc, (const T*)c->vel.p, n, mm, output ? 0 : 1, vel_zero);

@@ -761,6 +761,14 @@ __device__ __forceinline__ void grid_update_regs(const NView<T>& nd, long long i
     }
 }
 
+// The factor dt of what the particles gather: the FP64 form takes it once per
+// node, in the records (its FP64 operations bound it), the FP32 form in each
+// particle, after the sum (pass2_particle says why).
+__device__ __forceinline__ double record_dt(double x, double dt) { return x * dt; }
+__device__ __forceinline__ float record_dt(float x, float) { return x; }
+__device__ __forceinline__ double gather_dt(double x, double) { return x; }
+__device__ __forceinline__ float gather_dt(float x, float dt) { return x * dt; }
+
 // ---------------------------------------------------------------------------
 // G2P pass 1 (…MPLocks.cpp:489-510): v_p += N (f_i/m_i) dt over the corners
 // in findAdjacentGridPoints order, fused with the velocity remap (:539-564):
@@ -770,7 +778,7 @@ __device__ __forceinline__ void grid_update_regs(const NView<T>& nd, long long i
 template <typename T, int BATCH>
 __global__ void __launch_bounds__(256) k_pass1_remap(PView<T> P, NView<T> nd, Geom g,
                                                      const unsigned* __restrict__ skeys,
-                                                     const unsigned* __restrict__ perm, long long n, int contact) {
+                                                     const unsigned* __restrict__ perm, long long n, T dt, int contact) {
     step_enter<sizeof(T) == 4>();
     long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     unsigned key = (s < n) ? skeys[s] : 0xffffffffu;
@@ -812,9 +820,9 @@ __global__ void __launch_bounds__(256) k_pass1_remap(PView<T> P, NView<T> nd, Ge
                 if (!(r[k].w != (T)0)) continue;  // out of range or m <= mass_min
                 T N, G[3];
                 B.corner(k, N, G);
-                v[0] = v[0] + N * r[k].x;
-                v[1] = v[1] + N * r[k].y;
-                v[2] = v[2] + N * r[k].z;
+                v[0] = v[0] + gather_dt(N * r[k].x, dt);
+                v[1] = v[1] + gather_dt(N * r[k].y, dt);
+                v[2] = v[2] + gather_dt(N * r[k].z, dt);
             }
         } else {
 #pragma unroll 1
@@ -825,9 +833,9 @@ __global__ void __launch_bounds__(256) k_pass1_remap(PView<T> P, NView<T> nd, Ge
                 if (!(r.w != (T)0)) continue;
                 T N, G[3];
                 B.corner(k, N, G);
-                v[0] = v[0] + N * r.x;
-                v[1] = v[1] + N * r.y;
-                v[2] = v[2] + N * r.z;
+                v[0] = v[0] + gather_dt(N * r.x, dt);
+                v[1] = v[1] + gather_dt(N * r.y, dt);
+                v[2] = v[2] + gather_dt(N * r.z, dt);
             }
         }
 #pragma unroll
@@ -880,7 +888,7 @@ __host__ __device__ constexpr size_t pass1_cells_smem(int bs) {
 template <typename T, int CPT, int BS>
 __global__ void __launch_bounds__(BS, sizeof(T) == 4 && CPT < 4 ? 1536 / BS : 1) k_pass1_cells(PView<T> P, NView<T> nd, Geom g,
                                                      const unsigned* __restrict__ skeys,
-                                                     const unsigned* __restrict__ perm, long long n, int contact) {
+                                                     const unsigned* __restrict__ perm, long long n, T dt, int contact) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int bs = BS;
     const int t = threadIdx.x;
@@ -931,9 +939,9 @@ __global__ void __launch_bounds__(BS, sizeof(T) == 4 && CPT < 4 ? 1536 / BS : 1)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const T N = nx * ((j & 2) ? B.Ny[1] : B.Ny[0]) * ((j & 1) ? B.Nz[1] : B.Nz[0]);
-                    v[0] += N * rq[j].x;
-                    v[1] += N * rq[j].y;
-                    v[2] += N * rq[j].z;
+                    v[0] += gather_dt(N * rq[j].x, dt);
+                    v[1] += gather_dt(N * rq[j].y, dt);
+                    v[2] += gather_dt(N * rq[j].z, dt);
                 }
             }
 #pragma unroll
@@ -1029,10 +1037,9 @@ __device__ __forceinline__ void node_dc_regs(const unsigned own[3], const unsign
 // the node's values in registers: displacement control (non-contact: before
 // the update, …MPLocks.cpp:143-174), the grid update (IntegrateGrid, :90-142;
 // contact :242-277), displacement control (contact: after it), then the
-// record (dt f/m, m > m_min), G2P pass 1's increment (:508; the factor dt is
-// taken here once per node instead of in every particle).  The updated
-// momentum and the mass also go to the record's second half for phase B
-// (which overwrites it with p/m and v); clean (not an output step): the
+// record (f/m, m > m_min), G2P pass 1's increment (:508; FP64 form: with the
+// factor dt, record_dt).  The updated momentum and the mass also go to the
+// record's second half for phase B (which overwrites it with p/m and v); clean (not an output step): the
 // node's mass, momentum and force are zeroed here, for the next step's P2G.
 //
 // work (when given): the step's boundary work in FP64, added to work[0]
@@ -1141,9 +1148,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) k_node_phase_a(NV
         if (fx & 2u) nd.ftemp[nn + i] += ft_y;
         const bool has = m > mass_min;
         Quad<T> r, pm;
-        r.x = has ? f[0] / m * dt : (T)0;
-        r.y = has ? f[1] / m * dt : (T)0;
-        r.z = has ? f[2] / m * dt : (T)0;
+        r.x = has ? record_dt(f[0] / m, dt) : (T)0;
+        r.y = has ? record_dt(f[1] / m, dt) : (T)0;
+        r.z = has ? record_dt(f[2] / m, dt) : (T)0;
         r.w = has ? (T)1 : (T)0;
         pm.x = p[0];
         pm.y = p[1];
@@ -1158,9 +1165,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) k_node_phase_a(NV
 
 // The node work between pass 1 and pass 2, in registers: the remap v += q/m
 // (:559-560; phase A cleared q before pass 1 summed it), displacement
-// control and BC (:573-599) in the path's order, then the record (dt p/m,
-// m > m_min, dt v: the displacement and the velocity gradient that pass 2
-// gathers carry the factor dt).  The claims are cleared after this last use (every claimed
+// control and BC (:573-599) in the path's order, then the record (p/m,
+// m > m_min, v; FP64 form: both with the factor dt).  The claims are cleared after this last use (every claimed
 // node is active: platen particles take part in P2G).  clean: a step whose
 // node values nobody sees (not the last of an advance; pass 2 reads only the
 // records) leaves the node zeroed as the next step's grid reset would
@@ -1213,13 +1219,13 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_node_phase_b(NV
         }
         if (contact) node_dc_regs<T>(own, dclist, pvel, np, m, v, vset, p, fz);
         Quad<T> r, vq;
-        r.x = has ? p[0] / m * dt : (T)0;
-        r.y = has ? p[1] / m * dt : (T)0;
-        r.z = has ? p[2] / m * dt : (T)0;
+        r.x = has ? record_dt(p[0] / m, dt) : (T)0;
+        r.y = has ? record_dt(p[1] / m, dt) : (T)0;
+        r.z = has ? record_dt(p[2] / m, dt) : (T)0;
         r.w = has ? (T)1 : (T)0;
-        vq.x = v[0] * dt;
-        vq.y = v[1] * dt;
-        vq.z = v[2] * dt;
+        vq.x = record_dt(v[0], dt);
+        vq.y = record_dt(v[1], dt);
+        vq.z = record_dt(v[2], dt);
         vq.w = (T)0;
         *reinterpret_cast<Quad<T>*>(nd.rec + 8 * i) = r;
         *reinterpret_cast<Quad<T>*>(nd.rec + 8 * i + 4) = vq;
@@ -1640,17 +1646,27 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
             } else {
                 particle_bases<T>(P, gs, p, b, B);
             }
-            // The two corners of an (x, y) pair are summed along z first, with
-            // A = Nx Ny, Bx = Ny gx and By = Nx gy formed once per pair: a
-            // record's r is zero where m <= mass_min, and grad N =
-            // -(Bx Nz, By Nz, A gz), so
-            //   disp += A (Nz r), L_x -= Bx (Nz v), L_y -= By (Nz v), L_z -= A (gz v):
-            // 132 products and sums per particle instead of 168 corner by
-            // corner.  The records carry the factor dt.  FP32 form: the displacement sum is formed in FP32 and
-            // added to the FP64 position once.  FP64 form (bound by its FP64
-            // pipe): added per corner in the reference's order
-            // (…MPLocks.cpp:197-198), so positions keep its last bits, on
-            // which the ties of the contact normals turn.
+            // An (x, y) pair of corners shares A = Nx Ny, Bx = Ny gx and By =
+            // Nx gy; a record's r is zero where m <= mass_min, and grad N =
+            // -(Bx Nz, By Nz, A gz).
+            // FP32 form: displacement and L are summed corner by corner, the
+            // records hold p/m and v, and dt comes last, per particle.  Other
+            // orders have the same number of roundings, but some that do not
+            // change from step to step: with dt taken per node and the pair
+            // summed along z first, 99% of the positions of 300k particles
+            // in three materials stayed within 2.9e-9 h of corner order's
+            // after 120 steps, where two runs of one code stay within 1.1e-9
+            // (1.07M block 6.4e-10 and 4.7e-10, honeycombs 5.1M 3.4e-10 and
+            // 1.8e-10), and the error against the FP64 form grew by 1.4 to
+            // 1.6.  Corner order and dt here cost 2% (honeycombs 675 us per
+            // step, 659 the other way).
+            // FP64 form (bound by its FP64 pipe): the records carry dt; L is
+            // summed along z first,
+            //   L_x -= Bx (Nz v), L_y -= By (Nz v), L_z -= A (gz v),
+            // 132 products and sums per particle instead of 168; the position
+            // is added to per corner in the reference's order
+            // (…MPLocks.cpp:197-198), so it keeps its last bits, on which the
+            // ties of the contact normals turn.
             T disp[3] = {0, 0, 0};
             const CellNodes cn = cell_nodes(gs, b);
 #pragma unroll(sizeof(T) == 4 ? 4 : (BATCH ? 2 : 1))
@@ -1665,27 +1681,42 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
                 }
                 const bool ix = (h >> 1) & 1, iy = h & 1;
                 const T nx = ix ? B.Nx[1] : B.Nx[0], ny = iy ? B.Ny[1] : B.Ny[0];
-                const T A = nx * ny, Bx = ny * (ix ? B.gx[1] : B.gx[0]), By = nx * (iy ? B.gy[1] : B.gy[0]);
+                const T gx = ix ? B.gx[1] : B.gx[0], gy = iy ? B.gy[1] : B.gy[0], A = nx * ny;
                 const T r0[3] = {rq[0].x, rq[0].y, rq[0].z}, r1[3] = {rq[1].x, rq[1].y, rq[1].z};
                 const T v0[3] = {vq[0].x, vq[0].y, vq[0].z}, v1[3] = {vq[1].x, vq[1].y, vq[1].z};
+                // outerProduct(v_i, grad N): column c, row r = v_i[r] * G[c]
+                if constexpr (sizeof(T) == 4) {
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const T w = B.Nz[0] * v0[c] + B.Nz[1] * v1[c], d = B.gz[0] * v0[c] + B.gz[1] * v1[c];
-                    if constexpr (sizeof(T) == 4) {
-                        disp[c] += A * (B.Nz[0] * r0[c] + B.Nz[1] * r1[c]);
-                    } else {
+                    for (int j = 0; j < 2; ++j) {
+                        const float nz = B.Nz[j], N = A * nz;
+                        const float Gx = -(ny * nz) * gx, Gy = -(nx * nz) * gy, Gz = -A * B.gz[j];
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            const float v = j ? v1[c] : v0[c];
+                            disp[c] += N * (j ? r1[c] : r0[c]);
+                            Ldt[c] += v * Gx;
+                            Ldt[3 + c] += v * Gy;
+                            Ldt[6 + c] += v * Gz;
+                        }
+                    }
+                } else {
+                    const double Bx = ny * gx, By = nx * gy;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        const double w = B.Nz[0] * v0[c] + B.Nz[1] * v1[c], d = B.gz[0] * v0[c] + B.gz[1] * v1[c];
                         x[c] = x[c] + A * B.Nz[0] * r0[c];
                         x[c] = x[c] + A * B.Nz[1] * r1[c];
+                        Ldt[c] -= Bx * w;
+                        Ldt[3 + c] -= By * w;
+                        Ldt[6 + c] -= A * d;
                     }
-                    // outerProduct(v_i, grad N): column c, row r = v_i[r] * G[c]
-                    Ldt[c] -= Bx * w;
-                    Ldt[3 + c] -= By * w;
-                    Ldt[6 + c] -= A * d;
                 }
             }
             if constexpr (sizeof(T) == 4) {
 #pragma unroll
-                for (int c = 0; c < 3; ++c) x[c] += fps_f2d(disp[c]);
+                for (int c = 0; c < 3; ++c) x[c] += fps_f2d(disp[c] * dt);
+#pragma unroll
+                for (int k = 0; k < 9; ++k) Ldt[k] *= dt;
             }
         }
         if constexpr (LS) {

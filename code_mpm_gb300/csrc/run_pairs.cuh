@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(BS) k_p2g_pairs(PView<float> P, NView<float> n
 template <int BS>
 __global__ void __launch_bounds__(BS) k_pass1_pairs(PView<float> P, NView<float> nd, Geom g,
                                                      const unsigned* __restrict__ skeys,
-                                                     const unsigned* __restrict__ perm, long long n, int contact) {
+                                                     const unsigned* __restrict__ perm, long long n, float dt, int contact) {
     step_enter<true>();
     constexpr int TS = PAIR_TILE_PER_THREAD * BS;
     __shared__ unsigned skey[TS];
@@ -397,9 +397,9 @@ __global__ void __launch_bounds__(BS) k_pass1_pairs(PView<float> P, NView<float>
                 for (int k = 0; k < 8; ++k) {
                     Nk[k] = Nx[(k >> 2) & 1] * Ny[(k >> 1) & 1] * Nz[k & 1];
                     if (!(rq[k].w != 0.0f)) continue;  // out of range or m <= mass_min
-                    v[0] = v[0] + Nk[k] * rq[k].x;
-                    v[1] = v[1] + Nk[k] * rq[k].y;
-                    v[2] = v[2] + Nk[k] * rq[k].z;
+                    v[0] = v[0] + Nk[k] * rq[k].x * dt;
+                    v[1] = v[1] + Nk[k] * rq[k].y * dt;
+                    v[2] = v[2] + Nk[k] * rq[k].z * dt;
                 }
 #pragma unroll
                 for (int c = 0; c < 3; ++c) P.vel[c * np + p] = v[c];
