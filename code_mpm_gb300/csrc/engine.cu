@@ -98,6 +98,11 @@ struct mpm_ctx {
     DevBuf work_acc;  // boundary work since the last particle upload (FP64): displacement control, friction
     int nsurf = 0;
     bool have_mon = false;
+    // the caller's displacement-control list and monitor mask as uploaded, in the caller's numbering: dclist and
+    // mon_mask follow the slots (reorder) and are made from these again when particles are uploaded
+    std::vector<uint32_t> dc_caller;
+    DevBuf mon_caller;
+    long long mon_n = 0;
     // host pinned staging for the error word
     unsigned* h_err = nullptr;
     // profiling
@@ -157,7 +162,7 @@ struct mpm_ctx {
                           &e_strain, &e_strain_max, &e_strain_ti, &e_plastic, &backstress, &mp_mg, &strain_rate,
                           &material, &pflags, &dc_mult, &g_acc, &g_vel, &g_ftemp, &g_mg,
                           &g_state, &g_fixed, &g_friction, &g_ratio, &g_q, &g_owner, &g_nowner, &g_need, &g_list, &g_count, &cstart,
-                          &cend, &keys0, &vals0, &keys1, &vals1, &keys_copy, &counts, &dclist, &mats, &staging, &staging2, &tune_backup, &surf, &mon_mask, &mon_acc, &loc, &geom_tab, &sid, &alist, &acount,
+                          &cend, &keys0, &vals0, &keys1, &vals1, &keys_copy, &counts, &dclist, &mats, &staging, &staging2, &tune_backup, &surf, &mon_mask, &mon_caller, &mon_acc, &loc, &geom_tab, &sid, &alist, &acount,
                           &q_in, &q_out, &q_vol, &q_pidx, &q_count, &sg_acc, &hv_count,
                           &dsim, &tl_dev, &orig, &ptmp, &Fe, &work_acc, &fext_any, &g_amark};
         all.assign(std::begin(list), std::end(list));
@@ -1449,6 +1454,31 @@ int alloc_particles(mpm_ctx* c, long long n) {
     return ensure(c, c->counts, (size_t)1024 * (nblocks + 1) * 4);  // digit counts per tile, and totals
 }
 
+// The displacement-control list and the monitor mask of the particles just
+// uploaded, in the caller's order: entries of particles that the upload does not
+// have are left out, particles past the mask's end are in no monitor.  slots: the
+// device copies follow an order of the particles that is gone.
+int caller_lists(mpm_ctx* c, bool slots) {
+    std::vector<uint32_t> list;
+    for (uint32_t i : c->dc_caller)
+        if ((long long)i < c->n) list.push_back(i);
+    if (slots || (int)list.size() != c->ndc) {
+        c->ndc = 0;
+        if (!list.empty())
+            CK(cudaMemcpyAsync(c->dclist.p, list.data(), list.size() * 4, cudaMemcpyHostToDevice, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+        c->ndc = (int)list.size();
+    }
+    if (c->have_mon) {
+        int rc = ensure(c, c->mon_mask, (size_t)std::max<long long>(1, c->n));
+        if (rc) return rc;
+        const long long kept = std::min(c->n, c->mon_n);
+        CK(cudaMemsetAsync(c->mon_mask.p, 0, (size_t)c->n, c->stream));
+        CK(cudaMemcpyAsync(c->mon_mask.p, c->mon_caller.p, (size_t)kept, cudaMemcpyDeviceToDevice, c->stream));
+    }
+    return MPM_OK;
+}
+
 }  // namespace
 
 // =============================================================================
@@ -1818,6 +1848,10 @@ int mpm_upload_particles(mpm_ctx* c, const mpm_particles* p, int64_t n) {
     rc = alloc_particles(c, n);
     if (rc) return rc;
     c->n = n;
+    // the upload is in the caller's order, and so are the lists again
+    const bool slots = c->have_orig;
+    c->have_orig = false;
+    if ((rc = caller_lists(c, slots))) return rc;
     struct {
         DevBuf* b;
         const double* h;
@@ -1906,7 +1940,6 @@ int mpm_upload_particles(mpm_ctx* c, const mpm_particles* p, int64_t n) {
     c->have_fext = c->h_err[1] != 0u;
     c->have_particles = true;
     c->keys_valid = false;
-    c->have_orig = false;  // the upload is in the caller's order
     c->reorder_pending = c->reorder_interval >= 0;
     c->steps_asked = 0;
     c->last_perm = c->last_skeys = nullptr;
@@ -1940,6 +1973,7 @@ int mpm_upload_dc_list(mpm_ctx* c, const uint32_t* idx, int64_t n) {
                (uint8_t*)c->pflags.p);
     }
     CK(cudaStreamSynchronize(c->stream));
+    c->dc_caller.assign(idx, idx + n);
     c->ndc = (int)n;
     return MPM_OK;
 }
@@ -2216,15 +2250,20 @@ int mpm_upload_monitor_mask(mpm_ctx* c, const uint8_t* mask, int64_t n) {
     graph_reset(c);
     if (!c) return MPM_ERR_ARG;
     if (n != c->n || (n > 0 && !mask)) return fail(c, MPM_ERR_ARG, "monitor mask must have one entry per particle");
-    int rc = ensure(c, c->mon_mask, (size_t)std::max<int64_t>(1, n));
-    if (rc) return rc;
-    if (n > 0) CK(cudaMemcpyAsync(c->mon_mask.p, mask, (size_t)n, cudaMemcpyHostToDevice, c->stream));
-    if (n > 0 && c->have_orig) {  // slot s takes the caller's entry orig[s]
-        if ((rc = ensure(c, c->ptmp, (size_t)n))) return rc;
-        LAUNCH("fill", k_permute<1>, blocks_for(n), NTHREADS, c->mon_mask.p, c->ptmp.p, (const unsigned*)c->orig.p, n, 1);
-        CK(cudaMemcpyAsync(c->mon_mask.p, c->ptmp.p, (size_t)n, cudaMemcpyDeviceToDevice, c->stream));
+    const size_t bytes = (size_t)std::max<int64_t>(1, n);
+    c->have_mon = false;
+    int rc;
+    if ((rc = ensure(c, c->mon_caller, bytes)) || (rc = ensure(c, c->mon_mask, bytes))) return rc;
+    if (n > 0) {
+        CK(cudaMemcpyAsync(c->mon_caller.p, mask, (size_t)n, cudaMemcpyHostToDevice, c->stream));
+        if (c->have_orig)  // slot s takes the caller's entry orig[s]
+            LAUNCH("fill", k_permute<1>, blocks_for(n), NTHREADS, c->mon_caller.p, c->mon_mask.p, (const unsigned*)c->orig.p, n,
+                   1);
+        else
+            CK(cudaMemcpyAsync(c->mon_mask.p, c->mon_caller.p, (size_t)n, cudaMemcpyDeviceToDevice, c->stream));
     }
     CK(cudaStreamSynchronize(c->stream));
+    c->mon_n = n;
     c->have_mon = true;
     return MPM_OK;
 }

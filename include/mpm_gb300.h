@@ -187,7 +187,9 @@ int mpm_upload_materials(mpm_ctx* ctx, const mpm_material* mats, int32_t n);
 int mpm_upload_particles(mpm_ctx* ctx, const mpm_particles* p, int64_t n);
 /* Indices of displacement-controlled particles, in the order of
  * v_MarkedMaterialPoints_Displacement_Control (that order decides which
- * particle's velocity a shared node keeps).  Duplicates are rejected. */
+ * particle's velocity a shared node keeps).  Duplicates are rejected.  The list
+ * holds for later particle uploads, too, in the same numbering; entries of
+ * particles that such an upload does not have are left out. */
 int mpm_upload_dc_list(mpm_ctx* ctx, const uint32_t* idx, int64_t n);
 int mpm_upload_nodes(mpm_ctx* ctx, const mpm_nodes* nodes);
 int mpm_set_timeline(mpm_ctx* ctx, const double* t, const double* v3, int32_t n); /* TimeLine::addTimePoint */
@@ -303,6 +305,8 @@ typedef struct mpm_monitors {
     double platen_work;
     double friction_work;
 } mpm_monitors;
+/* One byte of MPM_MON_* bits per particle, in the caller's numbering; holds for
+ * later particle uploads, too (particles past its end are in no list). */
 int mpm_upload_monitor_mask(mpm_ctx* ctx, const uint8_t* mask, int64_t n);
 int mpm_monitors_read(mpm_ctx* ctx, mpm_monitors* out);
 
