@@ -18,6 +18,13 @@ constexpr unsigned FULL_MASK = 0xffffffffu;
 // the FP64 form, whose kernels last as long as the SM with the most warps,
 // does not: blocks placed one by one on the SMs that drain first spread
 // unevenly (a 40,000-particle bar took 98 us per step placed early, 76 us not).
+// So a kernel's lifetime begins while kernels before it still write what it
+// reads.  Such arrays are read by ordinary loads: no ld.global.nc, which wants
+// data that stays as it is for the whole kernel, and no __restrict__ on them in
+// the kernel's arguments, which would let the compiler use one, or move a load
+// above the wait.  (What only uploads, reorders and the optimiser write, by plain
+// launches, may have it, as they have ended before the next such kernel begins;
+// and arrays that the kernel only writes.)
 template <bool EARLY>
 __device__ __forceinline__ void step_enter() {
     if constexpr (EARLY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -295,19 +302,20 @@ __device__ __forceinline__ void acc_add(T* acc, long long i, T m, T p0, T p1, T 
 }
 
 template <typename T>
-__device__ __forceinline__ Quad<T> ld_quad(const T* __restrict__ p) {
+__device__ __forceinline__ Quad<T> ld_quad(const T* p) {
     return *reinterpret_cast<const Quad<T>*>(p);
 }
 
 // Both halves of a node record, a = p[0..3], b = p[4..7]: one 32-byte load in
-// FP32 (records are 32-byte aligned and not written while they are read),
-// two 32-byte loads in FP64.
+// FP32 (records are 32-byte aligned), two 32-byte loads in FP64.  An ordinary
+// (coherent) load, kept behind step_enter's wait: phase B may still be writing
+// the records when a block of pass 2 is placed.
 template <typename T>
-__device__ __forceinline__ void ld_record(const T* __restrict__ p, Quad<T>& a, Quad<T>& b) {
+__device__ __forceinline__ void ld_record(const T* p, Quad<T>& a, Quad<T>& b) {
     if constexpr (sizeof(T) == 4) {
-        asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-            : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-            : "l"(p));
+        asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                     : "l"(p));
     } else {
         a = ld_quad(p);
         b = ld_quad(p + 4);

@@ -853,7 +853,7 @@ struct ClaimArgs {
 };
 template <bool EARLY, int NPT>
 __global__ void __launch_bounds__(CS_THREADS) k_step_lists(uint8_t* amark, unsigned* state, long long nn,
-                                                           unsigned ncompact, unsigned* __restrict__ list,
+                                                           unsigned ncompact, unsigned* list,
                                                            unsigned* count, int output, ClaimArgs dc, Geom g,
                                                            DevSim* clock) {
     __shared__ unsigned woff[CS_THREADS / 32];

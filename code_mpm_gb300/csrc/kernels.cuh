@@ -83,9 +83,8 @@ __device__ __forceinline__ unsigned particle_key(const Geom& g, const double x[3
     return ok ? g.key_off + (unsigned)((b[0] + 1) + g.kd[0] * ((b[1] + 1) + g.kd[1] * (b[2] + 1))) : g.key_max;
 }
 
-static __global__ void k_cell_keys(const double* __restrict__ pos, long long n, Geom g, unsigned* keys,
-                            unsigned* __restrict__ vals, unsigned* keys_copy, unsigned* err,
-                            float* __restrict__ loc, const uint16_t* __restrict__ sid) {
+static __global__ void k_cell_keys(const double* pos, long long n, Geom g, unsigned* keys, unsigned* vals,
+                                   unsigned* keys_copy, unsigned* err, float* loc, const uint16_t* __restrict__ sid) {
     step_enter<true>();
     long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (p >= n) return;
@@ -195,8 +194,8 @@ __device__ __forceinline__ void prefetch_l2(const void* base, int es, long long 
 // The choice (and the block size) is made per form by the autotuner.
 // ---------------------------------------------------------------------------
 template <typename T, int REDUCE>
-__global__ void __launch_bounds__(512) k_p2g(PView<T> P, NView<T> nd, Geom g, const unsigned* __restrict__ skeys,
-                                             const unsigned* __restrict__ perm, long long n, int with_mg) {
+__global__ void __launch_bounds__(512) k_p2g(PView<T> P, NView<T> nd, Geom g, const unsigned* skeys,
+                                             const unsigned* perm, long long n, int with_mg) {
     step_enter<sizeof(T) == 4>();
     if (blockIdx.x == 0 && threadIdx.x == 0) *nd.acount = 0u;
     long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -296,7 +295,7 @@ __global__ void __launch_bounds__(512) k_p2g(PView<T> P, NView<T> nd, Geom g, co
 // from the keys, whose neighbours come by shuffle, and counts them; run_starts
 // (after a __syncthreads) numbers them and ends with a __syncthreads (four waits
 // before: P2G 135 -> 131 us on the 5.08M-particle batch, 33.1 -> 31.6 on the 1.07M block).
-__device__ __forceinline__ unsigned run_heads(unsigned key, const unsigned* __restrict__ skeys, long long s, long long n,
+__device__ __forceinline__ unsigned run_heads(unsigned key, const unsigned* skeys, long long s, long long n,
                                               int* wsum) {
     const int t = threadIdx.x, lane = t & 31;
     unsigned prev = __shfl_up_sync(FULL_MASK, key, 1);
@@ -452,7 +451,7 @@ struct P2GBlock {
     // honeycomb batch about three runs in four have such a neighbour, so a
     // third of the corner atomics go).
     __device__ __forceinline__ void scatter(const NView<T>& nd, const Geom& g, const uint16_t* __restrict__ sid,
-                                            const unsigned* __restrict__ perm, long long s0, int nslots,
+                                            const unsigned* perm, long long s0, int nslots,
                                             unsigned heads) const {
         const int t = threadIdx.x, lane = t & 31;
         const long long nn = nd.nn;
@@ -581,7 +580,7 @@ struct P2GBlock {
 // path's node mass gradients (output steps of the FP32 form).
 template <typename T, int BS, bool FE, bool MG>
 __device__ __forceinline__ void p2g_cells_run(const PView<T>& P, const NView<T>& nd, const Geom& g,
-                                              const unsigned* __restrict__ skeys, const unsigned* __restrict__ perm,
+                                              const unsigned* skeys, const unsigned* perm,
                                               long long n) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const P2GBlock<T, BS, FE, MG> blk(smem_raw);
@@ -622,14 +621,13 @@ __device__ __forceinline__ void p2g_cells_run(const PView<T>& P, const NView<T>&
 // form, a solid block of 286k particles: 233 us before, 112 now.
 template <typename T, int BS, bool FE>
 __global__ void __launch_bounds__(BS, sizeof(T) == 4 ? 1280 / BS : 1) k_p2g_cells(
-    PView<T> P, NView<T> nd, Geom g, const unsigned* __restrict__ skeys, const unsigned* __restrict__ perm, long long n) {
+    PView<T> P, NView<T> nd, Geom g, const unsigned* skeys, const unsigned* perm, long long n) {
     p2g_cells_run<T, BS, FE, false>(P, nd, g, skeys, perm, n);
 }
 
 template <int BS>
 __global__ void __launch_bounds__(BS) k_p2g_cells_mg(PView<float> P, NView<float> nd, Geom g,
-                                                      const unsigned* __restrict__ skeys,
-                                                      const unsigned* __restrict__ perm, long long n) {
+                                                      const unsigned* skeys, const unsigned* perm, long long n) {
     p2g_cells_run<float, BS, true, true>(P, nd, g, skeys, perm, n);
 }
 
@@ -648,7 +646,7 @@ __global__ void __launch_bounds__(BS) k_p2g_cells_mg(PView<float> P, NView<float
 // as neighbours in a platen's list mostly do, two to a cell: it is not made (the
 // atomics of one cell queue: 24.4 -> 17.4 us on the 5.08M-particle batch).
 __device__ __forceinline__ void dc_claim(int k, int ndc, const unsigned* __restrict__ dclist,
-                                         const unsigned* __restrict__ keys, const uint8_t* __restrict__ pflags,
+                                         const unsigned* keys, const uint8_t* pflags,
                                          const Geom& g, unsigned* owner, long long nn, int contact,
                                          const uint16_t* __restrict__ sid, unsigned* state) {
     const bool have = k < ndc;
@@ -777,8 +775,8 @@ __device__ __forceinline__ float gather_dt(float x, float dt) { return x * dt; }
 // ---------------------------------------------------------------------------
 template <typename T, int BATCH>
 __global__ void __launch_bounds__(256) k_pass1_remap(PView<T> P, NView<T> nd, Geom g,
-                                                     const unsigned* __restrict__ skeys,
-                                                     const unsigned* __restrict__ perm, long long n, T dt, int contact) {
+                                                     const unsigned* skeys, const unsigned* perm, long long n, T dt,
+                                                     int contact) {
     step_enter<sizeof(T) == 4>();
     long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     unsigned key = (s < n) ? skeys[s] : 0xffffffffu;
@@ -887,8 +885,8 @@ __host__ __device__ constexpr size_t pass1_cells_smem(int bs) {
 // -> 118 us there, 48.1 -> 44.7 on 1.89M particles, 26.9 -> 26.0 on 1.07M.
 template <typename T, int CPT, int BS>
 __global__ void __launch_bounds__(BS, sizeof(T) == 4 && CPT < 4 ? 1536 / BS : 1) k_pass1_cells(PView<T> P, NView<T> nd, Geom g,
-                                                     const unsigned* __restrict__ skeys,
-                                                     const unsigned* __restrict__ perm, long long n, T dt, int contact) {
+                                                     const unsigned* skeys, const unsigned* perm, long long n, T dt,
+                                                     int contact) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int bs = BS;
     const int t = threadIdx.x;
@@ -1020,7 +1018,7 @@ __global__ void __launch_bounds__(BS, sizeof(T) == 4 && CPT < 4 ? 1536 / BS : 1)
 // velocity v, momentum m v and zero force.
 template <typename T>
 __device__ __forceinline__ void node_dc_regs(const unsigned own[3], const unsigned* __restrict__ dclist,
-                                             const T* __restrict__ pvel, long long np, T m, T v[3], bool vset[3],
+                                             const T* pvel, long long np, T m, T v[3], bool vset[3],
                                              T p[3], bool fzero[3]) {
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -1090,7 +1088,7 @@ template <typename T>
 constexpr int NODE_THREADS = sizeof(T) == 8 ? 64 : 256;
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) k_node_phase_a(NView<T> nd, T dt, double damping, int contact, int floor_friction,
-                               const unsigned* __restrict__ dclist, int ndc, const T* __restrict__ pvel, long long np,
+                               const unsigned* __restrict__ dclist, int ndc, const T* pvel, long long np,
                                T mass_min, int clean, double* work, double dtd) {
     step_enter<sizeof(T) == 4>();
     const long long nn = nd.nn;
@@ -1173,7 +1171,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) k_node_phase_a(NV
 // (ResetGrid, …MPLocks.cpp:4-22), so that step needs no reset pass.
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_node_phase_b(NView<T> nd, T dt, int contact, const unsigned* __restrict__ dclist, int ndc,
-                               const T* __restrict__ pvel, long long np, T mass_min, int clean, int vel_zero) {
+                               const T* pvel, long long np, T mass_min, int clean, int vel_zero) {
     step_enter<sizeof(T) == 4>();
     const long long nn = nd.nn;
     NODE_LOOP_AHEAD(nd, i) {

@@ -32,8 +32,8 @@ constexpr long long RS_FEW = 3 << 18;  // up to so many keys
 constexpr int RS_TILE = RS_THREADS * RS_ITEMS, RS_FEW_TILE = RS_THREADS * RS_FEW_ITEMS;
 
 template <int DB, int ITEMS>
-static __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const unsigned* __restrict__ keys, long long n, int shift,
-                                                         unsigned* __restrict__ counts, int nblocks) {
+static __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const unsigned* keys, long long n, int shift, unsigned* counts,
+                                                         int nblocks) {
     constexpr unsigned NB = 1u << DB, MASK = NB - 1u;
     __shared__ unsigned h[NB];
     for (int i = threadIdx.x; i < (int)NB; i += RS_THREADS) h[i] = 0;
@@ -54,7 +54,7 @@ static __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const unsigned* _
 constexpr int RS_SCAN_THREADS = 256;
 constexpr int RS_SCAN_ITEMS = 4;
 
-static __global__ void __launch_bounds__(RS_SCAN_THREADS) k_rs_scan(unsigned* __restrict__ counts, int nblocks) {
+static __global__ void __launch_bounds__(RS_SCAN_THREADS) k_rs_scan(unsigned* counts, int nblocks) {
     __shared__ unsigned wsum[2][RS_SCAN_THREADS / 32];
     step_enter<true>();
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
@@ -95,11 +95,10 @@ static __global__ void __launch_bounds__(RS_SCAN_THREADS) k_rs_scan(unsigned* __
 }
 
 template <int DB, int ITEMS>
-static __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const unsigned* __restrict__ kin,
-                                                            const unsigned* __restrict__ vin,
+static __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const unsigned* kin, const unsigned* vin,
                                                             unsigned* __restrict__ kout, unsigned* __restrict__ vout,
-                                                            long long n, int shift,
-                                                            const unsigned* __restrict__ offs, int nblocks) {
+                                                            long long n, int shift, const unsigned* offs,
+                                                            int nblocks) {
     constexpr unsigned NB = 1u << DB, MASK = NB - 1u;
     __shared__ unsigned wcnt[RS_WARPS][NB];
     __shared__ unsigned gofs[NB];

@@ -161,7 +161,7 @@ struct PairStaged {
 // N = A Nz and G = -(Bx Nz, By Nz, A gz), so its force is Nz c + gz d with
 // c and d formed once per particle and (x, y) pair.
 template <bool MG, class SRC>
-__device__ __forceinline__ void pair_accumulate(const SRC& src, const unsigned* __restrict__ perm, long long s0,
+__device__ __forceinline__ void pair_accumulate(const SRC& src, const unsigned* perm, long long s0,
                                                 int a, int e, int par, const Geom& gs, float am[8], float ap0[8],
                                                 float ap1[8], float ap2[8], float af0[8], float af1[8],
                                                 float af2[8], float g0[8], float g1[8], float g2[8]) {
@@ -220,8 +220,8 @@ __device__ __forceinline__ void pair_exchange(float v[8], int par) {
 
 template <int BS, bool MG, bool STAGE>
 __global__ void __launch_bounds__(BS) k_p2g_pairs(PView<float> P, NView<float> nd, Geom g,
-                                                   const unsigned* __restrict__ skeys,
-                                                   const unsigned* __restrict__ perm, long long n,
+                                                   const unsigned* skeys,
+                                                   const unsigned* perm, long long n,
                                                    unsigned* err) {
     constexpr int TS = PAIR_TILE_PER_THREAD * BS;
     using S = PairStage<TS>;
@@ -338,8 +338,8 @@ __global__ void __launch_bounds__(BS) k_p2g_pairs(PView<float> P, NView<float> n
 // ---------------------------------------------------------------------------
 template <int BS>
 __global__ void __launch_bounds__(BS) k_pass1_pairs(PView<float> P, NView<float> nd, Geom g,
-                                                     const unsigned* __restrict__ skeys,
-                                                     const unsigned* __restrict__ perm, long long n, float dt, int contact) {
+                                                     const unsigned* skeys,
+                                                     const unsigned* perm, long long n, float dt, int contact) {
     step_enter<true>();
     constexpr int TS = PAIR_TILE_PER_THREAD * BS;
     __shared__ unsigned skey[TS];

@@ -261,8 +261,8 @@ __device__ __forceinline__ void tile_fma(const GemmTile& s, int buf, int ty, int
 // FWD: C = relu(A W^T + bias), A n x K, W 128 x K.
 // else: C = (A W) where H > 0 (else 0), A n x 128, W 128 x 128; the column sums of C added to gbias.
 template <bool FWD, int K>
-__global__ void __launch_bounds__(GT, 2) k_layer(int n, const float* __restrict__ A, const float* __restrict__ W,
-                                                 const float* __restrict__ bias, const float* __restrict__ H,
+__global__ void __launch_bounds__(GT, 2) k_layer(int n, const float* A, const float* __restrict__ W,
+                                                 const float* __restrict__ bias, const float* H,
                                                  float* __restrict__ C, float* __restrict__ gbias) {
     extern __shared__ __align__(16) unsigned char net_smem[];
     GemmTile& s = *reinterpret_cast<GemmTile*>(net_smem);
@@ -300,13 +300,14 @@ __global__ void __launch_bounds__(GT, 2) k_layer(int n, const float* __restrict_
     __align__(8) float acc[8][8] = {};
     load(0);
     store(0);
+    if (GK < K) load(GK);  // each slice is requested before the barrier in front of the one it follows
     __syncthreads();
 #pragma unroll 1
     for (int k0 = 0; k0 < K; k0 += GK) {
         const int buf = (k0 / GK) & 1;
-        if (k0 + GK < K) load(k0 + GK);
         tile_fma(s, buf, ty, tx, acc);
         if (k0 + GK < K) store(buf ^ 1);
+        if (k0 + 2 * GK < K) load(k0 + 2 * GK);
         __syncthreads();
     }
     float cs[8] = {};
@@ -349,8 +350,8 @@ __global__ void __launch_bounds__(GT, 2) k_layer(int n, const float* __restrict_
 
 // gW[128 x N] += D^T X over this block's rows (D n x 128, X n x N), N = 128 or 16.
 template <int N>
-__global__ void __launch_bounds__(GT, 2) k_weight_grad(int n, int rows, const float* __restrict__ D,
-                                                       const float* __restrict__ X, float* __restrict__ gW) {
+__global__ void __launch_bounds__(GT, 2) k_weight_grad(int n, int rows, const float* D,
+                                                       const float* X, float* __restrict__ gW) {
     static_assert(N == HID || N == IN, "layer widths");
     extern __shared__ __align__(16) unsigned char net_smem[];
     GemmTile& s = *reinterpret_cast<GemmTile*>(net_smem);
@@ -382,11 +383,11 @@ __global__ void __launch_bounds__(GT, 2) k_weight_grad(int n, int rows, const fl
     __align__(8) float acc[8][8] = {};  // N = 16: acc[i][0] of column tx
     load(beg);
     store(0);
+    if (beg + GK < end) load(beg + GK);
     __syncthreads();
     int buf = 0;
 #pragma unroll 1
     for (int r0 = beg; r0 < end; r0 += GK, buf ^= 1) {
-        if (r0 + GK < end) load(r0 + GK);
         if constexpr (N == HID) {
             tile_fma(s, buf, ty, tx, acc);
         } else {
@@ -401,6 +402,7 @@ __global__ void __launch_bounds__(GT, 2) k_weight_grad(int n, int rows, const fl
             }
         }
         if (r0 + GK < end) store(buf ^ 1);
+        if (r0 + 2 * GK < end) load(r0 + 2 * GK);
         __syncthreads();
     }
 #pragma unroll
@@ -423,9 +425,9 @@ __global__ void __launch_bounds__(GT, 2) k_weight_grad(int n, int rows, const fl
 // as the column sums of d, of layer 3's bias; without it y is written.
 constexpr int HEAD_WARPS = 16;
 template <bool GRAD>
-__global__ void __launch_bounds__(HEAD_WARPS * 32) k_head(long long n, const float* __restrict__ h,
+__global__ void __launch_bounds__(HEAD_WARPS * 32) k_head(long long n, const float* h,
                                                           const float* __restrict__ W4, const float* __restrict__ b4,
-                                                          const float* __restrict__ t, float* __restrict__ y,
+                                                          const float* t, float* __restrict__ y,
                                                           float* __restrict__ d, float* __restrict__ gW4,
                                                           float* __restrict__ gb4, float* __restrict__ gb3,
                                                           double* __restrict__ loss) {
