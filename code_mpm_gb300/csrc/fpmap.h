@@ -20,7 +20,10 @@
 //
 // Stresses are scaled by a power of two that brings k0 into [1, 2), so the
 // squares and their error terms stay far from the float range's ends for any
-// system of units.
+// system of units.  That needs a material whose moduli are within reach of its
+// yield stress, and a state within reach of its yield surface: fps_vmh_fits
+// says whether they are, and the caller takes the map in FP64 where not
+// (yield 0 or next to nothing, stresses far past the surface).
 //
 // Measured against the exact value in long double (tests/csrc/fpmap_check.c,
 // three runs of 4M random states from 0.9 to 1.02 of the surface, six
@@ -44,7 +47,9 @@ typedef struct {
 // The material's constants (stresses and moduli times `s`), from doubles on the host.
 typedef struct {
     fps_df twoG, lam, G, inv_2G, k0, s23C1, C0, third, irt2, f23;
+    float s23C1_ll;  // s23C1's bits below its pair: near saturation the difference from R is all there is
     float s, inv_s;
+    float rad_min, rad_max;  // radii the map is taken for (unscaled); none (1 and 0) for a material it does not suit
 } fps_map_const;
 
 typedef struct {
@@ -119,6 +124,16 @@ FPS_HD fps_df fps_df_div(fps_df a, fps_df b) {
     return fps_fast_sum(q, fps_mul(r, inv));
 }
 
+// Whether the pairs serve a state of this radius, stress and trial stress
+// (unscaled floats; the trial stress to float accuracy).  The bound, 1024 radii,
+// leaves the sums at 2^-36 of the radius or better, 2^12 below what the float
+// stress itself resolves; NaN fits (either map gives NaN).
+FPS_HD int fps_vmh_fits(const fps_map_const* m, float rad, const float sig[6], const float tr[6]) {
+    float a = 0.0f;
+    for (int i = 0; i < 6; ++i) a = fmaxf(a, fmaxf(fabsf(sig[i]), fabsf(tr[i])));
+    return rad >= m->rad_min && rad <= m->rad_max && a <= 1024.0f * rad;
+}
+
 // The map of (sig, R, de): the float state's increments, each rounded once.
 // Returns 1 for a plastic step, 0 for an elastic one (deps_p and dR are then
 // zero); elastic as in the reference when J2 <= rad^2.
@@ -167,7 +182,7 @@ FPS_HD int fps_vmh_map(const fps_map_const* m, float R, const float sig[6], cons
         if (i < 3) n2 = i == 0 ? w2 : fps_df_add(n2, w2);
         else s2 = i == 3 ? w2 : fps_df_add(s2, w2);
     }
-    const fps_df sat = fps_df_addf(m->s23C1, -Rs);
+    const fps_df sat = fps_df_addf(fps_df_addf(fps_two_sum(m->s23C1.h, -Rs), m->s23C1.l), m->s23C1_ll);
     if (sat.h > 0.0f) {
         s2.h = fps_mul(4.0f, s2.h);
         s2.l = fps_mul(4.0f, s2.l);
@@ -188,8 +203,7 @@ static inline fps_df fps_df_of(double v) {
 static inline void fps_map_constants(double E, double nu, double yield, double C0, double C1, fps_map_const* m) {
     const double k0 = yield / sqrt(3.0), G = 0.5 * E / (1.0 + nu);
     int ex = 0;
-    const double by = k0 > 0.0 ? k0 : G * 1.0e-3;  // the stress scale: the yield radius, or a strain of 1e-3
-    if (by > 0.0 && by < 1.0e300) (void)frexp(by, &ex);
+    if (k0 > 0.0 && k0 < 1.0e300) (void)frexp(k0, &ex);
     if (ex > 100) ex = 100;
     if (ex < -100) ex = -100;
     const double s = ldexp(1.0, 1 - ex);
@@ -201,10 +215,18 @@ static inline void fps_map_constants(double E, double nu, double yield, double C
     m->inv_2G = fps_df_of(1.0 / (2.0 * G * s));
     m->k0 = fps_df_of(k0 * s);
     m->s23C1 = fps_df_of(sqrt(2.0 / 3.0) * C1 * s);
+    m->s23C1_ll = (float)(sqrt(2.0 / 3.0) * C1 * s - (double)m->s23C1.h - (double)m->s23C1.l);
     m->C0 = fps_df_of(C0);
     m->third = fps_df_of(1.0 / 3.0);
     m->irt2 = fps_df_of(1.0 / sqrt(2.0));
     m->f23 = fps_df_of(2.0 / 3.0);
+    // suited: k0 within the scale's range; yield strains from 2^-45 (3e-14) to 2^20, saturation and hardening rate
+    // inside the float range with their low parts; Poisson ratios away from -1 and 0.5 (no modulus 2^12 of another)
+    const int fits = k0 * s >= 1.0 && k0 * s < 2.0 && G * s >= 0x1p-20 && G * s <= 0x1p45 && nu >= -0.95 &&
+                     1.0 - 2.0 * nu >= 0x1p-11 && fabs(C1) * s <= 0x1p60 && (C1 == 0.0 || fabs(C1) * s >= 0x1p-60) &&
+                     (C0 == 0.0 || (fabs(C0) >= 0x1p-60 && fabs(C0) <= 0x1p60));
+    m->rad_min = fits ? (float)(0.5 * k0) : 1.0f;
+    m->rad_max = fits ? (float)(0x1p40 * k0) : 0.0f;
 }
 
 #endif

@@ -1808,7 +1808,7 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
             } else {
                 if constexpr (sizeof(T) == 4) {
                     if (wide)
-                        plastic = cr_increment_pairs(M, R, sig, e, o);
+                        plastic = cr_increment_pairs(M, R, sig, e, tr, o);
                     else
                         plastic = cr_return<T>(M, R, sig, e, tr, o);
                 } else {

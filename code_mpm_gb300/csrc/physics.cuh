@@ -331,17 +331,17 @@ __device__ __forceinline__ bool cr_return(const MatConst& m, T R, const T sig[6]
 }
 
 template <typename T>
-__device__ __forceinline__ void cr_increment(const MatConst& m, T R, const T sig[6], const T e[6], CrOut<T>& o) {
+__device__ __forceinline__ bool cr_increment(const MatConst& m, T R, const T sig[6], const T e[6], CrOut<T>& o) {
     CrTrial<T> t;
     cr_trial<T>(m, R, sig, e, t);
-    cr_return<T>(m, R, sig, e, t, o);
+    return cr_return<T>(m, R, sig, e, t, o);
 }
 
 // The exact map in FP64 on FP32 state (the judge of the learned map and the
 // guard's replacement of its results): the float inputs widened exactly, the
 // increment computed in double (cr_increment<double>, the plain form's
 // arithmetic), each output rounded once to float.
-__device__ __forceinline__ void cr_increment_wide(const MatConst& m, float R, const float sig[6], const float e[6],
+__device__ __forceinline__ bool cr_increment_wide(const MatConst& m, float R, const float sig[6], const float e[6],
                                                   CrOut<double>& w) {
     double s64[6], e64[6];
 #pragma unroll
@@ -349,7 +349,7 @@ __device__ __forceinline__ void cr_increment_wide(const MatConst& m, float R, co
         s64[i] = fps_f2d(sig[i]);
         e64[i] = fps_f2d(e[i]);
     }
-    cr_increment<double>(m, fps_f2d(R), s64, e64, w);
+    return cr_increment<double>(m, fps_f2d(R), s64, e64, w);
 }
 
 __device__ __forceinline__ void cr_narrow(const CrOut<double>& w, CrOut<float>& o) {
@@ -361,14 +361,55 @@ __device__ __forceinline__ void cr_narrow(const CrOut<double>& w, CrOut<float>& 
     o.dR = __double2float_rn(w.dR);
 }
 
+// The exact map in FP64, outputs rounded to float, out of line: for the few
+// states that the path below does not take, whose registers it stays out of.
+// in: stress, R, strain increment; out: dsig, deps_p, dR.
+static __device__ __noinline__ bool cr_increment_apart(const MatConst* m, const float* in, float* out) {
+    float sig[6], e[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        sig[i] = in[i];
+        e[i] = in[7 + i];
+    }
+    CrOut<double> w;
+    const bool plastic = cr_increment_wide(*m, in[6], sig, e, w);
+    CrOut<float> o;
+    cr_narrow(w, o);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        out[i] = o.dsig[i];
+        out[6 + i] = o.deps_p[i];
+    }
+    out[12] = o.dR;
+    return plastic;
+}
+
 // The same map on the chosen form's fallback path, in pairs of floats
 // (fpmap.h).  In FP64 it held pass 2 to the FP64 pipe wherever a warp had one
 // particle near the yield surface: of a solid block of 1.07M particles with a
 // quarter of them on the surface, pass 2 took 212 us, 119 us with the pairs;
-// 5.08M particles of honeycombs, 536 and 408 us.  Returns whether the
-// increment is plastic.
+// 5.08M particles of honeycombs, 536 and 408 us.  States and materials that the
+// pairs do not suit (fps_vmh_fits, from the trial's radius and stress) take FP64
+// after all.  Returns whether the increment is plastic.
 __device__ __forceinline__ bool cr_increment_pairs(const MatConst& m, float R, const float sig[6], const float e[6],
-                                                   CrOut<float>& o) {
+                                                   const CrTrial<float>& t, CrOut<float>& o) {
+    if (!fps_vmh_fits(&m.map, t.rad, sig, t.tr)) {
+        float in[13], out[13];
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            in[i] = sig[i];
+            in[7 + i] = e[i];
+        }
+        in[6] = R;
+        const bool plastic = cr_increment_apart(&m, in, out);
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            o.dsig[i] = out[i];
+            o.deps_p[i] = out[6 + i];
+        }
+        o.dR = out[12];
+        return plastic;
+    }
     fps_map_out w;
     const int plastic = fps_vmh_map(&m.map, R, sig, e, &w);
 #pragma unroll

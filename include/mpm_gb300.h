@@ -84,7 +84,8 @@ extern "C" {
 #define MPM_OPT_LARGE_STRAIN 12  /* FP64 form, non-contact loop: 1 runs the large-strain pass 2 (G2P_P2_LargeStrain, PhysicsEngine_runSimulation_Classic_DoublePass_MPLocks.cpp:281-437), which the reference ships disabled (:605); 0 (default) the small-strain pass */
 #define MPM_OPT_FP64_FALLBACK 13 /* FP32 form: 1 (default) computes the von Mises hardening return map
                                     (…_VonMisesHardening.cpp:4-92) as FP64 gives it, rounded to float (in pairs of
-                                    floats, 48 bits), for particles whose FP32 trial yield
+                                    floats, 48 bits; in FP64 where those do not reach: yield strains under 3e-14,
+                                    stresses over 1024 radii), for particles whose FP32 trial yield
                                     function is above -0.001 x k0 and that the network does not take: with a
                                     network the states up to its band (mpm_attach_surrogate, 0.02 by default) past
                                     the surface, every plastic state without one, and the elastic states just
