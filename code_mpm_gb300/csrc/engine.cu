@@ -53,9 +53,8 @@ struct mpm_ctx {
     // options
     int floor_friction = 0;
     int profile = 0;
-    // block sizes: 0 = chosen by the particle count (auto_block) unless the
-    // caller or the autotuner sets one; modes: the autotuner's choice on the
-    // 256-specimen honeycomb batch
+    // block sizes: 0 until the caller or the autotuner sets one (auto_block,
+    // pass2_block); modes: the autotuner's choice on the 256-specimen honeycomb batch
     int p2g_reduce = 3, p2g_block = 0, pass_block = 0, gather_batch = 0;
     int pass1_corners = 2, pass1_block = 0;  // cell-run pass 1 (P2G modes 2-4)
     bool have_fext = false;  // some particle carries an external force
@@ -934,7 +933,9 @@ void graph_reset(mpm_ctx* c) {
 }
 
 // The block size of a particle kernel: the caller's (or the autotuner's), else
-// 128 threads in the FP32 form.  The FP64 form's kernels are bound by the FP64
+// 128 threads; in the FP64 form 128, chosen or not, is at most that, so that a
+// tuning's block sizes mean the same in the engine that they are handed to.  The
+// FP64 form's kernels are bound by the FP64
 // pipe, two lanes per clock of each SM, so what counts is that every SM gets
 // its share of the warps: smaller blocks until there are AUTO_WAVES of them
 // per SM.  A 40,000-particle bar took 129.5 us per step with 2, 122.8 with 4
@@ -942,7 +943,7 @@ void graph_reset(mpm_ctx* c) {
 // more often), 286k particles 475 us with 2 to 8, 490 with 16.
 constexpr int AUTO_WAVES = 4;
 int auto_block(const mpm_ctx* c, int chosen) {
-    if (chosen) return chosen;
+    if (chosen > 128) return chosen;
     if (c->form != MPM_FORM_FP64) return 128;
     int b = 128;
     while (b > 32 && c->n < (long long)AUTO_WAVES * b * c->sm_count) b >>= 1;
@@ -2386,8 +2387,7 @@ int mpm_autotune(mpm_ctx* c, int32_t steps, double dt, int contact, mpm_tune_res
         c->sim = sim0;
         return r;
     };
-    // block candidates: 0 is 128, or fewer where the FP64 form's auto_block says so
-    const int blocks[3] = {0, 256, 512}, corners[3] = {1, 2, 4};
+    const int blocks[3] = {128, 256, 512}, corners[3] = {1, 2, 4};
     const int p2g_modes = c->form == MPM_FORM_FP32 ? 7 : 5;
     for (int red = 0; red < p2g_modes && rc == MPM_OK; ++red)
         for (int pb = 0; pb < 3 && rc == MPM_OK; ++pb) rc = trial(0, red, 1, blocks[pb]);

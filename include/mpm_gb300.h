@@ -71,10 +71,10 @@ extern "C" {
 #define MPM_OPT_FLOOR_FRICTION 1 /* contact path: Coulomb friction on x/y of z-fixed nodes (extension; default 0) */
 #define MPM_OPT_PROFILE 2        /* 1: time every kernel with CUDA events (default 0) */
 #define MPM_OPT_P2G_REDUCE 3     /* P2G: 0 = one atomic per particle, 1 = sum each cell's run across lanes first, 2, 3 (default), 4 = stage the block in shared memory and sum each cell's run in four threads (one kernel; the three values differ in nothing any more), 5 / 6 (FP32 form) = sum the runs in registers by lane pairs, with the tile read from global memory / staged by bulk copies */
-#define MPM_OPT_P2G_BLOCK 4      /* P2G threads per block: 128 (default), 256 or 512; by default the FP64 form takes 64 or 32 where the particles are few */
-#define MPM_OPT_PASS_BLOCK 5     /* G2P pass-2 threads per block: 128 (default), 256 or 512; by default the FP64 form takes 64 or 32 where the particles are few */
+#define MPM_OPT_P2G_BLOCK 4      /* P2G threads per block: 128 (default; in the FP64 form at most: 64 or 32 where the particles are few), 256 or 512 */
+#define MPM_OPT_PASS_BLOCK 5     /* G2P pass-2 threads per block: 128 (default; FP64 form as MPM_OPT_P2G_BLOCK), 256 (the FP32 form's own choice in pass-2 mode 0) or 512 */
 #define MPM_OPT_GATHER 6         /* pass-2 (G2P) mode: 0 = node gathers one (x, y) pair of corners at a time, 1 = several
-                                    pairs' loads issued together, 2 = (FP32 form) as 0 with the block's particle fields
+                                    pairs' loads issued together (the FP32 form does so in 0, too), 2 = (FP32 form) as 0 with the block's particle fields
                                     brought into shared memory by bulk copies first.  Until set: FP64 form 0, FP32 form 2
                                     for few particles (under 512 per SM), else 0 */
 #define MPM_OPT_GRAPH 7          /* 1 (default): mpm_advance replays a captured two-step CUDA graph in the steady state; 0: launch every kernel */
@@ -220,10 +220,13 @@ int mpm_advance_timed(mpm_ctx* ctx, int32_t nsteps, double dt, int contact, floa
 /* Autotuner (no counterpart in the reference, which has one fixed OpenMP
  * loop): times `steps` steps of dt per candidate launch configuration on the
  * current state in three stages, each keeping the fastest so far: P2G mode x
- * P2G block (15), then pass-1 corners per thread x pass-1 block (9, cell-run
- * modes only), then pass-2 block x pass-2 mode (6; 9 in the FP32 form).  The particle and node
+ * P2G block (15; 21 in the FP32 form), then pass-1 corners per thread x pass-1 block (9, cell-run
+ * modes only), then pass-2 block x pass-2 mode (6; 9 in the FP32 form).  Values of an option that
+ * name one kernel (P2G modes 2 to 4) are timed all the same, as the count
+ * of candidates is part of the result.  The particle and node
  * state and the time are restored exactly as they were.  Results are the
- * chosen options and the best and worst candidate times per step. */
+ * chosen options, which set the same configuration in this engine or in another
+ * of its kind, and the best and worst candidate times per step. */
 typedef struct mpm_tune_result {
     int32_t p2g_reduce, p2g_block, pass_block, candidates;
     double best_ms_per_step, worst_ms_per_step;
