@@ -954,16 +954,15 @@ int auto_block(const mpm_ctx* c, int chosen) {
 // staged (2) for particles that fill less than half a wave of it (1024 threads
 // per SM), where each block's copies are all there is in flight, and direct (0)
 // beyond, where the staging only delays a block's first gathers.  Staged /
-// direct, us per step: 40,000 particles 25.7 / 26.7, 43,500 32.1 / 32.1, 89,000
-// 38.9 / 38.3, 209,000 46.4 / 45.1, 383,000 73.1 / 70.6, 1.07M 143.5 / 138.0,
-// 1.89M 255 / 247, 5.08M 669 / 657.
+// direct, us per step: 40,000 particles 25.3 / 25.9, 42,000 31.6 / 31.1, 87,000
+// 37.0 / 37.0, 207,000 47.0 / 46.0, 383,000 75.8 / 73.7, 1.07M 159.8 / 152.3.
 int gather_mode(const mpm_ctx* c) {
     if (c->gather_batch >= 0) return c->gather_batch;
     return c->n < 512LL * c->sm_count ? 2 : 0;
 }
-// And its block: 256 threads where nobody chose and it runs direct (128: 138.4
-// against 138.0 us with 1.07M particles, 71.2 against 70.6 with 383,000; 512: 666
-// against 658 with 5.08M).
+// And its block: 256 threads where nobody chose and it runs direct (128 / 256 /
+// 512: 47.0 / 46.0 / 46.3 us with 207,000 particles, 74.5 / 73.7 / 73.3 with
+// 383,000, 151.5 / 152.3 / 151.9 with 1.07M).
 int pass2_block(const mpm_ctx* c) {
     if (!c->pass_block && c->gather_batch < 0 && gather_mode(c) == 0) return 256;
     return auto_block(c, c->pass_block);

@@ -285,7 +285,8 @@ __global__ void __launch_bounds__(512) k_p2g(PView<T> P, NView<T> nd, Geom g, co
 // (GridPoint_Mediator.cpp:118-133).  Its quantities are then staged as zero for
 // that axis.  Where rounding leaves one of the axis' two factors (FP32: a
 // cell-local coordinate below 3e-8), the staging thread adds that factor's
-// share to the nodes itself (rare: one particle in some ten million).
+// share to the nodes itself (one particle in some ten million per step: every
+// other step among 5M).
 // ---------------------------------------------------------------------------
 // Runs of equal cell keys among a block's slots: run r covers slots
 // run_start[r] .. run_start[r + 1] - 1.  The slots need not be sorted (a cell met
@@ -1656,8 +1657,8 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
             // after 120 steps, where two runs of one code stay within 1.1e-9
             // (1.07M block 6.4e-10 and 4.7e-10, honeycombs 5.1M 3.4e-10 and
             // 1.8e-10), and the error against the FP64 form grew by 1.4 to
-            // 1.6.  Corner order and dt here cost 2% (honeycombs 675 us per
-            // step, 659 the other way).
+            // 1.6.  Corner order and dt here cost 2% (honeycombs 685 us per
+            // step, 668 the other way).
             // FP64 form (bound by its FP64 pipe): the records carry dt; L is
             // summed along z first,
             //   L_x -= Bx (Nz v), L_y -= By (Nz v), L_z -= A (gz v),
@@ -1856,7 +1857,8 @@ __device__ __forceinline__ unsigned pass2_particle(const PView<T>& P, const NVie
 // registers).  Blocks of 128, us per step of a 1.07M-particle block and of 5.08M
 // particles of honeycombs: 142.9 and 677 with 768 threads per SM, 140.3 and 665
 // with 896, 138.4 and 657 with 1024, 140.0 and 660 with 1152; 144.6 and 679 with
-// 1280 (256 threads per block; 48 registers and spills).  CONTACT: the loop's path, apart so that each kernel holds
+// 1280 (256 threads per block; 48 registers and spills); those with the pairs of
+// corners summed along z first, now 151.5 and 679 with 1024.  CONTACT: the loop's path, apart so that each kernel holds
 // one path's code (pass 2's warps also wait for instructions).
 template <typename T, int BATCH, int BS, bool CONTACT>
 __global__ void __launch_bounds__(BS, sizeof(T) == 4 ? 1024 / BS : 1) k_pass2(PView<T> P, NView<T> nd, Geom g, PassKeys keys,
@@ -1940,9 +1942,9 @@ __global__ void __launch_bounds__(BS) k_pass2_ls(PView<double> P, NView<double> 
 // Node mass gradients sum grad N m_p over all particles; the reference adds
 // them in particle index order (one thread), and the max-norm selection that
 // follows is sensitive to the last bit.  Only nodes adjacent to surface
-// particles are ever read, so those nodes are summed here by one thread each,
-// merging the (index-ordered) particle ranges of the eight surrounding cells
-// in index order, with the reference's exact per-pair gradient.
+// particles are ever read, so only those are summed here, over the particles of
+// the eight surrounding cells in index order, with the reference's exact
+// per-pair gradient.
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void k_contact_need(PView<T> P, const unsigned* __restrict__ keys, Geom g, unsigned* __restrict__ need,

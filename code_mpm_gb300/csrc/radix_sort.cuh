@@ -32,8 +32,8 @@ constexpr long long RS_FEW = 3 << 18;  // up to so many keys
 constexpr int RS_TILE = RS_THREADS * RS_ITEMS, RS_FEW_TILE = RS_THREADS * RS_FEW_ITEMS;
 
 template <int DB, int ITEMS>
-static __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const unsigned* keys, long long n, int shift, unsigned* counts,
-                                                         int nblocks) {
+static __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const unsigned* keys, long long n, int shift,
+                                                         unsigned* counts, int nblocks) {
     constexpr unsigned NB = 1u << DB, MASK = NB - 1u;
     __shared__ unsigned h[NB];
     for (int i = threadIdx.x; i < (int)NB; i += RS_THREADS) h[i] = 0;
