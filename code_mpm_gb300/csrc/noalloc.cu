@@ -115,7 +115,10 @@ extern "C" int mpm_cell_order_noalloc(const mpm_grid_desc* grid, const double* d
     // every scratch word the sort reads is written first by this call (keys by k_cell_keys, digit counts and
     // totals by each pass), so the previous call's contents need no clearing.  The keys go to the caller's
     // array and are the first pass's input; its values are the identity, the last pass's the caller's order.
-    launch_after(st, k_cell_keys, (unsigned)((n + 255) / 256), 256, d_pos, n, g, d_keys, (unsigned*)nullptr, d_keys, err,
+    // A caller that wants the order alone may give one array for both: the first pass, which may be the last
+    // as well, then reads the keys from the scratch.
+    unsigned* first = d_order == d_keys ? keysB : d_keys;
+    launch_after(st, k_cell_keys, (unsigned)((n + 255) / 256), 256, d_pos, n, g, first, (unsigned*)nullptr, d_keys, err,
                  (float*)nullptr, (const uint16_t*)nullptr);
     if (cudaGetLastError() != cudaSuccess) return MPM_ERR_CUDA;
     int bits = 1;
@@ -124,7 +127,7 @@ extern "C" int mpm_cell_order_noalloc(const mpm_grid_desc* grid, const double* d
     const int tile = few ? RS_FEW_TILE : RS_TILE, nblocks = (int)((n + tile - 1) / tile);
     const auto hist = few ? k_rs_hist<8, RS_FEW_ITEMS> : k_rs_hist<8, RS_ITEMS>;
     const auto scatter = few ? k_rs_scatter<8, RS_FEW_ITEMS> : k_rs_scatter<8, RS_ITEMS>;
-    const unsigned *kin = d_keys, *vin = nullptr;
+    const unsigned *kin = first, *vin = nullptr;
     unsigned *kout = keysA, *vout = valsA;
     for (int shift = 0; shift < bits; shift += 8) {
         const bool last = shift + 8 >= bits;
